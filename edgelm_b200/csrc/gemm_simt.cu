@@ -8,9 +8,12 @@
 //   EPI_RESIDUAL  out[M, N] (float) = residual[M, N] + acc   (out may be residual itself)
 //   EPI_SWIGLU    out[M, N] = silu(acc_gate) * acc_up with a second weight W2 (up) of W's shape
 //   EPI_RELU2     out[M, N] = max(acc, 0)^2
-// Two kernels: a 64x64 tile for many rows and a one-warp-per-output-column kernel for a few
+// Three kernels: register tiles of 8x8 outputs a thread for float32 operands in 16-byte pieces (the 32-bit path's products of
+// more than 16 rows), a 64x64 tile for any size and alignment, and a one-warp-per-output-column kernel for a few
 // rows (decode), which reads every weight once.  Each output element is summed over k in an
-// order that depends on K alone, never on M or on the row's place in the batch.
+// order that depends on the sizes alone (in the last two: on K alone), never on the row's place in the batch.
+#include <cooperative_groups.h>
+
 #include "common.cuh"
 
 namespace edgelm {
@@ -94,6 +97,240 @@ gemm_tile_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, co
   }
 }
 
+// ------------------------------------------------------------------ float32 register tiles
+// A block computes 8 TY x 8 TX outputs (a SwiGLU's gate and up columns side by side: 4 TX columns of either weight).  KG groups of
+// TY TX threads share K, and a cluster of CS blocks shares it again; a thread keeps 8 x 8 sums, rows ty + TY i and columns
+// tx + TX j, reading four k of a row at a time (16 reads of 16 bytes for 256 multiply-adds).  The multiply-adds are packed pairs
+// (`fma.rn.f32x2`: even and odd k in sums of their own; single ones waited for register ports).  Both operands come by
+// cp.async, S_STAGES stages of 16 k a group, a row's four pieces of 16 bytes exchanged by
+// the row's number so that eight neighbouring rows' reads lie in different banks.  After S_FLUSH stages the pairs join running sums
+// that lie in shared memory (a thread's own 64): the rounding error of a long row of products grows with the number of runs and the
+// run's length, not with their product.  The sums of groups and blocks are added in the order of K.  Measured beside the any-size
+// kernel: 1,143 rows, N 576, K 1536 176 -> 77 us; 2,048 rows, N 6144, K 2048 2,231 -> 1,259 us (41 TFLOP/s; the multiply-adds' pipe is
+// 55 % busy, what is left is the two warps a scheduler that 64 pairs of sums allow); 24 rows, N 960, K 2560 169 -> 10 us.
+constexpr int SK = 16, S_STAGES = 3, S_FLUSH = 8;
+
+__device__ __forceinline__ void cp_async16(unsigned dst, const float* src, bool there) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+
+template <int THREADS>
+__device__ __forceinline__ void group_sync(int group) {
+  if (THREADS == 32) __syncwarp();
+  else asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(THREADS) : "memory");
+}
+
+using pair_t = unsigned long long;       // two float32
+__device__ __forceinline__ void fma_pair(pair_t& c, pair_t a, pair_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
+__device__ __forceinline__ float pair_sum(pair_t c) { return __uint_as_float((uint32_t)c) + __uint_as_float((uint32_t)(c >> 32)); }
+
+template <int TY, int TX, int KG> constexpr size_t sgemm_smem() {
+  constexpr size_t ring = (size_t)KG * S_STAGES * 8 * (TY + TX) * SK * 4, sums = (size_t)TY * TX * KG * 64 * 4, red = (size_t)KG * 8 * TY * (8 * TX + 8) * 4;
+  return ring + sums > red ? ring + sums : red;
+}
+
+template <int TY, int TX, int KG, int EPI>
+__global__ void __launch_bounds__(TY * TX * KG)
+sgemm_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, const float* __restrict__ W2, float* out, int ldo,
+             const float* residual, int M, int N, int K, int CS) {
+  extern __shared__ __align__(128) float sm[];
+  constexpr int GT = TY * TX, BM = 8 * TY, BN = 8 * TX, NOUT = EPI == EPI_SWIGLU ? BN / 2 : BN, STAGE = (BM + BN) * SK;
+  constexpr int PIECES = (BM + BN) * 4 / GT, RP = BN + 8;
+  pdl_launch_dependents();
+  pdl_wait();
+  const int g = threadIdx.x / GT, t = threadIdx.x % GT, lane = t & 31, w = t >> 5;
+  // (a read of 16 bytes a lane takes two clocks where neighbouring lanes share their row or two rows alternate, four elsewhere)
+  const int tx = (w % (TX / 8)) * 8 + (lane >> 1 & 7), ty = (w / (TX / 8)) * 4 + (lane & 1) + (lane >> 4) * 2;
+  const int rank = blockIdx.x % CS, m0 = blockIdx.y * BM, n0 = (blockIdx.x / CS) * NOUT;
+  const int chunks = (K + SK - 1) / SK, parts = KG * CS, part_no = rank * KG + g;
+  const int c_end = (int)((long long)chunks * (part_no + 1) / parts), c_begin = (int)((long long)chunks * part_no / parts);
+  float* ring = sm + (size_t)g * S_STAGES * STAGE;
+  float4* sums = reinterpret_cast<float4*>(sm + KG * S_STAGES * STAGE) + threadIdx.x;      // [16][threads]
+  // this thread's pieces of a stage: row t / 4 + i GT / 4 of the tile's rows of A and then of W, 16 bytes t % 4 of its 64.
+  // (rows beyond M or N: the last row again, whose sums are not stored)
+  const int kp = (t & 3) * 4, k_end = K - kp;
+  const float* src[PIECES];
+  unsigned dst0 = (unsigned)__cvta_generic_to_shared(ring) + (t >> 2) * SK * 4;
+#pragma unroll
+  for (int i = 0; i < PIECES; ++i) {
+    const int r = (t >> 2) + i * (GT / 4);
+    if (r < BM) {
+      src[i] = A + (size_t)min(m0 + r, M - 1) * lda + kp + c_begin * SK;
+    } else {
+      const int c = r - BM;
+      const bool up = EPI == EPI_SWIGLU && c >= NOUT;
+      src[i] = (up ? W2 : W) + (size_t)min(n0 + (up ? c - NOUT : c), N - 1) * K + kp + c_begin * SK;
+    }
+  }
+  // the next stage's pieces on their way (a stage beyond this group's last: nothing); `src` moves on
+  int next = c_begin;
+  auto load = [&](int slot) {
+    if (next < c_end) {
+      const bool there = next * SK < k_end;      // (K is a multiple of 4)
+#pragma unroll
+      for (int i = 0; i < PIECES; ++i) {
+        const int sw = (((t >> 2) + i * (GT / 4)) >> 1 & 3) * 4;
+        cp_async16(dst0 + (slot * STAGE + i * (GT / 4) * SK + (kp ^ sw)) * 4, there ? src[i] : A, there);
+        src[i] += SK;
+      }
+    }
+    ++next;
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+#pragma unroll
+  for (int s = 0; s < S_STAGES - 1; ++s) load(s);
+  pair_t part[8][8] = {};
+  int run = 0, slot = 0;                 // stages since the pairs last joined the sums
+  bool kept = false;
+  int oa[4], ow[4];
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    oa[k] = ty * SK + (k * 4 ^ (ty >> 1 & 3) * 4);
+    ow[k] = (BM + tx) * SK + (k * 4 ^ (tx >> 1 & 3) * 4);
+  }
+  for (int c = c_begin; c < c_end; ++c) {
+    asm volatile("cp.async.wait_group %0;" ::"n"(S_STAGES - 2) : "memory");
+    group_sync<GT>(g);                   // the stage is there for all; the one computed last is free
+    load(slot == 0 ? S_STAGES - 1 : slot - 1);
+    if (run == S_FLUSH) {
+#pragma unroll
+      for (int q = 0; q < 16; ++q) {
+        float4 v = kept ? sums[q * GT * KG] : make_float4(0.f, 0.f, 0.f, 0.f);
+        const int i = q >> 1, j = (q & 1) * 4;
+        v.x += pair_sum(part[i][j]); v.y += pair_sum(part[i][j + 1]); v.z += pair_sum(part[i][j + 2]); v.w += pair_sum(part[i][j + 3]);
+        part[i][j] = part[i][j + 1] = part[i][j + 2] = part[i][j + 3] = 0;
+        sums[q * GT * KG] = v;
+      }
+      run = 0;
+      kept = true;
+    }
+    ++run;
+    const float* st = ring + slot * STAGE;
+    slot = slot == S_STAGES - 1 ? 0 : slot + 1;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+      ulonglong2 a[8];
+#pragma unroll
+      for (int i = 0; i < 8; ++i) a[i] = *reinterpret_cast<const ulonglong2*>(st + oa[k ^ (TY * i / 2 & 3)] + i * TY * SK);
+#pragma unroll
+      for (int j = 0; j < 8; ++j) {
+        const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(st + ow[k] + j * TX * SK);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma_pair(part[i][j], a[i].x, b.x);
+#pragma unroll
+        for (int i = 0; i < 8; ++i) fma_pair(part[i][j], a[i].y, b.y);
+      }
+    }
+  }
+  float acc[8][8];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) {
+    const float4 v = kept ? sums[q * GT * KG] : make_float4(0.f, 0.f, 0.f, 0.f);
+    const int i = q >> 1, j = (q & 1) * 4;
+    acc[i][j] = v.x + pair_sum(part[i][j]);
+    acc[i][j + 1] = v.y + pair_sum(part[i][j + 1]);
+    acc[i][j + 2] = v.z + pair_sum(part[i][j + 2]);
+    acc[i][j + 3] = v.w + pair_sum(part[i][j + 3]);
+  }
+  if (KG == 1 && CS == 1) {
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int m = m0 + ty + TY * i;
+      if (m >= M) continue;
+#pragma unroll
+      for (int j = 0; j < (EPI == EPI_SWIGLU ? 4 : 8); ++j) {
+        const int n = n0 + tx + TX * j;
+        if (n < N) epilogue_store<EPI, float>(out, residual, (size_t)m * ldo + n, acc[i][j], EPI == EPI_SWIGLU ? acc[i][(j + 4) & 7] : 0.f);
+      }
+    }
+    return;
+  }
+  // partial tiles into shared memory (over the rings and sums), the groups' added in every block, then the blocks'
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) sm[(g * BM + ty + TY * i) * RP + tx + TX * j] = acc[i][j];
+  __syncthreads();
+  if (KG > 1) {
+    for (int e = threadIdx.x; e < BM * BN; e += GT * KG) {
+      float* p = sm + e / BN * RP + e % BN;
+      float v = p[0];
+#pragma unroll
+      for (int q = 1; q < KG; ++q) v += p[q * BM * RP];
+      p[0] = v;
+    }
+    __syncthreads();
+  }
+  cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
+  if (CS > 1) cluster.sync();
+  const int r_begin = BM * rank / CS, r_end = BM * (rank + 1) / CS;
+  for (int e = r_begin * NOUT + threadIdx.x; e < r_end * NOUT; e += GT * KG) {
+    const int r = e / NOUT, c = e % NOUT, m = m0 + r, n = n0 + c;
+    if (m >= M || n >= N) continue;
+    float v = 0.f, v2 = 0.f;
+    for (int q = 0; q < CS; ++q) {
+      const float* p = (CS > 1 ? cluster.map_shared_rank(sm, q) : sm) + r * RP + c;
+      v += p[0];
+      if (EPI == EPI_SWIGLU) v2 += p[NOUT];
+    }
+    epilogue_store<EPI, float>(out, residual, (size_t)m * ldo + n, v, v2);
+  }
+  if (CS > 1) cluster.sync();            // (no block leaves while another reads its sums)
+}
+
+template <int TY, int TX, int KG, int EPI>
+int launch_sgemm(const float* a, int lda, const float* w, const float* w2, float* out, int ldo, const float* residual, int M, int N, int K,
+                 int CS, cudaStream_t stream) {
+  constexpr int NOUT = EPI == EPI_SWIGLU ? 4 * TX : 8 * TX;
+  constexpr size_t smem = sgemm_smem<TY, TX, KG>();
+  auto* kern = sgemm_kernel<TY, TX, KG, EPI>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+  EL_REFUSE(e == cudaSuccess, "gemm_simt: %zu bytes of shared memory: %s", smem, cudaGetErrorString(e));
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)((N + NOUT - 1) / NOUT * CS), (unsigned)((M + 8 * TY - 1) / (8 * TY)));
+  cfg.blockDim = dim3(TY * TX * KG);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream;
+  cudaLaunchAttribute attr[2];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = (unsigned)CS;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr[1].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = (pdl_enabled() & 1) ? 2 : 1;
+  cudaLaunchKernelEx(&cfg, kern, a, lda, w, w2, out, ldo, residual, M, N, K, CS);
+  return 0;
+}
+
+// The tile and the number of blocks that share K: what takes the least time by a count of waves of one block an SM (a block's
+// registers and rings fill it; clusters of eight find room for 120 blocks).  The constants are measured: a stage of all of a block's
+// groups takes 1.83, 1.95 and 2.1 us in the three tiles (one wave, K 960: 110, 31 and 18.6 us), a wave 2.5 us beside them, and 2.5 more
+// where blocks exchange sums.  24 rows, N 960, K 960: 12.4, 9.2 and 6.5 us with the middle tile in clusters of 4, of 8, and the small
+// one of 8; N 2560, K 960 (SwiGLU): 33, 19.5 and 23.7 us with the middle tile, the small one alone and in clusters of 4.
+template <int EPI>
+int launch_sgemm_best(const float* a, int lda, const float* w, const float* w2, float* out, int ldo, const float* residual, int M, int N,
+                      int K, cudaStream_t stream) {
+  const int chunks = (K + SK - 1) / SK;
+  struct Tile { int rows, columns, groups; float stage_us; };
+  constexpr Tile tiles[3] = {{128, 128, 1, 1.83f}, {64, 64, 4, 1.95f}, {32, 64, 8, 2.1f}};
+  float best = 0.f;
+  int best_t = -1, best_cs = 1;
+  for (int t = 0; t < 3; ++t)
+    for (int cs = 1; cs <= (t == 0 ? 1 : 8) && (cs == 1 || 2 * chunks >= tiles[t].groups * cs); cs *= 2) {
+      const int columns = tiles[t].columns / (EPI == EPI_SWIGLU ? 2 : 1), room = cs == 8 ? 120 : cs == 4 ? 136 : 148;
+      const long long blocks = (long long)((M + tiles[t].rows - 1) / tiles[t].rows) * ((N + columns - 1) / columns) * cs;
+      const int stages = (chunks + tiles[t].groups * cs - 1) / (tiles[t].groups * cs);
+      const float us = (float)((blocks + room - 1) / room) * ((float)stages * tiles[t].stage_us + 2.5f + (cs > 1 ? 2.5f : 0.f));
+      if (best_t < 0 || us < best) { best = us; best_t = t; best_cs = cs; }
+    }
+  if (best_t == 0) return launch_sgemm<16, 16, 1, EPI>(a, lda, w, w2, out, ldo, residual, M, N, K, best_cs, stream);
+  if (best_t == 1) return launch_sgemm<8, 8, 4, EPI>(a, lda, w, w2, out, ldo, residual, M, N, K, best_cs, stream);
+  return launch_sgemm<4, 8, 8, EPI>(a, lda, w, w2, out, ldo, residual, M, N, K, best_cs, stream);
+}
+
 // ------------------------------------------------------------------ few-rows kernel
 template <typename T, int VEC> struct VecLoad;
 template <> struct VecLoad<float, 4> {
@@ -170,6 +407,11 @@ int launch_gemm(const void* A, int lda, const void* W, const void* W2, void* out
   const TW* w2 = (const TW*)W2;
   TOut* o = (TOut*)out;
   const bool few = force_kernel == 1 || (force_kernel == 0 && M <= 2 * GEMV_ROWS);
+  if constexpr (sizeof(TA) == 4 && sizeof(TOut) == 4) {
+    const bool pieces = K % 4 == 0 && lda % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0 && (W2 == nullptr || (uintptr_t)W2 % 16 == 0);
+    if (pieces && (force_kernel == 3 || (force_kernel == 0 && !few)))
+      return launch_sgemm_best<EPI>(a, lda, w, w2, o, ldo, residual, M, N, K, stream);
+  }
   if (few) {
     constexpr int VEC = sizeof(TW) == 2 ? 8 : 4;
     const bool same_width = sizeof(TA) == sizeof(TW);
@@ -194,7 +436,8 @@ int launch_gemm(const void* A, int lda, const void* W, const void* W2, void* out
 using namespace edgelm;
 
 // a_dtype: dtype of `a` and of both weights; out_dtype: dtype of `out` (EPI_RESIDUAL: float).
-// force_kernel: 0 choose by M, 1 the few-rows kernel, 2 the tile kernel (tests call both).
+// force_kernel: 0 choose by sizes and alignment, 1 the few-rows kernel, 2 the any-size tile kernel, 3 the float32 register tiles where
+// the operands allow them, else 2 (tests call all).
 extern "C" int edgelm_gemm_simt(const void* a, int lda, const void* w, const void* w2, void* out, int ldo,
                                 const float* residual, int M, int N, int K, int a_dtype, int out_dtype, int epilogue,
                                 int force_kernel, cudaStream_t stream) {
@@ -203,12 +446,13 @@ extern "C" int edgelm_gemm_simt(const void* a, int lda, const void* w, const voi
   EL_REFUSE(epilogue != EPI_SWIGLU || w2 != nullptr, "gemm_simt: SwiGLU needs the second weight");
   EL_REFUSE(epilogue != EPI_RESIDUAL || (residual != nullptr && out_dtype == DT_F32), "gemm_simt: residual epilogue needs a float32 residual and output");
   EL_REFUSE((M + BM - 1) / BM <= 65535, "gemm_simt: too many rows (%d)", M);
+  int rc = 0;
 #define EL_GEMM_CASE(TA, TOUT)                                                                                      \
   switch (epilogue) {                                                                                                \
-    case EPI_STORE: launch_gemm<TA, TA, EPI_STORE, TOUT>(a, lda, w, w2, out, ldo, residual, M, N, K, force_kernel, stream); break;       \
-    case EPI_RESIDUAL: launch_gemm<TA, TA, EPI_RESIDUAL, float>(a, lda, w, w2, out, ldo, residual, M, N, K, force_kernel, stream); break; \
-    case EPI_SWIGLU: launch_gemm<TA, TA, EPI_SWIGLU, TOUT>(a, lda, w, w2, out, ldo, residual, M, N, K, force_kernel, stream); break;     \
-    case EPI_RELU2: launch_gemm<TA, TA, EPI_RELU2, TOUT>(a, lda, w, w2, out, ldo, residual, M, N, K, force_kernel, stream); break;       \
+    case EPI_STORE: rc = launch_gemm<TA, TA, EPI_STORE, TOUT>(a, lda, w, w2, out, ldo, residual, M, N, K, force_kernel, stream); break;       \
+    case EPI_RESIDUAL: rc = launch_gemm<TA, TA, EPI_RESIDUAL, float>(a, lda, w, w2, out, ldo, residual, M, N, K, force_kernel, stream); break; \
+    case EPI_SWIGLU: rc = launch_gemm<TA, TA, EPI_SWIGLU, TOUT>(a, lda, w, w2, out, ldo, residual, M, N, K, force_kernel, stream); break;     \
+    case EPI_RELU2: rc = launch_gemm<TA, TA, EPI_RELU2, TOUT>(a, lda, w, w2, out, ldo, residual, M, N, K, force_kernel, stream); break;       \
     default: EL_REFUSE(false, "gemm_simt: unknown epilogue %d", epilogue);                                           \
   }
   if (a_dtype == DT_F32 && out_dtype == DT_F32) {
@@ -221,6 +465,7 @@ extern "C" int edgelm_gemm_simt(const void* a, int lda, const void* w, const voi
     EL_REFUSE(false, "gemm_simt: unsupported dtypes a=%d out=%d", a_dtype, out_dtype);
   }
 #undef EL_GEMM_CASE
+  if (rc != 0) return rc;
   EL_LAUNCH_CHECK("gemm_simt");
   return 0;
 }

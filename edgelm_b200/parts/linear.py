@@ -5,7 +5,7 @@
                     on mma.sync tensor cores (gemv_mma.cu), float32 on the CUDA cores (gemv.cu);
   bfloat16, more    the tcgen05 tensor-core kernel (gemm_tc.cu): operands by TMA, accumulator in
                     tensor memory;
-  anything else     the CUDA-core kernels of gemm_simt.cu: the whole float32 path for many rows,
+  anything else     the CUDA-core kernels of gemm_simt.cu: the whole float32 path for many rows (register tiles),
                     and every size the other two do not take (K not a multiple of 8, unaligned rows).
 """
 import os

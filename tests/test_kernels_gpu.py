@@ -114,6 +114,27 @@ def test_gemm_simt_swiglu(dtype, M, N, K):
         assert rel_err(out, want) < tol(dtype)
 
 
+@pytest.mark.parametrize("M,N,K", [(17, 48, 64), (32, 64, 16), (33, 1000, 576), (65, 397, 132), (129, 65, 4), (24, 960, 2560), (64, 2000, 20),
+                                     (300, 130, 1028), (1000, 1100, 96)])
+def test_gemm_simt_register_tiles(M, N, K):
+    """Tiles' edges, parts of a stage, groups without a stage, clusters; 5e-7 is eight roundings of 2^-24 of the result's norm,
+    twice what sums of runs of 64 pairs can gather at K = 2560."""
+    o = ops()
+    a, w, w2, res = rnd((M, K + 4), torch.float32, 20)[:, :K], rnd((N, K), torch.float32, 21, 0.3), rnd((N, K), torch.float32, 22, 0.3), rnd((M, N), torch.float32, 23)
+    y, u = a.double() @ w.double().T, a.double() @ w2.double().T
+    wants = {o.EPI_STORE: y, o.EPI_RESIDUAL: y + res.double(), o.EPI_SWIGLU: y / (1 + torch.exp(-y)) * u, o.EPI_RELU2: y.clamp(min=0) ** 2}
+    for epilogue, want in wants.items():
+        out = res.clone() if epilogue == o.EPI_RESIDUAL else torch.full((M, N), float("nan"), device=dev())
+        o.gemm_simt(a, w, out, epilogue=epilogue, w2=w2 if epilogue == o.EPI_SWIGLU else None,
+                    residual=out if epilogue == o.EPI_RESIDUAL else None, force_kernel=3)
+        assert float((out.double() - want).norm() / want.norm()) < 5e-7
+    order = torch.randperm(M, device=dev())       # a row's sums do not depend on its place
+    out, moved = torch.empty(M, N, device=dev()), torch.empty(M, N, device=dev())
+    o.gemm_simt(a, w, out, force_kernel=3)
+    o.gemm_simt(a[order], w, moved, force_kernel=3)
+    assert torch.equal(moved, out[order])
+
+
 def test_gemm_row_independent_of_batch():
     """A row's result is the same bits whether it is computed alone or among others."""
     o = ops()
