@@ -154,6 +154,19 @@ def test_blend_convolution_and_norms(dtype):
 
 
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("T,C,L", [(1, 130, 5), (37, 2048, 64), (333, 1000, 24), (160, 2048, 513), (2500, 128, 7)])
+def test_lowrank_decay_tiles(T, C, L, dtype):
+    """One and sixteen tokens a block, ragged edges of both, ranks in and out of whole pieces.  The sum takes L
+    roundings of 2^-24 of partial sums under 2, of which exp(-exp(.)) passes on at most 0.37, and its own functions eight more."""
+    g = np.random.default_rng(T + L)
+    a, w2, w0 = g.normal(size=(T, L)), f32(g.normal(size=(C, L)) / np.sqrt(L)).to(dtype), g.uniform(-4, 1, C)
+    out = torch.full((T, C), float("nan"), device=DEV)
+    ops.lowrank_decay(f32(a), w2, f32(w0), out)
+    ref = torch.exp(-torch.exp(torch.tanh(f32(a).double()) @ w2.double().T + f32(w0).double()))
+    assert float((out.double() - ref).abs().max()) < (L + 8) * 2.0 ** -24
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("window,pool,dk,dv,H,G", [(9, 4, 20, 12, 4, 2), (3, 7, 40, 72, 2, 1), (70, 64, 16, 16, 3, 3), (5, 1, 33, 8, 2, 2)])
 def test_window_attention_with_pooled_blocks(dtype, window, pool, dk, dv, H, G):
     """Two sequences side by side through prompt pieces and single tokens.  In the first, key 37 (its block too) is far
