@@ -189,8 +189,8 @@ class MaskedAttention(Part):
 
     def _on_tensor_cores(self):
         """Whether prompt steps take the tensor-core kernel with float32 scores and weights (three bfloat16 terms for each
-        float32 operand): one map a head, a bfloat16 cache, head sizes that it takes."""
-        return self.maps == 1 and ops.attn_prefill_split_takes(self.dtype, self.dk, self.dv)
+        float32 operand): a bfloat16 cache, head sizes and maps that it takes."""
+        return ops.attn_prefill_split_takes(self.dtype, self.dk, self.dv, self.maps)
 
     def _whole_rows(self):
         """Whether the block-per-pair kernel of single tokens reads whole key and value rows at a time."""
@@ -336,7 +336,7 @@ class MaskedAttention(Part):
             elif self._on_tensor_cores():
                 tiles = ctx.tiles(ops.SPLIT_PREFILL_TILE)
                 ops.attn_prefill_split(q, a, cache.k, cache.v, table, tiles.seq, tiles.tok0, tiles.ntok, tiles.pos0, tiles.count, self.nh, self.nkv,
-                                       self.dk, self.dv, self.scale, gate=gate, mask=self.mask, mask_size=self.mask_size, sink=self.sink, keep=self.keep,
+                                       self.dk, self.dv, self.scale, gate=gate, mask=self.mask, mask_size=self.mask_size, sink=self.sink, keep=self.keep, maps=self.maps,
                                        max_keys=max(p + n for p, n in zip(ctx.seq_first_positions, ctx.seq_lengths)))
             else:
                 tiles = ctx.tiles(self.tile_tokens)

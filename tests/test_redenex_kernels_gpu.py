@@ -255,6 +255,31 @@ def test_two_maps_over_the_same_values(H, G, d, dv, size, dtype):
             assert np.abs(out2.cpu().numpy() - ref).max() < tol * max(1.0, np.abs(ref).max()), ("single, split", back, splits)
 
 
+@pytest.mark.parametrize("H,G,d,dv,size", [(4, 2, 32, 64, 100), (2, 2, 64, 128, 64), (3, 1, 64, 64, 0), (2, 1, 32, 32, 7)])
+def test_two_maps_on_the_tensor_cores(H, G, d, dv, size):
+    """Whole prompts and pieces that go on from the cache, at the edges of pages, tiles and chunks, one and two groups of warps a
+    block.  5e-6: float32 sums of up to 700 weighted values and the exponentials' roundings, 2^-24 each, of scores up to 30."""
+    g = np.random.default_rng(d + dv)
+    lengths, scale = [700, 64, 65, 1, 129], d ** -0.5
+    rnd = lambda a: torch.tensor(a, dtype=torch.bfloat16).double().numpy()
+    kv = PagedKV(lengths, G, 2 * d, dv, torch.bfloat16, seed=4)
+    Q, want = [], []
+    for s, n in enumerate(lengths):
+        q, k, v = f32(g.normal(size=(n, H, 2, d)) * 2).double().cpu().numpy(), rnd(g.normal(size=(n, G, 2, d))), rnd(g.normal(size=(n, G, dv)))
+        kv.put(s, k.reshape(n, G, 2 * d), v)
+        Q.append(q)
+        want.append(np.stack([plain.chunked_softmax_attention(q[:, :, j], k[:, :, j], v, scale, size or None) for j in range(2)], axis=2))
+    assert ops.attn_prefill_split_takes(torch.bfloat16, d, dv, 2)
+    for pieces in ([(0, n) for n in lengths], [(n // 3, n - n // 3) for n in lengths], [(699, 1), (0, 64), (64, 1), (0, 1), (63, 3)]):
+        tiles = make_tiles([n for _, n in pieces], [a for a, _ in pieces], ops.SPLIT_PREFILL_TILE)
+        cut = lambda rows, w: np.concatenate([r[a:a + n].reshape(n, w) for r, (a, n) in zip(rows, pieces)])
+        out = torch.full((sum(n for _, n in pieces), H * 2 * dv), float("nan"), device=DEV)
+        ops.attn_prefill_split(f32(cut(Q, H * 2 * d)), out, kv.k, kv.v, i32(kv.table), *tiles, H, G, d, dv, scale, max_keys=max(lengths),
+                               mask=ops.MASK_CHUNK if size else ops.MASK_CAUSAL, mask_size=size, maps=2)
+        ref = cut(want, H * 2 * dv)
+        assert np.abs(out.cpu().numpy() - ref).max() < 5e-6 * np.abs(ref).max(), pieces[0]
+
+
 @pytest.mark.parametrize("out_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,H,dv,lam,offset", [(37, 4, 24, 0.37, 0.3), (3, 1, 130, -0.2, 0.8), (130, 16, 80, 1.4, 0.7), (5, 3, 7, 0.5, 0.5)])
 def test_maps_combined(T, H, dv, lam, offset, out_dtype):
