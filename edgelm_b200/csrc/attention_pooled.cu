@@ -12,7 +12,7 @@
 //
 // Three kernels: (1) bias, partial rotation, per-head unit RMS norm of q and k, append of k and v; (2) the pooled
 // rows of the blocks that the step's tokens complete; (3) attention.  Scores, softmax, norms, angles: float32.
-#include "common.cuh"
+#include "mma_split.cuh"
 
 namespace edgelm {
 
@@ -477,6 +477,224 @@ pooled_window_attn_tiled_kernel(const T* __restrict__ q, T* __restrict__ out, co
   }
 }
 
+// ---- prompt steps on the tensor cores (bfloat16 cache, key and value heads of one size of 32, 64, 96 or 128)
+// A block of four warps: 64 consecutive new tokens of one sequence, one query head, 16 rows a warp; the keys 64 at a time for the
+// window's pages (copied by cp.async, two stages), 32 at a time for the pooled rows, which come first.  Scores of page keys are
+// products of bfloat16 numbers summed in float32; the float32 weights, and the pooled rows' float32 keys and values, go as three
+// bfloat16 terms (8 + 8 + 8 bits of their mantissas), weights times pooled values as the six products of terms that float32 can
+// tell from zero.  Scores, maxima, exponentials, denominators and outputs are float32, as on the CUDA cores.
+// 2,048 tokens, 32 heads of 64, a window of 1,024, blocks of 64: 1,131 us there, 145 us here (bound by the issue of the small
+// matrix instructions: three of them for every page value).
+constexpr int PM_WARPS = 4, PM_ROWS = 16 * PM_WARPS, PM_POOLED = 32;
+
+// S[NT tiles of 8 keys] = Q K^T, the keys in TERMS tiles of `tile` elements one after the other (the smallest term first)
+template <int HDT, int NT, int TERMS>
+__device__ __forceinline__ void pm_scores(float (&s)[NT][4], const uint32_t (&qa)[HDT][4], const __nv_bfloat16* ks, int tile, int lane) {
+  constexpr int PITCH = HDT * 16 + 8;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    s[nt][0] = s[nt][1] = s[nt][2] = s[nt][3] = 0.f;
+#pragma unroll
+    for (int t = TERMS - 1; t >= 0; --t)
+#pragma unroll
+      for (int d = 0; d < HDT; d += 2) {
+        const int mi = lane >> 3;
+        uint32_t b0, b1, b2, b3;
+        sp_ldmatrix_x4(sp_smem(ks + t * tile + (nt * 8 + (lane & 7)) * PITCH + (d + (mi >> 1)) * 16 + (mi & 1) * 8), b0, b1, b2, b3);
+        sp_mma(s[nt], qa[d][0], qa[d][1], qa[d][2], qa[d][3], b0, b1);
+        sp_mma(s[nt], qa[d + 1][0], qa[d + 1][1], qa[d + 1][2], qa[d + 1][3], b2, b3);
+      }
+  }
+}
+
+// running maximum, denominator and outputs of the lane's two rows over NT tiles of keys whose scores (in units of log 2, -inf: not
+// seen) are in `s`, with the values in TERMS tiles
+template <int VDT, int NT, int TERMS>
+__device__ __forceinline__ void pm_gather(float (&s)[NT][4], float (&o)[VDT * 2][4], float& mA, float& mB, float& lA, float& lB,
+                                          const __nv_bfloat16* vs, int tile, int lane) {
+  constexpr int PITCH = VDT * 16 + 8;
+  float mxA = -INFINITY, mxB = -INFINITY;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    mxA = fmaxf(mxA, fmaxf(s[nt][0], s[nt][1]));
+    mxB = fmaxf(mxB, fmaxf(s[nt][2], s[nt][3]));
+  }
+#pragma unroll
+  for (int off = 1; off < 4; off <<= 1) {
+    mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, off));
+    mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, off));
+  }
+  const float nmA = fmaxf(mA, mxA), nmB = fmaxf(mB, mxB);
+  const float refA = nmA == -INFINITY ? 0.f : nmA, refB = nmB == -INFINITY ? 0.f : nmB;      // (a row that sees no key yet)
+  const float corrA = exp2f(mA - refA), corrB = exp2f(mB - refB);
+  float sumA = 0.f, sumB = 0.f;
+#pragma unroll
+  for (int nt = 0; nt < NT; ++nt) {
+    s[nt][0] = exp2f(s[nt][0] - refA);
+    s[nt][1] = exp2f(s[nt][1] - refA);
+    s[nt][2] = exp2f(s[nt][2] - refB);
+    s[nt][3] = exp2f(s[nt][3] - refB);
+    sumA += s[nt][0] + s[nt][1];
+    sumB += s[nt][2] + s[nt][3];
+  }
+#pragma unroll
+  for (int off = 1; off < 4; off <<= 1) {
+    sumA += __shfl_xor_sync(0xffffffffu, sumA, off);
+    sumB += __shfl_xor_sync(0xffffffffu, sumB, off);
+  }
+  lA = lA * corrA + sumA;
+  lB = lB * corrB + sumB;
+  mA = nmA;
+  mB = nmB;
+  if (__any_sync(0xffffffffu, corrA != 1.f || corrB != 1.f)) {
+#pragma unroll
+    for (int i = 0; i < VDT * 2; ++i) {
+      o[i][0] *= corrA;
+      o[i][1] *= corrA;
+      o[i][2] *= corrB;
+      o[i][3] *= corrB;
+    }
+  }
+#pragma unroll
+  for (int kt = 0; kt < NT / 2; ++kt) {
+    uint32_t a[3][4];
+    sp_split(s[2 * kt][0], s[2 * kt][1], a[0][0], a[1][0], a[2][0]);
+    sp_split(s[2 * kt][2], s[2 * kt][3], a[0][1], a[1][1], a[2][1]);
+    sp_split(s[2 * kt + 1][0], s[2 * kt + 1][1], a[0][2], a[1][2], a[2][2]);
+    sp_split(s[2 * kt + 1][2], s[2 * kt + 1][3], a[0][3], a[1][3], a[2][3]);
+#pragma unroll
+    for (int v = TERMS - 1; v >= 0; --v)
+#pragma unroll
+      for (int dt = 0; dt < VDT * 2; dt += 2) {
+        const int mi = lane >> 3;
+        uint32_t b0, b1, b2, b3;
+        sp_ldmatrix_x4_trans(sp_smem(vs + v * tile + (kt * 16 + (mi & 1) * 8 + (lane & 7)) * PITCH + (dt + (mi >> 1)) * 8), b0, b1, b2, b3);
+#pragma unroll
+        for (int t = 2 - v; t >= 0; --t) {      // (terms whose places add up to more than 2 are under float32's last bit)
+          sp_mma(o[dt], a[t][0], a[t][1], a[t][2], a[t][3], b0, b1);
+          sp_mma(o[dt + 1], a[t][0], a[t][1], a[t][2], a[t][3], b2, b3);
+        }
+      }
+  }
+}
+
+template <int HDT>
+__global__ void __launch_bounds__(PM_WARPS * 32)
+pooled_window_attn_mma_kernel(const __nv_bfloat16* __restrict__ q, __nv_bfloat16* __restrict__ out, const __nv_bfloat16* __restrict__ kcache,
+                              const __nv_bfloat16* __restrict__ vcache, const float* __restrict__ pk, const float* __restrict__ pv,
+                              const int32_t* __restrict__ page_table, int table_stride, int n_pages, const int32_t* __restrict__ tile_seq,
+                              const int32_t* __restrict__ tile_tok0, const int32_t* __restrict__ tile_ntok,
+                              const int32_t* __restrict__ tile_pos0, int H, int G, float scale, int window, int P, int R) {
+  constexpr int HD = HDT * 16, PITCH = HD + 8, PIECES = HD / 8, STAGE = 2 * PAGE * PITCH, TERM = PM_POOLED * PITCH;
+  extern __shared__ __align__(16) uint8_t pm_raw[];
+  __nv_bfloat16* sm = reinterpret_cast<__nv_bfloat16*>(pm_raw);      // two stages (keys | values), or three terms of pooled keys | values
+  const int tile = blockIdx.x, head = blockIdx.y, g = head / (H / G);
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, gid = lane >> 2, tig = lane & 3;
+  const int tok0 = tile_tok0[tile], ntok = tile_ntok[tile], pos0 = tile_pos0[tile];
+  const int32_t* table = page_table + (size_t)tile_seq[tile] * table_stride;
+  const int rowA = warp * 16 + gid, rowB = rowA + 8;
+  const int posA = rowA < ntok ? pos0 + rowA : -1, posB = rowB < ntok ? pos0 + rowB : -1;      // (-1: no such row, nothing is seen)
+  const int n_keys = pos0 + ntok, first_page = max(0, pos0 - window + 1) / PAGE, end_page = (n_keys + PAGE - 1) / PAGE;
+  const float scale2 = scale * 1.4426950408889634f;                  // scores in units of log 2
+  auto page_of = [&](int i) {
+    const int page = table[i];
+    return page < n_pages ? page : -1;
+  };
+  auto load_page = [&](int i, int stage) {
+    const int page = page_of(i), valid = page >= 0 ? min(PAGE, n_keys - i * PAGE) : 0;      // (rows past the last key: zeros)
+    const size_t row0 = ((size_t)max(page, 0) * G + g) * PAGE;
+    __nv_bfloat16* ks = sm + stage * STAGE;
+    for (int e = threadIdx.x; e < PAGE * PIECES; e += PM_WARPS * 32) {
+      const int r = e / PIECES, c = (e - r * PIECES) * 8, bytes = r < valid ? 16 : 0;
+      sp_cp16(sp_smem(ks + r * PITCH + c), bytes ? kcache + (row0 + r) * HD + c : kcache, bytes);
+      sp_cp16(sp_smem(ks + PAGE * PITCH + r * PITCH + c), bytes ? vcache + (row0 + r) * HD + c : vcache, bytes);
+    }
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  uint32_t qa[HDT][4];
+  {
+    const uint32_t* qA = reinterpret_cast<const uint32_t*>(q + ((size_t)(tok0 + min(rowA, ntok - 1)) * H + head) * HD) + tig;
+    const uint32_t* qB = reinterpret_cast<const uint32_t*>(q + ((size_t)(tok0 + min(rowB, ntok - 1)) * H + head) * HD) + tig;
+#pragma unroll
+    for (int d = 0; d < HDT; ++d) {
+      qa[d][0] = qA[d * 8];
+      qa[d][1] = qB[d * 8];
+      qa[d][2] = qA[d * 8 + 4];
+      qa[d][3] = qB[d * 8 + 4];
+    }
+  }
+  float o[HDT * 2][4];
+#pragma unroll
+  for (int i = 0; i < HDT * 2; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
+  float mA = -INFINITY, mB = -INFINITY, lA = 0.f, lB = 0.f;
+
+  // the pooled rows of the blocks that the tile's last token sees, 32 at a time: each value as three terms
+  auto blocks_seen = [&](int pos) { return P > 0 && pos >= window ? (pos - window + 1) / P : 0; };
+  const int nbA = blocks_seen(posA), nbB = blocks_seen(posB), nb = blocks_seen(n_keys - 1);
+  for (int b0 = 0; b0 < nb; b0 += PM_POOLED) {
+    __syncthreads();
+    for (int e = threadIdx.x; e < PM_POOLED * (HD / 2) * 2; e += PM_WARPS * 32) {
+      const int which = e / (PM_POOLED * (HD / 2)), r = e / (HD / 2) % PM_POOLED, c = e % (HD / 2) * 2, b = b0 + r;
+      float2 x = make_float2(0.f, 0.f);
+      if (b < nb) {
+        const int end = b * P + P - 1, page = page_of(end / PAGE);
+        if (page >= 0) x = *reinterpret_cast<const float2*>((which ? pv : pk) + (((size_t)page * G + g) * R + b - PAGE * (end / PAGE) / P) * HD + c);
+      }
+      uint32_t t1, t2, t3;
+      sp_split(x.x, x.y, t1, t2, t3);
+      __nv_bfloat16* dst = sm + which * 3 * TERM + r * PITCH + c;
+      *reinterpret_cast<uint32_t*>(dst) = t1;
+      *reinterpret_cast<uint32_t*>(dst + TERM) = t2;
+      *reinterpret_cast<uint32_t*>(dst + 2 * TERM) = t3;
+    }
+    __syncthreads();
+    float s[PM_POOLED / 8][4];
+    pm_scores<HDT, PM_POOLED / 8, 3>(s, qa, sm, TERM, lane);
+#pragma unroll
+    for (int nt = 0; nt < PM_POOLED / 8; ++nt)
+#pragma unroll
+      for (int j = 0; j < 4; ++j) s[nt][j] = b0 + nt * 8 + tig * 2 + (j & 1) < (j < 2 ? nbA : nbB) ? s[nt][j] * scale2 : -INFINITY;
+    pm_gather<HDT, PM_POOLED / 8, 3>(s, o, mA, mB, lA, lB, sm + 3 * TERM, TERM, lane);
+  }
+  if (nb > 0) __syncthreads();
+  // the window's pages
+  const int warp_last = warp * 16 < ntok ? pos0 + min(ntok - 1, warp * 16 + 15) : -1, warp_first = pos0 + warp * 16 - window + 1;
+  load_page(first_page, 0);
+  for (int i = first_page; i < end_page; ++i) {
+    const int stage = (i - first_page) & 1;
+    if (i + 1 < end_page) {
+      load_page(i + 1, stage ^ 1);
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    if (i * PAGE <= warp_last && i * PAGE + PAGE > warp_first) {      // else: no row of this warp sees a key of the page
+      const __nv_bfloat16* ks = sm + stage * STAGE;
+      float s[PAGE / 8][4];
+      pm_scores<HDT, PAGE / 8, 1>(s, qa, ks, 0, lane);
+      // every row sees the whole page: no mask
+      const bool whole = warp * 16 + 15 < ntok && i * PAGE + PAGE - 1 <= pos0 + warp * 16 && i * PAGE >= warp_first + 15;
+#pragma unroll
+      for (int nt = 0; nt < PAGE / 8; ++nt)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+          const int key = i * PAGE + nt * 8 + tig * 2 + (j & 1), pos = j < 2 ? posA : posB;
+          s[nt][j] = whole || (key <= pos && key > pos - window) ? s[nt][j] * scale2 : -INFINITY;
+        }
+      pm_gather<HDT, PAGE / 8, 1>(s, o, mA, mB, lA, lB, ks + PAGE * PITCH, 0, lane);
+    }
+    __syncthreads();
+  }
+  const float invA = lA > 0.f ? 1.0f / lA : 0.f, invB = lB > 0.f ? 1.0f / lB : 0.f;
+#pragma unroll
+  for (int dt = 0; dt < HDT * 2; ++dt) {
+    const int d = dt * 8 + tig * 2;
+    if (rowA < ntok) *reinterpret_cast<__nv_bfloat162*>(out + ((size_t)(tok0 + rowA) * H + head) * HD + d) = __floats2bfloat162_rn(o[dt][0] * invA, o[dt][1] * invA);
+    if (rowB < ntok) *reinterpret_cast<__nv_bfloat162*>(out + ((size_t)(tok0 + rowB) * H + head) * HD + d) = __floats2bfloat162_rn(o[dt][2] * invB, o[dt][3] * invB);
+  }
+}
+
 }  // namespace edgelm
 
 using namespace edgelm;
@@ -588,5 +806,38 @@ extern "C" int edgelm_pooled_window_attn_tiled(const void* q, void* out, const v
 #undef EL_TW
   if (rc != 0) return rc;
   EL_LAUNCH_CHECK("pooled_window_attn_tiled");
+  return 0;
+}
+
+// 1 if the tensor-core kernel of prompt steps takes these head sizes, else 0.
+extern "C" int edgelm_pooled_window_attn_mma_takes(int dk, int dv) { return dk == dv && (dk == 32 || dk == 64 || dk == 96 || dk == 128) ? 1 : 0; }
+
+// `edgelm_pooled_window_attn_tiled` on the tensor cores: a bfloat16 cache, tiles of at most 64 consecutive tokens of one sequence.
+extern "C" int edgelm_pooled_window_attn_mma(const void* q, void* out, const void* kcache, const void* vcache, const float* pk, const float* pv,
+                                             const int32_t* page_table, int table_stride, int n_pages, const int32_t* tile_seq,
+                                             const int32_t* tile_tok0, const int32_t* tile_ntok, const int32_t* tile_pos0, int n_tiles, int H,
+                                             int G, int dk, int dv, float scale, int window, int P, int R, cudaStream_t stream) {
+  if (n_tiles == 0) return 0;
+  EL_REFUSE(n_tiles > 0 && H > 0 && H <= 65535 && G > 0 && H % G == 0, "pooled_window_attn_mma: %d query heads over %d key/value heads", H, G);
+  EL_REFUSE(edgelm_pooled_window_attn_mma_takes(dk, dv), "pooled_window_attn_mma: head sizes %d / %d are not taken (32, 64, 96 or 128, both alike)", dk, dv);
+  EL_REFUSE(window >= 1 && P >= 0 && (P == 0 || (R == (PAGE + P - 1) / P && pk != nullptr && pv != nullptr)), "pooled_window_attn_mma: window %d, block %d, rows a page %d", window, P, R);
+  EL_REFUSE((uintptr_t)q % 4 == 0 && (uintptr_t)out % 4 == 0 && (uintptr_t)kcache % 16 == 0 && (uintptr_t)vcache % 16 == 0 && (uintptr_t)pk % 8 == 0 && (uintptr_t)pv % 8 == 0,
+            "pooled_window_attn_mma: keys and values must be 16-byte aligned, pooled rows 8");
+  const size_t smem = (size_t)2 * 2 * PAGE * (dk + 8) * 2;      // (more than the pooled rows' six terms of 32 rows)
+#define EL_PM(HDT)                                                                                                                       \
+  do {                                                                                                                                   \
+    auto kern = pooled_window_attn_mma_kernel<HDT>;                                                                                      \
+    const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);                            \
+    EL_REFUSE(e == cudaSuccess, "pooled_window_attn_mma: %zu bytes of shared memory refused: %s", smem, cudaGetErrorString(e));          \
+    kern<<<dim3(n_tiles, H), PM_WARPS * 32, smem, stream>>>((const __nv_bfloat16*)q, (__nv_bfloat16*)out, (const __nv_bfloat16*)kcache,  \
+                                                           (const __nv_bfloat16*)vcache, pk, pv, page_table, table_stride, n_pages,      \
+                                                           tile_seq, tile_tok0, tile_ntok, tile_pos0, H, G, scale, window, P, R);        \
+  } while (0)
+  if (dk == 32) EL_PM(2);
+  else if (dk == 64) EL_PM(4);
+  else if (dk == 96) EL_PM(6);
+  else EL_PM(8);
+#undef EL_PM
+  EL_LAUNCH_CHECK("pooled_window_attn_mma");
   return 0;
 }

@@ -655,6 +655,31 @@ def pooled_window_attn_tiled(q, out, kcache, vcache, pooled_k, pooled_v, page_ta
                                                  nh, nkv, dk, dv, ctypes.c_float(scale), int(window), int(pool or 0), rows, _stream()))
 
 
+def pooled_window_attn_mma_takes(dtype, dk, dv):
+    """Whether the tensor-core form of `pooled_window_attn_tiled` takes a cache of this type and these head sizes."""
+    return dtype == torch.bfloat16 and dk == dv and dk in (32, 64, 96, 128)
+
+
+def pooled_window_attn_mma(q, out, kcache, vcache, pooled_k, pooled_v, page_table, tile_seq, tile_tok0, tile_ntok, tile_pos0, n_tiles,
+                           nh, nkv, dk, dv, scale, window, pool):
+    """`pooled_window_attn_tiled` on the tensor cores, over tiles of at most SPLIT_PREFILL_TILE tokens."""
+    T = q.shape[0]
+    _need(q.is_contiguous() and out.is_contiguous() and q.shape == (T, nh * dk) and out.shape == (T, nh * dv) and
+          q.dtype == out.dtype == kcache.dtype == torch.bfloat16, "pooled_window_attn_mma: shapes")
+    _pooled_cache_check(kcache, vcache, nkv, dk, dv, "pooled_window_attn_mma")
+    for t, n in ((page_table, "page_table"), (tile_seq, "tile_seq"), (tile_tok0, "tile_tok0"), (tile_ntok, "tile_ntok"), (tile_pos0, "tile_pos0")):
+        _i32(t, n)
+    rows = 0
+    if pool:
+        _f32(pooled_k, "pooled_k"); _f32(pooled_v, "pooled_v")
+        rows = pooled_k.shape[2]
+        _need(tuple(pooled_k.shape) == (kcache.shape[0], nkv, rows, dk) and tuple(pooled_v.shape) == (kcache.shape[0], nkv, rows, dv), "pooled_window_attn_mma: pooled layout")
+    _check(lib().edgelm_pooled_window_attn_mma(_p(q), _p(out), _p(kcache), _p(vcache), _p(pooled_k) if pool else _p(None),
+                                               _p(pooled_v) if pool else _p(None), _p(page_table), page_table.stride(0), kcache.shape[0],
+                                               _p(tile_seq), _p(tile_tok0), _p(tile_ntok), _p(tile_pos0), int(n_tiles), nh, nkv, dk, dv,
+                                               ctypes.c_float(scale), int(window), int(pool or 0), rows, _stream()))
+
+
 # ----------------------------------------------------------------------------- attention with a key range per query
 MASK_CAUSAL, MASK_WINDOW, MASK_CHUNK = 0, 1, 2
 

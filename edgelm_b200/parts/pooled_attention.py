@@ -47,8 +47,12 @@ class PooledWindowAttention(Part):
         self.freq = self.b_qkv = None
         self.tile_tokens = max(1, 32 // (self.nh // self.nkv))   # tokens whose heads fill one block of the prompt kernel
 
+    def _on_tensor_cores(self):
+        """Whether prompt steps take the tensor-core kernel: a bfloat16 cache and head sizes that it takes."""
+        return ops.pooled_window_attn_mma_takes(self.dtype, self.dk, self.dv)
+
     def tile_sizes(self):
-        return (self.tile_tokens,)
+        return (ops.SPLIT_PREFILL_TILE if self._on_tensor_cores() else self.tile_tokens,)
 
     def sizes(self):
         return {"heads": self.nh, "kv_heads": self.nkv, "head_dim": self.dk, "v_head_dim": self.dv, "window": self.window,
@@ -111,6 +115,10 @@ class PooledWindowAttention(Part):
             if ctx.all_single:      # one token a sequence: a block per (token, head), its warps sharing the keys
                 ops.pooled_window_attn(q, a, cache.k, cache.v, pooled_k, pooled_v, ctx.tok_pos, ctx.tok_seq, table, self.nh, self.nkv, self.dk,
                                        self.dv, self.scale, self.window, self.pool)
+            elif self._on_tensor_cores():
+                tiles = ctx.tiles(ops.SPLIT_PREFILL_TILE)
+                ops.pooled_window_attn_mma(q, a, cache.k, cache.v, pooled_k, pooled_v, table, tiles.seq, tiles.tok0, tiles.ntok, tiles.pos0,
+                                           tiles.count, self.nh, self.nkv, self.dk, self.dv, self.scale, self.window, self.pool)
             else:                   # a prompt step: keys staged once for the 32 rows of a tile
                 tiles = ctx.tiles(self.tile_tokens)
                 ops.pooled_window_attn_tiled(q, a, cache.k, cache.v, pooled_k, pooled_v, table, tiles.seq, tiles.tok0, tiles.ntok, tiles.pos0,

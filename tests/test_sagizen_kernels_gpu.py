@@ -228,6 +228,49 @@ def test_window_attention_with_pooled_blocks(dtype, window, pool, dk, dv, H, G):
         assert np.isfinite(ot).all() and np.abs(ot - w).max() < tol * max(1.0, np.abs(w).max())
 
 
+@pytest.mark.parametrize("window,pool,d,H,G", [(100, 64, 64, 4, 2), (7, 3, 32, 3, 1), (64, 1, 96, 2, 2), (200, 5, 128, 2, 1), (50, None, 64, 2, 1)])
+def test_pooled_attention_on_the_tensor_cores(window, pool, d, H, G):
+    """Prompts and pieces that go on from the cache, up to 300 pooled rows, edges of pages and tiles, unwritten rows poisoned.  The
+    output's bfloat16 rounding is 2^-9 of a value; beside the CUDA-core kernel, whose float32 sums differ in order only, a rounding
+    may fall the other way where a sum lies within 2^-20 of its edge (a share of 2^-9, measured under 0.002)."""
+    from edgelm_b200.engine.batch import make_tiles
+    g = np.random.default_rng(window)
+    PAGE, total, scale = 64, [333, 64, 1], 1.3 / np.sqrt(d)
+    bf = lambda a: torch.tensor(a, dtype=torch.bfloat16).double().numpy()
+    q = [bf(g.normal(size=(n, H, d)) * 2) for n in total]
+    k, v = ([bf(g.normal(size=(n, G, d))) for n in total] for _ in range(2))
+    want = [plain.pooled_window_attention(a, b, c, scale, window, pool) for a, b, c in zip(q, k, v)]
+    R = -(-PAGE // pool) if pool else 1
+    kc, vc = (torch.full((9, G, PAGE, d), float("nan"), dtype=torch.bfloat16, device=DEV) for _ in range(2))
+    pk, pv = (torch.full((9, G, R, d), float("nan"), device=DEV) for _ in range(2))
+    table, err = i32([[5, 2, 7, 8, 1, 3], [0] + [-1] * 5, [6] + [-1] * 5]), torch.zeros(1, dtype=torch.int32, device=DEV)
+    assert ops.pooled_window_attn_mma_takes(torch.bfloat16, d, d)
+    for step in steps_of(total, [[70, 1, 63, 199], [5, 2, 57], [1]]):
+        live = [(s, a, n) for s, (a, n) in enumerate(step) if n]
+        T = sum(n for _, _, n in live)
+        pos, seq = i32(np.concatenate([np.arange(a, a + n) for _, a, n in live])), i32(np.concatenate([np.full(n, s) for s, _, n in live]))
+        row = lambda s, a, n: np.concatenate([x[s][a:a + n].reshape(n, -1) for x in (q, k, v)], 1)
+        qd = torch.empty(T, H * d, dtype=torch.bfloat16, device=DEV)
+        ops.qk_rope_norm_append(f32(np.concatenate([row(*l) for l in live])), None, qd, pos, seq, table, kc, vc, H, G, d, d, 0, None, 0.0, False, err)
+        if pool:
+            ops.pool_blocks(pos, seq, table, kc, vc, pk, pv, T, G, d, d, pool, err)
+        outs = []
+        for tokens in (64, max(1, 32 // (H // G))):
+            cols = make_tiles([n for _, _, n in live], [a for _, a, _ in live], tokens)
+            out = torch.full((T, H * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+            call = (qd, out, kc, vc, pk if pool else None, pv if pool else None, table[[s for s, _, _ in live]].contiguous(), *map(i32, cols), len(cols[0]))
+            if tokens == 64:
+                ops.pooled_window_attn_mma(*call, H, G, d, d, scale, window, pool)
+            else:
+                ops.pooled_window_attn_tiled(*call, tokens, H, G, d, d, scale, window, pool)
+            outs.append(out.float().cpu().numpy())
+        ref = np.concatenate([want[s][a:a + n].reshape(n, -1) for s, a, n in live])
+        assert np.abs(outs[0] - ref).max() < 2.0 ** -8 * np.abs(ref).max()
+        assert (np.abs(outs[0] - ref) <= 2.0 ** -8 * np.abs(ref) + 1e-5).all()
+        assert (outs[0] != outs[1]).mean() < 0.01
+    assert int(err.item()) == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_rotation_bias_and_unit_norm(dtype):
     g = np.random.default_rng(9)
