@@ -1,0 +1,71 @@
+// Small float32 matrix products out of shared memory, for recurrences that are worked off chunk by chunk: both operands lie with the
+// summed index contiguous, in rows whose pitch is 4 floats times an odd number (eight neighbouring rows' pieces of 16 bytes then lie
+// in different banks).
+#pragma once
+#include "common.cuh"
+
+namespace edgelm {
+
+constexpr int CHUNK = 64;      // tokens of a chunk (the step's tiles of that size)
+
+__host__ __device__ constexpr int chunk_pitch(int n) { return ((n + 3) / 4 | 1) * 4; }
+
+// Thread (ty, tx) of a block of 16 NY threads: rows m = ty + NY a, columns n = tx + 16 b.  (Neighbouring threads are two rows of one
+// column: a read of 16 bytes a lane then takes two clocks for either operand.)
+__device__ __forceinline__ int chunk_tx() { return threadIdx.x >> 1 & 15; }
+__device__ __forceinline__ int chunk_ty() { return (threadIdx.x & 1) + (threadIdx.x >> 5) * 2; }
+
+// acc[a][b] += sum over k < K of A[m][k] B[n][k]; K a multiple of 4; rows from M and columns from N on: the last one's again.
+// Packed pairs of multiply-adds; the products are summed in two runs (four for small tiles) of their own before they join `acc`.
+template <int NY, int RM, int RN>
+__device__ __forceinline__ void chunk_mm(float (&acc)[RM][RN], const float* A, int pa, int M, const float* B, int pb, int N, int K) {
+  constexpr int RUNS = RM * RN <= 16 ? 2 : 1;
+  const int tx = chunk_tx(), ty = chunk_ty();
+  const float* ar[RM];
+  const float* br[RN];
+  unsigned long long sum[RUNS][RM][RN] = {};
+#pragma unroll
+  for (int a = 0; a < RM; ++a) ar[a] = A + min(ty + NY * a, M - 1) * pa;
+#pragma unroll
+  for (int b = 0; b < RN; ++b) br[b] = B + min(tx + 16 * b, N - 1) * pb;
+#pragma unroll 2
+  for (int k = 0; k < K; k += 4) {
+    ulonglong2 av[RM];
+#pragma unroll
+    for (int a = 0; a < RM; ++a) av[a] = *reinterpret_cast<const ulonglong2*>(ar[a] + k);
+#pragma unroll
+    for (int b = 0; b < RN; ++b) {
+      const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(br[b] + k);
+#pragma unroll
+      for (int a = 0; a < RM; ++a) {
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[0][a][b]) : "l"(av[a].x), "l"(bv.x));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[RUNS - 1][a][b]) : "l"(av[a].y), "l"(bv.y));
+      }
+    }
+  }
+#pragma unroll
+  for (int a = 0; a < RM; ++a)
+#pragma unroll
+    for (int b = 0; b < RN; ++b) {
+      float v = 0.f;
+#pragma unroll
+      for (int r = 0; r < RUNS; ++r) v += __uint_as_float((uint32_t)sum[r][a][b]) + __uint_as_float((uint32_t)(sum[r][a][b] >> 32));
+      acc[a][b] += v;
+    }
+}
+
+__device__ __forceinline__ void chunk_cp16(float* dst, const float* src, bool there) {
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
+}
+
+// rows [rows][n] of `src` (row pitch ld, n a multiple of 4, 16-byte aligned) on their way into dst [..][pitch]; zeros for the rows from
+// `valid` on
+__device__ __forceinline__ void chunk_rows(float* dst, int pitch, const float* src, size_t ld, int rows, int valid, int n) {
+  const int nv = n >> 2;
+  for (int i = threadIdx.x; i < rows * nv; i += blockDim.x) {
+    const int r = i / nv, c = (i - r * nv) * 4;
+    chunk_cp16(dst + r * pitch + c, r < valid ? src + (size_t)r * ld + c : src, r < valid);
+  }
+}
+
+}  // namespace edgelm

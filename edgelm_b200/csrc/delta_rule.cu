@@ -10,7 +10,7 @@
 //
 // Tokens of all sequences are packed along the first axis; `seq_tok0[s] .. seq_tok0[s + 1] - 1` are the packed rows of
 // the batch's sequence s, `seq_slot[s]` the row of its state.
-#include "common.cuh"
+#include "chunk_mm.cuh"
 
 namespace edgelm {
 
@@ -173,6 +173,269 @@ delta_scan_kernel(const float* __restrict__ qkv, int C, const float* __restrict_
     }
 }
 
+// ------------------------------------------------------------------ the recurrence chunk by chunk
+// For prompt steps: with L_t the sum of the logarithms of the decays of a chunk's tokens up to t, S0 the state before the chunk and
+// u_t the correction that token t writes,
+//
+//     u_t = beta_t (v_t - exp(L_t) S0^T k_t - sum_(s < t) exp(L_t - L_s) (k_t . k_s) u_s)
+//     o_t = exp(L_t) S0^T q_t + sum_(s <= t) exp(L_t - L_s) (q_t . k_s) u_s
+//     S   = exp(L_n) S0 + sum_s exp(L_n - L_s) k_s u_s^T
+//
+// so the corrections solve (I + A) U = beta V - (beta exp(L) K) S0 with A strictly lower triangular, and what goes from chunk to chunk is
+// two small matrix products instead of a chain through every token:
+//   1. `delta_chunk_solve`, every (chunk, head) at once: A, then U0 = (I + A)^-1 beta V and W = (I + A)^-1 (beta exp(L) K) by
+//      substitution, a thread a column with its 64 values in registers;
+//   2. `delta_chunk_states`, the chunks of a (sequence, head) in order, blocks of 16 value channels: U = U0 - W S0, then S;
+//   3. `delta_chunk_out`, every (chunk, head) at once: the outputs from U and the kept S0.
+// Logarithms and their sums are kept in double precision (a decay that is zero in float32 counts as exp(-200)), everything else is float32.
+// One (chunk, head) of the scratch: U0, later U, [e][64]; W [64][d]; the keys times exp(L_n - L_s) [d][64]; S0 [e][d].  Then exp(L_n) of each.
+// Bound by the substitution and the products out of shared memory.  Nine heads of 64, prompts of 333 to
+// 1,700 tokens (4,065 in all): the walk 548 us, this 197 (48 + 95 + 53).
+constexpr int DC_BLOCK = 16;       // value channels a block of `delta_chunk_states` owns
+constexpr int DC_STATE_THREADS = 128;
+
+__host__ __device__ inline size_t dc_floats(int d, int e) { return (size_t)(2 * CHUNK) * d + (size_t)CHUNK * e + (size_t)d * e; }
+
+// lg[t] = L_t of the chunk's tokens (from ntok on: the last one's), by the first warp; the block synchronises afterwards
+__device__ __forceinline__ void dc_logs(double* lg, const float* __restrict__ bg, int tok0, int ntok, int H, int h) {
+  if (threadIdx.x >= 32) return;
+  double x[2];
+#pragma unroll
+  for (int i = 0; i < 2; ++i) {
+    const int t = 2 * threadIdx.x + i;
+    x[i] = t < ntok ? fmax(log((double)bg[(size_t)(tok0 + t) * 2 * H + H + h]), -200.0) : 0.0;
+  }
+  double sum = x[0] + x[1];
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const double up = __shfl_up_sync(0xffffffffu, sum, off);
+    if (threadIdx.x >= off) sum += up;
+  }
+  lg[2 * threadIdx.x] = sum - x[1];
+  lg[2 * threadIdx.x + 1] = sum;
+}
+
+__global__ void __launch_bounds__(256)
+delta_chunk_solve_kernel(const float* __restrict__ qkv, int C, const float* __restrict__ bg, float* __restrict__ scratch,
+                         float* __restrict__ full, const int32_t* __restrict__ tile_tok0, const int32_t* __restrict__ tile_ntok, int H, int G,
+                         int d, int e) {
+  extern __shared__ __align__(16) float dc_smem[];
+  __shared__ double lg[CHUNK];
+  __shared__ float beta[CHUNK];
+  const int P = chunk_pitch(d);
+  float* ks = dc_smem;                       // [CHUNK][P]
+  float* at = ks + CHUNK * P;                // [s][t]: A[t][s]
+  constexpr int AP = CHUNK + 4;
+  const int tile = blockIdx.x, h = blockIdx.y, g = h / (H / G), tok0 = tile_tok0[tile], ntok = tile_ntok[tile];
+  chunk_rows(ks, P, qkv + (size_t)tok0 * C + G * d + g * d, C, CHUNK, ntok, d);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  dc_logs(lg, bg, tok0, ntok, H, h);
+  if (threadIdx.x >= 64 && threadIdx.x < 64 + CHUNK) {
+    const int t = threadIdx.x - 64;
+    beta[t] = t < ntok ? bg[(size_t)(tok0 + t) * 2 * H + h] : 0.f;
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  {
+    float acc[4][4] = {};
+    chunk_mm<16, 4, 4>(acc, ks, P, CHUNK, ks, P, CHUNK, d);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int s = chunk_ty() + 16 * a, t = chunk_tx() + 16 * b;
+        at[s * AP + t] = s < t ? beta[t] * expf((float)(lg[t] - lg[s])) * acc[a][b] : 0.f;
+      }
+  }
+  __syncthreads();
+  const int c = threadIdx.x;
+  float* base = scratch + ((size_t)tile * H + h) * dc_floats(d, e);
+  if (c == 0) full[(size_t)tile * H + h] = expf((float)lg[CHUNK - 1]);
+  if (c >= d + e) return;
+  float x[CHUNK];
+  if (c < e) {
+    const float* v = qkv + (size_t)tok0 * C + 2 * G * d + (size_t)h * e + c;
+#pragma unroll
+    for (int t = 0; t < CHUNK; ++t) x[t] = t < ntok ? v[(size_t)t * C] : 0.f;
+#pragma unroll
+    for (int t = 0; t < CHUNK; ++t) x[t] *= beta[t];
+  } else {
+    float* kt = base + (size_t)CHUNK * e + (size_t)CHUNK * d + (size_t)(c - e) * CHUNK;
+    const double last = lg[CHUNK - 1];
+#pragma unroll
+    for (int t = 0; t < CHUNK; ++t) x[t] = ks[t * P + c - e];
+#pragma unroll
+    for (int t = 0; t < CHUNK; t += 4)
+      *reinterpret_cast<float4*>(kt + t) = make_float4(x[t] * expf((float)(last - lg[t])), x[t + 1] * expf((float)(last - lg[t + 1])),
+                                                       x[t + 2] * expf((float)(last - lg[t + 2])), x[t + 3] * expf((float)(last - lg[t + 3])));
+#pragma unroll
+    for (int t = 0; t < CHUNK; ++t) x[t] *= beta[t] * expf((float)lg[t]);
+  }
+#pragma unroll
+  for (int s = 0; s < CHUNK - 1; ++s) {
+#pragma unroll
+    for (int t = (s + 1) & ~3; t < CHUNK; t += 4) {      // (at [s][t] is zero up to t = s)
+      const float4 a = *reinterpret_cast<const float4*>(at + s * AP + t);
+      if (t > s) x[t] = fmaf(-a.x, x[s], x[t]);
+      if (t + 1 > s) x[t + 1] = fmaf(-a.y, x[s], x[t + 1]);
+      if (t + 2 > s) x[t + 2] = fmaf(-a.z, x[s], x[t + 2]);
+      x[t + 3] = fmaf(-a.w, x[s], x[t + 3]);
+    }
+  }
+  if (c < e) {
+#pragma unroll
+    for (int t = 0; t < CHUNK; t += 4) *reinterpret_cast<float4*>(base + (size_t)c * CHUNK + t) = make_float4(x[t], x[t + 1], x[t + 2], x[t + 3]);
+  } else {
+#pragma unroll
+    for (int t = 0; t < CHUNK; ++t) base[(size_t)CHUNK * e + (size_t)t * d + c - e] = x[t];
+  }
+}
+
+template <int RN>      // ceil(d / 16)
+__global__ void __launch_bounds__(DC_STATE_THREADS)
+delta_chunk_states_kernel(float* __restrict__ scratch, const float* __restrict__ full, float* __restrict__ state,
+                          const int32_t* __restrict__ seq_tok0, const int32_t* __restrict__ seq_slot, int H, int d, int e) {
+  extern __shared__ __align__(16) float dc_smem[];
+  constexpr int AP = CHUNK + 4;
+  const int P = chunk_pitch(d), STAGE = CHUNK * P + d * AP + DC_BLOCK * CHUNK;
+  float* ss = dc_smem + 2 * STAGE;           // the state's rows [DC_BLOCK][P]
+  float* us = ss + DC_BLOCK * P;             // U [DC_BLOCK][AP]
+  const int s = blockIdx.x / H, h = blockIdx.x - s * H, j0 = blockIdx.y * DC_BLOCK, nj = min(DC_BLOCK, e - j0);
+  int first = 0;                             // the sequence's first tile: every earlier sequence has ceil(n / CHUNK)
+  for (int p = 0; p < s; ++p) first += (seq_tok0[p + 1] - seq_tok0[p] + CHUNK - 1) / CHUNK;
+  const int chunks = (seq_tok0[s + 1] - seq_tok0[s] + CHUNK - 1) / CHUNK;
+  if (chunks == 0) return;
+  const size_t FL = dc_floats(d, e);
+  float* st = state + ((size_t)seq_slot[s] * H + h) * e * d + (size_t)j0 * d;
+  auto load = [&](int c) {                   // W, the scaled keys, this block's rows of U0
+    float* dst = dc_smem + (c & 1) * STAGE;
+    const float* base = scratch + ((size_t)(first + c) * H + h) * FL;
+    chunk_rows(dst, P, base + (size_t)CHUNK * e, d, CHUNK, CHUNK, d);
+    chunk_rows(dst + CHUNK * P, AP, base + (size_t)CHUNK * e + (size_t)CHUNK * d, CHUNK, d, d, CHUNK);
+    chunk_rows(dst + CHUNK * P + d * AP, CHUNK, base + (size_t)j0 * CHUNK, CHUNK, DC_BLOCK, nj, CHUNK);
+    asm volatile("cp.async.commit_group;" ::: "memory");
+  };
+  load(0);
+  const int tx = chunk_tx(), ty = chunk_ty();
+  float S[2][RN];                            // rows ty + 8 a of the block's channels, key channels tx + 16 b
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < RN; ++b) {
+      const int j = ty + 8 * a, i = tx + 16 * b;
+      S[a][b] = j < nj && i < d ? st[(size_t)j * d + i] : 0.f;
+    }
+  float keep_next = full[(size_t)first * H + h];
+  for (int c = 0; c < chunks; ++c) {
+    float* base = scratch + ((size_t)(first + c) * H + h) * FL;
+    float* kept = base + (size_t)CHUNK * e + (size_t)(2 * CHUNK) * d + (size_t)j0 * d;
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < RN; ++b) {
+        const int j = ty + 8 * a, i = tx + 16 * b;
+        if (i < d) {
+          ss[j * P + i] = S[a][b];
+          if (j < nj) kept[(size_t)j * d + i] = S[a][b];
+        }
+      }
+    const float keep = keep_next;
+    if (c + 1 < chunks) {
+      load(c + 1);
+      keep_next = full[(size_t)(first + c + 1) * H + h];
+      asm volatile("cp.async.wait_group 1;" ::: "memory");
+    } else {
+      asm volatile("cp.async.wait_group 0;" ::: "memory");
+    }
+    __syncthreads();
+    const float* ws = dc_smem + (c & 1) * STAGE;
+    const float* u0 = ws + CHUNK * P + d * AP;
+    float acc[2][4] = {};
+    chunk_mm<8, 2, 4>(acc, ss, P, DC_BLOCK, ws, P, CHUNK, d);
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int j = ty + 8 * a, t = tx + 16 * b;
+        const float u = u0[j * CHUNK + t] - acc[a][b];
+        us[j * AP + t] = u;
+        if (j < nj) base[(size_t)(j0 + j) * CHUNK + t] = u;
+      }
+    __syncthreads();
+#pragma unroll
+    for (int a = 0; a < 2; ++a)
+#pragma unroll
+      for (int b = 0; b < RN; ++b) S[a][b] *= keep;
+    chunk_mm<8, 2, RN>(S, us, AP, DC_BLOCK, ws + CHUNK * P, AP, d, CHUNK);
+    __syncthreads();                         // `ss`, `us` and this stage are free
+  }
+#pragma unroll
+  for (int a = 0; a < 2; ++a)
+#pragma unroll
+    for (int b = 0; b < RN; ++b) {
+      const int j = ty + 8 * a, i = tx + 16 * b;
+      if (j < nj && i < d) st[(size_t)j * d + i] = S[a][b];
+    }
+}
+
+template <int RN>      // ceil(e / 16)
+__global__ void __launch_bounds__(256)
+delta_chunk_out_kernel(const float* __restrict__ qkv, int C, const float* __restrict__ bg, const float* __restrict__ scratch,
+                       float* __restrict__ o, const int32_t* __restrict__ tile_tok0, const int32_t* __restrict__ tile_ntok, int H, int G, int d,
+                       int e) {
+  extern __shared__ __align__(16) float dc_smem[];
+  __shared__ double lg[CHUNK];
+  constexpr int AP = CHUNK + 4;
+  const int P = chunk_pitch(d);
+  float* qs = dc_smem;                       // [CHUNK][P]
+  float* ks = qs + CHUNK * P;                // [CHUNK][P]
+  float* ss = ks + CHUNK * P;                // S0 [e][P]
+  float* us = ss + e * P;                    // U [e][AP]
+  float* ms = us + e * AP;                   // the chunk's own weights [t][s]
+  const int tile = blockIdx.x, h = blockIdx.y, g = h / (H / G), tok0 = tile_tok0[tile], ntok = tile_ntok[tile];
+  const float* base = scratch + ((size_t)tile * H + h) * dc_floats(d, e);
+  const float* row = qkv + (size_t)tok0 * C + g * d;
+  chunk_rows(qs, P, row, C, CHUNK, ntok, d);
+  chunk_rows(ks, P, row + G * d, C, CHUNK, ntok, d);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  chunk_rows(ss, P, base + (size_t)CHUNK * e + (size_t)(2 * CHUNK) * d, d, e, e, d);
+  chunk_rows(us, AP, base, CHUNK, e, e, CHUNK);
+  asm volatile("cp.async.commit_group;" ::: "memory");
+  dc_logs(lg, bg, tok0, ntok, H, h);
+  asm volatile("cp.async.wait_group 1;" ::: "memory");
+  __syncthreads();
+  const int tx = chunk_tx(), ty = chunk_ty();
+  {
+    float acc[4][4] = {};
+    chunk_mm<16, 4, 4>(acc, qs, P, CHUNK, ks, P, CHUNK, d);
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+#pragma unroll
+      for (int b = 0; b < 4; ++b) {
+        const int t = ty + 16 * a, s = tx + 16 * b;
+        ms[t * AP + s] = s <= t ? expf((float)(lg[t] - lg[s])) * acc[a][b] : 0.f;
+      }
+  }
+  asm volatile("cp.async.wait_group 0;" ::: "memory");
+  __syncthreads();
+  float acc[4][RN] = {};
+  chunk_mm<16, 4, RN>(acc, qs, P, CHUNK, ss, P, e, d);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) {
+    const float w = expf((float)lg[ty + 16 * a]);
+#pragma unroll
+    for (int b = 0; b < RN; ++b) acc[a][b] *= w;
+  }
+  chunk_mm<16, 4, RN>(acc, ms, AP, CHUNK, us, AP, e, CHUNK);
+#pragma unroll
+  for (int a = 0; a < 4; ++a)
+#pragma unroll
+    for (int b = 0; b < RN; ++b) {
+      const int t = ty + 16 * a, j = tx + 16 * b;
+      if (t < ntok && j < e) o[(size_t)(tok0 + t) * H * e + (size_t)h * e + j] = acc[a][b];
+    }
+}
+
 }  // namespace edgelm
 
 using namespace edgelm;
@@ -222,5 +485,40 @@ extern "C" int edgelm_delta_scan(const float* qkv, int C, const float* bg, float
 #undef EL_DS
 #undef EL_DS2
   EL_LAUNCH_CHECK("delta_scan");
+  return 0;
+}
+
+// 1 if the chunked form takes heads of these sizes (whole pieces of 16 bytes, its tiles in shared memory).
+extern "C" int edgelm_delta_chunked_takes(int d, int e) { return d >= 4 && d <= 128 && e >= 4 && e <= 128 && d % 4 == 0 && e % 4 == 0 ? 1 : 0; }
+
+// Floats of scratch that the chunked form takes for `n_tiles` chunks.
+extern "C" long long edgelm_delta_chunked_scratch(int n_tiles, int H, int d, int e) { return (long long)n_tiles * H * ((long long)dc_floats(d, e) + 4); }
+
+// `edgelm_delta_scan` chunk by chunk (three launches): the step's tokens come as tiles of at most CHUNK consecutive tokens of one
+// sequence, in the order of the sequences, every sequence cut from its first row of the step.  scratch: `edgelm_delta_chunked_scratch` floats.
+extern "C" int edgelm_delta_chunked(const float* qkv, int C, const float* bg, float* state, float* o, const int32_t* seq_tok0,
+                                    const int32_t* seq_slot, int n_seqs, const int32_t* tile_tok0, const int32_t* tile_ntok, int n_tiles, int H,
+                                    int G, int d, int e, float* scratch, cudaStream_t stream) {
+  if (n_seqs == 0 || n_tiles == 0) return 0;
+  EL_REFUSE(n_seqs > 0 && n_tiles > 0 && H > 0 && H <= 65535 && G > 0 && H % G == 0 && C == 2 * G * d + H * e, "delta_chunked: sizes do not fit (heads %d over %d, channels %d)", H, G, C);
+  EL_REFUSE(edgelm_delta_chunked_takes(d, e), "delta_chunked: heads of %d x %d are not taken (use the scan)", d, e);
+  EL_REFUSE(scratch != nullptr && (uintptr_t)scratch % 16 == 0 && (uintptr_t)qkv % 16 == 0, "delta_chunked: rows and scratch must be 16-byte aligned");
+  const int P = chunk_pitch(d), AP = CHUNK + 4;
+  float* full = scratch + (size_t)n_tiles * H * dc_floats(d, e);
+  const size_t smem1 = (size_t)(CHUNK * P + CHUNK * AP) * 4;
+  const size_t smem2 = (size_t)(2 * (CHUNK * P + d * AP + DC_BLOCK * CHUNK) + DC_BLOCK * P + DC_BLOCK * AP) * 4;
+  const size_t smem3 = (size_t)(2 * CHUNK * P + e * P + e * AP + CHUNK * AP) * 4;
+  auto k2 = d <= 64 ? delta_chunk_states_kernel<4> : delta_chunk_states_kernel<8>;
+  auto k3 = e <= 64 ? delta_chunk_out_kernel<4> : delta_chunk_out_kernel<8>;
+  cudaError_t err = cudaFuncSetAttribute(delta_chunk_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
+  if (err == cudaSuccess) err = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
+  EL_REFUSE(err == cudaSuccess, "delta_chunked: shared memory refused: %s", cudaGetErrorString(err));
+  delta_chunk_solve_kernel<<<dim3(n_tiles, H), 256, smem1, stream>>>(qkv, C, bg, scratch, full, tile_tok0, tile_ntok, H, G, d, e);
+  EL_LAUNCH_CHECK("delta_chunk_solve");
+  k2<<<dim3(n_seqs * H, (e + DC_BLOCK - 1) / DC_BLOCK), DC_STATE_THREADS, smem2, stream>>>(scratch, full, state, seq_tok0, seq_slot, H, d, e);
+  EL_LAUNCH_CHECK("delta_chunk_states");
+  k3<<<dim3(n_tiles, H), 256, smem3, stream>>>(qkv, C, bg, scratch, o, tile_tok0, tile_ntok, H, G, d, e);
+  EL_LAUNCH_CHECK("delta_chunk_out");
   return 0;
 }

@@ -997,6 +997,36 @@ def delta_scan(qkv, bg, state, o, seq_tok0, seq_slot, n_seqs, heads, kv_heads, d
                                    kv_heads, d, e, _stream()))
 
 
+def delta_chunked_takes(d, e):
+    """Whether the chunked form of `delta_scan` takes heads of d x e."""
+    return 4 <= d <= 128 and 4 <= e <= 128 and d % 4 == 0 and e % 4 == 0     # (the rule of `edgelm_delta_chunked_takes`)
+
+
+def delta_chunked_scratch_floats(n_tiles, heads, d, e):
+    return int(n_tiles) * heads * (2 * DELTA_CHUNK * d + DELTA_CHUNK * e + d * e + 4)     # (`edgelm_delta_chunked_scratch`)
+
+
+DELTA_CHUNK = 64     # tokens of a chunk (CHUNK in chunk_mm.cuh)
+
+
+def delta_chunked(qkv, bg, state, o, seq_tok0, seq_slot, n_seqs, tile_tok0, tile_ntok, n_tiles, heads, kv_heads, d, e, scratch=None):
+    """`delta_scan` for prompt steps, chunk by chunk (three launches): the step's tokens come as tiles of at most DELTA_CHUNK
+    consecutive tokens of one sequence, in the sequences' order, each sequence cut from its first row of the step.  `scratch`:
+    float32 room for `delta_chunked_scratch_floats` values."""
+    for t, n in ((qkv, "qkv"), (bg, "bg"), (state, "state"), (o, "o")):
+        _f32(t, n)
+    for t, n in ((seq_tok0, "seq_tok0"), (seq_slot, "seq_slot"), (tile_tok0, "tile_tok0"), (tile_ntok, "tile_ntok")):
+        _i32(t, n)
+    T = qkv.shape[0]
+    _need(tuple(state.shape[1:]) == (heads, e, d) and o.shape == (T, heads * e), "delta_chunked: state or output shape")
+    need = delta_chunked_scratch_floats(n_tiles, heads, d, e)
+    if scratch is None:
+        scratch = torch.empty(need, dtype=torch.float32, device=qkv.device)
+    _need(scratch.dtype == torch.float32 and scratch.is_contiguous() and scratch.numel() >= need, "delta_chunked: scratch too small")
+    _check(lib().edgelm_delta_chunked(_p(qkv), qkv.shape[1], _p(bg), _p(state), _p(o), _p(seq_tok0), _p(seq_slot), int(n_seqs), _p(tile_tok0),
+                                      _p(tile_ntok), int(n_tiles), heads, kv_heads, d, e, _p(scratch), _stream()), launches=3)
+
+
 # ----------------------------------------------------------------------------- mixture of experts
 def moe_tile_rows(tensor_cores=False):
     """Rows of a tile of the grouped products: every expert's rows start at a multiple of it (the CUDA-core kernels'

@@ -103,6 +103,50 @@ def test_delta_rule_over_steps(H, G, d, e, taps):
     assert torch.isnan(state[1]).all()
 
 
+@pytest.mark.parametrize("H,G,d,e", [(3, 1, 64, 64), (2, 2, 32, 20), (2, 1, 128, 96), (1, 1, 4, 128), (2, 1, 60, 64)])
+def test_delta_rule_chunk_by_chunk(H, G, d, e):
+    """Edges of chunks and of the blocks' channels, sequences without a token, states from earlier pieces; decays from nearly 1 to zero,
+    keys that repeat (the correction then undoes what an earlier token wrote).  Off float64 by at most
+    2^-24 of the largest value for each step of a chunk's substitution and each term of the two products behind it (64 + 2 * 64)."""
+    g = np.random.default_rng(d + e)
+    total, cuts = [200, 64, 65, 131], [[129, 71], [64], [1, 64], [0, 128, 3]]
+    unit = lambda x: x / np.sqrt((x * x).sum(-1, keepdims=True))
+    q, k = ([unit(g.normal(size=(n, G, d))) for n in total] for _ in range(2))
+    for x in k:
+        x[1::5] = x[0::5][:len(x[1::5])]
+    v, beta = [g.normal(size=(n, H, e)) for n in total], [g.uniform(0, 1, (n, H)) for n in total]
+    decay = [np.exp(-np.exp(g.uniform(-7, 1.5, (n, H)))) for n in total]
+    decay[0][77] = 0.0
+    held = lambda xs: [np.float32(x).astype(np.float64) for x in xs]
+    q, k, v, beta, decay = (held(x) for x in (q, k, v, beta, decay))
+    rep = lambda x: np.repeat(x, H // G, axis=1)
+    want = [plain.delta_recurrence(rep(a), rep(b), c, x, y) for a, b, c, x, y in zip(q, k, v, beta, decay)]
+    slots = [3, 0, 5, 2]
+    states = [torch.zeros(6, H, e, d, device=DEV) for _ in range(2)]
+    for s in states:
+        s[1] = s[4] = 7.0                       # (slots of nobody)
+    worst = [0.0, 0.0]
+    for step in steps_of(total, cuts):
+        n_new = [n for _, n in step]
+        tok0, _ = packed(n_new)
+        rows = lambda xs: np.concatenate([x[a:a + n].reshape(n, int(np.prod(x.shape[1:]))) for x, (a, n) in zip(xs, step)])
+        qkv, bg = f32(np.concatenate([rows(q), rows(k), rows(v)], 1)), f32(np.concatenate([rows(beta), rows(decay)], 1))
+        _, ttok0, tntok, _, count = make_tiles(n_new, [0] * 4, ops.DELTA_CHUNK)
+        ref = rows(want)
+        for i, s in enumerate(states):
+            o = torch.full((sum(n_new), H * e), float("nan"), device=DEV)
+            if i == 0:
+                ops.delta_chunked(qkv, bg, s, o, tok0, i32(slots), 4, ttok0, tntok, count, H, G, d, e)
+            else:
+                ops.delta_scan(qkv, bg, s, o, tok0, i32(slots), 4, H, G, d, e)
+            worst[i] = max(worst[i], np.abs(o.cpu().numpy() - ref).max())
+    scale = max(np.abs(w).max() for w in want)
+    assert worst[0] < 192 * 2.0 ** -24 * scale, worst
+    assert float((states[0] - states[1]).abs().max()) < 192 * 2.0 ** -24 * max(1.0, float(states[1][slots].abs().max()))
+    assert bool((states[0][1] == 7).all() and (states[0][4] == 7).all())
+
+
+
 # ----------------------------------------------------------------------------- attention with a key range and a sink
 class PagedKV:
     """Keys and values of a few sequences in pages handed out in a scrambled order, the rest poisoned."""
