@@ -16,14 +16,14 @@ __device__ __forceinline__ int chunk_tx() { return threadIdx.x >> 1 & 15; }
 __device__ __forceinline__ int chunk_ty() { return (threadIdx.x & 1) + (threadIdx.x >> 5) * 2; }
 
 // acc[a][b] += sum over k < K of A[m][k] B[n][k]; K a multiple of 4; rows from M and columns from N on: the last one's again.
-// Packed pairs of multiply-adds; the products are summed in two runs (four for small tiles) of their own before they join `acc`.
+// Packed pairs of multiply-adds: even and odd k in sums of their own before they join `acc`.  (Four runs instead of two took the
+// registers of a second block an SM, whose loads hide the first one's: the state-space outputs of state_chunks.cu 285 us against 126.)
 template <int NY, int RM, int RN>
 __device__ __forceinline__ void chunk_mm(float (&acc)[RM][RN], const float* A, int pa, int M, const float* B, int pb, int N, int K) {
-  constexpr int RUNS = RM * RN <= 16 ? 2 : 1;
   const int tx = chunk_tx(), ty = chunk_ty();
   const float* ar[RM];
   const float* br[RN];
-  unsigned long long sum[RUNS][RM][RN] = {};
+  unsigned long long sum[RM][RN] = {};
 #pragma unroll
   for (int a = 0; a < RM; ++a) ar[a] = A + min(ty + NY * a, M - 1) * pa;
 #pragma unroll
@@ -38,20 +38,15 @@ __device__ __forceinline__ void chunk_mm(float (&acc)[RM][RN], const float* A, i
       const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(br[b] + k);
 #pragma unroll
       for (int a = 0; a < RM; ++a) {
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[0][a][b]) : "l"(av[a].x), "l"(bv.x));
-        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[RUNS - 1][a][b]) : "l"(av[a].y), "l"(bv.y));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[a][b]) : "l"(av[a].x), "l"(bv.x));
+        asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[a][b]) : "l"(av[a].y), "l"(bv.y));
       }
     }
   }
 #pragma unroll
   for (int a = 0; a < RM; ++a)
 #pragma unroll
-    for (int b = 0; b < RN; ++b) {
-      float v = 0.f;
-#pragma unroll
-      for (int r = 0; r < RUNS; ++r) v += __uint_as_float((uint32_t)sum[r][a][b]) + __uint_as_float((uint32_t)(sum[r][a][b] >> 32));
-      acc[a][b] += v;
-    }
+    for (int b = 0; b < RN; ++b) acc[a][b] += __uint_as_float((uint32_t)sum[a][b]) + __uint_as_float((uint32_t)(sum[a][b] >> 32));
 }
 
 __device__ __forceinline__ void chunk_cp16(float* dst, const float* src, bool there) {

@@ -190,7 +190,7 @@ delta_scan_kernel(const float* __restrict__ qkv, int C, const float* __restrict_
 // Logarithms and their sums are kept in double precision (a decay that is zero in float32 counts as exp(-200)), everything else is float32.
 // One (chunk, head) of the scratch: U0, later U, [e][64]; W [64][d]; the keys times exp(L_n - L_s) [d][64]; S0 [e][d].  Then exp(L_n) of each.
 // Bound by the substitution and the products out of shared memory.  Nine heads of 64, prompts of 333 to
-// 1,700 tokens (4,065 in all): the walk 548 us, this 197 (48 + 95 + 53).
+// 1,700 tokens (4,065 in all): the walk 548 us, this 195 (49 + 106 + 40).
 constexpr int DC_BLOCK = 16;       // value channels a block of `delta_chunk_states` owns
 constexpr int DC_STATE_THREADS = 128;
 
@@ -379,7 +379,7 @@ delta_chunk_states_kernel(float* __restrict__ scratch, const float* __restrict__
 }
 
 template <int RN>      // ceil(e / 16)
-__global__ void __launch_bounds__(256)
+__global__ void __launch_bounds__(256, RN <= 4 ? 2 : 1)
 delta_chunk_out_kernel(const float* __restrict__ qkv, int C, const float* __restrict__ bg, const float* __restrict__ scratch,
                        float* __restrict__ o, const int32_t* __restrict__ tile_tok0, const int32_t* __restrict__ tile_ntok, int H, int G, int d,
                        int e) {

@@ -549,6 +549,65 @@ def wkv_scan(r, k, v, w, bonus, state, o, seq_tok0, seq_slot, n_seqs, heads, hea
                                  heads, head_dim, r.shape[0], _stream()))
 
 
+STATE_CHUNK = 64     # tokens of a chunk of the chunked recurrences (CHUNK in chunk_mm.cuh)
+
+
+def ssm_chunked_takes(n_state, head_dim):
+    """Whether the chunked form of `ssm_scan` takes a state of n_state x head_dim a head."""
+    return 4 <= n_state <= 128 and n_state % 4 == 0 and 4 <= head_dim <= 64 and head_dim % 4 == 0     # (the rule of `edgelm_ssm_chunked_takes`)
+
+
+def ssm_chunked_scratch_floats(n_tiles, heads, groups, n_state, head_dim):
+    return int(n_tiles) * (heads * head_dim * n_state + groups * STATE_CHUNK * (STATE_CHUNK + n_state) + (heads + 3) // 4 * 4)     # (`edgelm_ssm_chunked_scratch`)
+
+
+def _chunk_tiles(seq_tok0, seq_slot, tile_tok0, tile_ntok, scratch, need, like, what):
+    for t, n in ((seq_tok0, "seq_tok0"), (seq_slot, "seq_slot"), (tile_tok0, "tile_tok0"), (tile_ntok, "tile_ntok")):
+        _i32(t, n)
+    if scratch is None:
+        scratch = torch.empty(need, dtype=torch.float32, device=like.device)
+    _need(scratch.dtype == torch.float32 and scratch.is_contiguous() and scratch.numel() >= need, f"{what}: scratch too small")
+    return scratch
+
+
+def ssm_chunked(xbc, u, dt_off, dt_bias, a_log, d, state, y, seq_tok0, seq_slot, n_seqs, tile_tok0, tile_ntok, n_tiles, heads, groups, n_state,
+                head_dim, scratch=None):
+    """`ssm_scan` for prompt steps, chunk by chunk (four launches): the step's tokens come as tiles of at most STATE_CHUNK consecutive
+    tokens of one sequence, in the sequences' order, each sequence cut from its first row of the step.  The tail of the convolution
+    ahead is not touched.  `scratch`: float32 room for `ssm_chunked_scratch_floats` values."""
+    for t, n in ((xbc, "xbc"), (dt_bias, "dt_bias"), (a_log, "A_log"), (d, "D"), (state, "state"), (y, "y")):
+        _f32(t, n)
+    inner = heads * head_dim
+    _need(u.dtype == torch.float32 and u.is_cuda and u.stride(1) == 1 and dt_off + heads <= u.shape[1], "ssm_chunked: u must be float32 rows")
+    _need(xbc.shape[1] == inner + 2 * groups * n_state and y.shape == (xbc.shape[0], inner) and u.shape[0] == xbc.shape[0], "ssm_chunked: shapes")
+    _need(tuple(state.shape[1:]) == (heads, head_dim, n_state) and dt_bias.numel() == heads and a_log.numel() == heads and d.numel() == heads, "ssm_chunked: state or per-head vectors")
+    scratch = _chunk_tiles(seq_tok0, seq_slot, tile_tok0, tile_ntok, scratch, ssm_chunked_scratch_floats(n_tiles, heads, groups, n_state, head_dim), xbc, "ssm_chunked")
+    _check(lib().edgelm_ssm_chunked(_p(xbc), xbc.shape[1], inner, groups, n_state, _p(u), u.stride(0), int(dt_off), _p(dt_bias), _p(a_log), _p(d),
+                                    _p(state), _p(y), _p(seq_tok0), _p(seq_slot), int(n_seqs), _p(tile_tok0), _p(tile_ntok), int(n_tiles), heads,
+                                    head_dim, _p(scratch), _stream()), launches=4)
+
+
+def wkv_chunked_takes(head_dim):
+    """Whether the chunked form of `wkv_scan` takes heads of this size."""
+    return 4 <= head_dim <= 64 and head_dim % 4 == 0     # (the rule of `edgelm_wkv_chunked_takes`)
+
+
+def wkv_chunked_scratch_floats(n_tiles, heads, head_dim):
+    return int(n_tiles) * heads * head_dim * (head_dim + STATE_CHUNK + 1)     # (`edgelm_wkv_chunked_scratch`)
+
+
+def wkv_chunked(r, k, v, w, bonus, state, o, seq_tok0, seq_slot, n_seqs, tile_tok0, tile_ntok, n_tiles, heads, head_dim, scratch=None):
+    """`wkv_scan` for prompt steps, chunk by chunk (three launches), over tiles as in `ssm_chunked`; `scratch`: float32 room for
+    `wkv_chunked_scratch_floats` values."""
+    for t, n in ((r, "r"), (k, "k"), (v, "v"), (w, "w"), (bonus, "bonus"), (state, "state"), (o, "o")):
+        _f32(t, n)
+    _need(r.shape == k.shape == v.shape == w.shape == o.shape and r.shape[1] == heads * head_dim, "wkv_chunked: shapes")
+    _need(tuple(state.shape[1:]) == (heads, head_dim, head_dim) and bonus.numel() == heads * head_dim, "wkv_chunked: state or bonus")
+    scratch = _chunk_tiles(seq_tok0, seq_slot, tile_tok0, tile_ntok, scratch, wkv_chunked_scratch_floats(n_tiles, heads, head_dim), r, "wkv_chunked")
+    _check(lib().edgelm_wkv_chunked(_p(r), _p(k), _p(v), _p(w), _p(bonus), _p(state), _p(o), _p(seq_tok0), _p(seq_slot), int(n_seqs), _p(tile_tok0),
+                                    _p(tile_ntok), int(n_tiles), heads, head_dim, _p(scratch), _stream()), launches=3)
+
+
 def lowrank_decay(a, w2, w0, out):
     """out = exp(-exp(w0 + tanh(a) @ w2.T)) in float32; a [T, L] float32, w2 [C, L] float32 or bfloat16."""
     _f32(a, "a"); _f32(w0, "w0"); _f32(out, "out")

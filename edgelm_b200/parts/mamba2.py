@@ -79,9 +79,21 @@ class Mamba2(Part):
     def cache_need(self):
         return NeedSet.of(conv=StateNeed((self.taps - 1, self.channels)), ssm=StateNeed((self.heads, self.head_dim, self.n_state)))
 
+    # Steps of at least so many tokens a sequence on average take the chunked form.
+    CHUNKED_FROM = 16
+
+    def _chunked(self):
+        """Whether prompt steps may take the chunked form of the recurrence (float32 either way, and as close to float64 as the walk)."""
+        return ops.ssm_chunked_takes(self.n_state, self.head_dim)
+
+    def tile_sizes(self):
+        return (ops.STATE_CHUNK,) if self._chunked() else ()
+
     def workspace_bytes(self, n_tokens, n_seqs):
         f32 = torch.float32
-        return (nbytes((n_tokens, self.d_in), f32) + nbytes((n_tokens, self.channels), f32) + nbytes((n_tokens, self.inner), f32) +
+        chunks = n_tokens // ops.STATE_CHUNK + min(n_seqs, n_tokens // self.CHUNKED_FROM)
+        room = nbytes((ops.ssm_chunked_scratch_floats(chunks, self.heads, self.groups, self.n_state, self.head_dim),), f32) if self._chunked() else 0
+        return room + (nbytes((n_tokens, self.d_in), f32) + nbytes((n_tokens, self.channels), f32) + nbytes((n_tokens, self.inner), f32) +
                 nbytes((2 * n_tokens * self.heads,), f32) +
                 nbytes((n_tokens, self.inner), self.dtype) + nbytes((n_tokens, self.hidden), self.dtype))
 
@@ -92,15 +104,25 @@ class Mamba2(Part):
         with ctx.prof("ssm_in_proj"):
             linear.matmul(ctx, h, self.w_in, u, prefetch=(self.w_o,))
         xbc = ws.alloc((T, self.channels), f32)
+        chunked = not ctx.all_single and T >= self.CHUNKED_FROM * ctx.n_seqs and self._chunked()
         with ctx.prof("ssm_conv"):
             ops.conv_silu(u, self.inner, self.conv_w, self.conv_b, cache["conv"].state, xbc, ctx.tok_seq, ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs,
-                          update_state=False)     # (the scan kernel moves the tail on)
+                          update_state=chunked)     # (the scan kernel moves the tail on)
         y = ws.alloc((T, self.inner), f32)
-        steps = ws.alloc((2 * T * self.heads,), f32)
-        with ctx.prof("ssm_scan"):
-            ops.ssm_scan(xbc, u, 2 * self.inner + 2 * self.groups * self.n_state, self.dt_bias, self.a_log, self.d, cache["ssm"].state, y,
-                         ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs, self.heads, self.groups, self.n_state, self.head_dim,
-                         conv_state=cache["conv"].state, conv_off=self.inner, scratch=steps)
+        dt_off = 2 * self.inner + 2 * self.groups * self.n_state
+        if chunked:
+            tiles = ctx.tiles(ops.STATE_CHUNK)
+            with ws.frame():
+                scratch = ws.alloc((ops.ssm_chunked_scratch_floats(tiles.count, self.heads, self.groups, self.n_state, self.head_dim),), f32)
+                with ctx.prof("ssm_chunks"):
+                    ops.ssm_chunked(xbc, u, dt_off, self.dt_bias, self.a_log, self.d, cache["ssm"].state, y, ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs,
+                                    tiles.tok0, tiles.ntok, tiles.count, self.heads, self.groups, self.n_state, self.head_dim, scratch=scratch)
+        else:
+            steps = ws.alloc((2 * T * self.heads,), f32)
+            with ctx.prof("ssm_scan"):
+                ops.ssm_scan(xbc, u, dt_off, self.dt_bias, self.a_log, self.d, cache["ssm"].state, y, ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs,
+                             self.heads, self.groups, self.n_state, self.head_dim,
+                             conv_state=cache["conv"].state, conv_off=self.inner, scratch=steps)
         yn = ws.alloc((T, self.inner), self.dtype)
         with ctx.prof("ssm_gate_norm"):
             ops.gated_group_norm(y, u[:, :self.inner], self.norm_w, yn, self.norm_groups, self.eps, gate_first=True)

@@ -71,9 +71,21 @@ class DecayTimeMix(Part):
     def cache_need(self):
         return NeedSet.of(last=StateNeed((self.hidden,)), wkv=StateNeed((self.heads, self.head_dim, self.head_dim)))
 
+    # Steps of at least so many tokens a sequence on average take the chunked form.
+    CHUNKED_FROM = 16
+
+    def _chunked(self):
+        """Whether prompt steps may take the chunked form of the recurrence (float32 either way, and as close to float64 as the walk)."""
+        return ops.wkv_chunked_takes(self.head_dim)
+
+    def tile_sizes(self):
+        return (ops.STATE_CHUNK,) if self._chunked() else ()
+
     def workspace_bytes(self, n_tokens, n_seqs):
         f32 = torch.float32
-        return (nbytes((5, n_tokens, self.hidden), self.dtype) + 6 * nbytes((n_tokens, self.inner), f32) + nbytes((n_tokens, self.rank), f32) +
+        chunks = n_tokens // ops.STATE_CHUNK + min(n_seqs, n_tokens // self.CHUNKED_FROM)
+        room = nbytes((ops.wkv_chunked_scratch_floats(chunks, self.heads, self.head_dim),), f32) if self._chunked() else 0
+        return room + (nbytes((5, n_tokens, self.hidden), self.dtype) + 6 * nbytes((n_tokens, self.inner), f32) + nbytes((n_tokens, self.rank), f32) +
                 nbytes((n_tokens, self.inner), self.dtype) + nbytes((n_tokens, self.hidden), self.dtype))
 
     def forward(self, ctx, h, x, cache, accumulate=True):
@@ -94,9 +106,17 @@ class DecayTimeMix(Part):
         with ctx.prof("timemix_decay"):
             ops.lowrank_decay(low, self.w["w2"], self.w0, decay)
         o = ws.alloc((T, self.inner), f32)
-        with ctx.prof("timemix_scan"):
-            ops.wkv_scan(proj["r"], proj["k"], proj["v"], decay, self.bonus, cache["wkv"].state, o, ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs,
-                         self.heads, self.head_dim)
+        if not ctx.all_single and T >= self.CHUNKED_FROM * ctx.n_seqs and self._chunked():
+            tiles = ctx.tiles(ops.STATE_CHUNK)
+            with ws.frame():
+                scratch = ws.alloc((ops.wkv_chunked_scratch_floats(tiles.count, self.heads, self.head_dim),), f32)
+                with ctx.prof("timemix_chunks"):
+                    ops.wkv_chunked(proj["r"], proj["k"], proj["v"], decay, self.bonus, cache["wkv"].state, o, ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs,
+                                    tiles.tok0, tiles.ntok, tiles.count, self.heads, self.head_dim, scratch=scratch)
+        else:
+            with ctx.prof("timemix_scan"):
+                ops.wkv_scan(proj["r"], proj["k"], proj["v"], decay, self.bonus, cache["wkv"].state, o, ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs,
+                             self.heads, self.head_dim)
         on = ws.alloc((T, self.inner), self.dtype)
         with ctx.prof("timemix_gate_norm"):
             ops.gated_group_norm(o, proj["g"], self.norm_w, on, self.heads, self.eps, gate_first=False)

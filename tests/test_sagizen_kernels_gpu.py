@@ -153,6 +153,80 @@ def test_blend_convolution_and_norms(dtype):
     assert np.abs(dec.cpu().numpy() - ref).max() < 1e-5
 
 
+def chunk_steps(total, cuts):
+    """Per step the sequences' new tokens, `seq_tok0` and the tiles of STATE_CHUNK tokens (first row, tokens, count)."""
+    from edgelm_b200.engine.batch import make_tiles
+    for step in steps_of(total, cuts):
+        n_new = [n for _, n in step]
+        _, tok0, ntok, _ = make_tiles(n_new, [0] * len(n_new), ops.STATE_CHUNK)
+        yield step, packed(n_new)[0], (i32(tok0), i32(ntok), len(tok0))
+
+
+def rows_of(xs, step):
+    return np.concatenate([x[a:a + n].reshape(n, int(np.prod(x.shape[1:]))) for x, (a, n) in zip(xs, step)])
+
+
+CHUNK_TOTAL, CHUNK_CUTS = [200, 64, 65, 131], [[129, 71], [64], [1, 64], [0, 128, 3]]
+
+
+@pytest.mark.parametrize("H,G,N,P", [(4, 1, 128, 64), (4, 2, 16, 20), (3, 3, 60, 64), (2, 1, 100, 4)])
+def test_state_space_chunk_by_chunk(H, G, N, P):
+    """Edges of chunks, sequences without a token in a step, states from earlier pieces, decays from nearly 1 to zero; 2^-24 of the largest
+    value for each term of the three sums behind an output (64 tokens, N state rows, 64 again), and twice that in the state."""
+    g = np.random.default_rng(N + P)
+    total = CHUNK_TOTAL
+    x, B, C = [g.normal(size=(n, H, P)) for n in total], [g.normal(size=(n, G, N)) for n in total], [g.normal(size=(n, G, N)) / np.sqrt(N) for n in total]
+    raw = [g.normal(-3, 2, size=(n, H)) for n in total]
+    raw[0][77] = 200.0
+    bias, A_log, D = g.normal(size=H), g.uniform(-2, 2, H), g.normal(size=H)
+    want = [plain.ssm_recurrence(a, b, c, plain.softplus(r + bias), A_log, D, G) for a, b, c, r in zip(x, B, C, raw)]
+    slots, states = [3, 0, 5, 2], [torch.zeros(6, H, P, N, device=DEV) for _ in range(2)]
+    for s in states:
+        s[1] = s[4] = 7.0                       # (slots of nobody)
+    worst, scale = [0.0, 0.0], max(np.abs(w).max() for w in want)
+    for step, tok0, tiles in chunk_steps(total, CHUNK_CUTS):
+        xbc, u = f32(np.concatenate([rows_of(x, step), rows_of(B, step), rows_of(C, step)], 1)), f32(np.pad(rows_of(raw, step), ((0, 0), (3, 2))))
+        for i, s in enumerate(states):
+            y = torch.full((len(xbc), H * P), float("nan"), device=DEV)
+            args = (xbc, u, 3, f32(bias), f32(A_log), f32(D), s, y, tok0, i32(slots), 4)
+            if i == 0:
+                ops.ssm_chunked(*args, *tiles, H, G, N, P)
+            else:
+                ops.ssm_scan(*args, H, G, N, P)
+            worst[i] = max(worst[i], np.abs(y.cpu().numpy() - rows_of(want, step)).max())
+    assert worst[0] < (128 + N) * 2.0 ** -24 * scale, worst
+    assert float((states[0] - states[1]).abs().max()) < 2 * (128 + N) * 2.0 ** -24 * max(1.0, float(states[1][slots].abs().max()))
+    assert bool((states[0][1] == 7).all() and (states[0][4] == 7).all())
+
+
+@pytest.mark.parametrize("H,K", [(3, 64), (2, 20), (1, 4), (2, 36)])
+def test_time_mix_chunk_by_chunk(H, K):
+    """As above for a decay per key channel, down to zero: 64 terms of the walk, K of the product, in each output."""
+    g = np.random.default_rng(K)
+    total = CHUNK_TOTAL
+    r, k, v = ([g.normal(size=(n, H, K)) for n in total] for _ in range(3))
+    w = [np.float32(np.exp(-np.exp(g.uniform(-8, 2, size=(n, H, K))))).astype(np.float64) for n in total]
+    w[0][77] = 0.0
+    bonus = g.normal(size=(H, K))
+    want = [plain.wkv_recurrence(a, b, c, d, bonus) for a, b, c, d in zip(r, k, v, w)]
+    slots, states = [3, 0, 5, 2], [torch.zeros(6, H, K, K, device=DEV) for _ in range(2)]
+    for s in states:
+        s[1] = s[4] = 7.0                       # (slots of nobody)
+    worst, scale = [0.0, 0.0], max(np.abs(x).max() for x in want)
+    for step, tok0, tiles in chunk_steps(total, CHUNK_CUTS):
+        rows = [f32(rows_of(x, step)) for x in (r, k, v, w)]
+        for i, s in enumerate(states):
+            o = torch.full_like(rows[0], float("nan"))
+            if i == 0:
+                ops.wkv_chunked(*rows, f32(bonus), s, o, tok0, i32(slots), 4, *tiles, H, K)
+            else:
+                ops.wkv_scan(*rows, f32(bonus), s, o, tok0, i32(slots), 4, H, K)
+            worst[i] = max(worst[i], np.abs(o.cpu().numpy() - rows_of(want, step)).max())
+    assert worst[0] < (64 + K) * 2.0 ** -24 * scale, worst
+    assert float((states[0] - states[1]).abs().max()) < (64 + K) * 2.0 ** -24 * max(1.0, float(states[1][slots].abs().max()))
+    assert bool((states[0][1] == 7).all() and (states[0][4] == 7).all())
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("T,C,L", [(1, 130, 5), (37, 2048, 64), (333, 1000, 24), (160, 2048, 513), (2500, 128, 7)])
 def test_lowrank_decay_tiles(T, C, L, dtype):
