@@ -105,10 +105,12 @@ gemm_tile_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, co
 // cp.async, S_STAGES stages of 16 k a group, a row's four pieces of 16 bytes exchanged by
 // the row's number so that eight neighbouring rows' reads lie in different banks.  After S_FLUSH stages the pairs join running sums
 // that lie in shared memory (a thread's own 64): the rounding error of a long row of products grows with the number of runs and the
-// run's length, not with their product.  The sums of groups and blocks are added in the order of K.  Measured beside the any-size
-// kernel: 1,143 rows, N 576, K 1536 176 -> 77 us; 2,048 rows, N 6144, K 2048 2,231 -> 1,259 us (41 TFLOP/s; the multiply-adds' pipe is
-// 55 % busy, what is left is the two warps a scheduler that 64 pairs of sums allow); 24 rows, N 960, K 2560 169 -> 10 us.
-constexpr int SK = 16, S_STAGES = 3, S_FLUSH = 8;
+// run's length, not with their product.  (Two stages, runs of 16 products a pair: 1.13e-7 of the result at K 576, 1.82e-7 at K 2560, the
+// any-size kernel's 1.34e-7 and 2.41e-7; runs twice as long are 7 % faster and less exact than it at K under 300.)  The sums of groups and
+// blocks are added in the order of K.  Measured beside the any-size kernel: 2,000 rows, N 1000, K 2560 680 -> 326 us; 300 rows, N 576,
+// K 2560 173 -> 47 us; 24 rows, N 960, K 2560 169 -> 10 us.  Bound by the issue of the multiply-adds (their pipe is about 55 % busy: 64
+// pairs of sums leave a scheduler two warps).
+constexpr int SK = 16, S_STAGES = 3, S_FLUSH = 2;
 
 __device__ __forceinline__ void cp_async16(unsigned dst, const float* src, bool there) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(there ? 16 : 0) : "memory");
@@ -409,7 +411,10 @@ int launch_gemm(const void* A, int lda, const void* W, const void* W2, void* out
   const bool few = force_kernel == 1 || (force_kernel == 0 && M <= 2 * GEMV_ROWS);
   if constexpr (sizeof(TA) == 4 && sizeof(TOut) == 4) {
     const bool pieces = K % 4 == 0 && lda % 4 == 0 && (uintptr_t)A % 16 == 0 && (uintptr_t)W % 16 == 0 && (W2 == nullptr || (uintptr_t)W2 % 16 == 0);
-    if (pieces && (force_kernel == 3 || (force_kernel == 0 && !few)))
+    // (short K in one wave of the any-size kernel's blocks: that kernel has done before the other's stages are on their way; 100 rows,
+    // N 200: 5.1 against 5.8 us at K 48, 6.3 against 5.9 at K 64, 8.4 against 5.3 at K 96)
+    const bool short_k = K < 96 && (long long)((M + BM - 1) / BM) * ((N + BN - 1) / BN) <= 148;
+    if (pieces && (force_kernel == 3 || (force_kernel == 0 && !few && !short_k)))
       return launch_sgemm_best<EPI>(a, lda, w, w2, o, ldo, residual, M, N, K, stream);
   }
   if (few) {
