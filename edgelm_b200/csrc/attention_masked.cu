@@ -20,7 +20,7 @@
 // space, weighted latents out of it); `masked_attn` (a block per token and head: steps of one token a sequence);
 // `masked_attn_tiled` (prompt steps: keys staged once for 32 rows, from the cache's pages or from the step's own rows);
 // `latent_expand_keys`; `add_row_bias`.
-#include "common.cuh"
+#include "rotate_rows.cuh"
 
 namespace edgelm {
 
@@ -957,17 +957,24 @@ extern "C" int edgelm_rotate_append(const float* qkv, const float* bias, float* 
   EL_REFUSE(n_tokens > 0 && H > 0 && G > 0 && H % G == 0, "rotate_append: %d query heads over %d key/value heads", H, G);
   EL_REFUSE(dk >= 1 && dk <= 2048 && dv >= 1, "rotate_append: head sizes %d / %d are not taken", dk, dv);
   EL_REFUSE(rot >= 0 && rot <= dk && rot % 2 == 0 && (rot == 0 || freq != nullptr), "rotate_append: %d rotated dimensions of %d", rot, dk);
+  EL_REFUSE(dtype == DT_F32 || dtype == DT_BF16, "rotate_append: unknown dtype code %d", dtype);
+  if (!move_tail && rotate_rows_takes(n_tokens, H, G, dk, dv, maps, rot, interleaved, conv_w ? taps : 0)) {      // (prompt steps, heads of whole runs of 32)
+    const RotateRows rows{qkv, ldq, bias, tok_pos, tok_seq, page_table, table_stride, n_pages, n_tokens, H, G, dv, maps, rot, interleaved, freq, err,
+                          q_norm, k_norm, eps, mult, 0, conv_w, conv_state, seq_tok0, seq_slot, taps};
+    if (dtype == DT_F32) launch_rotate_rows(rows, dk, q_out, (float*)kcache, (float*)vcache, stream);
+    else launch_rotate_rows(rows, dk, q_out, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, stream);
+    EL_LAUNCH_CHECK("rotate_rows");
+    return 0;
+  }
   const size_t smem = (size_t)MA_WARPS * dk * sizeof(float);
   const dim3 grid(n_tokens, (H + G + MA_WARPS - 1) / MA_WARPS), block(MA_WARPS * 32);
   const int bit = pdl_bit_for_tokens(n_tokens);
   if (dtype == DT_F32)
     launch_pdl(bit, rotate_append_kernel<float>, grid, block, smem, stream, qkv, bias, q_out, tok_pos, tok_seq, page_table, table_stride,
                n_pages, (float*)kcache, (float*)vcache, H, G, dk, dv, rot, interleaved, freq, err, maps, q_norm, k_norm, eps, ldq, conv, mult);
-  else if (dtype == DT_BF16)
+  else
     launch_pdl(bit, rotate_append_kernel<__nv_bfloat16>, grid, block, smem, stream, qkv, bias, q_out, tok_pos, tok_seq, page_table,
                table_stride, n_pages, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, H, G, dk, dv, rot, interleaved, freq, err, maps, q_norm, k_norm, eps, ldq, conv, mult);
-  else
-    EL_REFUSE(false, "rotate_append: unknown dtype code %d", dtype);
   EL_LAUNCH_CHECK("rotate_append");
   return 0;
 }

@@ -13,6 +13,7 @@
 // Three kernels: (1) bias, partial rotation, per-head unit RMS norm of q and k, append of k and v; (2) the pooled
 // rows of the blocks that the step's tokens complete; (3) attention.  Scores, softmax, norms, angles: float32.
 #include "mma_split.cuh"
+#include "rotate_rows.cuh"
 
 namespace edgelm {
 
@@ -93,43 +94,48 @@ qk_rope_norm_append_kernel(const float* __restrict__ qkv, const float* __restric
   }
 }
 
-// The pooled rows of the blocks that end at a token of this step.
+// The pooled rows of the blocks that end at a token of this step.  A block of threads looks at `run` consecutive tokens (POOL_RUN in prompt
+// steps), of which one in P ends a block.  (A block of threads a token: 2,048 tokens of 32 heads 86 us, most of it blocks that found nothing
+// to do; now 40.)
+constexpr int POOL_RUN = 16;
+
 template <typename T>
 __global__ void pool_blocks_kernel(const int32_t* __restrict__ tok_pos, const int32_t* __restrict__ tok_seq,
                                    const int32_t* __restrict__ page_table, int table_stride, int n_pages,
                                    const T* __restrict__ kcache, const T* __restrict__ vcache, float* __restrict__ pk,
-                                   float* __restrict__ pv, int G, int dk, int dv, int P, int R, int* __restrict__ err) {
+                                   float* __restrict__ pv, int G, int dk, int dv, int P, int R, int* __restrict__ err, int n_tokens, int run) {
   pdl_launch_dependents();
   pdl_wait();   // (launched as a programmatic dependent: nothing is read or written before the kernel ahead is done)
-  const int t = blockIdx.x;
-  const int pos = tok_pos[t];
-  if (pos < 0 || (pos + 1) % P != 0) return;
-  const int b = (pos + 1) / P - 1;
-  const int32_t* table = page_table + (size_t)tok_seq[t] * table_stride;
-  const int dst_page = table[pos / PAGE];
-  if (dst_page < 0 || dst_page >= n_pages) {
-    if (threadIdx.x == 0 && blockIdx.y == 0) atomicOr(err, ERR_PAGE_RANGE);
-    return;
-  }
-  const int rowi = b - (PAGE * (pos / PAGE)) / P;
-  const float invP = 1.0f / (float)P;
-  // a block per (token that ends a block, key/value head); a thread a channel of the key, then of the value: the rows
-  // of a block lie side by side in a page, so neighbouring threads read neighbouring addresses, eight rows in flight
-  const int g = blockIdx.y;
-  for (int i = threadIdx.x; i < dk + dv; i += blockDim.x) {
-    const bool is_k = i < dk;
-    const int d = is_k ? dk : dv, c = is_k ? i : i - dk;
-    const T* base = is_k ? kcache : vcache;
-    float acc = 0.f;
-#pragma unroll 8
-    for (int j = 0; j < P; ++j) {
-      const int p = b * P + j;
-      const int page = table[p / PAGE];
-      if (page < 0 || page >= n_pages) continue;   // (flagged by the append of that token's step)
-      acc += to_f32(base[(((size_t)page * G + g) * PAGE + p % PAGE) * d + c]);
+  for (int t = blockIdx.x * run; t < min(n_tokens, (int)(blockIdx.x + 1) * run); ++t) {
+    const int pos = tok_pos[t];
+    if (pos < 0 || (pos + 1) % P != 0) continue;
+    const int b = (pos + 1) / P - 1;
+    const int32_t* table = page_table + (size_t)tok_seq[t] * table_stride;
+    const int dst_page = table[pos / PAGE];
+    if (dst_page < 0 || dst_page >= n_pages) {
+      if (threadIdx.x == 0 && blockIdx.y == 0) atomicOr(err, ERR_PAGE_RANGE);
+      continue;
     }
-    float* dst = is_k ? pk : pv;
-    dst[(((size_t)dst_page * G + g) * R + rowi) * d + c] = acc * invP;
+    const int rowi = b - (PAGE * (pos / PAGE)) / P;
+    const float invP = 1.0f / (float)P;
+    // a block per (token that ends a block, key/value head); a thread a channel of the key, then of the value: the rows
+    // of a block lie side by side in a page, so neighbouring threads read neighbouring addresses, eight rows in flight
+    const int g = blockIdx.y;
+    for (int i = threadIdx.x; i < dk + dv; i += blockDim.x) {
+      const bool is_k = i < dk;
+      const int d = is_k ? dk : dv, c = is_k ? i : i - dk;
+      const T* base = is_k ? kcache : vcache;
+      float acc = 0.f;
+#pragma unroll 8
+      for (int j = 0; j < P; ++j) {
+        const int p = b * P + j;
+        const int page = table[p / PAGE];
+        if (page < 0 || page >= n_pages) continue;   // (flagged by the append of that token's step)
+        acc += to_f32(base[(((size_t)page * G + g) * PAGE + p % PAGE) * d + c]);
+      }
+      float* dst = is_k ? pk : pv;
+      dst[(((size_t)dst_page * G + g) * R + rowi) * d + c] = acc * invP;
+    }
   }
 }
 
@@ -707,15 +713,22 @@ extern "C" int edgelm_qk_rope_norm_append(const float* qkv, const float* bias, v
   EL_REFUSE(n_tokens > 0 && H > 0 && G > 0 && H % G == 0, "qk_rope_norm_append: %d query heads over %d key/value heads", H, G);
   EL_REFUSE(dk >= 1 && dk <= 256 && dv >= 1 && dv <= 256, "qk_rope_norm_append: head sizes %d / %d are not taken (1 to 256)", dk, dv);
   EL_REFUSE(rot >= 0 && rot <= dk && rot % 2 == 0, "qk_rope_norm_append: %d rotated dimensions of %d", rot, dk);
+  EL_REFUSE(dtype == DT_F32 || dtype == DT_BF16, "qk_rope_norm_append: unknown dtype code %d", dtype);
+  if (rotate_rows_takes(n_tokens, H, G, dk, dv, 1, rot, 0, 0)) {      // (prompt steps, heads of whole runs of 32)
+    const RotateRows rows{qkv, (H + G) * dk + G * dv, bias, tok_pos, tok_seq, page_table, table_stride, n_pages, n_tokens, H, G, dv, 1, rot, 0, freq, err,
+                          nullptr, nullptr, eps, 1.f, unit_norm, nullptr, nullptr, nullptr, nullptr, 0};
+    if (dtype == DT_F32) launch_rotate_rows(rows, dk, (float*)q_out, (float*)kcache, (float*)vcache, stream);
+    else launch_rotate_rows(rows, dk, (__nv_bfloat16*)q_out, (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, stream);
+    EL_LAUNCH_CHECK("rotate_rows");
+    return 0;
+  }
   const size_t smem = (size_t)PW_WARPS * dk * sizeof(float);
   if (dtype == DT_F32)
     launch_pdl(pdl_bit_for_tokens(n_tokens), qk_rope_norm_append_kernel<float>, dim3(n_tokens, (H + G + PW_WARPS - 1) / PW_WARPS), dim3(PW_WARPS * 32), (size_t)(smem), stream, qkv, bias, (float*)q_out, tok_pos, tok_seq, page_table, table_stride, n_pages,
                                                                               (float*)kcache, (float*)vcache, H, G, dk, dv, rot, freq, eps, unit_norm, err);
-  else if (dtype == DT_BF16)
+  else
     launch_pdl(pdl_bit_for_tokens(n_tokens), qk_rope_norm_append_kernel<__nv_bfloat16>, dim3(n_tokens, (H + G + PW_WARPS - 1) / PW_WARPS), dim3(PW_WARPS * 32), (size_t)(smem), stream, qkv, bias, (__nv_bfloat16*)q_out, tok_pos, tok_seq, page_table, table_stride, n_pages,
                                                                                       (__nv_bfloat16*)kcache, (__nv_bfloat16*)vcache, H, G, dk, dv, rot, freq, eps, unit_norm, err);
-  else
-    EL_REFUSE(false, "qk_rope_norm_append: unknown dtype code %d", dtype);
   EL_LAUNCH_CHECK("qk_rope_norm_append");
   return 0;
 }
@@ -725,10 +738,11 @@ extern "C" int edgelm_pool_blocks(const int32_t* tok_pos, const int32_t* tok_seq
                                   int n_tokens, int G, int dk, int dv, int P, int R, int* err, cudaStream_t stream) {
   if (n_tokens == 0) return 0;
   EL_REFUSE(n_tokens > 0 && G > 0 && dk > 0 && dv > 0 && P >= 1 && R == (PAGE + P - 1) / P, "pool_blocks: bad sizes (block %d, rows a page %d)", P, R);
+  const int run = n_tokens > 64 ? POOL_RUN : 1, runs = (n_tokens + run - 1) / run;
   if (dtype == DT_F32)
-    launch_pdl(pdl_bit_for_tokens(n_tokens), pool_blocks_kernel<float>, dim3(n_tokens, G), dim3(128), (size_t)(0), stream, tok_pos, tok_seq, page_table, table_stride, n_pages, (const float*)kcache, (const float*)vcache, pk, pv, G, dk, dv, P, R, err);
+    launch_pdl(pdl_bit_for_tokens(n_tokens), pool_blocks_kernel<float>, dim3(runs, G), dim3(128), (size_t)(0), stream, tok_pos, tok_seq, page_table, table_stride, n_pages, (const float*)kcache, (const float*)vcache, pk, pv, G, dk, dv, P, R, err, n_tokens, run);
   else if (dtype == DT_BF16)
-    launch_pdl(pdl_bit_for_tokens(n_tokens), pool_blocks_kernel<__nv_bfloat16>, dim3(n_tokens, G), dim3(128), (size_t)(0), stream, tok_pos, tok_seq, page_table, table_stride, n_pages, (const __nv_bfloat16*)kcache, (const __nv_bfloat16*)vcache, pk, pv, G, dk, dv, P, R, err);
+    launch_pdl(pdl_bit_for_tokens(n_tokens), pool_blocks_kernel<__nv_bfloat16>, dim3(runs, G), dim3(128), (size_t)(0), stream, tok_pos, tok_seq, page_table, table_stride, n_pages, (const __nv_bfloat16*)kcache, (const __nv_bfloat16*)vcache, pk, pv, G, dk, dv, P, R, err, n_tokens, run);
   else
     EL_REFUSE(false, "pool_blocks: unknown dtype code %d", dtype);
   EL_LAUNCH_CHECK("pool_blocks");

@@ -89,6 +89,62 @@ __global__ void conv_silu_kernel(const float* __restrict__ u, int ldu, int off, 
   }
 }
 
+// The filter over many tokens: a thread owns four neighbouring channels of CONV_RUN consecutive tokens, with the taps and the last inputs
+// in registers, so that an input is read once (16 bytes at a time, eight tokens' requests together) and not once a tap.  At most four taps;
+// rows and columns in whole pieces of 16 bytes.  Bound by memory: 2,048 tokens of 4,352 channels, four taps: a token a block 74 us, this
+// 26.
+constexpr int CONV_RUN = 16, CONV_THREADS = 128;
+
+__global__ void __launch_bounds__(CONV_THREADS)
+conv_rows_kernel(const float* __restrict__ u, int ldu, int off, const float* __restrict__ w, const float* __restrict__ b,
+                 const float* __restrict__ state, float* __restrict__ out, const int32_t* __restrict__ tok_seq,
+                 const int32_t* __restrict__ seq_tok0, const int32_t* __restrict__ seq_slot, int n_tokens, int C, int taps,
+                 const float* __restrict__ in_bias, int act) {
+  const int c = (blockIdx.y * CONV_THREADS + threadIdx.x) * 4;
+  if (c >= C) return;
+  float wt[4][4], past[3][4], bias[4], ib[4];      // taps aligned to the end: wt[3] multiplies the current token
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    bias[q] = b ? b[c + q] : 0.f;
+    ib[q] = in_bias ? in_bias[c + q] : 0.f;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) wt[j][q] = j >= 4 - taps ? w[(size_t)(c + q) * taps + j - (4 - taps)] : 0.f;
+  }
+  const int t_end = min(n_tokens, (int)(blockIdx.x + 1) * CONV_RUN);
+  for (int base = blockIdx.x * CONV_RUN; base < t_end; base += 8) {
+    float4 in[8];
+#pragma unroll
+    for (int x = 0; x < 8; ++x) in[x] = base + x < t_end ? *reinterpret_cast<const float4*>(u + (size_t)(base + x) * ldu + off + c) : make_float4(0.f, 0.f, 0.f, 0.f);
+#pragma unroll
+    for (int x = 0; x < 8; ++x) {
+      const int t = base + x;
+      if (t >= t_end) break;
+      const int s = tok_seq[t], k = t - seq_tok0[s];
+      if (t == blockIdx.x * CONV_RUN || k == 0) {      // the inputs before this token: rows of the step, or the sequence's tail
+        const float* tail = state + (size_t)seq_slot[s] * (taps - 1) * C;
+#pragma unroll
+        for (int j = 0; j < 3; ++j) {
+          const int r = k - 3 + j, row = taps - 1 + r;
+#pragma unroll
+          for (int q = 0; q < 4; ++q)
+            past[j][q] = r >= 0 ? u[(size_t)(t - k + r) * ldu + off + c + q] + ib[q] : (row >= 0 ? tail[(size_t)row * C + c + q] : 0.f);
+        }
+      }
+      const float now[4] = {in[x].x + ib[0], in[x].y + ib[1], in[x].z + ib[2], in[x].w + ib[3]};
+      float y[4];
+#pragma unroll
+      for (int q = 0; q < 4; ++q) {
+        const float acc = fmaf(wt[3][q], now[q], fmaf(wt[2][q], past[2][q], fmaf(wt[1][q], past[1][q], fmaf(wt[0][q], past[0][q], bias[q]))));
+        y[q] = act ? silu_exact(acc) : acc;
+        past[0][q] = past[1][q];
+        past[1][q] = past[2][q];
+        past[2][q] = now[q];
+      }
+      *reinterpret_cast<float4*>(out + (size_t)t * C + c) = make_float4(y[0], y[1], y[2], y[3]);
+    }
+  }
+}
+
 // The state after the step: the last taps - 1 inputs of each sequence.  A thread owns a channel and walks the
 // rows upwards, so that a row it still has to read (one further on) is never overwritten before.
 __global__ void conv_state_update_kernel(const float* __restrict__ u, int ldu, int off, float* __restrict__ state,
@@ -483,6 +539,81 @@ __global__ void gated_group_norm_kernel(const float* __restrict__ y, const float
   }
 }
 
+// The same for many rows, 16 bytes at a time: L = 4, 8, .. 256 neighbouring threads hold a group (up to 32: several groups a warp, their
+// sum by shuffles; 256: a block a group) with PIECES pieces each in registers between the sum and the scaling, so that values and gates
+// are read once.  Bound by memory: 2,048 rows of 4,096 in one group, and of 2,048 in 32: a block a group with single reads 108 us the two,
+// this 29.
+template <typename TOut, int L, int PIECES>
+__global__ void __launch_bounds__(256)
+gated_group_norm_vec_kernel(const float* __restrict__ y, const float* __restrict__ gate, int ldg, const float* __restrict__ w,
+                            TOut* __restrict__ out, long long n_groups, int inner, int groups, float eps, int gate_first, int gate_sigmoid) {
+  __shared__ float red[33];
+  const long long item = ((long long)blockIdx.x * 256 + threadIdx.x) / L;
+  const int l = threadIdx.x % L, gs = inner / groups;
+  const bool in = item < n_groups;
+  const long long t = in ? item / groups : 0;
+  const int g = in ? (int)(item - t * groups) : 0;
+  const float* yr = y + t * inner + (long long)g * gs;
+  const float* gr = gate + t * ldg + (long long)g * gs;
+  float v[PIECES][4], a[PIECES][4];
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int i = (l + p * L) * 4;
+    const bool there = in && i < gs;
+    *reinterpret_cast<float4*>(v[p]) = there ? *reinterpret_cast<const float4*>(yr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+    *reinterpret_cast<float4*>(a[p]) = there ? *reinterpret_cast<const float4*>(gr + i) : make_float4(0.f, 0.f, 0.f, 0.f);
+  }
+  float ss = 0.f;
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      a[p][q] = gate_sigmoid ? 1.0f / (1.0f + expf(-a[p][q])) : silu_exact(a[p][q]);
+      if (gate_first) v[p][q] *= a[p][q];
+      ss = fmaf(v[p][q], v[p][q], ss);
+    }
+  if (L <= 32) {
+#pragma unroll
+    for (int off = L / 2; off > 0; off >>= 1) ss += __shfl_xor_sync(0xffffffffu, ss, off);
+  } else {
+    ss = block_sum(ss, red);
+  }
+  const float inv = 1.0f / sqrtf(ss / (float)gs + eps);
+  if (!in) return;
+#pragma unroll
+  for (int p = 0; p < PIECES; ++p) {
+    const int i = (l + p * L) * 4;
+    if (i >= gs) break;
+    const float4 wp = *reinterpret_cast<const float4*>(w + (long long)g * gs + i);
+    float4 o = make_float4(v[p][0] * inv * wp.x, v[p][1] * inv * wp.y, v[p][2] * inv * wp.z, v[p][3] * inv * wp.w);
+    if (!gate_first) o = make_float4(o.x * a[p][0], o.y * a[p][1], o.z * a[p][2], o.w * a[p][3]);
+    store_piece(out + t * inner + (long long)g * gs + i, o);
+  }
+}
+
+// launches it if it takes these sizes
+template <typename TOut>
+static bool launch_group_norm_vec(const float* y, const float* gate, int ldg, const float* w, TOut* out, int n_tokens, int inner, int groups,
+                                  float eps, int gate_first, int gate_sigmoid, cudaStream_t stream) {
+  const int gs = inner / groups, pieces = gs / 4;
+  if (n_tokens <= 64 || gs % 4 || inner % 4 || ldg % 4 || (((uintptr_t)y | (uintptr_t)gate | (uintptr_t)w | (uintptr_t)out) & 15)) return false;
+  const long long n_groups = (long long)n_tokens * groups;
+  if (n_groups >= (1ll << 30)) return false;
+#define EL_GN(L, PIECES) gated_group_norm_vec_kernel<TOut, L, PIECES><<<(unsigned)((n_groups * L + 255) / 256), 256, 0, stream>>>(y, gate, ldg, w, out, n_groups, inner, groups, eps, gate_first, gate_sigmoid)
+  if (pieces <= 4) EL_GN(4, 1);
+  else if (pieces <= 8) EL_GN(8, 1);
+  else if (pieces <= 16) EL_GN(16, 1);
+  else if (pieces <= 32) EL_GN(32, 1);
+  else if (pieces <= 64) EL_GN(32, 2);
+  else if (pieces <= 256) EL_GN(256, 1);
+  else if (pieces <= 512) EL_GN(256, 2);
+  else if (pieces <= 1024) EL_GN(256, 4);
+  else if (pieces <= 2048) EL_GN(256, 8);
+  else return false;
+#undef EL_GN
+  return true;
+}
+
 // ------------------------------------------------------------------ x += rmsnorm(a y1 + b y2) * w  (+ a copy of x in the compute type)
 template <typename TCast>
 __global__ void rmsnorm_add_kernel(float* __restrict__ x, const float* __restrict__ y1, float a, const float* __restrict__ y2, float b,
@@ -617,7 +748,10 @@ extern "C" int edgelm_conv_act(const float* u, int ldu, int off, const float* w,
   const int col_blocks = (C + per_thread * row_threads(C) - 1) / (per_thread * row_threads(C));
   // a step of one token a sequence (as many tokens as sequences) moves the tail on in the same launch
   const int fused_tail = taps > 1 && update_state && n_tokens == n_seqs;
-  launch_pdl(pdl_bit_for_tokens(n_tokens), conv_silu_kernel, dim3(n_tokens, col_blocks), dim3(row_threads(C)), (size_t)(0), stream, u, ldu, off, w, b, state, out, tok_seq, seq_tok0, seq_slot, C, taps, in_bias, act, fused_tail);
+  const bool rows = n_tokens > 64 && !fused_tail && taps <= 4 && C % 4 == 0 && off % 4 == 0 && ldu % 4 == 0 && (uintptr_t)u % 16 == 0 && (uintptr_t)out % 16 == 0;
+  if (rows) conv_rows_kernel<<<dim3((n_tokens + CONV_RUN - 1) / CONV_RUN, (C + 4 * CONV_THREADS - 1) / (4 * CONV_THREADS)), CONV_THREADS, 0, stream>>>(
+      u, ldu, off, w, b, state, out, tok_seq, seq_tok0, seq_slot, n_tokens, C, taps, in_bias, act);
+  else launch_pdl(pdl_bit_for_tokens(n_tokens), conv_silu_kernel, dim3(n_tokens, col_blocks), dim3(row_threads(C)), (size_t)(0), stream, u, ldu, off, w, b, state, out, tok_seq, seq_tok0, seq_slot, C, taps, in_bias, act, fused_tail);
   EL_LAUNCH_CHECK("conv_silu");
   if (taps > 1 && update_state && !fused_tail) {
     launch_pdl(pdl_bit_for_tokens(n_tokens), conv_state_update_kernel, dim3(dim3(n_seqs, (C + 255) / 256)), dim3(256), (size_t)(0), stream, u, ldu, off, state, seq_tok0, seq_slot, C, taps, in_bias);
@@ -720,6 +854,11 @@ extern "C" int edgelm_gated_group_norm(const float* y, const float* gate, int ld
                                        int n_tokens, int inner, int groups, float eps, int gate_first, int gate_sigmoid, cudaStream_t stream) {
   if (n_tokens == 0) return 0;
   EL_REFUSE(n_tokens > 0 && inner > 0 && groups > 0 && inner % groups == 0, "gated_group_norm: %d values do not split into %d equal groups", inner, groups);
+  if ((out_dtype == DT_F32 && launch_group_norm_vec(y, gate, ldg, w, (float*)out, n_tokens, inner, groups, eps, gate_first, gate_sigmoid, stream)) ||
+      (out_dtype == DT_BF16 && launch_group_norm_vec(y, gate, ldg, w, (__nv_bfloat16*)out, n_tokens, inner, groups, eps, gate_first, gate_sigmoid, stream))) {
+    EL_LAUNCH_CHECK("gated_group_norm");
+    return 0;
+  }
   // (few rows of many values: a block of 1,024 threads walks a row in a quarter of the trips to memory)
   const int gs = inner / groups;
   const dim3 grid(n_tokens, groups), block(gs >= 1024 ? ((long long)n_tokens * groups <= 64 ? 1024 : 256) : (gs >= 128 ? 128 : 32));

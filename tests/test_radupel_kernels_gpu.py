@@ -320,6 +320,65 @@ def test_filter_over_time_inside_rotation_and_append(taps):
     assert int(err.item()) == 0 and (taps == 1 or torch.isnan(tails[1]).all())
 
 
+@pytest.mark.parametrize("H,G,dk,dv,maps,rot,inter,norm,taps,bias", [
+    (4, 2, 64, 64, 1, 64, True, False, 0, True), (3, 1, 64, 64, 1, 32, False, False, 4, False), (2, 2, 128, 128, 2, 64, False, True, 3, True),
+    (2, 1, 32, 64, 1, 16, False, True, 1, False), (2, 1, 96, 96, 1, 0, False, False, 2, True), (5, 1, 128, 128, 1, 128, False, False, 0, False)])
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+def test_rotation_and_append_of_many_tokens(H, G, dk, dv, maps, rot, inter, norm, taps, bias, dtype):
+    """Steps of more than 64 tokens: sequences that start and end inside a run of tokens, shorter than the filter, going on from a tail,
+    rows wider than the heads; every kind of partner.  3e-6: a dozen float32 roundings of values up to 5."""
+    g = torch.Generator().manual_seed(dk + rot + taps)
+    rnd = lambda *s: torch.randn(*s, generator=g, dtype=torch.float32)
+    lengths, first = [70, 1, 2, 33], [0, 100, 5, 62]
+    T, C, ds = sum(lengths), (H + G) * dk + G * dv, dk // maps
+    wide, b = rnd(T, C + 12), rnd(C) if bias else None
+    w, tail = rnd(C, taps) if taps else None, rnd(6, max(taps - 1, 0), C)
+    qn, kn = (rnd(ds).abs() + 0.5 for _ in range(2))
+    freq, slots = torch.rand(rot // 2, generator=g, dtype=torch.float64), [3, 0, 5, 2]
+    x = wide[:, :C].double() + (b.double() if bias else 0)
+    if taps:
+        rows, t0 = [], 0
+        for n, s in zip(lengths, slots):
+            u = torch.cat([tail[s].double(), x[t0:t0 + n]])
+            rows.append(sum(u[j:j + n] * w[:, j].double() for j in range(taps)))
+            t0 += n
+        x = torch.cat(rows)
+    pos = torch.cat([torch.arange(a, a + n) for a, n in zip(first, lengths)])
+    qk, v = x[:, :(H + G) * dk].reshape(T, H + G, maps, ds), x[:, (H + G) * dk:].reshape(T, G, dv)
+    if norm:
+        weight = torch.cat([qn.expand(H, maps, ds), kn.expand(G, maps, ds)]).double()
+        qk = qk / torch.sqrt(qk.square().mean(-1, keepdim=True) + 1e-3) * weight
+    if rot:
+        ang = pos.double()[:, None] * freq
+        c, sn = (f(ang)[:, None, None, :] * 1.1 for f in (torch.cos, torch.sin))
+        a, o = (qk[..., 0:rot:2], qk[..., 1:rot:2]) if inter else (qk[..., :rot // 2], qk[..., rot // 2:rot])
+        turned = torch.stack([a * c - o * sn, o * c + a * sn], -1).flatten(-2) if inter else torch.cat([a * c - o * sn, o * c + a * sn], -1)
+        qk = torch.cat([turned, qk[..., rot:]], -1)
+    qk = qk.reshape(T, H + G, dk)
+    kc, vc = (torch.zeros(12, G, PAGE, d, dtype=dtype, device=DEV) for d in (dk, dv))
+    table = torch.tensor([[7, 2, -1], [-1, 9, -1], [4, -1, -1], [1, 11, -1]], dtype=torch.int32, device=DEV)
+    seq = torch.repeat_interleave(torch.arange(4), torch.tensor(lengths))
+    tok0, q, err = i32([0, 70, 71, 73, 106]), torch.full((T, H * dk), float("nan"), device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    dev = lambda t: t.to(DEV) if t is not None else None
+    state = dev(tail)
+    ops.rotate_append(wide.to(DEV)[:, :C], dev(b), q, i32(pos), i32(seq), table, kc, vc, H, G, dk, dv, rot, inter, freq.to(DEV) if rot else None, err, maps=maps,
+                      q_norm=dev(qn) if norm else None, k_norm=dev(kn) if norm else None, eps=1e-3, conv_w=dev(w), conv_state=state if taps > 1 else None,
+                      seq_tok0=tok0 if taps else None, seq_slot=i32(slots) if taps else None, n_seqs=4, rot_mult=1.1)
+    assert int(err.item()) == 0
+    assert float((q.cpu().double().view(T, H, dk) - qk[:, :H]).abs().max()) < 3e-6
+    page = table.cpu()[seq, pos // PAGE].long()
+    for got, want in ((kc, qk[:, H:]), (vc, v)):
+        off = (got.cpu()[page, :, pos % PAGE].double() - want).abs()
+        assert bool((off < (3e-6 if dtype == torch.float32 else 3e-6 + 2.0 ** -8 * want.abs())).all())      # (a rounding to eight bits)
+        assert int((got != 0).any(-1).any(1).sum()) == T          # no other row was written
+    if taps > 1:
+        t0 = 0
+        for n, s in zip(lengths, slots):
+            u = torch.cat([tail[s], wide[t0:t0 + n, :C] + (b if bias else 0)])
+            assert torch.allclose(state[s].cpu(), u[-(taps - 1):], atol=1e-6)
+            t0 += n
+
+
 def test_tensor_core_attention_keeps_float32_scores_and_weights():
     """Queries so large that their rounding to bfloat16 would move the scores by a good part of 1, and values of very
     different sizes under weights of very different sizes: the kernel's output follows the float64 attention of the float32

@@ -153,6 +153,42 @@ def test_blend_convolution_and_norms(dtype):
     assert np.abs(dec.cpu().numpy() - ref).max() < 1e-5
 
 
+@pytest.mark.parametrize("C,taps,bias,act", [(260, 4, True, "silu"), (64, 2, False, None), (512, 1, True, "silu"), (1028, 3, True, None)])
+def test_filter_over_many_tokens(C, taps, bias, act):
+    """Steps of more than 64 tokens: sequences that start inside a run of tokens, shorter than the filter, going on from a tail."""
+    g = np.random.default_rng(C)
+    lengths, slots = [70, 1, 2, 33], [3, 0, 5, 2]
+    u, w, b, ib, tail = g.normal(size=(106, C + 8)), g.normal(size=(C, taps)), g.normal(size=C), g.normal(size=C), g.normal(size=(6, taps - 1, C))
+    tok0, tok_seq = packed(lengths)
+    state, y = f32(tail), torch.full((106, C), float("nan"), device=DEV)
+    ops.conv_act(f32(u), 4, f32(w), f32(b) if bias else None, state, y, tok_seq, tok0, i32(slots), 4, in_bias=f32(ib), act=act)
+    for s, (a, e) in enumerate(zip(tok0.tolist(), tok0.tolist()[1:])):
+        full = np.concatenate([tail[slots[s]], u[a:e, 4:4 + C] + ib])
+        ref = sum(full[j:j + e - a] * w[:, j] for j in range(taps)) + (b if bias else 0.0)
+        ref = plain.silu(ref) if act else ref
+        assert np.abs(y[a:e].cpu().numpy() - ref).max() < 3e-6 * max(1.0, np.abs(ref).max())      # (five roundings of sums up to 16)
+        if taps > 1:
+            assert np.allclose(state[slots[s]].cpu().numpy(), full[-(taps - 1):], atol=1e-6)
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("gs,groups", [(4, 3), (64, 5), (128, 2), (100, 3), (576, 1), (1028, 2), (4096, 1), (8192, 1), (8200, 1), (66, 2)])
+def test_gated_group_norm_of_many_rows(gs, groups, dtype):
+    """Every way a group is shared by threads, the last one ragged; sizes that no vector form takes too."""
+    g = np.random.default_rng(gs)
+    T, inner = 67, gs * groups
+    y, gate, w = g.normal(size=(T, inner)), g.normal(size=(T, inner + 4)), g.uniform(0.5, 1.5, inner)
+    for first in (True, False):
+        for act in ("silu", "sigmoid"):
+            o = torch.full((T, inner), float("nan"), dtype=dtype, device=DEV)
+            ops.gated_group_norm(f32(y), f32(gate)[:, 4:], f32(w), o, groups, 1e-4, first, gate_act=act)
+            a = plain.silu(gate[:, 4:]) if act == "silu" else 1.0 / (1.0 + np.exp(-gate[:, 4:]))
+            norm = lambda v: plain.unit_rms(v.reshape(T, groups, gs), 1e-4).reshape(T, inner) * w
+            ref = norm(y * a) if first else norm(y) * a
+            off = np.abs(o.float().cpu().numpy() - ref)
+            assert (off < 3e-6 * max(1.0, np.abs(ref).max()) + (0 if dtype == torch.float32 else 2.0 ** -8 * np.abs(ref))).all()
+
+
 def chunk_steps(total, cuts):
     """Per step the sequences' new tokens, `seq_tok0` and the tiles of STATE_CHUNK tokens (first row, tokens, count)."""
     from edgelm_b200.engine.batch import make_tiles
