@@ -118,6 +118,89 @@ __device__ __forceinline__ void fetch_residual(ResidualAhead& ra, const float* r
   }
 }
 
+// Eight sums of a row (columns col0 ..) through the epilogue, up to the residual
+template <int EPI>
+__device__ __forceinline__ void epilogue_values(float* v, const uint32_t* r, const uint32_t* r2, int col0, int N, const RopeAppend& form, float row_weight) {
+#pragma unroll
+  for (int j = 0; j < 8; ++j) {
+    const float acc = __uint_as_float(r[j]);
+    if (EPI == TC_EPI_SWIGLU) {
+      float g = acc * row_weight, u = __uint_as_float(r2[j]) * row_weight;
+      if (form.glu_bias != nullptr) {     // (every thread of a tile asks for the same 2 x 32 values: they come out of L1)
+        const int c = min(col0 + j, N - 1);
+        g += form.glu_bias[c];
+        u += form.glu_bias[N + c];
+      }
+      v[j] = glu_tc(g, u, form.glu_limit, form.glu_alpha, form.glu_shift);
+    } else if (EPI == TC_EPI_STORE && form.square_relu) {
+      const float z = fmaxf(acc, 0.f);
+      v[j] = z * z;
+    } else v[j] = acc;
+  }
+}
+
+// The epilogue of products of more than one row tile: a warp lays its 32 rows of 128 bytes (32 float32 columns, 64 bfloat16 ones) into
+// one of its two 4 KB buffers, in the 128-byte swizzle, and one lane hands them to TMA, which stores them or adds them to the residual in
+// place, whole rows of sectors at a time.  (A thread's own 16-byte stores and residual loads touch 32 rows an instruction: the epilogue
+// of a 128 x 256 float32 tile took 14 us, more than its MMAs at K 2048.  6,881 rows, N 2048 with the residual: K 2048 81 -> 50 us, K 8192
+// 218 -> 176; 2,048 rows, N 8512, K 2048 to float32 73 -> 62; 2,048 rows, N 576, K 576 with the residual 7.6 -> 5.3.)  TC_OUT: how the tile leaves.
+enum : int { TC_OUT_DIRECT = 0, TC_OUT_STORE = 1, TC_OUT_ADD = 2 };
+constexpr int TC_OUT_WARP = 8192;      // bytes of a warp's two buffers
+
+// What the one-tile kernel is told about it.  Its own form with the threads' stores has none of it: a 64-row decode step of 24 layers is
+// a hundred such products, and with the map and the second epilogue in them it took 879 us instead of 864.
+template <bool BY_TMA>
+struct OutTiles {};
+template <>
+struct OutTiles<true> {
+  CUtensorMap map;
+  int how;
+};
+
+template <int EPI, typename TOut, int BN>
+__device__ __forceinline__ void epilogue_tma_tile(uint32_t taddr, uint8_t* buffers, const CUtensorMap* map, int how, int row0, int n0, int M, int N,
+                                                  const RopeAppend& form, float row_weight, int lane) {
+  constexpr int NB = EPI == TC_EPI_SWIGLU ? 2 : 1, COLS = 128 / sizeof(TOut);
+  if (lane == 0) bulk_wait_read<0>();  // (a tile before may have ended on either buffer)
+  __syncwarp();
+#pragma unroll 1
+  for (int c0 = 0; c0 < BN; c0 += 32) {
+    if (n0 + c0 >= N) break;           // uniform over the block
+    uint32_t r[32], r2[32];
+    tmem_ld32(taddr + (uint32_t)c0, r);
+    if (NB == 2) tmem_ld32(taddr + (uint32_t)(c0 + BN), r2);
+    uint8_t* buf = buffers + (c0 / COLS & 1) * 4096;
+    if (c0 % COLS == 0) {              // the group before the last has read this buffer
+      if (lane == 0) bulk_wait_read<1>();
+      __syncwarp();
+    }
+    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+    for (int j0 = 0; j0 < 32; j0 += 8) {
+      float v[8];
+      epilogue_values<EPI>(v, r + j0, r2 + j0, n0 + c0 + j0, N, form, row_weight);
+      if constexpr (sizeof(TOut) == 4) {
+        float4* row = reinterpret_cast<float4*>(buf + lane * 128);
+        row[(j0 / 4) ^ (lane & 7)] = make_float4(v[0], v[1], v[2], v[3]);
+        row[(j0 / 4 + 1) ^ (lane & 7)] = make_float4(v[4], v[5], v[6], v[7]);
+      } else {
+        OutVec<TOut>::store8(reinterpret_cast<TOut*>(buf + lane * 128 + (((c0 % COLS + j0) / 8) ^ (lane & 7)) * 16), v);
+      }
+    }
+    if ((c0 + 32) % COLS == 0 || n0 + c0 + 32 >= N) {
+      asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) {
+        if (row0 < M) {
+          if (how == TC_OUT_ADD) tma_add_2d(map, smem_u32(buf), n0 + c0 / COLS * COLS, row0);
+          else tma_store_2d(map, smem_u32(buf), n0 + c0 / COLS * COLS, row0);
+        }
+        bulk_commit();
+      }
+    }
+  }
+}
+
 template <int EPI, typename TOut>
 __device__ __forceinline__ void epilogue_piece(const uint32_t* r, const uint32_t* r2, TOut* out, int ldo,
                                                const float* residual, int row, int col0, int M, int N, int vec_ok,
@@ -128,22 +211,7 @@ __device__ __forceinline__ void epilogue_piece(const uint32_t* r, const uint32_t
 #pragma unroll
   for (int j0 = 0; j0 < 32; j0 += 8) {
     float v[8];
-#pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const float acc = __uint_as_float(r[j0 + j]);
-      if (EPI == TC_EPI_SWIGLU) {
-        float g = acc * row_weight, u = __uint_as_float(r2[j0 + j]) * row_weight;
-        if (form.glu_bias != nullptr) {     // (every thread of a tile asks for the same 2 x 32 values: they come out of L1)
-          const int c = min(col0 + j0 + j, N - 1);
-          g += form.glu_bias[c];
-          u += form.glu_bias[N + c];
-        }
-        v[j] = glu_tc(g, u, form.glu_limit, form.glu_alpha, form.glu_shift);
-      } else if (EPI == TC_EPI_STORE && form.square_relu) {
-        const float z = fmaxf(acc, 0.f);
-        v[j] = z * z;
-      } else v[j] = acc;
-    }
+    epilogue_values<EPI>(v, r + j0, r2 + j0, col0 + j0, N, form, row_weight);
     if (full) {
       if (EPI == TC_EPI_RESIDUAL) {
         const bool pre = ahead != nullptr && ahead->have;
@@ -263,12 +331,12 @@ __device__ __forceinline__ void epilogue_rope_tile(uint32_t taddr, const RopeApp
   }
 }
 
-template <int BN, int EPI, typename TOut, int STAGES>
+template <int BN, int EPI, typename TOut, int STAGES, bool BY_TMA>
 __global__ void __launch_bounds__(TC_THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_b2, TOut* out, int ldo, const float* residual,
                int M, int N, int K, int vec_ok, int* err, int k_splits, float* partial, const RopeAppend rope,
-               const GroupedTiles grp) {
+               const GroupedTiles grp, const __grid_constant__ OutTiles<BY_TMA> out_tiles) {
   // a grouped product is launched without programmatic dependence: the kernel that wrote `tile_group` is complete
   int w_row0 = blockIdx.x * BN;           // the first row of the weight tile (its output columns start at n0)
   if (grp.tile_group != nullptr) {
@@ -389,7 +457,7 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     const int q = warp & 3;  // a warp reads the 32 lanes of tensor memory that its index modulo 4 selects
     ResidualAhead ra[2];
     ra[0].have = ra[1].have = false;
-    if (EPI == TC_EPI_RESIDUAL && k_splits == 1) fetch_residual(ra[0], residual, ldo, m0 + q * 32 + lane, n0, M, N, vec_ok);  // while the MMAs run
+    if (EPI == TC_EPI_RESIDUAL && !BY_TMA && k_splits == 1) fetch_residual(ra[0], residual, ldo, m0 + q * 32 + lane, n0, M, N, vec_ok);  // while the MMAs run
     RopeRow rr;
     if constexpr (EPI == TC_EPI_ROPE) rope_row_fetch(rr, rope, m0 + q * 32 + lane, M, n0 + BN > rope.nh * rope.hd, err);   // likewise
     float row_weight = 1.f;
@@ -402,6 +470,12 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (ok && EPI == TC_EPI_ROPE) {
       if constexpr (EPI == TC_EPI_ROPE)
         epilogue_rope_tile<BN>(tmem_base + ((uint32_t)(q * 32) << 16), rope, rr, out, ldo, m0 + q * 32 + lane, n0, N);
+    } else if (ok && BY_TMA) {
+      // (the ring is the buffers' room: the MMAs that read its last stage are done)
+      if constexpr (BY_TMA)
+        epilogue_tma_tile<EPI, TOut, BN>(tmem_base + ((uint32_t)(q * 32) << 16), smem + q * TC_OUT_WARP, &out_tiles.map, out_tiles.how, m0 + q * 32, n0, M, N, rope,
+                                         row_weight, lane);
+      if (lane == 0) bulk_wait_all();
     } else if (ok) {
 #pragma unroll
       for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -479,7 +553,8 @@ template <int BN, int EPI, typename TOut>
 __global__ void __launch_bounds__(TC_THREADS, 1)
 gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                           const __grid_constant__ CUtensorMap map_b2, TOut* out, int ldo, const float* residual,
-                          int M, int N, int K, int vec_ok, int* err, const RopeAppend rope) {
+                          int M, int N, int K, int vec_ok, int* err, const RopeAppend rope, const __grid_constant__ CUtensorMap map_out,
+                          int how_out) {
   constexpr int NB = EPI == TC_EPI_SWIGLU ? 2 : 1;
   constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2;
   constexpr int STAGE_BYTES = A_BYTES + NB * B_BYTES;
@@ -490,7 +565,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~(uintptr_t)1023);
-  uint64_t* bars = reinterpret_cast<uint64_t*>(smem + TCP_STAGES * STAGE_BYTES);
+  uint8_t* out_buffers = smem + TCP_STAGES * STAGE_BYTES;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(out_buffers + 4 * TC_OUT_WARP);
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + TCP_STAGES;
   uint64_t* tmem_full_bar = bars + 2 * TCP_STAGES;       // [2]
@@ -594,6 +670,8 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       const uint32_t acc_addr = tmem_base + (uint32_t)as * ACC_COLS + ((uint32_t)(q * 32) << 16);
       if constexpr (EPI == TC_EPI_ROPE) {
         epilogue_rope_tile<BN>(acc_addr, rope, rr, out, ldo, m0 + q * 32 + lane, n0, N);
+      } else if (how_out != TC_OUT_DIRECT) {
+        epilogue_tma_tile<EPI, TOut, BN>(acc_addr, out_buffers + q * TC_OUT_WARP, &map_out, how_out, m0 + q * 32, n0, M, N, rope, 1.f, lane);
       } else {
 #pragma unroll 1
         for (int c0 = 0; c0 < BN; c0 += 32) {
@@ -610,6 +688,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
       __syncwarp();
       if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(smem_u32(&tmem_empty_bar[as])) : "memory");
     }
+    if (lane == 0) bulk_wait_all();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
@@ -624,7 +703,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // 128 x 256 tiles and two accumulator stages (1.10 to 1.16 PFLOP/s at 2048 x 8192 x 2048 against 0.88 to 0.91
 // of the other), everything else to the one-tile-per-CTA kernel with 128 x 128 tiles, two CTAs per SM (the
 // persistent kernel with narrow tiles starves on shared-memory bandwidth: 0.68 to 0.78).  Forced for comparisons.
-static int g_tc_auto = 1, g_tc_persistent = 1, g_tc_wide = 1, g_tc_narrow = 1, g_tc_deep = 1, g_tc_tiny = 1;
+static int g_tc_auto = 1, g_tc_persistent = 1, g_tc_wide = 1, g_tc_narrow = 1, g_tc_deep = 1, g_tc_tiny = 1, g_tc_out = 1;
 
 // Scratch for split-K launches (set by the caller once; nothing is allocated here): without it no product is split.
 static float* g_splitk_ws = nullptr;
@@ -650,13 +729,24 @@ static int splitk_for(int tiles, int n_k, size_t bytes_per_split) {
   return (n_k + k_per - 1) / k_per;   // every split gets a share
 }
 
+static bool leaves_by_tma(int M, int N, const void* out, const float* residual, int epilogue, int vec_ok) {
+  return g_tc_out && M > TC_BM && N >= 64 && vec_ok && (epilogue != TC_EPI_RESIDUAL || residual == out);
+}
+
 template <int BN, int EPI, typename TOut>
 static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtensorMap& mb2, void* out, int ldo,
                      const float* residual, int M, int N, int K, int vec_ok, int* err, cudaStream_t stream, bool persistent,
                      const RopeAppend& rope, const GroupedTiles& grp = GroupedTiles{}) {
   constexpr int NB = EPI == TC_EPI_SWIGLU ? 2 : 1;
+  // products of more than one row tile hand their tiles to TMA: rows in whole pieces of 16 bytes, the residual added in place
+  OutTiles<true> mo{ma, TC_OUT_DIRECT};
+  constexpr bool CAN_TMA = EPI != TC_EPI_ROPE && BN >= 64;
+  if (CAN_TMA && leaves_by_tma(M, N, out, residual, EPI, vec_ok)) {
+    if (tensor_map(out, M, N, ldo, 32, &mo.map, (int)sizeof(TOut))) return -1;
+    mo.how = EPI == TC_EPI_RESIDUAL ? TC_OUT_ADD : TC_OUT_STORE;
+  }
   if (persistent) {
-    constexpr int smem = TCP_STAGES * (TC_BM * TC_BK * 2 + NB * BN * TC_BK * 2) + 1024 + 256;
+    constexpr int smem = TCP_STAGES * (TC_BM * TC_BK * 2 + NB * BN * TC_BK * 2) + 4 * TC_OUT_WARP + 1024 + 256;
     auto kern = gemm_tc_persistent_kernel<BN, EPI, TOut>;
     static bool configured = false;
     static int n_sms = 0;
@@ -677,7 +767,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
     g_last_launches = 1;
     g_last_kernel = BN | (1 << 12) | (1 << 16);
     cudaError_t le = launch_pdl(32, kern, dim3(grid), dim3(TC_THREADS), (size_t)smem, stream, ma, mb, mb2, (TOut*)out, ldo, residual, M, N, K,
-                                vec_ok, err, rope);
+                                vec_ok, err, rope, mo.map, mo.how);
     if (le != cudaSuccess) {
       set_error("gemm_tc: launch failed: %s", cudaGetErrorString(le));
       return -2;
@@ -701,22 +791,29 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
   }
   const bool deep = g_tc_deep && (long long)grid.x * grid.y * grid.z <= n_sms;
   g_last_kernel = BN | ((deep ? 1 : 0) << 13) | (splits << 16);
-  auto go = [&](auto kern, int smem) -> int {
+  auto go = [&](auto kern, int smem, const auto& out_tiles) -> int {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) {
       set_error("gemm_tc: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
       return -2;
     }
     cudaError_t le = launch_pdl(grp.tile_group != nullptr ? 0 : 8, kern, grid, dim3(TC_THREADS), (size_t)smem, stream, ma, mb, mb2, (TOut*)out, ldo,
-                                residual, M, N, K, vec_ok, err, splits, g_splitk_ws, rope, grp);
+                                residual, M, N, K, vec_ok, err, splits, g_splitk_ws, rope, grp, out_tiles);
     if (le != cudaSuccess) {
       set_error("gemm_tc: launch failed: %s", cudaGetErrorString(le));
       return -2;
     }
     return 0;
   };
-  const int rc = deep ? go(gemm_tc_kernel<BN, EPI, TOut, DEEP>, DEEP * STAGE_BYTES + 1024 + 256)
-                      : go(gemm_tc_kernel<BN, EPI, TOut, TC_STAGES>, TC_STAGES * STAGE_BYTES + 1024 + 256);
+  const int deep_smem = DEEP * STAGE_BYTES + 1024 + 256, smem = TC_STAGES * STAGE_BYTES + 1024 + 256;
+  int rc;
+  if constexpr (CAN_TMA) {
+    if (mo.how != TC_OUT_DIRECT && splits == 1) {   // (the shares of a split product are raw sums in the scratch)
+      return deep ? go(gemm_tc_kernel<BN, EPI, TOut, DEEP, true>, deep_smem, mo) : go(gemm_tc_kernel<BN, EPI, TOut, TC_STAGES, true>, smem, mo);
+    }
+  }
+  rc = deep ? go(gemm_tc_kernel<BN, EPI, TOut, DEEP, false>, deep_smem, OutTiles<false>{})
+            : go(gemm_tc_kernel<BN, EPI, TOut, TC_STAGES, false>, smem, OutTiles<false>{});
   if (rc) return rc;
   if (EPI != TC_EPI_ROPE && splits > 1) {
     const size_t plane = (size_t)M * N;
@@ -758,6 +855,12 @@ extern "C" int edgelm_gemm_tc_tiny(int on) {
   return 0;
 }
 
+// 1 (default): products of more than one row tile leave by TMA; 0: by the threads' own stores (comparisons).
+extern "C" int edgelm_gemm_tc_out(int on) {
+  g_tc_out = on & 1;
+  return 0;
+}
+
 extern "C" int edgelm_gemm_tc_narrow(int on) {
   g_tc_narrow = on & 1;
   g_tc_deep = (on >> 1) & 1;
@@ -783,13 +886,21 @@ static int gemm_tc_run(const void* a, int lda, const void* w, const void* w2, vo
   EL_REFUSE(epilogue != TC_EPI_RESIDUAL || (residual != nullptr && out_dtype == DT_F32), "gemm_tc: residual epilogue needs a float32 residual and output");
   EL_REFUSE(err != nullptr, "gemm_tc: needs the error word");
   EL_REFUSE((M + TC_BM - 1) / TC_BM <= 65535, "gemm_tc: too many rows (%d)", M);
+  const size_t esz = out_dtype == DT_F32 ? 4 : 2;
+  const int vec_ok = ((uintptr_t)out % 16 == 0) && ((size_t)ldo * esz % 16 == 0) &&
+                     (residual == nullptr || (uintptr_t)residual % 16 == 0);
   // wide tiles (128 x 256, or 2 x 128 for SwiGLU) when the output is wide enough to fill the device with
   // them: twice the multiply-adds per byte that comes through shared memory
   const long long wide_tiles = (long long)((M + TC_BM - 1) / TC_BM) * ((N + (epilogue == TC_EPI_SWIGLU ? 127 : 255)) / (epilogue == TC_EPI_SWIGLU ? 128 : 256));
-  const bool wide = g_tc_auto ? (wide_tiles >= 120 && N >= 1024 && K >= 1024) : (g_tc_wide && wide_tiles >= 120 && N >= 1024);
-  // (with a residual the wide tiles go one to a block: measured at 2,048 rows, N 2048: K 8192 65.9 -> 60.0 us, K 2048
-  // 25.3 -> 24.0 us; persistent 69.0 and 31.3 us)
-  const bool persistent = g_tc_auto ? (wide && epilogue != TC_EPI_RESIDUAL) : g_tc_persistent != 0;
+  // Several of them to a block (the persistent kernel), whose epilogues then run beside the next tile's MMAs.  With a residual only if it
+  // leaves by TMA and there is a wave and a half of tiles: one to a block and several, N 2048, at 2,048 rows and K 8192 53.8 and 54.3 us,
+  // at 3,900 rows 127 and 107, at 6,881 rows 196 and 176, K 2048 59 and 50.  A short K (512 to 1,023) only then too, and without a residual:
+  // 128-column tiles and several wide ones, 6,000 rows, K 576: N 3000 to float32 31.7 and 25.0 us, gated N 1536 31.6 and 22.3;
+  // 4,096 rows, K 960, gated N 2560 51 and 37.5; 1,792 rows (168 tiles), K 576, gated N 1536 14.5 and 12.6.
+  const bool residual_tiles = epilogue == TC_EPI_RESIDUAL, by_tma = epilogue != TC_EPI_ROPE && leaves_by_tma(M, N, out, residual, epilogue, vec_ok);
+  const bool fits = wide_tiles >= 120 && N >= 1024;
+  const bool wide = g_tc_auto ? fits && (K >= 1024 || (K >= 512 && wide_tiles >= 160 && by_tma && !residual_tiles)) : g_tc_wide && fits;
+  const bool persistent = g_tc_auto ? wide && (!residual_tiles || (by_tma && wide_tiles >= 222)) : g_tc_persistent != 0;
   // tiles of 64 columns for a single weight when 128-column tiles would not fill one wave of SMs and there are
   // several row tiles to share a weight tile in L2 (measured at 2,048 rows: N 576, K 576: 11.6 -> 8.8 us; N 576,
   // K 1536: 16.1 -> 13.5 us; with 256 tiles of 128 columns and K 8192 the narrow tiles lose: 68 -> 107 us)
@@ -808,9 +919,6 @@ static int gemm_tc_run(const void* a, int lda, const void* w, const void* w2, vo
   if (tensor_map(w, N, K, K, bn, &mb)) return -1;
   mb2 = mb;
   if (w2 && tensor_map(w2, N, K, K, bn, &mb2)) return -1;
-  const size_t esz = out_dtype == DT_F32 ? 4 : 2;
-  const int vec_ok = ((uintptr_t)out % 16 == 0) && ((size_t)ldo * esz % 16 == 0) &&
-                     (residual == nullptr || (uintptr_t)residual % 16 == 0);
   int rc = 0;
   if (wide) {
     if (epilogue == TC_EPI_STORE && out_dtype == DT_BF16)

@@ -61,6 +61,17 @@ __device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map
                ::"r"(dst), "l"((uint64_t)map), "r"(bar), "r"(x), "r"(y)
                : "memory");
 }
+// A tile from shared memory (128-byte swizzle) to where the tensor map says, what lies outside the tensor left out: stored, or added to
+// what is there (float32, round to nearest; a subnormal counts as zero).  Bulk groups belong to the issuing thread.
+__device__ __forceinline__ void tma_store_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+  asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void tma_add_2d(const CUtensorMap* map, uint32_t src, int x, int y) {
+  asm volatile("cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.tile.bulk_group [%0, {%2, %3}], [%1];" ::"l"((uint64_t)map), "r"(src), "r"(x), "r"(y) : "memory");
+}
+__device__ __forceinline__ void bulk_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
+template <int N> __device__ __forceinline__ void bulk_wait_read() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
+__device__ __forceinline__ void bulk_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 // Shared-memory matrix descriptor of a K-major tile with 128-byte swizzle: rows of 128 bytes,
 // groups of 8 rows 1024 bytes apart (stride byte offset), descriptor version 1.
 __device__ __forceinline__ uint64_t umma_desc(uint32_t saddr) {
@@ -117,23 +128,23 @@ static EncodeTiledFn encode_fn() {
 
 struct MapKey {
   const void* ptr;
-  int rows, cols, ld, box_rows;
-  bool operator==(const MapKey& o) const { return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows; }
+  int rows, cols, ld, box_rows, esz;
+  bool operator==(const MapKey& o) const { return ptr == o.ptr && rows == o.rows && cols == o.cols && ld == o.ld && box_rows == o.box_rows && esz == o.esz; }
 };
 struct MapKeyHash {
   size_t operator()(const MapKey& k) const {
     size_t h = reinterpret_cast<size_t>(k.ptr);
-    for (int v : {k.rows, k.cols, k.ld, k.box_rows}) h = h * 1000003u ^ (size_t)v;
+    for (int v : {k.rows, k.cols, k.ld, k.box_rows, k.esz}) h = h * 1000003u ^ (size_t)v;
     return h;
   }
 };
 
-// Tensor map of a row-major bfloat16 matrix [rows, cols] with row pitch ld, boxes of box_rows x 64,
+// Tensor map of a row-major matrix [rows, cols] of bfloat16 (`esz` 2) or float32 (4) with row pitch ld, boxes of box_rows x 128 bytes,
 // 128-byte swizzle, zero fill outside.  Cached: activations live at fixed workspace addresses.
-static int tensor_map(const void* ptr, int rows, int cols, int ld, int box_rows, CUtensorMap* out) {
+static int tensor_map(const void* ptr, int rows, int cols, int ld, int box_rows, CUtensorMap* out, int esz = 2) {
   static std::unordered_map<MapKey, CUtensorMap, MapKeyHash> cache;
   static std::mutex mu;
-  const MapKey key{ptr, rows, cols, ld, box_rows};
+  const MapKey key{ptr, rows, cols, ld, box_rows, esz};
   std::lock_guard<std::mutex> lock(mu);
   auto it = cache.find(key);
   if (it != cache.end()) {
@@ -143,11 +154,11 @@ static int tensor_map(const void* ptr, int rows, int cols, int ld, int box_rows,
   EncodeTiledFn enc = encode_fn();
   EL_REFUSE(enc != nullptr, "gemm_tc: the driver does not provide cuTensorMapEncodeTiled");
   const cuuint64_t dims[2] = {(cuuint64_t)cols, (cuuint64_t)rows};
-  const cuuint64_t strides[1] = {(cuuint64_t)ld * 2};
-  const cuuint32_t box[2] = {(cuuint32_t)TC_BK, (cuuint32_t)box_rows};
+  const cuuint64_t strides[1] = {(cuuint64_t)ld * esz};
+  const cuuint32_t box[2] = {(cuuint32_t)(128 / esz), (cuuint32_t)box_rows};
   const cuuint32_t estr[2] = {1, 1};
   CUtensorMap m;
-  const CUresult r = enc(&m, CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
+  const CUresult r = enc(&m, esz == 4 ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32 : CU_TENSOR_MAP_DATA_TYPE_BFLOAT16, 2, const_cast<void*>(ptr), dims, strides, box, estr,
                          CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B, CU_TENSOR_MAP_L2_PROMOTION_L2_128B,
                          CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   EL_REFUSE(r == CUDA_SUCCESS, "gemm_tc: cuTensorMapEncodeTiled failed with code %d for a [%d, %d] matrix of pitch %d", (int)r, rows, cols, ld);

@@ -504,6 +504,39 @@ def test_gemm_tc_store_and_residual(M, N, K):
     assert rel_err(out32, simt) < 2e-5
 
 
+@pytest.mark.parametrize("M,N,K", [(129, 64, 64), (200, 200, 96), (300, 68, 1024), (1000, 2072, 64), (2000, 2048, 1032), (1290, 2080, 1024), (2100, 2904, 520)])
+@pytest.mark.parametrize("persistent", [-1, 1])
+def test_gemm_tc_tiles_that_leave_by_tma(M, N, K, persistent):
+    """Ragged last rows and columns, an odd number of pieces in the last tile, rows wider than the product, split products beside;
+    each output beside the threads' own stores: the same bits.  What lies outside stays as it was."""
+    o = ops()
+    a, w, w2 = rnd((M, K), torch.bfloat16, 70), rnd((N, K), torch.bfloat16, 71, 0.2), rnd((N, K), torch.bfloat16, 72, 0.2)
+    err, x0 = torch.zeros(1, dtype=torch.int32, device=dev()), rnd((M + 1, N + 24), torch.float32, 73)
+    runs = []
+    try:
+        o.lib().edgelm_gemm_tc_persistent(persistent)
+        for on in (1, 0):
+            o.lib().edgelm_gemm_tc_out(on)
+            outs = []
+            for dtype, epilogue in ((torch.float32, o.EPI_STORE), (torch.bfloat16, o.EPI_STORE), (torch.float32, o.EPI_RESIDUAL), (torch.bfloat16, o.EPI_SWIGLU),
+                                    (torch.float32, o.EPI_RELU2)):
+                whole = x0.to(dtype, copy=True)
+                out = whole[:M, 8:8 + N]
+                o.gemm_tc(a, w, out, err, epilogue=epilogue, w2=w2 if epilogue == o.EPI_SWIGLU else None, residual=out if epilogue == o.EPI_RESIDUAL else None)
+                outs.append(whole)
+            runs.append(outs)
+    finally:
+        o.lib().edgelm_gemm_tc_out(1)
+        o.lib().edgelm_gemm_tc_persistent(-1)
+    assert int(err.item()) == 0
+    want = a.double() @ w.double().T
+    assert rel_err(runs[0][0][:M, 8:8 + N], want.cpu()) < 2e-5
+    assert rel_err(runs[0][2][:M, 8:8 + N], (x0[:M, 8:8 + N].double() + want).cpu()) < 2e-5
+    for got, ref in zip(*runs):
+        assert torch.equal(got, ref)
+        assert torch.equal(got[M:], x0[M:].to(got.dtype)) and torch.equal(got[:, :8], x0[:, :8].to(got.dtype)) and torch.equal(got[:, 8 + N:], x0[:, 8 + N:].to(got.dtype))
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 64, 64), (200, 200, 96), (2048, 1536, 576), (33, 130, 40), (64, 520, 1024), (40, 1536, 2048)])
 def test_gemm_tc_swiglu(M, N, K):
     o = ops()
