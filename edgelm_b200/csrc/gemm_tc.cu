@@ -729,8 +729,9 @@ static int splitk_for(int tiles, int n_k, size_t bytes_per_split) {
   return (n_k + k_per - 1) / k_per;   // every split gets a share
 }
 
-static bool leaves_by_tma(int M, int N, const void* out, const float* residual, int epilogue, int vec_ok) {
-  return g_tc_out && M > TC_BM && N >= 64 && vec_ok && (epilogue != TC_EPI_RESIDUAL || residual == out);
+// (a row that ends inside a piece of 16 bytes does not: TMA cuts a box off at whole pieces, and the rest of the last one was overwritten)
+static bool leaves_by_tma(int M, int N, size_t esz, const void* out, const float* residual, int epilogue, int vec_ok) {
+  return g_tc_out && M > TC_BM && N >= 64 && vec_ok && (size_t)N * esz % 16 == 0 && (epilogue != TC_EPI_RESIDUAL || residual == out);
 }
 
 template <int BN, int EPI, typename TOut>
@@ -741,7 +742,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
   // products of more than one row tile hand their tiles to TMA: rows in whole pieces of 16 bytes, the residual added in place
   OutTiles<true> mo{ma, TC_OUT_DIRECT};
   constexpr bool CAN_TMA = EPI != TC_EPI_ROPE && BN >= 64;
-  if (CAN_TMA && leaves_by_tma(M, N, out, residual, EPI, vec_ok)) {
+  if (CAN_TMA && leaves_by_tma(M, N, sizeof(TOut), out, residual, EPI, vec_ok)) {
     if (tensor_map(out, M, N, ldo, 32, &mo.map, (int)sizeof(TOut))) return -1;
     mo.how = EPI == TC_EPI_RESIDUAL ? TC_OUT_ADD : TC_OUT_STORE;
   }
@@ -897,7 +898,7 @@ static int gemm_tc_run(const void* a, int lda, const void* w, const void* w2, vo
   // at 3,900 rows 127 and 107, at 6,881 rows 196 and 176, K 2048 59 and 50.  A short K (512 to 1,023) only then too, and without a residual:
   // 128-column tiles and several wide ones, 6,000 rows, K 576: N 3000 to float32 31.7 and 25.0 us, gated N 1536 31.6 and 22.3;
   // 4,096 rows, K 960, gated N 2560 51 and 37.5; 1,792 rows (168 tiles), K 576, gated N 1536 14.5 and 12.6.
-  const bool residual_tiles = epilogue == TC_EPI_RESIDUAL, by_tma = epilogue != TC_EPI_ROPE && leaves_by_tma(M, N, out, residual, epilogue, vec_ok);
+  const bool residual_tiles = epilogue == TC_EPI_RESIDUAL, by_tma = epilogue != TC_EPI_ROPE && leaves_by_tma(M, N, esz, out, residual, epilogue, vec_ok);
   const bool fits = wide_tiles >= 120 && N >= 1024;
   const bool wide = g_tc_auto ? fits && (K >= 1024 || (K >= 512 && wide_tiles >= 160 && by_tma && !residual_tiles)) : g_tc_wide && fits;
   const bool persistent = g_tc_auto ? wide && (!residual_tiles || (by_tma && wide_tiles >= 222)) : g_tc_persistent != 0;

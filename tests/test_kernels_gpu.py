@@ -537,6 +537,22 @@ def test_gemm_tc_tiles_that_leave_by_tma(M, N, K, persistent):
         assert torch.equal(got[M:], x0[M:].to(got.dtype)) and torch.equal(got[:, :8], x0[:, :8].to(got.dtype)) and torch.equal(got[:, 8 + N:], x0[:, 8 + N:].to(got.dtype))
 
 
+@pytest.mark.parametrize("N", [570, 1030, 2050])
+def test_gemm_tc_columns_that_end_inside_a_piece(N):
+    """Rows that end inside 16 bytes, in a wider matrix: what lies behind them stays as it was."""
+    o = ops()
+    M, K = 2100, 520
+    a, w = rnd((M, K), torch.bfloat16, 85), rnd((N, K), torch.bfloat16, 86, 0.05)
+    err, x0 = torch.zeros(1, dtype=torch.int32, device=dev()), rnd((M, N + 14), torch.float32, 87)
+    for dtype, epilogue in ((torch.float32, o.EPI_STORE), (torch.bfloat16, o.EPI_STORE), (torch.float32, o.EPI_RESIDUAL)):
+        whole = x0.to(dtype, copy=True)
+        out = whole[:, 8:8 + N]
+        want = a.double() @ w.double().T + (out.double() if epilogue == o.EPI_RESIDUAL else 0)
+        o.gemm_tc(a, w, out, err, epilogue=epilogue, residual=out if epilogue == o.EPI_RESIDUAL else None)
+        assert rel_err(out, want) < tol(dtype)
+        assert torch.equal(whole[:, :8], x0[:, :8].to(dtype)) and torch.equal(whole[:, 8 + N:], x0[:, 8 + N:].to(dtype))
+
+
 @pytest.mark.parametrize("M,N,K", [(128, 64, 64), (200, 200, 96), (2048, 1536, 576), (33, 130, 40), (64, 520, 1024), (40, 1536, 2048)])
 def test_gemm_tc_swiglu(M, N, K):
     o = ops()
