@@ -331,11 +331,85 @@ __device__ __forceinline__ void epilogue_rope_tile(uint32_t taddr, const RopeApp
   }
 }
 
+// The blocks of a tile that share K: each holds raw sums [weight][128][SHARE_PITCH] in its shared memory, and block z of n
+// adds all blocks' sums of its pieces of four columns, in the blocks' order, and finishes them.  (The sums went through
+// global memory to a second kernel before, launched after them: 64 rows, weights from memory, N 6144, K 2048 16.4 -> 10.0 us; N 2048,
+// K 2048 8.2 -> 6.8, K 8192 14.6 -> 13.1.)
+constexpr int MAX_SHARES = 4;              // blocks of a cluster
+template <int BN>
+constexpr int SHARE_PITCH = BN + 4;        // (a thread lays down a row: eight rows' pieces of 16 bytes fall on all banks)
+
+__device__ __forceinline__ void cluster_barrier() {
+  asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
+}
+
+__device__ __forceinline__ float4 add_shares(uint32_t addr, int n) {
+  float4 v[MAX_SHARES];
+#pragma unroll
+  for (int z = 0; z < MAX_SHARES; ++z) {
+    if (z < n) {
+      uint32_t at;
+      asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(z));
+      asm volatile("ld.shared::cluster.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(v[z].x), "=f"(v[z].y), "=f"(v[z].z), "=f"(v[z].w) : "r"(at) : "memory");
+    }
+  }
+  float4 sum = v[0];
+#pragma unroll
+  for (int z = 1; z < MAX_SHARES; ++z)
+    if (z < n) sum = make_float4(sum.x + v[z].x, sum.y + v[z].y, sum.z + v[z].z, sum.w + v[z].w);
+  return sum;
+}
+
+template <int EPI, typename TOut, int BN>
+__device__ __forceinline__ void finish_shares(uint32_t sums, int n, int z, TOut* out, int ldo, const float* residual, int m0, int n0, int M, int N,
+                                              int vec_ok, const RopeAppend& form) {
+  constexpr int PER_ROW = BN / 4;
+  const int total = min(TC_BM, M - m0) * PER_ROW;
+  for (int p = z * TC_THREADS + threadIdx.x; p < total; p += n * TC_THREADS) {
+    const int r = p / PER_ROW, c = p % PER_ROW * 4, col = n0 + c;
+    if (col >= N) continue;
+    const size_t at = (size_t)(m0 + r) * ldo + col;
+    const bool whole = vec_ok && col + 4 <= N;
+    const int left = min(4, N - col);
+    float res[4] = {};
+    if constexpr (EPI == TC_EPI_RESIDUAL) {
+      if (whole) *reinterpret_cast<float4*>(res) = *reinterpret_cast<const float4*>(residual + at);
+      else for (int j = 0; j < left; ++j) res[j] = residual[at + j];
+    }
+    const uint32_t mine = sums + (uint32_t)(r * SHARE_PITCH<BN> + c) * 4;
+    const float4 a = add_shares(mine, n);
+    float4 b = a;
+    if constexpr (EPI == TC_EPI_SWIGLU) b = add_shares(mine + TC_BM * SHARE_PITCH<BN> * 4, n);
+    const float va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
+    float v[4];
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      if (EPI == TC_EPI_SWIGLU) {
+        const bool biased = form.glu_bias != nullptr && j < left;
+        v[j] = glu_tc(va[j] + (biased ? form.glu_bias[col + j] : 0.f), vb[j] + (biased ? form.glu_bias[N + col + j] : 0.f), form.glu_limit, form.glu_alpha,
+                      form.glu_shift);
+      } else if (EPI == TC_EPI_RESIDUAL) v[j] = res[j] + va[j];
+      else if (form.square_relu) v[j] = fmaxf(va[j], 0.f) * fmaxf(va[j], 0.f);
+      else v[j] = va[j];
+    }
+    if (whole) {
+      if constexpr (sizeof(TOut) == 4) {
+        *reinterpret_cast<float4*>(out + at) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+        __align__(8) TOut o[4] = {from_f32<TOut>(v[0]), from_f32<TOut>(v[1]), from_f32<TOut>(v[2]), from_f32<TOut>(v[3])};
+        *reinterpret_cast<uint2*>(out + at) = *reinterpret_cast<const uint2*>(o);
+      }
+    } else {
+      for (int j = 0; j < left; ++j) out[at + j] = from_f32<TOut>(v[j]);
+    }
+  }
+}
+
 template <int BN, int EPI, typename TOut, int STAGES, bool BY_TMA>
 __global__ void __launch_bounds__(TC_THREADS)
 gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b,
                const __grid_constant__ CUtensorMap map_b2, TOut* out, int ldo, const float* residual,
-               int M, int N, int K, int vec_ok, int* err, int k_splits, float* partial, const RopeAppend rope,
+               int M, int N, int K, int vec_ok, int* err, int k_splits, const RopeAppend rope,
                const GroupedTiles grp, const __grid_constant__ OutTiles<BY_TMA> out_tiles) {
   // a grouped product is launched without programmatic dependence: the kernel that wrote `tile_group` is complete
   int w_row0 = blockIdx.x * BN;           // the first row of the weight tile (its output columns start at n0)
@@ -344,10 +418,9 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     if (group < 0) return;                // (the whole block, before it holds anything)
     w_row0 += group * grp.rows_per_group;
   }
-  // k_splits > 1: block z of the grid accumulates its share of K only and leaves the raw sums in
-  // `partial` [split][weight][M][N] (float32); splitk_reduce_kernel adds the splits in their order and
-  // applies the epilogue.  For products of few tiles and long K (decoding 17 to 128 sequences), which
-  // would otherwise run on a handful of SMs.
+  // k_splits > 1: the blocks z of a tile are a cluster; each accumulates its share of K only and lays the raw sums into
+  // its shared memory, and after a barrier each finishes a share of the tile (`finish_shares`).  For products of few tiles
+  // and long K (decoding 17 to 128 sequences), which would otherwise run on a handful of SMs.
   constexpr int NB = EPI == TC_EPI_SWIGLU ? 2 : 1;
   constexpr int A_BYTES = TC_BM * TC_BK * 2, B_BYTES = BN * TC_BK * 2;
   constexpr int STAGE_BYTES = A_BYTES + NB * B_BYTES;
@@ -487,22 +560,15 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
         if (EPI == TC_EPI_RESIDUAL && k_splits == 1 && c0 + 32 < BN)   // the next piece's residual is on its way while this one is finished
           fetch_residual(ra[((c0 >> 5) + 1) & 1], residual, ldo, m0 + q * 32 + lane, n0 + c0 + 32, M, N, vec_ok);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (k_splits > 1) {   // raw sums of this share of K
-          const int row = m0 + q * 32 + lane;
-          if (row < M) {
+        if (k_splits > 1) {   // raw sums of this share of K (the ring is their room: the MMAs that read its last stage are done)
+          if (m0 + q * 32 + lane < M) {
 #pragma unroll
             for (int b = 0; b < NB; ++b) {
-              float* dst = partial + (((size_t)blockIdx.z * NB + b) * M + row) * N + n0 + c0;
+              float4* dst = reinterpret_cast<float4*>(smem) + ((b * TC_BM + q * 32 + lane) * SHARE_PITCH<BN> + c0) / 4;
               const uint32_t* src = b == 0 ? r : r2;
-              if (n0 + c0 + 32 <= N && N % 4 == 0) {
 #pragma unroll
-                for (int j = 0; j < 32; j += 4)
-                  *reinterpret_cast<float4*>(dst + j) = make_float4(__uint_as_float(src[j]), __uint_as_float(src[j + 1]), __uint_as_float(src[j + 2]), __uint_as_float(src[j + 3]));
-              } else {
-#pragma unroll
-                for (int j = 0; j < 32; ++j)
-                  if (n0 + c0 + j < N) dst[j] = __uint_as_float(src[j]);
-              }
+              for (int j = 0; j < 8; ++j)
+                dst[j] = make_float4(__uint_as_float(src[4 * j]), __uint_as_float(src[4 * j + 1]), __uint_as_float(src[4 * j + 2]), __uint_as_float(src[4 * j + 3]));
             }
           }
           continue;
@@ -513,30 +579,17 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
+  if constexpr (!BY_TMA && EPI != TC_EPI_ROPE) {
+    static_assert(NB * TC_BM * SHARE_PITCH<BN> * 4 <= STAGES * STAGE_BYTES, "a block's sums fit into its ring");
+    if (k_splits > 1) {
+      cluster_barrier();
+      finish_shares<EPI, TOut, BN>(smem_u32(smem), k_splits, blockIdx.z, out, ldo, residual, m0, n0, M, N, vec_ok, rope);
+      cluster_barrier();   // (no block leaves while another reads its sums)
+    }
+  }
   if (warp == 1) {
     asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_base), "r"(TMEM_COLS) : "memory");
-  }
-}
-
-// out = epilogue(sum over the splits, in their order, of the raw sums a split-K launch left).
-template <int EPI, typename TOut>
-__global__ void splitk_reduce_kernel(const float* __restrict__ partial, int splits, TOut* out, int ldo, const float* residual,
-                                     int M, int N, float glu_limit, float glu_alpha, float glu_shift, const float* __restrict__ glu_bias, int square_relu) {
-  constexpr int NB = EPI == TC_EPI_SWIGLU ? 2 : 1;
-  const size_t plane = (size_t)M * N;
-  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < plane; i += (size_t)gridDim.x * blockDim.x) {
-    float a = 0.f, b = 0.f;
-    for (int z = 0; z < splits; ++z) {
-      a += partial[(size_t)z * NB * plane + i];
-      if (NB == 2) b += partial[((size_t)z * NB + 1) * plane + i];
-    }
-    const int m = (int)(i / N), n = (int)(i - (size_t)m * N);
-    const size_t o = (size_t)m * ldo + n;
-    if (EPI == TC_EPI_SWIGLU) out[o] = from_f32<TOut>(glu_tc(a + (glu_bias ? glu_bias[n] : 0.f), b + (glu_bias ? glu_bias[N + n] : 0.f), glu_limit, glu_alpha, glu_shift));
-    else if (EPI == TC_EPI_RESIDUAL) out[o] = from_f32<TOut>(residual[o] + a);
-    else if (square_relu) out[o] = from_f32<TOut>(fmaxf(a, 0.f) * fmaxf(a, 0.f));
-    else out[o] = from_f32<TOut>(a);
   }
 }
 
@@ -705,26 +758,19 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // persistent kernel with narrow tiles starves on shared-memory bandwidth: 0.68 to 0.78).  Forced for comparisons.
 static int g_tc_auto = 1, g_tc_persistent = 1, g_tc_wide = 1, g_tc_narrow = 1, g_tc_deep = 1, g_tc_tiny = 1, g_tc_out = 1;
 
-// Scratch for split-K launches (set by the caller once; nothing is allocated here): without it no product is split.
-static float* g_splitk_ws = nullptr;
-static size_t g_splitk_bytes = 0;
-static int g_splitk_on = 1;
-static int g_last_launches = 1;   // kernels the last edgelm_gemm_tc call launched (2 when it split K)
 // Which kernel the last edgelm_gemm_tc call took: tile columns | persistent << 12 | deep ring << 13 | K splits << 16.
 // Tests read it so that a product meant for one kernel cannot pass on another.
 static int g_last_kernel = 0;
 
-// Splits of K for a product of `tiles` one-tile blocks and `n_k` K blocks of 64: none unless the tiles would leave
-// more than half of the SMs idle and K is at least 1,024 (below that the second kernel costs more than the idle
-// SMs: measured at 64 rows, N 960, K 576: 6.1 us whole against 7.7 us split); then enough splits for about one and
-// a half blocks an SM, at least four K blocks each, within the scratch.  Measured at 64 rows: N 2048, K 8192:
-// 60.9 -> 15.5 us; N 2048, K 2048: 16.9 -> 8.5 us; N 576, K 1536: 12.9 -> 9.2 us.
-static int splitk_for(int tiles, int n_k, size_t bytes_per_split) {
-  if (!g_splitk_on || g_splitk_ws == nullptr || tiles >= 74 || n_k < 16) return 1;
-  int s = (222 + tiles - 1) / tiles;
-  if (s > n_k / 4) s = n_k / 4;
-  while (s > 1 && (size_t)s * bytes_per_split > g_splitk_bytes) --s;
-  if (s < 2) return 1;
+// Splits of K for a product of `tiles` one-tile blocks and `n_k` K blocks of 64: four, of at least four K blocks each, if the tiles are a
+// third of the SMs at most and K is at least 1,024.  Whole and in four, 64 rows: N 6144 (48 tiles), K 2048 11.0 and 10.0 us; N 4096 10.4 and
+// 8.8; N 2048 11.8 and 6.8; 1,000 rows of N 576, K 1536 (72 tiles) 7.9 and 12.7.  In eight, one block an SM, clusters find room for 120
+// blocks only: N 2048, K 8192 in 16 x 8 blocks 20 us, two an SM with short rings 13.7, 16 x 4 blocks with deep rings 13.1.
+static int g_splitk_most = MAX_SHARES;
+constexpr int SPLIT_TILES = 48, SPLIT_DEEP = 120;   // (blocks of a split product that have the deep ring: N 960, K 2560 9.3 -> 7.3 us)
+static int splitk_for(int tiles, int n_k) {
+  if (tiles > SPLIT_TILES || n_k < 16 || g_splitk_most < 2) return 1;
+  const int s = n_k / 4 < g_splitk_most ? n_k / 4 : g_splitk_most;
   const int k_per = (n_k + s - 1) / s;
   return (n_k + k_per - 1) / k_per;   // every split gets a share
 }
@@ -765,7 +811,6 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
     }
     const int tiles = ((N + BN - 1) / BN) * ((M + TC_BM - 1) / TC_BM);
     const int grid = tiles < n_sms ? tiles : n_sms;
-    g_last_launches = 1;
     g_last_kernel = BN | (1 << 12) | (1 << 16);
     cudaError_t le = launch_pdl(32, kern, dim3(grid), dim3(TC_THREADS), (size_t)smem, stream, ma, mb, mb2, (TOut*)out, ldo, residual, M, N, K,
                                 vec_ok, err, rope, mo.map, mo.how);
@@ -778,10 +823,9 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
   constexpr int STAGE_BYTES = TC_BM * TC_BK * 2 + NB * BN * TC_BK * 2;
   constexpr int DEEP = TC_DEEP_BYTES / STAGE_BYTES;   // 6 stages of 32 KB, 8 of 24 KB
   dim3 grid((N + BN - 1) / BN, (M + TC_BM - 1) / TC_BM);
-  // (the rotation epilogue is not one the reduce kernel of split products knows: such a product stays whole)
-  const int splits = (EPI == TC_EPI_ROPE || grp.tile_group != nullptr) ? 1 : splitk_for((int)(grid.x * grid.y), (K + TC_BK - 1) / TC_BK, (size_t)NB * M * N * sizeof(float));
+  // (the rotation epilogue is not one that `finish_shares` knows: such a product stays whole)
+  const int splits = (EPI == TC_EPI_ROPE || grp.tile_group != nullptr) ? 1 : splitk_for((int)(grid.x * grid.y), (K + TC_BK - 1) / TC_BK);
   grid.z = splits;
-  g_last_launches = splits > 1 ? 2 : 1;
   // a grid of at most one block an SM has the shared memory to itself: a deeper ring hides more of the loads' latency
   // (a short K is a few loads behind one another: 9 of them at K 576)
   static int n_sms = 0;
@@ -790,7 +834,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
     cudaGetDevice(&dev);
     cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
   }
-  const bool deep = g_tc_deep && (long long)grid.x * grid.y * grid.z <= n_sms;
+  const bool deep = g_tc_deep && (long long)grid.x * grid.y * grid.z <= (splits > 1 ? SPLIT_DEEP : n_sms);
   g_last_kernel = BN | ((deep ? 1 : 0) << 13) | (splits << 16);
   auto go = [&](auto kern, int smem, const auto& out_tiles) -> int {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
@@ -798,8 +842,23 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
       set_error("gemm_tc: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
       return -2;
     }
-    cudaError_t le = launch_pdl(grp.tile_group != nullptr ? 0 : 8, kern, grid, dim3(TC_THREADS), (size_t)smem, stream, ma, mb, mb2, (TOut*)out, ldo,
-                                residual, M, N, K, vec_ok, err, splits, g_splitk_ws, rope, grp, out_tiles);
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = dim3(TC_THREADS);
+    cfg.dynamicSmemBytes = (size_t)smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr[2];
+    cfg.attrs = attr;
+    if (grp.tile_group == nullptr && (pdl_enabled() & 8)) {
+      attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+      attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+    }
+    if (splits > 1) {
+      attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+      attr[cfg.numAttrs].val.clusterDim.x = attr[cfg.numAttrs].val.clusterDim.y = 1;
+      attr[cfg.numAttrs++].val.clusterDim.z = (unsigned)splits;
+    }
+    cudaError_t le = cudaLaunchKernelEx(&cfg, kern, ma, mb, mb2, (TOut*)out, ldo, residual, M, N, K, vec_ok, err, splits, rope, grp, out_tiles);
     if (le != cudaSuccess) {
       set_error("gemm_tc: launch failed: %s", cudaGetErrorString(le));
       return -2;
@@ -807,21 +866,13 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
     return 0;
   };
   const int deep_smem = DEEP * STAGE_BYTES + 1024 + 256, smem = TC_STAGES * STAGE_BYTES + 1024 + 256;
-  int rc;
   if constexpr (CAN_TMA) {
-    if (mo.how != TC_OUT_DIRECT && splits == 1) {   // (the shares of a split product are raw sums in the scratch)
+    if (mo.how != TC_OUT_DIRECT && splits == 1) {   // (a split product's tiles are finished by several blocks)
       return deep ? go(gemm_tc_kernel<BN, EPI, TOut, DEEP, true>, deep_smem, mo) : go(gemm_tc_kernel<BN, EPI, TOut, TC_STAGES, true>, smem, mo);
     }
   }
-  rc = deep ? go(gemm_tc_kernel<BN, EPI, TOut, DEEP, false>, deep_smem, OutTiles<false>{})
-            : go(gemm_tc_kernel<BN, EPI, TOut, TC_STAGES, false>, smem, OutTiles<false>{});
-  if (rc) return rc;
-  if (EPI != TC_EPI_ROPE && splits > 1) {
-    const size_t plane = (size_t)M * N;
-    const int blocks = (int)((plane + 255) / 256 < 1184 ? (plane + 255) / 256 : 1184);
-    splitk_reduce_kernel<EPI, TOut><<<blocks, 256, 0, stream>>>(g_splitk_ws, splits, (TOut*)out, ldo, residual, M, N, rope.glu_limit, rope.glu_alpha, rope.glu_shift, rope.glu_bias, rope.square_relu);
-  }
-  return 0;
+  return deep ? go(gemm_tc_kernel<BN, EPI, TOut, DEEP, false>, deep_smem, OutTiles<false>{})
+              : go(gemm_tc_kernel<BN, EPI, TOut, TC_STAGES, false>, smem, OutTiles<false>{});
 }
 
 }  // namespace edgelm
@@ -840,12 +891,9 @@ extern "C" int edgelm_gemm_tc_persistent(int on) {
   return 0;
 }
 
-// Float32 scratch for split-K launches (raw sums of every split); the library only keeps the pointer.  bytes 0: none.
-// `on` 0 switches splitting off (comparisons).
-extern "C" int edgelm_gemm_tc_splitk(float* scratch, size_t bytes, int on) {
-  g_splitk_ws = bytes ? scratch : nullptr;
-  g_splitk_bytes = bytes;
-  g_splitk_on = on;
+// The most blocks that share a tile's K (1: never split; comparisons)
+extern "C" int edgelm_gemm_tc_splitk(int most) {
+  g_splitk_most = most < 1 ? 1 : most > MAX_SHARES ? MAX_SHARES : most;
   return 0;
 }
 
@@ -868,7 +916,6 @@ extern "C" int edgelm_gemm_tc_narrow(int on) {
   return 0;
 }
 
-extern "C" int edgelm_gemm_tc_last_launches() { return g_last_launches; }
 extern "C" int edgelm_gemm_tc_last_kernel() { return g_last_kernel; }
 
 // 1 if the tensor-core kernel takes these operands (alignment and pitch rules of TMA), else 0.

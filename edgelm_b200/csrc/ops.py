@@ -211,25 +211,10 @@ def gemm_tc_takes(a, w, out, w2=None):
     return bool(lib().edgelm_gemm_tc_takes(_p(a), a.stride(0), _p(w), _p(w2), a.shape[1]))
 
 
-SPLITK_SCRATCH_BYTES = 32 << 20
-_splitk_scratch = None
-
-
-def _splitk_ready():
-    """The scratch that lets products of few tiles and long K spread over the device (split-K): allocated once, at
-    the first product outside of a graph capture, and handed to the library."""
-    global _splitk_scratch
-    if _splitk_scratch is None and not torch.cuda.is_current_stream_capturing():
-        _splitk_scratch = torch.empty(SPLITK_SCRATCH_BYTES // 4, dtype=torch.float32, device="cuda")
-        lib().edgelm_gemm_tc_splitk.argtypes = [ctypes.c_void_p, ctypes.c_size_t, ctypes.c_int]
-        lib().edgelm_gemm_tc_splitk(_p(_splitk_scratch), SPLITK_SCRATCH_BYTES, 1)
-
-
 def gemm_tc(a, w, out, err, epilogue=EPI_STORE, w2=None, residual=None, glu=None, glu_bias=None):
     """out = a @ w.T (+ epilogue) on the tcgen05 tensor cores: bfloat16 operands, float32 accumulation.  `glu` (limit, alpha,
     shift) with the gated epilogue: out = g sigmoid(alpha g) (v + shift), g = min(a @ w.T, limit), v = clamp(a @ w2.T, -limit, limit)
     (limit 0: no clamps); `glu_bias` [2 N] float32: the two branches' biases, added before the unit."""
-    _splitk_ready()
     _need(a.dim() == 2 and w.dim() == 2 and out.dim() == 2, "gemm_tc: 2-D operands")
     M, K = a.shape
     N = w.shape[0]
@@ -248,7 +233,7 @@ def gemm_tc(a, w, out, err, epilogue=EPI_STORE, w2=None, residual=None, glu=None
     else:
         _check(lib().edgelm_gemm_tc(_p(a), a.stride(0), _p(w), _p(w2), _p(out), out.stride(0), _p(residual), M, N, K, _dt(out),
                                     epilogue, _p(err), _stream()), launches=0)
-    count_launches(lib().edgelm_gemm_tc_last_launches())
+    count_launches(1)
 
 
 def gemm_tc_rope_takes(a, w, qkv, kcache, vcache, cos, sin, hd):
@@ -265,7 +250,6 @@ def gemm_tc_rope(a, w, qkv, tok_pos, tok_seq, seq_slot, page_table, cos, sin, kc
     """The stacked q, k, v projection of a prompt step with rotation and cache append in its epilogue:
     qkv[:, :nh hd] = rotated query heads of a @ w.T; the rotated keys and the values go to each token's place in the
     cache pages.  The k and v columns of `qkv` are left as they were."""
-    _splitk_ready()
     M, K = a.shape
     _need(w.shape == ((nh + 2 * nkv) * hd, K) and qkv.shape == (M, (nh + 2 * nkv) * hd), "gemm_tc_rope: shapes")
     _need(gemm_tc_rope_takes(a, w, qkv, kcache, vcache, cos, sin, hd), "gemm_tc_rope: these operands are not taken (bfloat16, head size 64 or 128, aligned)")
@@ -277,7 +261,7 @@ def gemm_tc_rope(a, w, qkv, tok_pos, tok_seq, seq_slot, page_table, cos, sin, kc
     _check(lib().edgelm_gemm_tc_rope(_p(a), a.stride(0), _p(w), _p(qkv), qkv.stride(0), M, K, _p(tok_pos), _p(tok_seq), _p(seq_slot),
                                      _p(page_table), page_table.stride(0), kcache.shape[0], _p(cos), _p(sin), cos.shape[0],
                                      _p(kcache), _p(vcache), nh, nkv, hd, _p(err), _stream()), launches=0)
-    count_launches(lib().edgelm_gemm_tc_last_launches())
+    count_launches(1)
 
 
 def gemm_tc_last_kernel():

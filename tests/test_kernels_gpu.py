@@ -654,6 +654,36 @@ def test_gemm_tc_dispatch_names_its_kernel():
     assert k["k_splits"] > 1, k   # 64 rows, N 2048, K 8192: sixteen tiles, split over K
 
 
+@pytest.mark.parametrize("M,N,K", [(17, 576, 1536), (64, 2048, 2048), (33, 1030, 1032), (128, 3100, 1992), (300, 570, 1544), (640, 570, 8192)])
+def test_gemm_tc_shared_k_in_clusters(M, N, K):
+    """Few tiles and a long K: the blocks of a tile add their shares in shared memory.  Ragged rows, columns (also no whole pieces of four)
+    and K, a last share that is shorter, rows wider than the product; every epilogue beside float64 and the float32 ones beside the whole product."""
+    o = ops()
+    a, w, w2 = rnd((M, K), torch.bfloat16, 80), rnd((N, K), torch.bfloat16, 81, 0.05), rnd((N, K), torch.bfloat16, 82, 0.05)
+    err, x0, bias = torch.zeros(1, dtype=torch.int32, device=dev()), rnd((M + 1, N + 6), torch.float32, 83), rnd((2 * N,), torch.float32, 84)
+    g, u = a.double() @ w.double().T, a.double() @ w2.double().T
+    x = x0[:M, 4:4 + N].double()
+    gb, ub = g + bias[:N].double(), u + bias[N:].double()
+    for dtype, epilogue, glu_bias, want in ((torch.float32, o.EPI_STORE, None, g), (torch.bfloat16, o.EPI_STORE, None, g), (torch.float32, o.EPI_RESIDUAL, None, x + g),
+                                            (torch.float32, o.EPI_RELU2, None, g.clamp(min=0) ** 2), (torch.bfloat16, o.EPI_SWIGLU, None, g / (1 + torch.exp(-g)) * u),
+                                            (torch.bfloat16, o.EPI_SWIGLU, bias, gb / (1 + torch.exp(-gb)) * ub)):
+        outs = []
+        try:
+            for most in (4, 1):
+                o.lib().edgelm_gemm_tc_splitk(most)
+                whole = x0.to(dtype, copy=True)
+                out = whole[:M, 4:4 + N]
+                o.gemm_tc(a, w, out, err, epilogue=epilogue, w2=w2 if epilogue == o.EPI_SWIGLU else None, residual=out if epilogue == o.EPI_RESIDUAL else None, glu_bias=glu_bias)
+                assert (o.gemm_tc_last_kernel()["k_splits"] > 1) == (most > 1) or epilogue == o.EPI_SWIGLU   # (two weights: tiles half as wide)
+                outs.append(whole)
+        finally:
+            o.lib().edgelm_gemm_tc_splitk(4)
+        assert int(err.item()) == 0
+        tol_ = 1.6e-2 if dtype == torch.bfloat16 else 2e-5
+        assert rel_err(outs[0][:M, 4:4 + N], want.cpu()) < tol_ and rel_err(outs[0], outs[1]) < tol_
+        assert torch.equal(outs[0][M:], x0[M:].to(dtype)) and torch.equal(outs[0][:, :4], x0[:, :4].to(dtype)) and torch.equal(outs[0][:, 4 + N:], x0[:, 4 + N:].to(dtype))
+
+
 @pytest.mark.parametrize("M,N,K", [(17, 576, 576), (64, 960, 576), (128, 1536, 576), (64, 576, 1536), (33, 100, 200), (64, 4704, 96),
                                      (100, 2040, 2048)])
 def test_gemm_tc_tiles_of_32_columns_when_all_rows_are_one_tile(M, N, K):
