@@ -762,15 +762,17 @@ static int g_tc_auto = 1, g_tc_persistent = 1, g_tc_wide = 1, g_tc_narrow = 1, g
 // Tests read it so that a product meant for one kernel cannot pass on another.
 static int g_last_kernel = 0;
 
-// Splits of K for a product of `tiles` one-tile blocks and `n_k` K blocks of 64: four, of at least four K blocks each, if the tiles are a
-// third of the SMs at most and K is at least 1,024.  Whole and in four, 64 rows: N 6144 (48 tiles), K 2048 11.0 and 10.0 us; N 4096 10.4 and
-// 8.8; N 2048 11.8 and 6.8; 1,000 rows of N 576, K 1536 (72 tiles) 7.9 and 12.7.  In eight, one block an SM, clusters find room for 120
-// blocks only: N 2048, K 8192 in 16 x 8 blocks 20 us, two an SM with short rings 13.7, 16 x 4 blocks with deep rings 13.1.
+// Splits of K for a product of `tiles` one-tile blocks and `n_k` K blocks of 64: four, of at least four K blocks each, if the tiles are
+// half of the SMs at most and K is at least 1,024; three from 65 tiles on (clusters of four find no room for all).  Whole and in four, 64
+// rows: N 2048 (16 tiles), K 2048 11.8 and 6.8 us; N 6144 (48), K 2048 11.0 and 10.0; 200 rows, N 2048 (64), K 2048 9.9 and 8.4, K 8192
+// 31.0 and 18.2; 1,000 rows, N 576 (72), K 8192 whole, in three and in four 30.5, 20.3 and 27.3, K 1536 7.9, 8.0 and 12.6.  In eight, one
+// block an SM, clusters find room for 120 blocks only: N 2048, K 8192 in 16 x 8 blocks 20 us, two an SM with short rings 13.7, 16 x 4 blocks
+// with deep rings 13.1.
 static int g_splitk_most = MAX_SHARES;
-constexpr int SPLIT_TILES = 48, SPLIT_DEEP = 120;   // (blocks of a split product that have the deep ring: N 960, K 2560 9.3 -> 7.3 us)
+constexpr int SPLIT_TILES = 74, SPLIT_DEEP = 120;   // (blocks of a split product that have the deep ring: N 960, K 2560 9.3 -> 7.3 us)
 static int splitk_for(int tiles, int n_k) {
   if (tiles > SPLIT_TILES || n_k < 16 || g_splitk_most < 2) return 1;
-  const int s = n_k / 4 < g_splitk_most ? n_k / 4 : g_splitk_most;
+  const int room = tiles > 64 && g_splitk_most > 3 ? 3 : g_splitk_most, s = n_k / 4 < room ? n_k / 4 : room;
   const int k_per = (n_k + s - 1) / s;
   return (n_k + k_per - 1) / k_per;   // every split gets a share
 }

@@ -654,7 +654,8 @@ def test_gemm_tc_dispatch_names_its_kernel():
     assert k["k_splits"] > 1, k   # 64 rows, N 2048, K 8192: sixteen tiles, split over K
 
 
-@pytest.mark.parametrize("M,N,K", [(17, 576, 1536), (64, 2048, 2048), (33, 1030, 1032), (128, 3100, 1992), (300, 570, 1544), (640, 570, 8192)])
+@pytest.mark.parametrize("M,N,K", [(17, 576, 1536), (64, 2048, 2048), (33, 1030, 1032), (128, 3100, 1992), (300, 570, 1544), (640, 570, 8192),
+                                     (250, 2048, 1032), (1000, 576, 1032)])
 def test_gemm_tc_shared_k_in_clusters(M, N, K):
     """Few tiles and a long K: the blocks of a tile add their shares in shared memory.  Ragged rows, columns (also no whole pieces of four)
     and K, a last share that is shorter, rows wider than the product; every epilogue beside float64 and the float32 ones beside the whole product."""
