@@ -127,7 +127,7 @@ conv_rows_kernel(const float* __restrict__ u, int ldu, int off, const float* __r
           const int r = k - 3 + j, row = taps - 1 + r;
 #pragma unroll
           for (int q = 0; q < 4; ++q)
-            past[j][q] = r >= 0 ? u[(size_t)(t - k + r) * ldu + off + c + q] + ib[q] : (row >= 0 ? tail[(size_t)row * C + c + q] : 0.f);
+            past[j][q] = j < 4 - taps ? 0.f : r >= 0 ? u[(size_t)(t - k + r) * ldu + off + c + q] + ib[q] : (row >= 0 ? tail[(size_t)row * C + c + q] : 0.f);
         }
       }
       const float now[4] = {in[x].x + ib[0], in[x].y + ib[1], in[x].z + ib[2], in[x].w + ib[3]};
@@ -136,9 +136,9 @@ conv_rows_kernel(const float* __restrict__ u, int ldu, int off, const float* __r
       for (int q = 0; q < 4; ++q) {
         const float acc = fmaf(wt[3][q], now[q], fmaf(wt[2][q], past[2][q], fmaf(wt[1][q], past[1][q], fmaf(wt[0][q], past[0][q], bias[q]))));
         y[q] = act ? silu_exact(acc) : acc;
-        past[0][q] = past[1][q];
-        past[1][q] = past[2][q];
-        past[2][q] = now[q];
+        past[0][q] = taps > 3 ? past[1][q] : 0.f;      // (inputs in front of the filter count as zeros: 0 times an infinity is none)
+        past[1][q] = taps > 2 ? past[2][q] : 0.f;
+        past[2][q] = taps > 1 ? now[q] : 0.f;
       }
       *reinterpret_cast<float4*>(out + (size_t)t * C + c) = make_float4(y[0], y[1], y[2], y[3]);
     }

@@ -94,7 +94,7 @@ rotate_rows_kernel(const RotateRows a, TQ* __restrict__ q_out, T* __restrict__ k
           const int r = k - 3 + j, row = a.taps - 1 + r;
 #pragma unroll
           for (int m = 0; m < M; ++m)
-            past[m][j] = r >= 0 ? a.qkv[(size_t)(t0 + x - k + r) * a.ldq + ch0 + 32 * m] + ib[m]
+            past[m][j] = j < 4 - a.taps ? 0.f : r >= 0 ? a.qkv[(size_t)(t0 + x - k + r) * a.ldq + ch0 + 32 * m] + ib[m]
                                 : (row >= 0 ? tail[(size_t)row * C + ch0 + 32 * m] : 0.f);
         }
       }
@@ -102,9 +102,9 @@ rotate_rows_kernel(const RotateRows a, TQ* __restrict__ q_out, T* __restrict__ k
       for (int m = 0; m < M; ++m) {
         const float now = in[x][m];
         in[x][m] = fmaf(w[m][3], now, fmaf(w[m][2], past[m][2], fmaf(w[m][1], past[m][1], w[m][0] * past[m][0])));
-        past[m][0] = past[m][1];
-        past[m][1] = past[m][2];
-        past[m][2] = now;
+        past[m][0] = a.taps > 3 ? past[m][1] : 0.f;      // (inputs in front of the filter count as zeros: 0 times an infinity is none)
+        past[m][1] = a.taps > 2 ? past[m][2] : 0.f;
+        past[m][2] = a.taps > 1 ? now : 0.f;
       }
     }
   }

@@ -379,6 +379,26 @@ def test_rotation_and_append_of_many_tokens(H, G, dk, dv, maps, rot, inter, norm
             t0 += n
 
 
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+def test_filter_inside_rotation_reads_no_token_in_front_of_its_taps(taps):
+    """Steps of more than 64 tokens: an infinity in a value channel and a NaN in a query and a key channel reach `taps` tokens each."""
+    g = torch.Generator().manual_seed(taps)
+    T, H, G, d = 130, 2, 1, 32
+    C, bad = (H + G) * d + G * d, {20: 100, 61: 3, 90: 70}      # (token: channel of the value, of query head 0, of the key)
+    x, w = torch.randn(T, C, generator=g), torch.randn(C, taps, generator=g) + 2.0
+    for (t, c), value in zip(bad.items(), (float("inf"), float("nan"), float("nan"))):
+        x[t, c] = value
+    kc, vc = (torch.zeros(3, G, PAGE, d, device=DEV) for _ in range(2))
+    q, err, tail = torch.empty(T, H * d, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV), torch.zeros(1, taps - 1, C, device=DEV)
+    ops.rotate_append(x.to(DEV), None, q, i32(torch.arange(T)), i32(torch.zeros(T)), i32([[0, 1, 2]]), kc, vc, H, G, d, d, 0, False, None, err, conv_w=w.to(DEV),
+                      conv_state=tail if taps > 1 else None, seq_tok0=i32([0, T]), seq_slot=i32([0]), n_seqs=1)
+    got = torch.cat([q] + [c.view(-1, d)[:T] for c in (kc, vc)], 1).isfinite().cpu()
+    want = torch.ones(T, C, dtype=torch.bool)
+    for t, c in bad.items():
+        want[t:t + taps, c] = False
+    assert int(err.item()) == 0 and torch.equal(got, want)
+
+
 def test_tensor_core_attention_keeps_float32_scores_and_weights():
     """Queries so large that their rounding to bfloat16 would move the scores by a good part of 1, and values of very
     different sizes under weights of very different sizes: the kernel's output follows the float64 attention of the float32

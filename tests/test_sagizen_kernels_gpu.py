@@ -171,6 +171,29 @@ def test_filter_over_many_tokens(C, taps, bias, act):
             assert np.allclose(state[slots[s]].cpu().numpy(), full[-(taps - 1):], atol=1e-6)
 
 
+@pytest.mark.parametrize("taps", [1, 2, 3, 4])
+@pytest.mark.parametrize("cut", [0, 21, 23])
+def test_filter_reads_no_token_in_front_of_its_taps(taps, cut):
+    """An infinity and a NaN reach `taps` tokens each, in one step and where the step is cut behind the infinity."""
+    g = np.random.default_rng(taps)
+    T, C, bad = 180, 64, {20: np.inf, 99: np.nan}
+    u, w = g.normal(size=(T, C)), g.normal(size=(C, taps)) + 2.0
+    for t, value in bad.items():
+        u[t, 5] = value
+    state, got = torch.zeros(1, taps - 1, C, device=DEV), []
+    for a, e in ((0, cut), (cut, T)):
+        if a == e:
+            continue
+        tok0, tok_seq = packed([e - a])
+        y = torch.empty(e - a, C, device=DEV)
+        ops.conv_act(f32(u[a:e]), 0, f32(w), None, state, y, tok_seq, tok0, i32([0]), 1)
+        got.append(y.isfinite().cpu().numpy())
+    want = np.ones((T, C), bool)
+    for t in bad:
+        want[t:t + taps, 5] = False
+    assert (np.concatenate(got) == want).all()
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("gs,groups", [(4, 3), (64, 5), (128, 2), (100, 3), (576, 1), (1028, 2), (4096, 1), (8192, 1), (8200, 1), (66, 2)])
 def test_gated_group_norm_of_many_rows(gs, groups, dtype):
