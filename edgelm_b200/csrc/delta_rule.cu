@@ -203,7 +203,8 @@ __device__ __forceinline__ void dc_logs(double* lg, const float* __restrict__ bg
 #pragma unroll
   for (int i = 0; i < 2; ++i) {
     const int t = 2 * threadIdx.x + i;
-    x[i] = t < ntok ? fmax(log((double)bg[(size_t)(tok0 + t) * 2 * H + H + h]), -200.0) : 0.0;
+    const double z = t < ntok ? log((double)bg[(size_t)(tok0 + t) * 2 * H + H + h]) : 0.0;
+    x[i] = z < -200.0 ? -200.0 : z;        // (a NaN stays one)
   }
   double sum = x[0] + x[1];
 #pragma unroll

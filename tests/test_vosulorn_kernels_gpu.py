@@ -147,6 +147,36 @@ def test_delta_rule_chunk_by_chunk(H, G, d, e):
 
 
 
+DELTA_NOT_FINITE = {"decay": ("decay", (slice(None), 2), np.nan)}
+
+
+@pytest.mark.parametrize("what", DELTA_NOT_FINITE)
+def test_delta_rule_chunks_are_finite_where_the_walk_is(what):
+    """... and agree with it there (2e-5: the bound of the walk beside float64)."""
+    g = np.random.default_rng(5)
+    lengths, H, G, d, e = [20, 150], 3, 1, 32, 20
+    T = sum(lengths)
+    unit = lambda x: x / np.sqrt((x * x).sum(-1, keepdims=True))
+    c = {"q": unit(g.normal(size=(T, G, d))), "k": unit(g.normal(size=(T, G, d))), "v": g.normal(size=(T, H, e)), "beta": g.uniform(0.1, 1, (T, H)),
+         "decay": np.exp(-np.exp(g.uniform(-5, 0, (T, H))))}
+    name, at, value = DELTA_NOT_FINITE[what]
+    c[name][at] = value
+    qkv, bg = (f32(np.concatenate([c[k].reshape(T, -1) for k in ks], 1)) for ks in ("qkv", ("beta", "decay")))
+    tok0, (_, ttok0, tntok, _, count) = packed(lengths)[0], make_tiles(lengths, [0, 0], ops.DELTA_CHUNK)
+    outs = []
+    for chunked in (True, False):
+        state, o = torch.zeros(2, H, e, d, device=DEV), torch.full((T, H * e), float("nan"), device=DEV)
+        args = (qkv, bg, state, o, tok0, i32([1, 0]), 2)
+        if chunked:
+            ops.delta_chunked(*args, ttok0, tntok, count, H, G, d, e)
+        else:
+            ops.delta_scan(*args, H, G, d, e)
+        outs.append((o.isfinite(), state.isfinite(), o.nan_to_num(0, 0, 0)))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert float((outs[0][2] - outs[1][2]).abs().max()) < 2e-5 * float(outs[1][2].abs().max())
+
+
+
 # ----------------------------------------------------------------------------- attention with a key range and a sink
 class PagedKV:
     """Keys and values of a few sequences in pages handed out in a scrambled order, the rest poisoned."""
