@@ -62,7 +62,8 @@ __device__ __forceinline__ void ssm_logs(double* lg, float* dts, const float* __
     const float z = t < ntok ? raw[(size_t)(tok0 + t) * ldu] + bias : 0.f;
     const float dt = t < ntok ? log1pf(expf(-fabsf(z))) + fmaxf(z, 0.f) : 0.f;
     dts[t] = dt;
-    x[i] = rate * dt;
+    const double l = t < ntok ? rate * dt : 0.0;
+    x[i] = l < -200.0 ? -200.0 : l;      // (a decay that is zero in float32: sums and differences stay finite; a NaN stays one)
   }
   double sum = x[0] + x[1];
 #pragma unroll

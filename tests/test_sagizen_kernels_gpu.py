@@ -258,6 +258,35 @@ def test_state_space_chunk_by_chunk(H, G, N, P):
     assert bool((states[0][1] == 7).all() and (states[0][4] == 7).all())
 
 
+NOT_FINITE = {"rate": ("A_log", (1,), 100.0), "rate_nan": ("A_log", (1,), np.nan), "bias_nan": ("dt_bias", (2,), np.nan), "step": ("raw", (58, 1), np.inf)}
+
+
+@pytest.mark.parametrize("what", NOT_FINITE)
+def test_state_space_chunks_are_finite_where_the_walk_is(what):
+    """... and agree with it there (2e-5: the bound of the walk beside float64)."""
+    from edgelm_b200.engine.batch import make_tiles
+    g = np.random.default_rng(3)
+    lengths, H, G, N, P = [20, 150], 3, 1, 16, 8
+    T = sum(lengths)
+    c = {"x": g.normal(size=(T, H, P)), "B": g.normal(size=(T, G, N)), "C": g.normal(size=(T, G, N)), "raw": g.normal(-3, 1, size=(T, H)),
+         "A_log": g.uniform(-1, 1, H), "dt_bias": g.normal(size=H)}
+    name, at, value = NOT_FINITE[what]
+    c[name][at] = value
+    xbc, tok0 = f32(np.concatenate([c[k].reshape(T, -1) for k in ("x", "B", "C")], 1)), packed(lengths)[0]
+    _, ttok0, tntok, _ = make_tiles(lengths, [0, 0], ops.STATE_CHUNK)
+    outs = []
+    for chunked in (True, False):
+        state, y = torch.zeros(2, H, P, N, device=DEV), torch.full((T, H * P), float("nan"), device=DEV)
+        args = (xbc, f32(c["raw"]), 0, f32(c["dt_bias"]), f32(c["A_log"]), f32(np.ones(H)), state, y, tok0, i32([1, 0]), 2)
+        if chunked:
+            ops.ssm_chunked(*args, i32(ttok0), i32(tntok), len(ttok0), H, G, N, P)
+        else:
+            ops.ssm_scan(*args, H, G, N, P)
+        outs.append((y.isfinite(), state.isfinite(), y.nan_to_num(0, 0, 0)))
+    assert torch.equal(outs[0][0], outs[1][0]) and torch.equal(outs[0][1], outs[1][1])
+    assert float((outs[0][2] - outs[1][2]).abs().max()) < 2e-5 * float(outs[1][2].abs().max())
+
+
 @pytest.mark.parametrize("H,K", [(3, 64), (2, 20), (1, 4), (2, 36)])
 def test_time_mix_chunk_by_chunk(H, K):
     """As above for a decay per key channel, down to zero: 64 terms of the walk, K of the product, in each output."""
