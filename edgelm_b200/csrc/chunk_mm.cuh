@@ -49,6 +49,31 @@ __device__ __forceinline__ void chunk_mm(float (&acc)[RM][RN], const float* A, i
     for (int b = 0; b < RN; ++b) acc[a][b] += __uint_as_float((uint32_t)sum[a][b]) + __uint_as_float((uint32_t)(sum[a][b] >> 32));
 }
 
+// The logarithms of a chunk's decays: lg[t] = l_0 + .. + l_t, lane i of the calling warp bringing tokens 2 i and 2 i + 1.  No token's
+// sum holds a later one's value, so that what is not finite stays at its token and behind.
+__device__ __forceinline__ void chunk_log_sums(double* lg, double l0, double l1) {
+  const int lane = threadIdx.x & 31;
+  double sum = l0 + l1;
+#pragma unroll
+  for (int off = 1; off < 32; off <<= 1) {
+    const double up = __shfl_up_sync(0xffffffffu, sum, off);
+    if (lane >= off) sum += up;
+  }
+  const double before = __shfl_up_sync(0xffffffffu, sum, 1);
+  lg[2 * lane] = lane == 0 ? l0 : before + l0;
+  lg[2 * lane + 1] = sum;
+}
+
+// An output that a product over all tokens of the chunk left not finite, over its own and the earlier ones alone: first . second + sum over
+// s <= t of weights[s] values[s].  (A weight of zero times a later token's infinity is a NaN, where the walk has not met that token.)
+__device__ __forceinline__ float chunk_causal(const float* first, const float* second, int K, float scale, const float* weights, const float* values, int t) {
+  float v = 0.f;
+  for (int k = 0; k < K; ++k) v = fmaf(first[k], second[k], v);
+  v *= scale;
+  for (int s = 0; s <= t; ++s) v = fmaf(weights[s], values[s], v);
+  return v;
+}
+
 __device__ __forceinline__ void chunk_cp16(float* dst, const float* src, bool there) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
 }

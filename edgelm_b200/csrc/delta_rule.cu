@@ -206,14 +206,7 @@ __device__ __forceinline__ void dc_logs(double* lg, const float* __restrict__ bg
     const double z = t < ntok ? log((double)bg[(size_t)(tok0 + t) * 2 * H + H + h]) : 0.0;
     x[i] = z < -200.0 ? -200.0 : z;        // (a NaN stays one)
   }
-  double sum = x[0] + x[1];
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const double up = __shfl_up_sync(0xffffffffu, sum, off);
-    if (threadIdx.x >= off) sum += up;
-  }
-  lg[2 * threadIdx.x] = sum - x[1];
-  lg[2 * threadIdx.x + 1] = sum;
+  chunk_log_sums(lg, x[0], x[1]);
 }
 
 __global__ void __launch_bounds__(256)
@@ -428,13 +421,23 @@ delta_chunk_out_kernel(const float* __restrict__ qkv, int C, const float* __rest
     for (int b = 0; b < RN; ++b) acc[a][b] *= w;
   }
   chunk_mm<16, 4, RN>(acc, ms, AP, CHUNK, us, AP, e, CHUNK);
+  bool all_finite = true;
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int b = 0; b < RN; ++b) {
       const int t = ty + 16 * a, j = tx + 16 * b;
-      if (t < ntok && j < e) o[(size_t)(tok0 + t) * H * e + (size_t)h * e + j] = acc[a][b];
+      if (t >= ntok || j >= e) continue;
+      o[(size_t)(tok0 + t) * H * e + (size_t)h * e + j] = acc[a][b];
+      all_finite = all_finite && isfinite(acc[a][b]);
     }
+  if (all_finite) return;
+#pragma unroll 1
+  for (int i = 0; i < 4 * RN; ++i) {
+    const int t = ty + 16 * (i / RN), j = tx + 16 * (i % RN);
+    float* out = o + (size_t)(tok0 + t) * H * e + (size_t)h * e + j;
+    if (t < ntok && j < e && !isfinite(*out)) *out = chunk_causal(qs + t * P, ss + j * P, d, expf((float)lg[t]), ms + t * AP, us + j * AP, t);
+  }
 }
 
 }  // namespace edgelm

@@ -65,14 +65,7 @@ __device__ __forceinline__ void ssm_logs(double* lg, float* dts, const float* __
     const double l = t < ntok ? rate * dt : 0.0;
     x[i] = l < -200.0 ? -200.0 : l;      // (a decay that is zero in float32: sums and differences stay finite; a NaN stays one)
   }
-  double sum = x[0] + x[1];
-#pragma unroll
-  for (int off = 1; off < 32; off <<= 1) {
-    const double up = __shfl_up_sync(0xffffffffu, sum, off);
-    if (threadIdx.x >= off) sum += up;
-  }
-  lg[2 * threadIdx.x] = sum - x[1];
-  lg[2 * threadIdx.x + 1] = sum;
+  chunk_log_sums(lg, x[0], x[1]);
 }
 
 constexpr int SC_PITCH = CHUNK + 4;
@@ -209,13 +202,25 @@ ssm_chunk_out_kernel(const float* __restrict__ xbc, int C, int inner, const floa
   }
   chunk_mm<16, 4, 4>(acc, ms, SC_PITCH, CHUNK, xt, SC_PITCH, P, CHUNK);
   const float D = Dp[h];
+  bool all_finite = true;
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int t = chunk_ty() + 16 * a, p = chunk_tx() + 16 * b;
-      if (t < ntok && p < P) y[(size_t)(tok0 + t) * H * P + (size_t)h * P + p] = acc[a][b] + D * xt[p * SC_PITCH + t];
+      if (t >= ntok || p >= P) continue;
+      const float v = acc[a][b] + D * xt[p * SC_PITCH + t];
+      y[(size_t)(tok0 + t) * H * P + (size_t)h * P + p] = v;
+      all_finite = all_finite && isfinite(v);
     }
+  if (all_finite) return;
+#pragma unroll 1
+  for (int i = 0; i < 16; ++i) {
+    const int t = chunk_ty() + 16 * (i >> 2), p = chunk_tx() + 16 * (i & 3);
+    float* out = y + (size_t)(tok0 + t) * H * P + (size_t)h * P + p;
+    if (t < ntok && p < P && !isfinite(*out))
+      *out = chunk_causal(cs + t * NP, ss + p * NP, N, expf((float)lg[t]), ms + t * SC_PITCH, xt + p * SC_PITCH, t) + D * xt[p * SC_PITCH + t];
+  }
 }
 
 // ------------------------------------------------------------------ a decay per key channel

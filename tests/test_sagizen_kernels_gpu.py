@@ -258,7 +258,9 @@ def test_state_space_chunk_by_chunk(H, G, N, P):
     assert bool((states[0][1] == 7).all() and (states[0][4] == 7).all())
 
 
-NOT_FINITE = {"rate": ("A_log", (1,), 100.0), "rate_nan": ("A_log", (1,), np.nan), "bias_nan": ("dt_bias", (2,), np.nan), "step": ("raw", (58, 1), np.inf)}
+NOT_FINITE = {"rate": ("A_log", (1,), 100.0), "rate_nan": ("A_log", (1,), np.nan), "bias_nan": ("dt_bias", (2,), np.nan), "step": ("raw", (58, 1), np.inf),
+              "step_nan": ("raw", (57, 1), np.nan), "x": ("x", (57, 1, 3), np.inf), "x_nan": ("x", (30, 0, 7), np.nan), "B": ("B", (57, 0, 2), -np.inf),
+              "C": ("C", (57, 0, 2), np.nan)}
 
 
 @pytest.mark.parametrize("what", NOT_FINITE)

@@ -146,8 +146,9 @@ def test_delta_rule_chunk_by_chunk(H, G, d, e):
     assert bool((states[0][1] == 7).all() and (states[0][4] == 7).all())
 
 
-
-DELTA_NOT_FINITE = {"decay": ("decay", (slice(None), 2), np.nan)}
+DELTA_NOT_FINITE = {"decay": ("decay", (slice(None), 2), np.nan), "decay_even": ("decay", (30, 1), np.nan), "decay_odd": ("decay", (57, 1), np.nan),
+                    "beta": ("beta", (57, 0), np.nan), "q": ("q", (57, 0, 3), np.inf), "k": ("k", (57, 0, 3), np.inf), "k_first": ("k", (20, 0, 3), np.nan),
+                    "v": ("v", (57, 1, 5), np.inf), "v_nan": ("v", (30, 2, 19), np.nan)}
 
 
 @pytest.mark.parametrize("what", DELTA_NOT_FINITE)
