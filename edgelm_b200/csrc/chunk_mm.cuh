@@ -74,6 +74,42 @@ __device__ __forceinline__ float chunk_causal(const float* first, const float* s
   return v;
 }
 
+// acc[a][b] = the same sum in runs of eight products, which join in double.  (For products whose error travels on or whose terms largely
+// cancel: scores between a chunk's tokens.  With sums as in `chunk_mm` they alone put the delta rule's and the state-space outputs further
+// from float64 than a walk over the tokens is.)
+template <int NY, int RM, int RN>
+__device__ __forceinline__ void chunk_mm_runs(double (&acc)[RM][RN], const float* A, int pa, int M, const float* B, int pb, int N, int K) {
+  const int tx = chunk_tx(), ty = chunk_ty();
+#pragma unroll
+  for (int a = 0; a < RM; ++a)
+#pragma unroll
+    for (int b = 0; b < RN; ++b) acc[a][b] = 0.0;
+#pragma unroll 1
+  for (int k0 = 0; k0 < K; k0 += 8) {
+    unsigned long long sum[RM][RN] = {};
+#pragma unroll
+    for (int k = k0; k < k0 + 8; k += 4) {
+      if (k >= K) break;
+      ulonglong2 av[RM];
+#pragma unroll
+      for (int a = 0; a < RM; ++a) av[a] = *reinterpret_cast<const ulonglong2*>(A + min(ty + NY * a, M - 1) * pa + k);
+#pragma unroll
+      for (int b = 0; b < RN; ++b) {
+        const ulonglong2 bv = *reinterpret_cast<const ulonglong2*>(B + min(tx + 16 * b, N - 1) * pb + k);
+#pragma unroll
+        for (int a = 0; a < RM; ++a) {
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[a][b]) : "l"(av[a].x), "l"(bv.x));
+          asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(sum[a][b]) : "l"(av[a].y), "l"(bv.y));
+        }
+      }
+    }
+#pragma unroll
+    for (int a = 0; a < RM; ++a)
+#pragma unroll
+      for (int b = 0; b < RN; ++b) acc[a][b] += (double)(__uint_as_float((uint32_t)sum[a][b]) + __uint_as_float((uint32_t)(sum[a][b] >> 32)));
+  }
+}
+
 __device__ __forceinline__ void chunk_cp16(float* dst, const float* src, bool there) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((unsigned)__cvta_generic_to_shared(dst)), "l"(src), "r"(there ? 16 : 0) : "memory");
 }

@@ -187,12 +187,15 @@ delta_scan_kernel(const float* __restrict__ qkv, int C, const float* __restrict_
 //      substitution, a thread a column with its 64 values in registers;
 //   2. `delta_chunk_states`, the chunks of a (sequence, head) in order, blocks of 16 value channels: U = U0 - W S0, then S;
 //   3. `delta_chunk_out`, every (chunk, head) at once: the outputs from U and the kept S0.
-// Logarithms and their sums are kept in double precision (a decay that is zero in float32 counts as exp(-200)), everything else is float32.
+// Logarithms, their sums and exponentials and the substitution are double (a decay that is zero in float32 counts as exp(-200)), scores join
+// runs of eight float32 products in double, everything else is float32.  (All but the logarithms in float32: outputs 1.7 to 2.2 times as far
+// from float64 as the walk's.)
 // One (chunk, head) of the scratch: U0, later U, [e][64]; W [64][d]; the keys times exp(L_n - L_s) [d][64]; S0 [e][d].  Then exp(L_n) of each.
-// Bound by the substitution and the products out of shared memory.  Nine heads of 64, prompts of 333 to
-// 1,700 tokens (4,065 in all): the walk 548 us, this 195 (49 + 106 + 40).
+// Nine heads of 64, prompts of 333 to 1,700 tokens (4,065 in all): the walk 548 us, this 232 (77 + 106 + 49; all but the logarithms in
+// float32 195).
 constexpr int DC_BLOCK = 16;       // value channels a block of `delta_chunk_states` owns
 constexpr int DC_STATE_THREADS = 128;
+constexpr int DC_SOLVE_PITCH = CHUNK + 2;
 
 __host__ __device__ inline size_t dc_floats(int d, int e) { return (size_t)(2 * CHUNK) * d + (size_t)CHUNK * e + (size_t)d * e; }
 
@@ -209,17 +212,19 @@ __device__ __forceinline__ void dc_logs(double* lg, const float* __restrict__ bg
   chunk_log_sums(lg, x[0], x[1]);
 }
 
-__global__ void __launch_bounds__(256)
+// NT 128 threads where the columns fit (two blocks an SM: a thread's 64 doubles are half of its registers), else 256
+template <int NT>
+__global__ void __launch_bounds__(NT)
 delta_chunk_solve_kernel(const float* __restrict__ qkv, int C, const float* __restrict__ bg, float* __restrict__ scratch,
                          float* __restrict__ full, const int32_t* __restrict__ tile_tok0, const int32_t* __restrict__ tile_ntok, int H, int G,
                          int d, int e) {
   extern __shared__ __align__(16) float dc_smem[];
-  __shared__ double lg[CHUNK];
+  __shared__ double lg[CHUNK], to_start[CHUNK], to_end[CHUNK];      // L_t, exp(L_t), exp(L_n - L_t)
   __shared__ float beta[CHUNK];
+  constexpr int AP = DC_SOLVE_PITCH, NY = NT / 16, RM = CHUNK / NY;
   const int P = chunk_pitch(d);
-  float* ks = dc_smem;                       // [CHUNK][P]
-  float* at = ks + CHUNK * P;                // [s][t]: A[t][s]
-  constexpr int AP = CHUNK + 4;
+  double* at = reinterpret_cast<double*>(dc_smem);       // [s][t]: A[t][s]
+  float* ks = reinterpret_cast<float*>(at + CHUNK * AP); // [CHUNK][P]
   const int tile = blockIdx.x, h = blockIdx.y, g = h / (H / G), tok0 = tile_tok0[tile], ntok = tile_ntok[tile];
   chunk_rows(ks, P, qkv + (size_t)tok0 * C + G * d + g * d, C, CHUNK, ntok, d);
   asm volatile("cp.async.commit_group;" ::: "memory");
@@ -230,23 +235,25 @@ delta_chunk_solve_kernel(const float* __restrict__ qkv, int C, const float* __re
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
+  if (threadIdx.x < CHUNK) to_start[threadIdx.x] = exp(lg[threadIdx.x]);
+  else if (threadIdx.x < 2 * CHUNK) to_end[threadIdx.x - CHUNK] = exp(lg[CHUNK - 1] - lg[threadIdx.x - CHUNK]);
   {
-    float acc[4][4] = {};
-    chunk_mm<16, 4, 4>(acc, ks, P, CHUNK, ks, P, CHUNK, d);
+    double acc[RM][4];
+    chunk_mm_runs<NY, RM, 4>(acc, ks, P, CHUNK, ks, P, CHUNK, d);
 #pragma unroll
-    for (int a = 0; a < 4; ++a)
+    for (int a = 0; a < RM; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
-        const int s = chunk_ty() + 16 * a, t = chunk_tx() + 16 * b;
-        at[s * AP + t] = s < t ? beta[t] * expf((float)(lg[t] - lg[s])) * acc[a][b] : 0.f;
+        const int s = chunk_ty() + NY * a, t = chunk_tx() + 16 * b;
+        at[s * AP + t] = s < t ? (double)beta[t] * exp(lg[t] - lg[s]) * acc[a][b] : 0.0;
       }
   }
   __syncthreads();
   const int c = threadIdx.x;
   float* base = scratch + ((size_t)tile * H + h) * dc_floats(d, e);
-  if (c == 0) full[(size_t)tile * H + h] = expf((float)lg[CHUNK - 1]);
+  if (c == 0) full[(size_t)tile * H + h] = (float)to_start[CHUNK - 1];
   if (c >= d + e) return;
-  float x[CHUNK];
+  double x[CHUNK];
   if (c < e) {
     const float* v = qkv + (size_t)tok0 * C + 2 * G * d + (size_t)h * e + c;
 #pragma unroll
@@ -255,33 +262,34 @@ delta_chunk_solve_kernel(const float* __restrict__ qkv, int C, const float* __re
     for (int t = 0; t < CHUNK; ++t) x[t] *= beta[t];
   } else {
     float* kt = base + (size_t)CHUNK * e + (size_t)CHUNK * d + (size_t)(c - e) * CHUNK;
-    const double last = lg[CHUNK - 1];
 #pragma unroll
-    for (int t = 0; t < CHUNK; ++t) x[t] = ks[t * P + c - e];
+    for (int t = 0; t < CHUNK; t += 4) {
+      float k[4], out[4];
 #pragma unroll
-    for (int t = 0; t < CHUNK; t += 4)
-      *reinterpret_cast<float4*>(kt + t) = make_float4(x[t] * expf((float)(last - lg[t])), x[t + 1] * expf((float)(last - lg[t + 1])),
-                                                       x[t + 2] * expf((float)(last - lg[t + 2])), x[t + 3] * expf((float)(last - lg[t + 3])));
-#pragma unroll
-    for (int t = 0; t < CHUNK; ++t) x[t] *= beta[t] * expf((float)lg[t]);
+      for (int i = 0; i < 4; ++i) {
+        k[i] = ks[(t + i) * P + c - e];
+        out[i] = (float)(k[i] * to_end[t + i]);
+        x[t + i] = k[i] * (beta[t + i] * to_start[t + i]);
+      }
+      *reinterpret_cast<float4*>(kt + t) = make_float4(out[0], out[1], out[2], out[3]);
+    }
   }
 #pragma unroll
   for (int s = 0; s < CHUNK - 1; ++s) {
 #pragma unroll
-    for (int t = (s + 1) & ~3; t < CHUNK; t += 4) {      // (at [s][t] is zero up to t = s)
-      const float4 a = *reinterpret_cast<const float4*>(at + s * AP + t);
-      if (t > s) x[t] = fmaf(-a.x, x[s], x[t]);
-      if (t + 1 > s) x[t + 1] = fmaf(-a.y, x[s], x[t + 1]);
-      if (t + 2 > s) x[t + 2] = fmaf(-a.z, x[s], x[t + 2]);
-      x[t + 3] = fmaf(-a.w, x[s], x[t + 3]);
+    for (int t = (s + 1) & ~1; t < CHUNK; t += 2) {      // (at [s][t] is zero up to t = s)
+      const double2 a = *reinterpret_cast<const double2*>(at + s * AP + t);
+      if (t > s) x[t] = fma(-a.x, x[s], x[t]);
+      x[t + 1] = fma(-a.y, x[s], x[t + 1]);
     }
   }
   if (c < e) {
 #pragma unroll
-    for (int t = 0; t < CHUNK; t += 4) *reinterpret_cast<float4*>(base + (size_t)c * CHUNK + t) = make_float4(x[t], x[t + 1], x[t + 2], x[t + 3]);
+    for (int t = 0; t < CHUNK; t += 4)
+      *reinterpret_cast<float4*>(base + (size_t)c * CHUNK + t) = make_float4((float)x[t], (float)x[t + 1], (float)x[t + 2], (float)x[t + 3]);
   } else {
 #pragma unroll
-    for (int t = 0; t < CHUNK; ++t) base[(size_t)CHUNK * e + (size_t)t * d + c - e] = x[t];
+    for (int t = 0; t < CHUNK; ++t) base[(size_t)CHUNK * e + (size_t)t * d + c - e] = (float)x[t];
   }
 }
 
@@ -400,14 +408,14 @@ delta_chunk_out_kernel(const float* __restrict__ qkv, int C, const float* __rest
   __syncthreads();
   const int tx = chunk_tx(), ty = chunk_ty();
   {
-    float acc[4][4] = {};
-    chunk_mm<16, 4, 4>(acc, qs, P, CHUNK, ks, P, CHUNK, d);
+    double acc[4][4];
+    chunk_mm_runs<16, 4, 4>(acc, qs, P, CHUNK, ks, P, CHUNK, d);
 #pragma unroll
     for (int a = 0; a < 4; ++a)
 #pragma unroll
       for (int b = 0; b < 4; ++b) {
         const int t = ty + 16 * a, s = tx + 16 * b;
-        ms[t * AP + s] = s <= t ? expf((float)(lg[t] - lg[s])) * acc[a][b] : 0.f;
+        ms[t * AP + s] = s <= t ? (float)(exp(lg[t] - lg[s]) * acc[a][b]) : 0.f;
       }
   }
   asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -416,7 +424,7 @@ delta_chunk_out_kernel(const float* __restrict__ qkv, int C, const float* __rest
   chunk_mm<16, 4, RN>(acc, qs, P, CHUNK, ss, P, e, d);
 #pragma unroll
   for (int a = 0; a < 4; ++a) {
-    const float w = expf((float)lg[ty + 16 * a]);
+    const float w = (float)exp(lg[ty + 16 * a]);
 #pragma unroll
     for (int b = 0; b < RN; ++b) acc[a][b] *= w;
   }
@@ -436,7 +444,7 @@ delta_chunk_out_kernel(const float* __restrict__ qkv, int C, const float* __rest
   for (int i = 0; i < 4 * RN; ++i) {
     const int t = ty + 16 * (i / RN), j = tx + 16 * (i % RN);
     float* out = o + (size_t)(tok0 + t) * H * e + (size_t)h * e + j;
-    if (t < ntok && j < e && !isfinite(*out)) *out = chunk_causal(qs + t * P, ss + j * P, d, expf((float)lg[t]), ms + t * AP, us + j * AP, t);
+    if (t < ntok && j < e && !isfinite(*out)) *out = chunk_causal(qs + t * P, ss + j * P, d, (float)exp(lg[t]), ms + t * AP, us + j * AP, t);
   }
 }
 
@@ -509,16 +517,17 @@ extern "C" int edgelm_delta_chunked(const float* qkv, int C, const float* bg, fl
   EL_REFUSE(scratch != nullptr && (uintptr_t)scratch % 16 == 0 && (uintptr_t)qkv % 16 == 0, "delta_chunked: rows and scratch must be 16-byte aligned");
   const int P = chunk_pitch(d), AP = CHUNK + 4;
   float* full = scratch + (size_t)n_tiles * H * dc_floats(d, e);
-  const size_t smem1 = (size_t)(CHUNK * P + CHUNK * AP) * 4;
+  const size_t smem1 = (size_t)CHUNK * DC_SOLVE_PITCH * 8 + (size_t)CHUNK * P * 4;
+  auto k1 = d + e <= 128 ? delta_chunk_solve_kernel<128> : delta_chunk_solve_kernel<256>;
   const size_t smem2 = (size_t)(2 * (CHUNK * P + d * AP + DC_BLOCK * CHUNK) + DC_BLOCK * P + DC_BLOCK * AP) * 4;
   const size_t smem3 = (size_t)(2 * CHUNK * P + e * P + e * AP + CHUNK * AP) * 4;
   auto k2 = d <= 64 ? delta_chunk_states_kernel<4> : delta_chunk_states_kernel<8>;
   auto k3 = e <= 64 ? delta_chunk_out_kernel<4> : delta_chunk_out_kernel<8>;
-  cudaError_t err = cudaFuncSetAttribute(delta_chunk_solve_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
+  cudaError_t err = cudaFuncSetAttribute(k1, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem1);
   if (err == cudaSuccess) err = cudaFuncSetAttribute(k2, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem2);
   if (err == cudaSuccess) err = cudaFuncSetAttribute(k3, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem3);
   EL_REFUSE(err == cudaSuccess, "delta_chunked: shared memory refused: %s", cudaGetErrorString(err));
-  delta_chunk_solve_kernel<<<dim3(n_tiles, H), 256, smem1, stream>>>(qkv, C, bg, scratch, full, tile_tok0, tile_ntok, H, G, d, e);
+  k1<<<dim3(n_tiles, H), d + e <= 128 ? 128 : 256, smem1, stream>>>(qkv, C, bg, scratch, full, tile_tok0, tile_ntok, H, G, d, e);
   EL_LAUNCH_CHECK("delta_chunk_solve");
   k2<<<dim3(n_seqs * H, (e + DC_BLOCK - 1) / DC_BLOCK), DC_STATE_THREADS, smem2, stream>>>(scratch, full, state, seq_tok0, seq_slot, H, d, e);
   EL_LAUNCH_CHECK("delta_chunk_states");
