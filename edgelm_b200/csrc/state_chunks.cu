@@ -1,7 +1,7 @@
 // Prompt steps of the state mixers chunk by chunk: the step's tokens come as tiles of at most CHUNK consecutive tokens of one sequence,
 // in the order of the sequences, every sequence cut from its first row of the step.  The walks of recurrent.cu take a token after the
 // other (0.27 us each); here everything but a multiply-add per state element and chunk runs for all chunks at once.  States, decays,
-// step sizes and sums are float32, logarithms of decays double.
+// step sizes and sums are float32, logarithms of decays double; scores join runs of eight float32 products in double.
 //
 // Selective state-space recurrence (S <- a_t S + dt_t B_t x_t^T, y_t = S^T C_t + D x_t, a_t = exp(-exp(A_log) dt_t)), with L_t the sum of
 // log a up to token t of the chunk and S0 the state before it:
@@ -85,12 +85,12 @@ ssm_chunk_scores_kernel(const float* __restrict__ xbc, int C, int inner, float* 
   asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
   float* out = shared_part + ((size_t)tile * G + g) * (CHUNK * CHUNK + (size_t)CHUNK * N);
-  float acc[4][4] = {};
-  chunk_mm<16, 4, 4>(acc, cs, P, CHUNK, bs, P, CHUNK, N);
+  double acc[4][4];
+  chunk_mm_runs<16, 4, 4>(acc, cs, P, CHUNK, bs, P, CHUNK, N);
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
-    for (int b = 0; b < 4; ++b) out[(chunk_ty() + 16 * a) * CHUNK + chunk_tx() + 16 * b] = acc[a][b];
+    for (int b = 0; b < 4; ++b) out[(chunk_ty() + 16 * a) * CHUNK + chunk_tx() + 16 * b] = (float)acc[a][b];
   out += CHUNK * CHUNK;
   for (int i = threadIdx.x; i < CHUNK * N; i += blockDim.x) out[i] = bs[(i % CHUNK) * P + i / CHUNK];
 }
