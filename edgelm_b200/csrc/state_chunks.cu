@@ -254,21 +254,24 @@ wkv_chunk_local_kernel(const float* __restrict__ r, const float* __restrict__ kk
     // the outputs' share of S0: r_t times the decays of the tokens before it, two halves of the chunk side by side
     const int i = threadIdx.x & 63, half = threadIdx.x >> 6, begin = half ? min(CHUNK / 2, ntok) : 0, end = half ? ntok : min(CHUNK / 2, ntok);
     if (i < K) {
-      float d = 1.f;
+      double d = 1.0;                        // (in float32 the product's roundings alone were a tenth of the outputs' error)
       for (int t = 0; t < begin; ++t) d *= ws[t * WK + i];
       float* out = faded + (((size_t)tile * H + h) * CHUNK) * K + i;
       for (int t = begin; t < end; ++t) {
-        out[(size_t)t * K] = rs[t * WK + i] * d;
+        out[(size_t)t * K] = (float)(rs[t * WK + i] * d);
         d *= ws[t * WK + i];
       }
-      if (half) keep[((size_t)tile * H + h) * K + i] = d;
+      if (half) keep[((size_t)tile * H + h) * K + i] = (float)d;
     }
   }
   {
     const int t = threadIdx.x >> 1, c0 = (threadIdx.x & 1) * (WK / 2);
-    float b = 0.f;
+    float part[8] = {};                      // (eight short runs: one of 32 was less exact than the walk's sums)
     if (t < ntok)
-      for (int c = c0; c < min(c0 + WK / 2, K); ++c) b = fmaf(bonus[h * K + c], rs[t * WK + c] * ks[t * WK + c], b);
+#pragma unroll
+      for (int c = 0; c < WK / 2; ++c)
+        if (c0 + c < K) part[c & 7] = fmaf(bonus[h * K + c0 + c], rs[t * WK + c0 + c] * ks[t * WK + c0 + c], part[c & 7]);
+    float b = ((part[0] + part[4]) + (part[1] + part[5])) + ((part[2] + part[6]) + (part[3] + part[7]));
     b += __shfl_xor_sync(0xffffffffu, b, 1);
     if ((threadIdx.x & 1) == 0) own[t] = b;
   }
@@ -326,14 +329,16 @@ wkv_chunk_out_kernel(const float* __restrict__ before, const float* __restrict__
   chunk_rows(ss, P, before + ((size_t)tile * H + h) * K * K, K, K, K, K);
   asm volatile("cp.async.commit_group;\n cp.async.wait_group 0;" ::: "memory");
   __syncthreads();
-  float acc[4][4] = {};
-  chunk_mm<16, 4, 4>(acc, fs, P, CHUNK, ss, P, K, K);
+  double acc[4][4];
+  chunk_mm_runs<16, 4, 4>(acc, fs, P, CHUNK, ss, P, K, K);
 #pragma unroll
   for (int a = 0; a < 4; ++a)
 #pragma unroll
     for (int b = 0; b < 4; ++b) {
       const int t = chunk_ty() + 16 * a, j = chunk_tx() + 16 * b;
-      if (t < ntok && j < K) o[(size_t)(tok0 + t) * H * K + (size_t)h * K + j] += acc[a][b];
+      if (t >= ntok || j >= K) continue;
+      float* out = o + (size_t)(tok0 + t) * H * K + (size_t)h * K + j;
+      *out = (float)(*out + acc[a][b]);
     }
 }
 
