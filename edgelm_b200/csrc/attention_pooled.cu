@@ -94,9 +94,10 @@ qk_rope_norm_append_kernel(const float* __restrict__ qkv, const float* __restric
   }
 }
 
-// The pooled rows of the blocks that end at a token of this step.  A block of threads looks at `run` consecutive tokens (POOL_RUN in prompt
-// steps), of which one in P ends a block.  (A block of threads a token: 2,048 tokens of 32 heads 86 us, most of it blocks that found nothing
-// to do; now 40.)
+// The pooled rows of the blocks that end at a token of this step.  A block of threads looks at `run` consecutive tokens, a lane a token; in
+// prompt steps as many as a block has, up to POOL_RUN, so that there is about one pooled row to a block of threads and few find nothing to
+// do.  (A token a block, 16 a block and so many: 2,048 tokens, 32 heads, blocks of 64 82, 37 and 29 us, blocks of 4 69, 32 and 25; two heads,
+// blocks of 4 5.6, 9.8 and 3.9; 65 tokens, blocks of 4 3.2, 9.4 and 3.3.)
 constexpr int POOL_RUN = 16;
 
 template <typename T>
@@ -106,9 +107,10 @@ __global__ void pool_blocks_kernel(const int32_t* __restrict__ tok_pos, const in
                                    float* __restrict__ pv, int G, int dk, int dv, int P, int R, int* __restrict__ err, int n_tokens, int run) {
   pdl_launch_dependents();
   pdl_wait();   // (launched as a programmatic dependent: nothing is read or written before the kernel ahead is done)
-  for (int t = blockIdx.x * run; t < min(n_tokens, (int)(blockIdx.x + 1) * run); ++t) {
-    const int pos = tok_pos[t];
-    if (pos < 0 || (pos + 1) % P != 0) continue;
+  const int t0 = blockIdx.x * run, lane = threadIdx.x & 31;
+  const int mine = lane < run && t0 + lane < n_tokens ? tok_pos[t0 + lane] : -1;
+  for (unsigned ends = __ballot_sync(0xffffffffu, mine >= 0 && (mine + 1) % P == 0); ends != 0; ends &= ends - 1) {
+    const int x = __ffs(ends) - 1, t = t0 + x, pos = __shfl_sync(0xffffffffu, mine, x);
     const int b = (pos + 1) / P - 1;
     const int32_t* table = page_table + (size_t)tok_seq[t] * table_stride;
     const int dst_page = table[pos / PAGE];
@@ -738,7 +740,9 @@ extern "C" int edgelm_pool_blocks(const int32_t* tok_pos, const int32_t* tok_seq
                                   int n_tokens, int G, int dk, int dv, int P, int R, int* err, cudaStream_t stream) {
   if (n_tokens == 0) return 0;
   EL_REFUSE(n_tokens > 0 && G > 0 && dk > 0 && dv > 0 && P >= 1 && R == (PAGE + P - 1) / P, "pool_blocks: bad sizes (block %d, rows a page %d)", P, R);
-  const int run = n_tokens > 64 ? POOL_RUN : 1, runs = (n_tokens + run - 1) / run;
+  // (blocks of few tokens: as long a run as leaves eight blocks of threads an SM)
+  const long long shared = (long long)n_tokens * G / (8 * 148);
+  const int want = P > shared ? P : (int)shared, run = n_tokens <= 64 ? 1 : want < POOL_RUN ? want : POOL_RUN, runs = (n_tokens + run - 1) / run;
   if (dtype == DT_F32)
     launch_pdl(pdl_bit_for_tokens(n_tokens), pool_blocks_kernel<float>, dim3(runs, G), dim3(128), (size_t)(0), stream, tok_pos, tok_seq, page_table, table_stride, n_pages, (const float*)kcache, (const float*)vcache, pk, pv, G, dk, dv, P, R, err, n_tokens, run);
   else if (dtype == DT_BF16)

@@ -439,6 +439,32 @@ def test_pooled_attention_on_the_tensor_cores(window, pool, d, H, G):
     assert int(err.item()) == 0
 
 
+@pytest.mark.parametrize("pool,G", [(1, 1), (1, 20), (3, 16), (7, 2), (16, 1), (64, 2), (100, 3)])
+def test_pooled_rows_of_many_tokens(pool, G):
+    """Runs of one token to sixteen a block, with none, one and several ends of blocks in a run; sequences that start inside a run, one of
+    them going on; a mean of 100 values in float32."""
+    g = torch.Generator().manual_seed(pool)
+    lengths, first, d = [170, 33, 97], [0, 5, 150], 20
+    pos, seq = (np.concatenate(x) for x in ([np.arange(a, a + n) for a, n in zip(first, lengths)], [np.full(n, s) for s, n in enumerate(lengths)]))
+    R = -(-64 // pool)
+    kc, vc = (torch.randn(8, G, 64, d, generator=g).to(DEV) for _ in range(2))
+    pk, pv = (torch.full((8, G, R, d), float("nan"), device=DEV) for _ in range(2))
+    table, err = i32([[5, 2, 7, -1], [0, -1, -1, -1], [6, 1, 3, 4]]), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.pool_blocks(i32(pos), i32(seq), table, kc, vc, pk, pv, len(pos), G, d, d, pool, err)
+    want = {}
+    for p, s in zip(pos, seq):
+        if (p + 1) % pool == 0:
+            b, rows = p // pool, [(int(table[s, j // 64]), j % 64) for j in range(p + 1 - pool, p + 1)]
+            want[(int(table[s, p // 64]), int(b - 64 * (p // 64) // pool))] = rows
+    for got, c in ((pk, kc.cpu()), (pv, vc.cpu())):
+        written = (~got.isnan()).all(-1).all(1).cpu()
+        assert sorted(map(tuple, written.nonzero().tolist())) == sorted(want)
+        for (page, row), rows in want.items():
+            mean = torch.stack([c[a, :, j].double() for a, j in rows]).mean(0)
+            assert float((got[page, :, row].cpu().double() - mean).abs().max()) < 1e-6
+    assert int(err.item()) == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 def test_rotation_bias_and_unit_norm(dtype):
     g = np.random.default_rng(9)
