@@ -335,7 +335,7 @@ __device__ __forceinline__ void epilogue_rope_tile(uint32_t taddr, const RopeApp
 // adds all blocks' sums of its pieces of four columns, in the blocks' order, and finishes them.  (The sums went through
 // global memory to a second kernel before, launched after them: 64 rows, weights from memory, N 6144, K 2048 16.4 -> 10.0 us; N 2048,
 // K 2048 8.2 -> 6.8, K 8192 14.6 -> 13.1.)
-constexpr int MAX_SHARES = 4;              // blocks of a cluster
+constexpr int MAX_SHARES = 8, FEW_SHARES = 4;      // blocks of a cluster; the most of those where tiles are many
 template <int BN>
 constexpr int SHARE_PITCH = BN + 4;        // (a thread lays down a row: eight rows' pieces of 16 bytes fall on all banks)
 
@@ -343,10 +343,11 @@ __device__ __forceinline__ void cluster_barrier() {
   asm volatile("barrier.cluster.arrive.release;\nbarrier.cluster.wait.acquire;" ::: "memory");
 }
 
+template <int MOST>
 __device__ __forceinline__ float4 add_shares(uint32_t addr, int n) {
-  float4 v[MAX_SHARES];
+  float4 v[MOST];
 #pragma unroll
-  for (int z = 0; z < MAX_SHARES; ++z) {
+  for (int z = 0; z < MOST; ++z) {
     if (z < n) {
       uint32_t at;
       asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(at) : "r"(addr), "r"(z));
@@ -355,12 +356,12 @@ __device__ __forceinline__ float4 add_shares(uint32_t addr, int n) {
   }
   float4 sum = v[0];
 #pragma unroll
-  for (int z = 1; z < MAX_SHARES; ++z)
+  for (int z = 1; z < MOST; ++z)
     if (z < n) sum = make_float4(sum.x + v[z].x, sum.y + v[z].y, sum.z + v[z].z, sum.w + v[z].w);
   return sum;
 }
 
-template <int EPI, typename TOut, int BN>
+template <int EPI, typename TOut, int BN, int MOST>
 __device__ __forceinline__ void finish_shares(uint32_t sums, int n, int z, TOut* out, int ldo, const float* residual, int m0, int n0, int M, int N,
                                               int vec_ok, const RopeAppend& form) {
   constexpr int PER_ROW = BN / 4;
@@ -377,9 +378,9 @@ __device__ __forceinline__ void finish_shares(uint32_t sums, int n, int z, TOut*
       else for (int j = 0; j < left; ++j) res[j] = residual[at + j];
     }
     const uint32_t mine = sums + (uint32_t)(r * SHARE_PITCH<BN> + c) * 4;
-    const float4 a = add_shares(mine, n);
+    const float4 a = add_shares<MOST>(mine, n);
     float4 b = a;
-    if constexpr (EPI == TC_EPI_SWIGLU) b = add_shares(mine + TC_BM * SHARE_PITCH<BN> * 4, n);
+    if constexpr (EPI == TC_EPI_SWIGLU) b = add_shares<MOST>(mine + TC_BM * SHARE_PITCH<BN> * 4, n);
     const float va[4] = {a.x, a.y, a.z, a.w}, vb[4] = {b.x, b.y, b.z, b.w};
     float v[4];
 #pragma unroll
@@ -583,7 +584,8 @@ gemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant_
     static_assert(NB * TC_BM * SHARE_PITCH<BN> * 4 <= STAGES * STAGE_BYTES, "a block's sums fit into its ring");
     if (k_splits > 1) {
       cluster_barrier();
-      finish_shares<EPI, TOut, BN>(smem_u32(smem), k_splits, blockIdx.z, out, ldo, residual, m0, n0, M, N, vec_ok, rope);
+      if (k_splits <= FEW_SHARES) finish_shares<EPI, TOut, BN, FEW_SHARES>(smem_u32(smem), k_splits, blockIdx.z, out, ldo, residual, m0, n0, M, N, vec_ok, rope);
+      else finish_shares<EPI, TOut, BN, MAX_SHARES>(smem_u32(smem), k_splits, blockIdx.z, out, ldo, residual, m0, n0, M, N, vec_ok, rope);
       cluster_barrier();   // (no block leaves while another reads its sums)
     }
   }
@@ -767,12 +769,16 @@ static int g_last_kernel = 0;
 // rows: N 2048 (16 tiles), K 2048 11.8 and 6.8 us; N 6144 (48), K 2048 11.0 and 10.0; 200 rows, N 2048 (64), K 2048 9.9 and 8.4, K 8192
 // 31.0 and 18.2; 1,000 rows, N 576 (72), K 8192 whole, in three and in four 30.5, 20.3 and 27.3, K 1536 7.9, 8.0 and 12.6.  In eight, one
 // block an SM, clusters find room for 120 blocks only: N 2048, K 8192 in 16 x 8 blocks 20 us, two an SM with short rings 13.7, 16 x 4 blocks
-// with deep rings 13.1.
+// with deep rings 13.1.  Up to 15 tiles, which leave room for it, eight, of at least eight K blocks each: 64 rows, N 64 (2 tiles), K 4096 6.5 us in
+// four and 5.0 in eight, K 8192 9.8 and 6.7; N 384, K 8192 10.2 and 7.4; 500 rows, N 128, K 8192 11.3 and 8.4.
 static int g_splitk_most = MAX_SHARES;
 constexpr int SPLIT_TILES = 74, SPLIT_DEEP = 120;   // (blocks of a split product that have the deep ring: N 960, K 2560 9.3 -> 7.3 us)
 static int splitk_for(int tiles, int n_k) {
   if (tiles > SPLIT_TILES || n_k < 16 || g_splitk_most < 2) return 1;
-  const int room = tiles > 64 && g_splitk_most > 3 ? 3 : g_splitk_most, s = n_k / 4 < room ? n_k / 4 : room;
+  int s = tiles > 64 ? 3 : FEW_SHARES;
+  if (s > n_k / 4) s = n_k / 4;
+  if (tiles <= SPLIT_DEEP / MAX_SHARES && s < n_k / 8) s = n_k / 8 < MAX_SHARES ? n_k / 8 : MAX_SHARES;
+  if (s > g_splitk_most) s = g_splitk_most;
   const int k_per = (n_k + s - 1) / s;
   return (n_k + k_per - 1) / k_per;   // every split gets a share
 }
@@ -893,7 +899,7 @@ extern "C" int edgelm_gemm_tc_persistent(int on) {
   return 0;
 }
 
-// The most blocks that share a tile's K (1: never split; comparisons)
+// The most blocks that share a tile's K (1: never split, 8: as the rule says; comparisons)
 extern "C" int edgelm_gemm_tc_splitk(int most) {
   g_splitk_most = most < 1 ? 1 : most > MAX_SHARES ? MAX_SHARES : most;
   return 0;

@@ -655,9 +655,9 @@ def test_gemm_tc_dispatch_names_its_kernel():
 
 
 @pytest.mark.parametrize("M,N,K", [(17, 576, 1536), (64, 2048, 2048), (33, 1030, 1032), (128, 3100, 1992), (300, 570, 1544), (640, 570, 8192),
-                                     (250, 2048, 1032), (1000, 576, 1032)])
+                                     (250, 2048, 1032), (1000, 576, 1032), (17, 64, 8192), (40, 200, 4104), (64, 390, 2056), (140, 130, 4552)])
 def test_gemm_tc_shared_k_in_clusters(M, N, K):
-    """Few tiles and a long K: the blocks of a tile add their shares in shared memory.  Ragged rows, columns (also no whole pieces of four)
+    """Few tiles and a long K: the blocks of a tile, up to four and up to eight, add their shares in shared memory.  Ragged rows, columns (also no whole pieces of four)
     and K, a last share that is shorter, rows wider than the product; every epilogue beside float64 and the float32 ones beside the whole product."""
     o = ops()
     a, w, w2 = rnd((M, K), torch.bfloat16, 80), rnd((N, K), torch.bfloat16, 81, 0.05), rnd((N, K), torch.bfloat16, 82, 0.05)
@@ -670,7 +670,7 @@ def test_gemm_tc_shared_k_in_clusters(M, N, K):
                                             (torch.bfloat16, o.EPI_SWIGLU, bias, gb / (1 + torch.exp(-gb)) * ub)):
         outs = []
         try:
-            for most in (4, 1):
+            for most in (8, 1):
                 o.lib().edgelm_gemm_tc_splitk(most)
                 whole = x0.to(dtype, copy=True)
                 out = whole[:M, 4:4 + N]
@@ -678,7 +678,7 @@ def test_gemm_tc_shared_k_in_clusters(M, N, K):
                 assert (o.gemm_tc_last_kernel()["k_splits"] > 1) == (most > 1) or epilogue == o.EPI_SWIGLU   # (two weights: tiles half as wide)
                 outs.append(whole)
         finally:
-            o.lib().edgelm_gemm_tc_splitk(4)
+            o.lib().edgelm_gemm_tc_splitk(8)
         assert int(err.item()) == 0
         tol_ = 1.6e-2 if dtype == torch.bfloat16 else 2e-5
         assert rel_err(outs[0][:M, 4:4 + N], want.cpu()) < tol_ and rel_err(outs[0], outs[1]) < tol_
