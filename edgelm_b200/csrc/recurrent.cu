@@ -94,6 +94,10 @@ __global__ void conv_silu_kernel(const float* __restrict__ u, int ldu, int off, 
 // rows and columns in whole pieces of 16 bytes.  Bound by memory: 2,048 tokens of 4,352 channels, four taps: a token a block 74 us, this
 // 26.
 constexpr int CONV_RUN = 16, CONV_THREADS = 128;
+// The blocks from which on it is ahead: sixteen tokens are a chain of 9 us (14 where each is a sequence of its own), whatever the step.
+// (A token a block against this, four taps: 768 channels, 1,024 tokens, 128 blocks 8.9 and 9.3 to 15.1 us; 2,048 tokens, 256 blocks 14.7
+// and 9.9 to 15.2; 4,352 channels, 512 tokens, 288 blocks 19.4 and 10.4 to 15.3.)
+constexpr int CONV_BLOCKS = 256;
 
 __global__ void __launch_bounds__(CONV_THREADS)
 conv_rows_kernel(const float* __restrict__ u, int ldu, int off, const float* __restrict__ w, const float* __restrict__ b,
@@ -748,8 +752,9 @@ extern "C" int edgelm_conv_act(const float* u, int ldu, int off, const float* w,
   const int col_blocks = (C + per_thread * row_threads(C) - 1) / (per_thread * row_threads(C));
   // a step of one token a sequence (as many tokens as sequences) moves the tail on in the same launch
   const int fused_tail = taps > 1 && update_state && n_tokens == n_seqs;
-  const bool rows = n_tokens > 64 && !fused_tail && taps <= 4 && C % 4 == 0 && off % 4 == 0 && ldu % 4 == 0 && (uintptr_t)u % 16 == 0 && (uintptr_t)out % 16 == 0;
-  if (rows) conv_rows_kernel<<<dim3((n_tokens + CONV_RUN - 1) / CONV_RUN, (C + 4 * CONV_THREADS - 1) / (4 * CONV_THREADS)), CONV_THREADS, 0, stream>>>(
+  const dim3 row_grid((n_tokens + CONV_RUN - 1) / CONV_RUN, (C + 4 * CONV_THREADS - 1) / (4 * CONV_THREADS));
+  const bool rows = n_tokens > 64 && (long long)row_grid.x * row_grid.y >= CONV_BLOCKS && !fused_tail && taps <= 4 && C % 4 == 0 && off % 4 == 0 && ldu % 4 == 0 && (uintptr_t)u % 16 == 0 && (uintptr_t)out % 16 == 0;
+  if (rows) conv_rows_kernel<<<row_grid, CONV_THREADS, 0, stream>>>(
       u, ldu, off, w, b, state, out, tok_seq, seq_tok0, seq_slot, n_tokens, C, taps, in_bias, act);
   else launch_pdl(pdl_bit_for_tokens(n_tokens), conv_silu_kernel, dim3(n_tokens, col_blocks), dim3(row_threads(C)), (size_t)(0), stream, u, ldu, off, w, b, state, out, tok_seq, seq_tok0, seq_slot, C, taps, in_bias, act, fused_tail);
   EL_LAUNCH_CHECK("conv_silu");

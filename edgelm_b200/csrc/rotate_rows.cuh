@@ -28,8 +28,15 @@ struct RotateRows {
   int taps;
 };
 
+// The blocks from which on it is ahead of a block a token and four heads: a warp's eight tokens are a chain of some 8 us (with three taps
+// 11 to 15), whatever the step.  (A block a token
+// and four heads against this: 9 heads of 64, 384 tokens, 336 blocks 7.2 and 8.1 us; 512 tokens, 448 blocks 8.3 and 8.2; 768 tokens, 672
+// blocks 11.7 and 9.6; from 500 to 600 blocks 0.59 to 0.88 of the time over ten shapes of heads, 250 to 300 blocks 0.87 to 1.31.)
+constexpr int ROT_BLOCKS = 450;
+
 // whether the kernel takes these sizes (dk: what a head's queries and a key row hold, all maps)
 inline bool rotate_rows_takes(int n_tokens, int H, int G, int dk, int dv, int maps, int rot, int interleaved, int taps) {
+  if (dk < 1 || (long long)((n_tokens + ROT_TOKENS - 1) / ROT_TOKENS) * ((H + G + G * dv / dk + ROT_WARPS - 1) / ROT_WARPS) < ROT_BLOCKS) return false;
   if (n_tokens <= 64 || dk % 32 || dk > 128 || maps < 1 || dk % maps || (dk / maps) % 32 || rot > 128 || (G * dv) % dk || taps > 4) return false;
   const int half = rot / 2;
   return rot == 0 || interleaved || half % 32 == 0 || (half < 32 && (half & (half - 1)) == 0);

@@ -153,9 +153,11 @@ def test_blend_convolution_and_norms(dtype):
     assert np.abs(dec.cpu().numpy() - ref).max() < 1e-5
 
 
-@pytest.mark.parametrize("C,taps,bias,act", [(260, 4, True, "silu"), (64, 2, False, None), (512, 1, True, "silu"), (1028, 3, True, None)])
+@pytest.mark.parametrize("C,taps,bias,act", [(260, 4, True, "silu"), (64, 2, False, None), (512, 1, True, "silu"), (1028, 3, True, None),
+                                             (18948, 4, True, "silu"), (18948, 3, False, None), (19200, 2, True, None), (18948, 1, True, "silu")])
 def test_filter_over_many_tokens(C, taps, bias, act):
-    """Steps of more than 64 tokens: sequences that start inside a run of tokens, shorter than the filter, going on from a tail."""
+    """Steps of more than 64 tokens, few channels and enough for the kernel of many tokens: sequences that start inside a run of tokens,
+    shorter than the filter, going on from a tail."""
     g = np.random.default_rng(C)
     lengths, slots = [70, 1, 2, 33], [3, 0, 5, 2]
     u, w, b, ib, tail = g.normal(size=(106, C + 8)), g.normal(size=(C, taps)), g.normal(size=C), g.normal(size=C), g.normal(size=(6, taps - 1, C))
@@ -176,7 +178,7 @@ def test_filter_over_many_tokens(C, taps, bias, act):
 def test_filter_reads_no_token_in_front_of_its_taps(taps, cut):
     """An infinity and a NaN reach `taps` tokens each, in one step and where the step is cut behind the infinity."""
     g = np.random.default_rng(taps)
-    T, C, bad = 180, 64, {20: np.inf, 99: np.nan}
+    T, C, bad = 180, 13400, {20: np.inf, 99: np.nan}        # (channels enough for the kernel of many tokens)
     u, w = g.normal(size=(T, C)), g.normal(size=(C, taps)) + 2.0
     for t, value in bad.items():
         u[t, 5] = value
