@@ -126,6 +126,14 @@ using pair_t = unsigned long long;       // two float32
 __device__ __forceinline__ void fma_pair(pair_t& c, pair_t a, pair_t b) { asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b)); }
 __device__ __forceinline__ float pair_sum(pair_t c) { return __uint_as_float((uint32_t)c) + __uint_as_float((uint32_t)(c >> 32)); }
 
+template <int EPI>
+__device__ __forceinline__ void epilogue_put(float* out, float residual, float acc, float acc2) {
+  if (EPI == EPI_STORE) *out = acc;
+  if (EPI == EPI_RESIDUAL) *out = residual + acc;
+  if (EPI == EPI_SWIGLU) *out = silu_f32(acc) * acc2;
+  if (EPI == EPI_RELU2) *out = fmaxf(acc, 0.f) * fmaxf(acc, 0.f);
+}
+
 template <int TY, int TX, int KG> constexpr size_t sgemm_smem() {
   constexpr size_t ring = (size_t)KG * S_STAGES * 8 * (TY + TX) * SK * 4, sums = (size_t)TY * TX * KG * 64 * 4, red = (size_t)KG * 8 * TY * (8 * TX + 8) * 4;
   return ring + sums > red ? ring + sums : red;
@@ -235,14 +243,25 @@ sgemm_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, 
     acc[i][j + 3] = v.w + pair_sum(part[i][j + 3]);
   }
   if (KG == 1 && CS == 1) {
+    // (`out` may be the residual itself: a row's residuals are requested before the row ahead of it is stored, or every load would
+    // wait for the store before it)
+    float ahead[2][8] = {};
+    auto fetch = [&](int i) {
+      const int m = m0 + ty + TY * i;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        if (m < M && n0 + tx + TX * j < N) ahead[i & 1][j] = residual[(size_t)m * ldo + n0 + tx + TX * j];
+    };
+    if (EPI == EPI_RESIDUAL) fetch(0);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
       const int m = m0 + ty + TY * i;
+      if (EPI == EPI_RESIDUAL && i < 7) fetch(i + 1);
       if (m >= M) continue;
 #pragma unroll
       for (int j = 0; j < (EPI == EPI_SWIGLU ? 4 : 8); ++j) {
         const int n = n0 + tx + TX * j;
-        if (n < N) epilogue_store<EPI, float>(out, residual, (size_t)m * ldo + n, acc[i][j], EPI == EPI_SWIGLU ? acc[i][(j + 4) & 7] : 0.f);
+        if (n < N) epilogue_put<EPI>(out + (size_t)m * ldo + n, ahead[i & 1][j], acc[i][j], EPI == EPI_SWIGLU ? acc[i][(j + 4) & 7] : 0.f);
       }
     }
     return;
@@ -268,16 +287,27 @@ sgemm_kernel(const float* __restrict__ A, int lda, const float* __restrict__ W, 
   cooperative_groups::cluster_group cluster = cooperative_groups::this_cluster();
   if (CS > 1) cluster.sync();
   const int r_begin = BM * rank / CS, r_end = BM * (rank + 1) / CS;
-  for (int e = r_begin * NOUT + threadIdx.x; e < r_end * NOUT; e += GT * KG) {
-    const int r = e / NOUT, c = e % NOUT, m = m0 + r, n = n0 + c;
-    if (m >= M || n >= N) continue;
-    float v = 0.f, v2 = 0.f;
-    for (int q = 0; q < CS; ++q) {
-      const float* p = (CS > 1 ? cluster.map_shared_rank(sm, q) : sm) + r * RP + c;
-      v += p[0];
-      if (EPI == EPI_SWIGLU) v2 += p[NOUT];
+  constexpr int AHEAD = 4;               // (residuals requested together: `out` may be the residual itself)
+  for (int e0 = r_begin * NOUT + threadIdx.x; e0 < r_end * NOUT; e0 += AHEAD * GT * KG) {
+    float ahead[AHEAD] = {};
+    auto at = [&](int e) { return (size_t)(m0 + e / NOUT) * ldo + n0 + e % NOUT; };
+    auto there = [&](int e) { return e < r_end * NOUT && m0 + e / NOUT < M && n0 + e % NOUT < N; };
+    if (EPI == EPI_RESIDUAL)
+#pragma unroll
+      for (int x = 0; x < AHEAD; ++x)
+        if (there(e0 + x * GT * KG)) ahead[x] = residual[at(e0 + x * GT * KG)];
+#pragma unroll
+    for (int x = 0; x < AHEAD; ++x) {
+      const int e = e0 + x * GT * KG;
+      if (!there(e)) continue;
+      float v = 0.f, v2 = 0.f;
+      for (int q = 0; q < CS; ++q) {
+        const float* p = (CS > 1 ? cluster.map_shared_rank(sm, q) : sm) + e / NOUT * RP + e % NOUT;
+        v += p[0];
+        if (EPI == EPI_SWIGLU) v2 += p[NOUT];
+      }
+      epilogue_put<EPI>(out + at(e), ahead[x], v, v2);
     }
-    epilogue_store<EPI, float>(out, residual, (size_t)m * ldo + n, v, v2);
   }
   if (CS > 1) cluster.sync();            // (no block leaves while another reads its sums)
 }

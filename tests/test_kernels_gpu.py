@@ -115,7 +115,7 @@ def test_gemm_simt_swiglu(dtype, M, N, K):
 
 
 @pytest.mark.parametrize("M,N,K", [(17, 48, 64), (32, 64, 16), (33, 1000, 576), (65, 397, 132), (129, 65, 4), (24, 960, 2560), (64, 2000, 20),
-                                     (300, 130, 1028), (1000, 1100, 96)])
+                                     (300, 130, 1028), (1000, 1100, 96), (1000, 2250, 644)])
 def test_gemm_simt_register_tiles(M, N, K):
     """Tiles' edges, parts of a stage, groups without a stage, clusters; 5e-7 is eight roundings of 2^-24 of the result's norm,
     twice what sums of runs of 64 pairs can gather at K = 2560."""
