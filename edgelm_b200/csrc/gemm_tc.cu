@@ -760,7 +760,7 @@ gemm_tc_persistent_kernel(const __grid_constant__ CUtensorMap map_a, const __gri
 // persistent kernel with narrow tiles starves on shared-memory bandwidth: 0.68 to 0.78).  Forced for comparisons.
 static int g_tc_auto = 1, g_tc_persistent = 1, g_tc_wide = 1, g_tc_narrow = 1, g_tc_deep = 1, g_tc_tiny = 1, g_tc_out = 1;
 
-// Which kernel the last edgelm_gemm_tc call took: tile columns | persistent << 12 | deep ring << 13 | K splits << 16.
+// Which kernel the last edgelm_gemm_tc call took: tile columns | persistent << 12 | deep ring << 13 | how the tiles left << 14 | K splits << 16.
 // Tests read it so that a product meant for one kernel cannot pass on another.
 static int g_last_kernel = 0;
 
@@ -819,7 +819,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
     }
     const int tiles = ((N + BN - 1) / BN) * ((M + TC_BM - 1) / TC_BM);
     const int grid = tiles < n_sms ? tiles : n_sms;
-    g_last_kernel = BN | (1 << 12) | (1 << 16);
+    g_last_kernel = BN | (1 << 12) | (mo.how << 14) | (1 << 16);
     cudaError_t le = launch_pdl(32, kern, dim3(grid), dim3(TC_THREADS), (size_t)smem, stream, ma, mb, mb2, (TOut*)out, ldo, residual, M, N, K,
                                 vec_ok, err, rope, mo.map, mo.how);
     if (le != cudaSuccess) {
@@ -843,7 +843,7 @@ static int launch_tc(const CUtensorMap& ma, const CUtensorMap& mb, const CUtenso
     cudaDeviceGetAttribute(&n_sms, cudaDevAttrMultiProcessorCount, dev);
   }
   const bool deep = g_tc_deep && (long long)grid.x * grid.y * grid.z <= (splits > 1 ? SPLIT_DEEP : n_sms);
-  g_last_kernel = BN | ((deep ? 1 : 0) << 13) | (splits << 16);
+  g_last_kernel = BN | ((deep ? 1 : 0) << 13) | ((splits == 1 ? mo.how : TC_OUT_DIRECT) << 14) | (splits << 16);
   auto go = [&](auto kern, int smem, const auto& out_tiles) -> int {
     cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) {

@@ -265,9 +265,11 @@ def gemm_tc_rope(a, w, qkv, tok_pos, tok_seq, seq_slot, page_table, cos, sin, kc
 
 
 def gemm_tc_last_kernel():
-    """Which kernel the last `gemm_tc` call took: {"tile_columns", "persistent", "deep_ring", "k_splits"}."""
+    """Which kernel the last `gemm_tc` call took: {"tile_columns", "persistent", "deep_ring", "left" ("stores", "tma" or
+    "tma_add"), "k_splits"}."""
     v = int(lib().edgelm_gemm_tc_last_kernel())
-    return {"tile_columns": v & 0xFFF, "persistent": bool(v >> 12 & 1), "deep_ring": bool(v >> 13 & 1), "k_splits": v >> 16}
+    return {"tile_columns": v & 0xFFF, "persistent": bool(v >> 12 & 1), "deep_ring": bool(v >> 13 & 1),
+            "left": ("stores", "tma", "tma_add")[v >> 14 & 3], "k_splits": v >> 16}
 
 
 def rope_kv_append(qkv, tok_pos, tok_seq, seq_slot, page_table, cos, sin, kcache, vcache, nh, nkv, hd, err):
