@@ -503,11 +503,8 @@ extern "C" int edgelm_delta_scan(const float* qkv, int C, const float* bg, float
 // 1 if the chunked form takes heads of these sizes (whole pieces of 16 bytes, its tiles in shared memory).
 extern "C" int edgelm_delta_chunked_takes(int d, int e) { return d >= 4 && d <= 128 && e >= 4 && e <= 128 && d % 4 == 0 && e % 4 == 0 ? 1 : 0; }
 
-// Floats of scratch that the chunked form takes for `n_tiles` chunks.
-extern "C" long long edgelm_delta_chunked_scratch(int n_tiles, int H, int d, int e) { return (long long)n_tiles * H * ((long long)dc_floats(d, e) + 4); }
-
 // `edgelm_delta_scan` chunk by chunk (three launches): the step's tokens come as tiles of at most CHUNK consecutive tokens of one
-// sequence, in the order of the sequences, every sequence cut from its first row of the step.  scratch: `edgelm_delta_chunked_scratch` floats.
+// sequence, in the order of the sequences, every sequence cut from its first row of the step.  scratch: n_tiles H (`dc_floats` + 4) floats.
 extern "C" int edgelm_delta_chunked(const float* qkv, int C, const float* bg, float* state, float* o, const int32_t* seq_tok0,
                                     const int32_t* seq_slot, int n_seqs, const int32_t* tile_tok0, const int32_t* tile_ntok, int n_tiles, int H,
                                     int G, int d, int e, float* scratch, cudaStream_t stream) {

@@ -544,7 +544,7 @@ def ssm_chunked_takes(n_state, head_dim):
 
 
 def ssm_chunked_scratch_floats(n_tiles, heads, groups, n_state, head_dim):
-    return int(n_tiles) * (heads * head_dim * n_state + groups * STATE_CHUNK * (STATE_CHUNK + n_state) + (heads + 3) // 4 * 4)     # (`edgelm_ssm_chunked_scratch`)
+    return int(n_tiles) * (heads * head_dim * n_state + groups * STATE_CHUNK * (STATE_CHUNK + n_state) + (heads + 3) // 4 * 4)     # (laid out in `edgelm_ssm_chunked`)
 
 
 def _chunk_tiles(seq_tok0, seq_slot, tile_tok0, tile_ntok, scratch, need, like, what):
@@ -579,7 +579,7 @@ def wkv_chunked_takes(head_dim):
 
 
 def wkv_chunked_scratch_floats(n_tiles, heads, head_dim):
-    return int(n_tiles) * heads * head_dim * (head_dim + STATE_CHUNK + 1)     # (`edgelm_wkv_chunked_scratch`)
+    return int(n_tiles) * heads * head_dim * (head_dim + STATE_CHUNK + 1)     # (laid out in `edgelm_wkv_chunked`)
 
 
 def wkv_chunked(r, k, v, w, bonus, state, o, seq_tok0, seq_slot, n_seqs, tile_tok0, tile_ntok, n_tiles, heads, head_dim, scratch=None):
@@ -1048,7 +1048,7 @@ def delta_chunked_takes(d, e):
 
 
 def delta_chunked_scratch_floats(n_tiles, heads, d, e):
-    return int(n_tiles) * heads * (2 * DELTA_CHUNK * d + DELTA_CHUNK * e + d * e + 4)     # (`edgelm_delta_chunked_scratch`)
+    return int(n_tiles) * heads * (2 * DELTA_CHUNK * d + DELTA_CHUNK * e + d * e + 4)     # (`dc_floats` and a decay of every (chunk, head))
 
 
 DELTA_CHUNK = 64     # tokens of a chunk (CHUNK in chunk_mm.cuh)

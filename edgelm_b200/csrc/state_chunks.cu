@@ -350,13 +350,8 @@ using namespace edgelm;
 extern "C" int edgelm_ssm_chunked_takes(int N, int P) { return N >= 4 && N <= 128 && N % 4 == 0 && P >= 4 && P <= 64 && P % 4 == 0 ? 1 : 0; }
 extern "C" int edgelm_wkv_chunked_takes(int K) { return K >= 4 && K <= WK && K % 4 == 0 ? 1 : 0; }
 
-// Floats of scratch that they take for `n_tiles` chunks.
-extern "C" long long edgelm_ssm_chunked_scratch(int n_tiles, int H, int G, int N, int P) {
-  return (long long)n_tiles * ((long long)H * P * N + (long long)G * (CHUNK * CHUNK + CHUNK * N) + (H + 3) / 4 * 4);
-}
-extern "C" long long edgelm_wkv_chunked_scratch(int n_tiles, int H, int K) { return (long long)n_tiles * H * ((long long)K * K + CHUNK * K + K); }
-
 // The recurrence of `edgelm_ssm_scan` over tiles: the raw step sizes at u[t][dt_off + h].  (The tail of the convolution ahead stays as it is.)
+// scratch: n_tiles times H P N, G CHUNK (CHUNK + N) and H (in fours) floats.
 extern "C" int edgelm_ssm_chunked(const float* xbc, int C, int inner, int G, int N, const float* u, int ldu, int dt_off, const float* dt_bias,
                                   const float* A_log, const float* D, float* state, float* y, const int32_t* seq_tok0, const int32_t* seq_slot, int n_seqs,
                                   const int32_t* tile_tok0, const int32_t* tile_ntok, int n_tiles, int H, int P, float* scratch,
@@ -389,7 +384,7 @@ extern "C" int edgelm_ssm_chunked(const float* xbc, int C, int inner, int G, int
   return 0;
 }
 
-// The recurrence of `edgelm_wkv_scan` over tiles.
+// The recurrence of `edgelm_wkv_scan` over tiles; scratch: n_tiles H K (K + CHUNK + 1) floats.
 extern "C" int edgelm_wkv_chunked(const float* r, const float* k, const float* v, const float* w, const float* bonus, float* state, float* o,
                                   const int32_t* seq_tok0, const int32_t* seq_slot, int n_seqs, const int32_t* tile_tok0,
                                   const int32_t* tile_ntok, int n_tiles, int H, int K, float* scratch, cudaStream_t stream) {
