@@ -41,8 +41,14 @@ CFG_B = {"architecture": "Sagizen", "vocab": 97, "width": 50, "norm": {"eps": 3e
     mamba(2, 24, 8, 2, 1, 2, 30),
     parallel(2, 2, 32, 32, 33, 5, None, 0.2, 1, 40, 0.9, 1.1, 64),
 ]}
-DECAY_RANK = {"a": 24, "b": 5}     # the rank of the decay's projection is a size that only the tensors' shapes give
-CONFIGS = {"a": CFG_A, "b": CFG_B}
+# Heads of 64, states of 128 x 64, and channels enough for a prompt of 1,210 tokens to reach the kernels that the presets' prompt
+# steps take.
+CFG_C = {"architecture": "Sagizen", "vocab": 131, "width": 96, "norm": {"eps": 1e-5}, "layers": [
+    mamba(24, 64, 128, 1, 4, 1, 96),
+    parallel(3, 3, 64, 64, 70, 64, {"base": 10000.0, "dims": 64, "scaling": {"factor": 4.0}}, 0.2, 2, 64, 0.7, 1.3, 96),
+]}
+DECAY_RANK = {"a": 24, "b": 5, "c": 24}     # the rank of the decay's projection is a size that only the tensors' shapes give
+CONFIGS = {"a": CFG_A, "b": CFG_B, "c": CFG_C}
 
 
 def tensors_for(cfg, seed, decay_rank):

@@ -135,6 +135,28 @@ def test_unequal_batches_on_reused_slots(dirs, oracles, name, dtype):
     eng.check_device_errors()
 
 
+@pytest.mark.parametrize("dtype", DTYPES)
+def test_heads_of_64_and_a_prompt_of_1210_tokens(tmp_path, dtype):
+    """The sizes of the presets' heads: rotation and append of many tokens, window attention on the tensor cores (bfloat16) and both
+    recurrences in chunks, in whole prompts, in pieces that start inside a chunk, and several prompts in a step."""
+    from edgelm_b200.engine.engine import Engine, StepEntry
+    d = M.write_dir(str(tmp_path / "c"), M.CFG_C, seed=31, decay_rank=M.DECAY_RANK["c"])
+    eng, oracle = Engine.from_dir(d, dtype=dtype, max_tokens=2048), Oracle(d)
+    requests = [M.tokens(M.CFG_C, n, 90 + i) for i, n in enumerate((1210, 65, 17, 129))]
+    for r in requests:
+        close(H.run_whole(eng, r), oracle.logits(r), dtype, len(r))
+    for cuts in ([100, 1110], [65, 1, 1144]):
+        slot, rows, at = eng.open(1)[0], [], 0
+        for c in cuts:
+            rows.append(eng.step([StepEntry(slot, requests[0][at:at + c], list(range(c)))]).cpu().numpy())
+            at += c
+        eng.close([slot])
+        close(np.concatenate(rows, 0), oracle.logits(requests[0]), dtype, cuts)
+    for r, g in zip(requests, H.run_batches(eng, requests, batch_size=4, decode_tail=12)):
+        close(g, oracle.logits(r), dtype, len(r))
+    eng.check_device_errors()
+
+
 @pytest.mark.parametrize("name", NAMES)
 def test_steps_cut_by_the_engine(dirs, oracles, name):
     """An engine that runs at most 64 tokens at a time cuts a step of three prompts into consecutive smaller ones."""

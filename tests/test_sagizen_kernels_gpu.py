@@ -492,3 +492,30 @@ def test_rotation_bias_and_unit_norm(dtype):
         assert np.abs(kc[p // 64, 0, p % 64].float().cpu().numpy() - qk[i, H]).max() < tol
         assert np.abs(vc[p // 64, 0, p % 64].float().cpu().numpy() - x[i, (H + G) * dk:]).max() < tol
     assert int(err.item()) == 0
+
+
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("H,G,dk,dv,rot", [(66, 3, 64, 64, 64), (68, 2, 64, 64, 32), (68, 1, 128, 128, 64), (66, 2, 96, 192, 0)])
+def test_rotation_bias_and_unit_norm_of_many_tokens(H, G, dk, dv, rot, dtype):
+    """Heads of whole runs of 32 in steps of more than 64 tokens, two sequences, the last run of tokens a part.  3e-6: a dozen float32
+    roundings of values up to 5 (a unit row's largest); a bfloat16 value is off by 2^-9 of itself beside that."""
+    g = np.random.default_rng(dk + rot)
+    eps, lengths, first = 1e-4, [70, 130], [0, 1000]
+    T, pos = sum(lengths), np.concatenate([np.arange(a, a + n) for a, n in zip(first, lengths)])
+    qkv, bias = g.normal(size=(T, (H + G) * dk + G * dv)), g.normal(size=(H + G) * dk + G * dv)
+    freq = 1e4 ** (-2.0 * np.arange(rot // 2) / max(rot, 1)) / 3.0
+    kc, vc = (torch.zeros((5, G, 64, d), dtype=dtype, device=DEV) for d in (dk, dv))
+    table = torch.full((2, 18), -1, dtype=torch.int32, device=DEV)
+    table[0, :2], table[1, 15:18] = i32([3, 0]), i32([4, 1, 2])
+    seq = np.repeat([0, 1], lengths)
+    qd, err = torch.full((T, H * dk), float("nan"), dtype=dtype, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.qk_rope_norm_append(f32(qkv), f32(bias), qd, i32(pos), i32(seq), table, kc, vc, H, G, dk, dv, rot,
+                            torch.tensor(freq, dtype=torch.float64, device=DEV) if rot else None, eps, True, err)
+    x = qkv.astype(np.float32).astype(np.float64) + bias.astype(np.float32)
+    qk = x[:, :(H + G) * dk].reshape(T, H + G, dk)
+    qk = plain.unit_rms(plain.rotate_partial(qk, pos, rot, 1e4, 3.0) if rot else qk, eps)
+    page, row = table.cpu().numpy()[seq, pos // 64], pos % 64
+    for got, want in ((qd.view(T, H, dk), qk[:, :H]), (kc[page, :, row], qk[:, H:]), (vc[page, :, row], x[:, (H + G) * dk:].reshape(T, G, dv))):
+        off = np.abs(got.float().cpu().numpy() - want)
+        assert (off < 3e-6 + (0 if dtype == torch.float32 else 2.0 ** -8 * np.abs(want))).all()
+    assert int(err.item()) == 0 and int((kc != 0).any(-1).any(1).sum()) == T
