@@ -491,8 +491,8 @@ pooled_window_attn_tiled_kernel(const T* __restrict__ q, T* __restrict__ out, co
 // products of bfloat16 numbers summed in float32; the float32 weights, and the pooled rows' float32 keys and values, go as three
 // bfloat16 terms (8 + 8 + 8 bits of their mantissas), weights times pooled values as the six products of terms that float32 can
 // tell from zero.  Scores, maxima, exponentials, denominators and outputs are float32, as on the CUDA cores.
-// 2,048 tokens, 32 heads of 64, a window of 1,024, blocks of 64: 1,131 us there, 145 us here (bound by the issue of the small
-// matrix instructions: three of them for every page value).
+// 2,048 tokens, 32 heads of 64, a window of 1,024, blocks of 64: 1,131 us there, 145 us here (three small matrix
+// instructions for every page value, in chains with the exponentials: the tensor pipe is active 44 % of the time, half of the issue slots used).
 constexpr int PM_WARPS = 4, PM_ROWS = 16 * PM_WARPS, PM_POOLED = 32;
 
 // S[NT tiles of 8 keys] = Q K^T, the keys in TERMS tiles of `tile` elements one after the other (the smallest term first)

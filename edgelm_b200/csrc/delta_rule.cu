@@ -192,7 +192,7 @@ delta_scan_kernel(const float* __restrict__ qkv, int C, const float* __restrict_
 // from float64 as the walk's.)
 // One (chunk, head) of the scratch: U0, later U, [e][64]; W [64][d]; the keys times exp(L_n - L_s) [d][64]; S0 [e][d].  Then exp(L_n) of each.
 // Nine heads of 64, prompts of 333 to 1,700 tokens (4,065 in all): the walk 548 us, this 232 (77 + 106 + 49; all but the logarithms in
-// float32 195).
+// float32 195).  The first waits for its loads, results and unrolled code (double pipe 17 % active), the second is the longest sequence's chain.
 constexpr int DC_BLOCK = 16;       // value channels a block of `delta_chunk_states` owns
 constexpr int DC_STATE_THREADS = 128;
 constexpr int DC_SOLVE_PITCH = CHUNK + 2;

@@ -108,8 +108,8 @@ gemm_tile_kernel(const TA* __restrict__ A, int lda, const TW* __restrict__ W, co
 // run's length, not with their product.  (Two stages, runs of 16 products a pair: 1.13e-7 of the result at K 576, 1.82e-7 at K 2560, the
 // any-size kernel's 1.34e-7 and 2.41e-7; runs twice as long are 7 % faster and less exact than it at K under 300.)  The sums of groups and
 // blocks are added in the order of K.  Measured beside the any-size kernel: 2,000 rows, N 1000, K 2560 680 -> 326 us; 300 rows, N 576,
-// K 2560 173 -> 47 us; 24 rows, N 960, K 2560 169 -> 10 us.  Bound by the issue of the multiply-adds (their pipe is about 55 % busy: 64
-// pairs of sums leave a scheduler two warps).
+// K 2560 173 -> 47 us; 24 rows, N 960, K 2560 169 -> 10 us.  Bound by the chains of two warps a scheduler, which is what 64
+// pairs of sums leave room for (1,143 rows, N 1536, K 576: the multiply-adds' pipe active 52 %, issue slots 45 %, memory 1 %).
 constexpr int SK = 16, S_STAGES = 3, S_FLUSH = 2;
 
 __device__ __forceinline__ void cp_async16(unsigned dst, const float* src, bool there) {

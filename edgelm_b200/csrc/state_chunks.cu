@@ -11,7 +11,7 @@
 //   2. `ssm_chunk_state`, per (chunk, head): the chunk's own sum of the second line;
 //   3. `chunk_fold`: the chunks of a sequence in order, element by element: S0 in place of that sum, the state moved on;
 //   4. `ssm_chunk_out`, per (chunk, head): the first line.
-// Bound by the multiply-adds of 2. and 4. (products out of shared memory).  2,048 tokens of one sequence, 64 heads of 128 x 64: the walk
+// Most of the time goes to the products out of shared memory of 2. and 4.  2,048 tokens of one sequence, 64 heads of 128 x 64: the walk
 // 597 us, this 230 (state 80, out 126, the other two 24).
 //
 // Decayed outer-product recurrence with a bonus (o_t = (S + diag(u) k_t v_t^T)^T r_t, S <- diag(w_t) S + k_t v_t^T; a decay per key channel):
@@ -19,8 +19,8 @@
 //      channels in registers; its outputs, its last state, and r_t times the product of the decays before t;
 //   2. `chunk_fold`;
 //   3. `wkv_chunk_out`, per (chunk, head): what S0 adds to the outputs, one product.
-// Bound by the issue of the walk's multiply-adds (three a state element and token).  2,048 tokens, 32 heads of 64: the walk 562 us, this
-// about 130 (local 85).
+// Most of the time goes to 1. (three multiply-adds a state element and token).  2,048 tokens, 32 heads of 64: the walk 562 us, this
+// 148.
 #include "chunk_mm.cuh"
 
 namespace edgelm {
