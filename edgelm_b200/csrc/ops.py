@@ -119,8 +119,9 @@ def rmsnorm(x, w, eps, out, rows_idx=None):
     _check(lib().edgelm_rmsnorm(_p(x), _p(w), _p(out), _dt(out), _p(rows_idx), rows, dim, ctypes.c_float(eps), _stream()))
 
 
-def gemm_simt(a, w, out, epilogue=EPI_STORE, w2=None, residual=None, force_kernel=0):
-    """out = a @ w.T (+ epilogue) with float32 accumulation on the CUDA cores."""
+def gemm_simt(a, w, out, epilogue=EPI_STORE, w2=None, residual=None, force_kernel=0, err=None):
+    """out = a @ w.T (+ epilogue) with float32 accumulation: on the CUDA cores, or (float32 operands in 16-byte pieces, more than
+    16 rows) on the tensor cores at float32's precision, whose bounded waits report to `err`."""
     _need(a.dim() == 2 and w.dim() == 2 and out.dim() == 2, "gemm: 2-D operands")
     M, K = a.shape
     N = w.shape[0]
@@ -130,7 +131,22 @@ def gemm_simt(a, w, out, epilogue=EPI_STORE, w2=None, residual=None, force_kerne
     if residual is not None:
         _need(residual.dtype == torch.float32 and residual.shape == out.shape and residual.stride() == out.stride(), "gemm: residual layout")
     _check(lib().edgelm_gemm_simt(_p(a), a.stride(0), _p(w), _p(w2), _p(out), out.stride(0), _p(residual), M, N, K,
-                                  _dt(a), _dt(out), epilogue, force_kernel, _stream()))
+                                  _dt(a), _dt(out), epilogue, force_kernel, _p(err), _stream()))
+
+
+def gemm_split(a, w, out, err=None, epilogue=EPI_STORE, w2=None, residual=None, form=0):
+    """out = a @ w.T (+ epilogue), all float32, as tensor-core products of three bfloat16 terms an operand.  `err`: the device
+    error word (None: sums behind a wait that ran out are only not-a-numbers).  `form`: 0 by sizes, else rows of the
+    tile (32, 64) + 256 * blocks that share K."""
+    _need(a.dim() == 2 and w.dim() == 2 and out.dim() == 2, "gemm: 2-D operands")
+    M, K = a.shape
+    N = w.shape[0]
+    _need(w.shape[1] == K and out.shape == (M, N), f"gemm: shapes a{tuple(a.shape)} w{tuple(w.shape)} out{tuple(out.shape)}")
+    _need(a.dtype == w.dtype == out.dtype == torch.float32 and (w2 is None or (w2.dtype == w.dtype and w2.shape == w.shape and w2.is_contiguous())), "gemm_split: float32 operands")
+    _need(a.stride(1) == 1 and out.stride(1) == 1 and w.is_contiguous(), "gemm: rows must be contiguous")
+    if residual is not None:
+        _need(residual.dtype == torch.float32 and residual.shape == out.shape and residual.stride() == out.stride(), "gemm: residual layout")
+    _check(lib().edgelm_gemm_split(_p(a), a.stride(0), _p(w), _p(w2), _p(out), out.stride(0), _p(residual), M, N, K, epilogue, form, _p(err), _stream()))
 
 
 def gemv_takes(a, w, w2=None, normed=False):

@@ -1,12 +1,13 @@
 """out = a . W^T with an epilogue, on the kernel that fits the sizes.
 
-  rows <= 16        the few-rows kernels: weights streamed once, activations in shared memory, the
+  rows <= 16        the few-rows kernels (float32: up to where the tensor cores win, `_few_rows_f32`): weights streamed once, activations in shared memory, the
                     preceding RMSNorm computed in the prologue (`NormedInput`).  bfloat16 runs
                     on mma.sync tensor cores (gemv_mma.cu), float32 on the CUDA cores (gemv.cu);
   bfloat16, more    the tcgen05 tensor-core kernel (gemm_tc.cu): operands by TMA, accumulator in
                     tensor memory;
-  anything else     the CUDA-core kernels of gemm_simt.cu: the whole float32 path for many rows (register tiles),
-                    and every size the other two do not take (K not a multiple of 8, unaligned rows).
+  float32, more     the tensor cores as well, three bfloat16 terms an operand (gemm_split.cu): as exact as float32 sums;
+  anything else     the CUDA-core kernels of gemm_simt.cu: every size that the others do not take (K not a
+                    multiple of 8 or 4, unaligned rows).
 """
 import os
 
@@ -24,6 +25,14 @@ MMA_WIDE_COLUMNS = 8192  # from here on (the vocabulary) the tensor-core kernel 
 
 def _few_rows_on_mma(rows, n_cols):
     return rows >= MMA_MIN_ROWS or n_cols >= MMA_WIDE_COLUMNS
+
+
+def _few_rows_f32(rows, w, w2, fused_norm):
+    """Whether a float32 product of up to 16 rows stays on the few-rows kernel, whose time grows with the rows; the tensor-core
+    product's does not, but it starts later and wants a fused norm computed ahead (2 us).  Measured, few rows | tensor cores, us: N 576, K 576 at 8
+    and 16 rows 5.6 | 6.3, 6.7 | 6.3; N 576, K 1536 at 4 and 8 7.4 | 6.8, 10.9 | 6.7; N 2560 SwiGLU, K 960 with the norm at 4, 8 and 16
+    11.4, 16.1, 23.4 | 10.5; N 49152, K 576 at 2, 4, 8, 16 34.7, 42.4, 59, 110 | 35."""
+    return rows < 4 or rows * w.numel() * (2 if w2 is not None else 1) < (24_000_000 if fused_norm else 5_000_000)
 
 
 class NormedInput:
@@ -71,7 +80,7 @@ def matmul(ctx, a, w, out, epilogue=EPI_STORE, w2=None, residual=None, prefetch=
                 ops.gemv_mma(a.x, w, out, epilogue=epilogue, w2=w2, residual=residual, norm_weight=a.norm.weight, eps=a.norm.eps,
                              prefetch=prefetch)
                 return
-            if ops.gemv_takes(a.x, w, w2, normed=True):
+            if _few_rows_f32(rows, w, w2, True) and ops.gemv_takes(a.x, w, w2, normed=True):
                 ops.gemv(a.x, w, out, epilogue=epilogue, w2=w2, residual=residual, norm_weight=a.norm.weight, eps=a.norm.eps,
                          n_sms=ctx.n_sms)
                 return
@@ -79,8 +88,11 @@ def matmul(ctx, a, w, out, epilogue=EPI_STORE, w2=None, residual=None, prefetch=
     if rows <= FEW_ROWS and _few_rows_on_mma(rows, w.shape[0]) and ops.gemv_mma_takes(a, w, w2):
         ops.gemv_mma(a, w, out, epilogue=epilogue, w2=w2, residual=residual, prefetch=prefetch)
     elif rows <= FEW_ROWS and ops.gemv_takes(a, w, w2):
-        ops.gemv(a, w, out, epilogue=epilogue, w2=w2, residual=residual, n_sms=ctx.n_sms)
+        if a.dtype != torch.float32 or _few_rows_f32(rows, w, w2, False):
+            ops.gemv(a, w, out, epilogue=epilogue, w2=w2, residual=residual, n_sms=ctx.n_sms)
+        else:
+            ops.gemm_split(a, w, out, ctx.err, epilogue=epilogue, w2=w2, residual=residual)
     elif a.dtype == torch.bfloat16 and rows > FEW_ROWS and ops.gemm_tc_takes(a, w, out, w2):
         ops.gemm_tc(a, w, out, ctx.err, epilogue=epilogue, w2=w2, residual=residual)
     else:
-        ops.gemm_simt(a, w, out, epilogue=epilogue, w2=w2, residual=residual)
+        ops.gemm_simt(a, w, out, epilogue=epilogue, w2=w2, residual=residual, err=ctx.err)

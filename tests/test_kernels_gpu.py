@@ -137,6 +137,46 @@ def test_gemm_simt_register_tiles(M, N, K):
     assert torch.equal(moved, out[order])
 
 
+@pytest.mark.parametrize("M,N,K", [(31, 127, 36), (33, 129, 64), (65, 260, 100), (96, 192, 1000)])
+@pytest.mark.parametrize("form", [32 + 256, 32 + 2 * 256, 32 + 8 * 256, 64 + 256, 64 + 3 * 256])
+def test_gemm_split_forms(M, N, K, form):
+    """Both tiles and clusters at the edges of rows, columns and units of k.  Each sum: up to eight cut-offs of a leading run
+    (2^-24 of it on average), K / 32 roundings of runs, eight of blocks and the epilogue's: 2^-24 sqrt((8 + 32 + 8 + 2) / 3) = 2.4e-7."""
+    o = ops()
+    if form >> 8 > (K + 63) // 64:
+        pytest.skip("more blocks than stages of K")
+    a, w, w2, res = rnd((M, K + 8), torch.float32, 24)[:, 4:K + 4], rnd((N, K), torch.float32, 25, 0.3), rnd((N, K), torch.float32, 26, 0.3), rnd((M, N), torch.float32, 27)
+    err = torch.zeros(1, dtype=torch.int32, device=dev())
+    y, u = a.double() @ w.double().T, a.double() @ w2.double().T
+    for epilogue, want in ((o.EPI_STORE, y), (o.EPI_RESIDUAL, y + res.double()), (o.EPI_SWIGLU, y / (1 + torch.exp(-y)) * u)):
+        out = res.clone() if epilogue == o.EPI_RESIDUAL else torch.full((M, N), float("nan"), device=dev())
+        o.gemm_split(a, w, out, err, epilogue=epilogue, w2=w2 if epilogue == o.EPI_SWIGLU else None,
+                     residual=out if epilogue == o.EPI_RESIDUAL else None, form=form)
+        assert int(err.item()) == 0
+        assert float((out.double() - want).norm() / want.norm()) < 2.4e-7 * (2 if epilogue == o.EPI_SWIGLU else 1)
+
+
+def test_gemm_split_values_that_bfloat16_has_not():
+    """Infinities, not-a-numbers, numbers that bfloat16 rounds to infinity and numbers whose later terms are too small for it come out as
+    float32 multiply-adds give them."""
+    o = ops()
+    M, N, K = 40, 140, 96
+    a, w = rnd((M, K), torch.float32, 28), rnd((N, K), torch.float32, 29)
+    a[1, 5], a[2, 7], a[3, 9], w[4, 3], w[5, 5] = float("inf"), float("nan"), -float("inf"), float("inf"), 0.0
+    a[6] = 0.0
+    a[7, 11] = 3.4e38
+    a[8] *= 1e-34
+    w[9] *= 1e-30
+    got, want = torch.empty(M, N, device=dev()), torch.empty(M, N, device=dev())
+    o.gemm_split(a, w, got)
+    o.gemm_simt(a, w, want, force_kernel=2)
+    assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf())
+    assert torch.equal(got[got.isinf()], want[want.isinf()])
+    finite = want.isfinite()
+    scale = (a.double().abs() @ w.double().abs().T)[finite]       # (K roundings of partial sums, each up to 2^-24 of the absolute values' sum)
+    assert bool(((got.double() - want.double())[finite].abs() <= K * 2.0 ** -24 * scale).all())
+
+
 def test_gemm_row_independent_of_batch():
     """A row's result is the same bits whether it is computed alone or among others."""
     o = ops()
