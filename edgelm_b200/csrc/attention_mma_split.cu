@@ -23,7 +23,9 @@
 // Takes key head sizes 32, 64, 96, 128 over value head sizes of these that are not larger; with two maps a head (a key row holds a
 // head's two keys side by side, each softmax runs over the same values; every (head, map) is a head of its own here, and its output
 // stays float32) key sizes 32 and 64 over values as large or twice as large.  Two maps of 64 over values of 128, 16 heads, chunks of
-// 1,024, prompts of 1,000 and 2,900 tokens: 1,614 us on the CUDA cores, 271 us here.
+// 1,024, prompts of 1,000 and 2,900 tokens: 1,614 us on the CUDA cores, 248 us here.  One sequence of 6,000 tokens, 9 heads of 64:
+// 577 -> 448 us with one conversion a pair of terms, the scale folded into the exponent's multiply-add, a row's sum added over its lanes at
+// the end and the tiles of many keys first.
 #include <math_constants.h>
 
 #include "mma_split.cuh"
@@ -58,7 +60,8 @@ attn_prefill_split_kernel(const float* __restrict__ q, int ldq, void* __restrict
   const int group = threadIdx.x / (SP_WARPS * 32), gtid = threadIdx.x % (SP_WARPS * 32);
   __nv_bfloat16* sm = reinterpret_cast<__nv_bfloat16*>(sp_raw) + (size_t)group * 2 * STAGE;  // this group's [2 stages][K: 64 x PITCH | V: 64 x VPITCH]
 
-  const int tile = blockIdx.x, head = blockIdx.y;       // (head: of nh MAPS, a head's maps next to each other)
+  // (the last tiles of a sequence see the most keys: they go first, or the launch ends with them alone)
+  const int tile = gridDim.x - 1 - blockIdx.x, head = blockIdx.y;       // (head: of nh MAPS, a head's maps next to each other)
   const int kvh = head / (nh / nkv * MAPS), map = head % MAPS;
   const int lane = threadIdx.x & 31, warp = (threadIdx.x >> 5) % SP_WARPS, gid = lane >> 2, tig = lane & 3;
   const int seq = tile_seq[tile], tok0 = tile_tok0[tile], ntok = tile_ntok[tile], pos0 = tile_pos0[tile];
@@ -77,7 +80,9 @@ attn_prefill_split_kernel(const float* __restrict__ q, int ldq, void* __restrict
   const int first_page = sp_first_key(pos0, mask, mask_size) / PAGE, kept_pages = min(first_page, (keep + PAGE - 1) / PAGE);
   const int n_visit = kept_pages + n_pages - first_page;
   auto page_at = [&](int i) { return i < kept_pages ? i : first_page + i - kept_pages; };
-  const float scale2 = scale * 1.4426950408889634f;                     // scores in units of log 2
+  // scores in units of log 2; the sign of the scale (or a scale of 0) goes to the queries, so that the largest score has the largest weight
+  // and a masked one stays at minus infinity
+  const float scale2 = scale == 0.f ? 1.f : fabsf(scale) * 1.4426950408889634f, turn = scale < 0.f ? -1.f : scale > 0.f ? 1.f : 0.f;
 
   auto load_page = [&](int pg, int stage) {
     const int page = pages ? pages[pg] : 0;
@@ -116,10 +121,10 @@ attn_prefill_split_kernel(const float* __restrict__ q, int ldq, void* __restrict
       const float2 b0 = rowB < ntok ? *reinterpret_cast<const float2*>(qB + d) : make_float2(0.f, 0.f);
       const float2 a1 = rowA < ntok ? *reinterpret_cast<const float2*>(qA + d + 8) : make_float2(0.f, 0.f);
       const float2 b1 = rowB < ntok ? *reinterpret_cast<const float2*>(qB + d + 8) : make_float2(0.f, 0.f);
-      sp_split(a0.x, a0.y, qa[0][ks][0], qa[1][ks][0], qa[2][ks][0]);
-      sp_split(b0.x, b0.y, qa[0][ks][1], qa[1][ks][1], qa[2][ks][1]);
-      sp_split(a1.x, a1.y, qa[0][ks][2], qa[1][ks][2], qa[2][ks][2]);
-      sp_split(b1.x, b1.y, qa[0][ks][3], qa[1][ks][3], qa[2][ks][3]);
+      sp_split(turn * a0.x, turn * a0.y, qa[0][ks][0], qa[1][ks][0], qa[2][ks][0]);
+      sp_split(turn * b0.x, turn * b0.y, qa[0][ks][1], qa[1][ks][1], qa[2][ks][1]);
+      sp_split(turn * a1.x, turn * a1.y, qa[0][ks][2], qa[1][ks][2], qa[2][ks][2]);
+      sp_split(turn * b1.x, turn * b1.y, qa[0][ks][3], qa[1][ks][3], qa[2][ks][3]);
     }
   }
   float o[VD / 8][4];
@@ -163,23 +168,22 @@ attn_prefill_split_kernel(const float* __restrict__ q, int ldq, void* __restrict
           }
         }
       }
-      // ---- scale, mask, running max and sum (float32), scores in units of log 2
+      // ---- mask, running maximum and sum (float32); the maxima are of the scores as they come, the weights 2^(score scale - maximum
+      // scale) with one rounding of the exponent; the sums are this lane's keys' only, added over a row's four lanes at the end
       const bool masked = pg * PAGE + PAGE - 1 > warp_min_limit || (pg * PAGE < warp_last_first && pg * PAGE + PAGE > keep);
+      if (masked) {
+#pragma unroll
+        for (int nt = 0; nt < 8; ++nt) {
+          const int key = pg * PAGE + nt * 8 + tig * 2;
+          if (!((key >= firstA || key < keep) && key <= limA)) s[nt][0] = -CUDART_INF_F;
+          if (!((key + 1 >= firstA || key + 1 < keep) && key + 1 <= limA)) s[nt][1] = -CUDART_INF_F;
+          if (!((key >= firstB || key < keep) && key <= limB)) s[nt][2] = -CUDART_INF_F;
+          if (!((key + 1 >= firstB || key + 1 < keep) && key + 1 <= limB)) s[nt][3] = -CUDART_INF_F;
+        }
+      }
       float mxA = -CUDART_INF_F, mxB = -CUDART_INF_F;
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt) {
-        const int key = pg * PAGE + nt * 8 + tig * 2;
-        if (masked) {
-          s[nt][0] = (key >= firstA || key < keep) && key <= limA ? s[nt][0] * scale2 : -CUDART_INF_F;
-          s[nt][1] = (key + 1 >= firstA || key + 1 < keep) && key + 1 <= limA ? s[nt][1] * scale2 : -CUDART_INF_F;
-          s[nt][2] = (key >= firstB || key < keep) && key <= limB ? s[nt][2] * scale2 : -CUDART_INF_F;
-          s[nt][3] = (key + 1 >= firstB || key + 1 < keep) && key + 1 <= limB ? s[nt][3] * scale2 : -CUDART_INF_F;
-        } else {
-          s[nt][0] *= scale2;
-          s[nt][1] *= scale2;
-          s[nt][2] *= scale2;
-          s[nt][3] *= scale2;
-        }
         mxA = fmaxf(mxA, fmaxf(s[nt][0], s[nt][1]));
         mxB = fmaxf(mxB, fmaxf(s[nt][2], s[nt][3]));
       }
@@ -187,25 +191,21 @@ attn_prefill_split_kernel(const float* __restrict__ q, int ldq, void* __restrict
       mxA = fmaxf(mxA, __shfl_xor_sync(0xffffffffu, mxA, 2));
       mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 1));
       mxB = fmaxf(mxB, __shfl_xor_sync(0xffffffffu, mxB, 2));
-      const float nmA = fmaxf(mA, mxA), nmB = fmaxf(mB, mxB);
-      const float refA = nmA == -CUDART_INF_F ? 0.f : nmA, refB = nmB == -CUDART_INF_F ? 0.f : nmB;  // a row that sees no key yet
+      // (a row that sees no key yet: -inf stays its maximum, 0 its reference)
+      const float nmA = mxA == -CUDART_INF_F ? mA : fmaxf(mA, mxA * scale2), nmB = mxB == -CUDART_INF_F ? mB : fmaxf(mB, mxB * scale2);
+      const float refA = nmA == -CUDART_INF_F ? 0.f : nmA, refB = nmB == -CUDART_INF_F ? 0.f : nmB;
       const float corrA = exp2f(mA - refA), corrB = exp2f(mB - refB);  // exp2(-inf) = 0 on the first page
-      float sumA = 0.f, sumB = 0.f;
+      lA *= corrA;
+      lB *= corrB;
 #pragma unroll
       for (int nt = 0; nt < 8; ++nt) {
-        s[nt][0] = exp2f(s[nt][0] - refA);
-        s[nt][1] = exp2f(s[nt][1] - refA);
-        s[nt][2] = exp2f(s[nt][2] - refB);
-        s[nt][3] = exp2f(s[nt][3] - refB);
-        sumA += s[nt][0] + s[nt][1];
-        sumB += s[nt][2] + s[nt][3];
+        s[nt][0] = sp_exp2(fmaf(s[nt][0], scale2, -refA));
+        s[nt][1] = sp_exp2(fmaf(s[nt][1], scale2, -refA));
+        s[nt][2] = sp_exp2(fmaf(s[nt][2], scale2, -refB));
+        s[nt][3] = sp_exp2(fmaf(s[nt][3], scale2, -refB));
+        lA += s[nt][0] + s[nt][1];
+        lB += s[nt][2] + s[nt][3];
       }
-      sumA += __shfl_xor_sync(0xffffffffu, sumA, 1);
-      sumA += __shfl_xor_sync(0xffffffffu, sumA, 2);
-      sumB += __shfl_xor_sync(0xffffffffu, sumB, 1);
-      sumB += __shfl_xor_sync(0xffffffffu, sumB, 2);
-      lA = lA * corrA + sumA;
-      lB = lB * corrB + sumB;
       mA = nmA;
       mB = nmB;
       if (__any_sync(0xffffffffu, corrA != 1.f || corrB != 1.f)) {   // some row's maximum moved: rescale what is gathered
@@ -242,6 +242,10 @@ attn_prefill_split_kernel(const float* __restrict__ q, int ldq, void* __restrict
     }
     group_sync();  // this stage is free for the page after next
   }
+  lA += __shfl_xor_sync(0xffffffffu, lA, 1);
+  lA += __shfl_xor_sync(0xffffffffu, lA, 2);
+  lB += __shfl_xor_sync(0xffffffffu, lB, 1);
+  lB += __shfl_xor_sync(0xffffffffu, lB, 2);
   if (NG > 1) {
     // ---- merge the groups: groups 1.. leave (max, sum, output) in shared memory, group 0 folds them in order
     __syncthreads();

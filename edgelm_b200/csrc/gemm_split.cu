@@ -34,6 +34,7 @@
 // multiply-adds, so they come out as the CUDA-core kernels give them.
 #include <cooperative_groups.h>
 
+#include "mma_split.cuh"
 #include "tc_common.cuh"
 
 namespace edgelm {
@@ -49,32 +50,8 @@ template <int BN> constexpr int sp_split_groups() { return BN == 64 ? 2 : 4; }  
 template <int BN> constexpr int sp_threads() { return 64 + 128 * sp_split_groups<BN>() + 256; }
 template <int BN> constexpr int sp_slot_bytes() { return SP_W_BYTES + BN * 128; }
 template <int BN> constexpr int sp_term_bytes() { return BN * 128; }
-template <int BN> constexpr size_t sp_smem() { return 1024 + 6 * sp_term_bytes<BN>() + sp_slots<BN>() * sp_slot_bytes<BN>() + 512; }
+template <int BN> constexpr size_t split_smem() { return 1024 + 6 * sp_term_bytes<BN>() + sp_slots<BN>() * sp_slot_bytes<BN>() + 512; }
 
-__device__ __forceinline__ uint32_t pack_bf16(float lo, float hi) {
-  const __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
-  return *reinterpret_cast<const uint32_t*>(&v);
-}
-// two neighbouring k's -> their three terms, packed.  (What a term leaves is exact; both of a pair in one packed multiply-add.)
-__device__ __forceinline__ uint32_t next_term(unsigned long long& xy) {
-  uint32_t t;
-  asm("{\n\t.reg .b32 x, y, hx, hy;\n\t.reg .b64 h;\n\t"
-      "mov.b64 {x, y}, %1;\n\t"
-      "cvt.rn.bf16x2.f32 %0, y, x;\n\t"
-      "shl.b32 hx, %0, 16;\n\t"
-      "and.b32 hy, %0, 0xffff0000;\n\t"
-      "mov.b64 h, {hx, hy};\n\t"
-      "fma.rn.f32x2 %1, h, %2, %1;\n\t}"
-      : "=&r"(t), "+l"(xy)
-      : "l"(0xbf800000bf800000ull));
-  return t;
-}
-__device__ __forceinline__ void split_pair(float x, float y, uint32_t& t1, uint32_t& t2, uint32_t& t3) {
-  unsigned long long xy = (unsigned long long)__float_as_uint(y) << 32 | __float_as_uint(x);
-  t1 = next_term(xy);
-  t2 = next_term(xy);
-  t3 = pack_bf16(__uint_as_float((uint32_t)xy), __uint_as_float((uint32_t)(xy >> 32)));
-}
 __device__ __forceinline__ void mbar_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void tmem_st8(uint32_t taddr, const uint32_t* r) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
@@ -257,8 +234,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
 #pragma unroll
         for (int u = 0; u < 4; ++u) {
           const float4 v = row[(g * 4 + u) ^ (w_row & 7)];
-          split_pair(v.x, v.y, t[0][2 * u], t[1][2 * u], t[2][2 * u]);
-          split_pair(v.z, v.w, t[0][2 * u + 1], t[1][2 * u + 1], t[2][2 * u + 1]);
+          sp_split(v.x, v.y, t[0][2 * u], t[1][2 * u], t[2][2 * u]);
+          sp_split(v.z, v.w, t[0][2 * u + 1], t[1][2 * u + 1], t[2][2 * u + 1]);
         }
 #pragma unroll
         for (int q = 0; q < 3; ++q) tmem_st8(tmem + lanes + SP_A_BASE + st * SP_A_COLS + q * 32 + half * 16 + g * 8, t[q]);
@@ -269,10 +246,10 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap map_w, const __grid_consta
         const float4* ar = reinterpret_cast<const float4*>(slot + SP_W_BYTES + r * 128);
         const float4 v = ar[(2 * p) ^ (r & 7)], w = ar[(2 * p + 1) ^ (r & 7)];
         uint4 t1, t2, t3;
-        split_pair(v.x, v.y, t1.x, t2.x, t3.x);
-        split_pair(v.z, v.w, t1.y, t2.y, t3.y);
-        split_pair(w.x, w.y, t1.z, t2.z, t3.z);
-        split_pair(w.z, w.w, t1.w, t2.w, t3.w);
+        sp_split(v.x, v.y, t1.x, t2.x, t3.x);
+        sp_split(v.z, v.w, t1.y, t2.y, t3.y);
+        sp_split(w.x, w.y, t1.z, t2.z, t3.z);
+        sp_split(w.z, w.w, t1.w, t2.w, t3.w);
         uint8_t* dst = smem + st * 3 * TERM + r * 128 + ((half * 4 + p) ^ (r & 7)) * 16;
         *reinterpret_cast<uint4*>(dst) = t1;
         *reinterpret_cast<uint4*>(dst + TERM) = t2;
@@ -381,7 +358,7 @@ template <int BN, int EPI>
 int launch_split(const float* a, int lda, const float* w, const float* w2, float* out, int ldo, const float* residual, int M, int N, int K,
                  int CS, int* err, cudaStream_t stream) {
   constexpr int NOUT = EPI == EPI_SWIGLU ? SP_ROWS / 2 : SP_ROWS;
-  constexpr size_t smem = sp_smem<BN>();
+  constexpr size_t smem = split_smem<BN>();
   CUtensorMap mw, mw2, ma;
   if (tensor_map(w, N, K, K, NOUT, &mw, 4)) return -1;
   mw2 = mw;

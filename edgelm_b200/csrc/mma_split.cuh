@@ -27,16 +27,33 @@ __device__ __forceinline__ void sp_cp16(uint32_t dst, const void* src, int src_b
 }
 
 // Two float32 values as three packed pairs of bfloat16 terms: x = t1 + t2 + t3 up to float32 rounding (each term the
-// rounding of what the terms before left over; the remainders are exact in float32).
+// rounding of what the terms before left over; the remainders are exact in float32).  Both values of a pair in one conversion and one
+// packed multiply-add a term: 9 instructions a pair (17 with a conversion a value; the attention below was bound by these).
+__device__ __forceinline__ uint32_t sp_next_term(unsigned long long& xy) {
+  uint32_t t;
+  asm("{\n\t.reg .b32 x, y, hx, hy;\n\t.reg .b64 h;\n\t"
+      "mov.b64 {x, y}, %1;\n\t"
+      "cvt.rn.bf16x2.f32 %0, y, x;\n\t"
+      "shl.b32 hx, %0, 16;\n\t"
+      "and.b32 hy, %0, 0xffff0000;\n\t"
+      "mov.b64 h, {hx, hy};\n\t"
+      "fma.rn.f32x2 %1, h, %2, %1;\n\t}"
+      : "=&r"(t), "+l"(xy)
+      : "l"(0xbf800000bf800000ull));
+  return t;
+}
 __device__ __forceinline__ void sp_split(float x, float y, uint32_t& t1, uint32_t& t2, uint32_t& t3) {
-  const __nv_bfloat16 x1 = __float2bfloat16_rn(x), y1 = __float2bfloat16_rn(y);
-  const float xr = x - __bfloat162float(x1), yr = y - __bfloat162float(y1);
-  const __nv_bfloat16 x2 = __float2bfloat16_rn(xr), y2 = __float2bfloat16_rn(yr);
-  const __nv_bfloat16 x3 = __float2bfloat16_rn(xr - __bfloat162float(x2)), y3 = __float2bfloat16_rn(yr - __bfloat162float(y2));
-  const __nv_bfloat162 p1 = __halves2bfloat162(x1, y1), p2 = __halves2bfloat162(x2, y2), p3 = __halves2bfloat162(x3, y3);
-  t1 = *reinterpret_cast<const uint32_t*>(&p1);
-  t2 = *reinterpret_cast<const uint32_t*>(&p2);
-  t3 = *reinterpret_cast<const uint32_t*>(&p3);
+  unsigned long long xy = (unsigned long long)__float_as_uint(y) << 32 | __float_as_uint(x);
+  t1 = sp_next_term(xy);
+  t2 = sp_next_term(xy);
+  const __nv_bfloat162 last = __floats2bfloat162_rn(__uint_as_float((uint32_t)xy), __uint_as_float((uint32_t)(xy >> 32)));
+  t3 = *reinterpret_cast<const uint32_t*>(&last);
+}
+// 2^x on the special-function unit (results under 2^-126 count as zero)
+__device__ __forceinline__ float sp_exp2(float x) {
+  float y;
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
+  return y;
 }
 
 }  // namespace edgelm

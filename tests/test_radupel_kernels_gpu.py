@@ -426,6 +426,26 @@ def test_tensor_core_attention_keeps_float32_scores_and_weights():
     assert ours < 6e-3 and theirs > 5 * ours, (ours, theirs)       # (6e-3: the output's own rounding to bfloat16)
 
 
+@pytest.mark.parametrize("scale", [-0.2, 0.0, 0.125])
+def test_tensor_core_attention_scale_of_any_sign(scale):
+    """The running maximum is one of unscaled scores: against the CUDA-core kernel, which scales first."""
+    g = np.random.default_rng(6)
+    H, G, d, n = 3, 1, 64, 190
+    q = f32(g.normal(size=(n, H * d)) * 4.0)
+    kv = PagedKV([n], G, d, d, torch.bfloat16, seed=2)
+    kv.put(0, g.normal(size=(n, G, d)), g.normal(size=(n, G, d)))
+    outs = []
+    for tile, fn in ((ops.SPLIT_PREFILL_TILE, ops.attn_prefill_split), (8, ops.masked_attn_tiled)):
+        tiles = make_tiles([n], [0], tile)
+        out = torch.full((n, H * d), float("nan"), dtype=torch.bfloat16, device=DEV)
+        extra = (8,) if fn is ops.masked_attn_tiled else ()
+        rest = (ops.MASK_CAUSAL, 0, None) if extra else ()
+        fn(q, out, kv.k, kv.v, i32(kv.table), *tiles, *extra, H, G, d, d, scale, *rest)
+        outs.append(out.float())
+    # (both round to bfloat16: a difference of one step of 2^-8)
+    assert float((outs[0] - outs[1]).abs().max()) <= 2.0 ** -7 * float(outs[1].abs().max())
+
+
 # ----------------------------------------------------------------------------- the scoring router and its experts
 @pytest.mark.parametrize("E,ident,top,groups,keep,negative", [(6, 3, 3, 3, 2, False), (3, 0, 1, 1, 1, False), (5, 1, 2, 2, 1, True), (7, 2, 2, 3, 1, True),
                                                               (8, 0, 4, 4, 2, False), (2, 2, 2, 1, 1, True), (12, 4, 3, 8, 2, False), (4, 2, 3, 3, 1, True)])
