@@ -338,6 +338,27 @@ def attn_prefill_mma(qkv, out, kcache, vcache, page_table, seq_slot, tile_seq, t
                                          int(force_groups), _stream()))
 
 
+F32_PREFILL_TILE = 64  # new tokens per tile of the float32 tensor-core prefill kernel (AF_ROWS in attention_f32.cu)
+
+
+def attn_prefill_f32_takes(dtype, hd):
+    """Whether the tensor-core prefill attention of float32 models takes this dtype and head size (float32; 32, 64, 96, 128)."""
+    return dtype == torch.float32 and bool(lib().edgelm_attn_prefill_f32_takes(int(hd)))
+
+
+def attn_prefill_f32(qkv, out, kcache, vcache, page_table, seq_slot, tile_seq, tile_tok0, tile_ntok, tile_pos0, n_tiles, nh, nkv, hd, scale):
+    """Causal attention of new tokens over a paged float32 cache on mma.sync tensor cores, three bfloat16 terms an operand; tiles of
+    at most 64 tokens."""
+    _need(qkv.dtype == out.dtype == kcache.dtype == vcache.dtype == torch.float32 and qkv.stride(1) == 1 and out.stride(1) == 1 and
+          kcache.is_contiguous() and vcache.is_contiguous(), "attn_prefill_f32: layout")
+    for t, n in ((page_table, "page_table"), (seq_slot, "seq_slot"), (tile_seq, "tile_seq"), (tile_tok0, "tile_tok0"),
+                 (tile_ntok, "tile_ntok"), (tile_pos0, "tile_pos0")):
+        _i32(t, n)
+    _check(lib().edgelm_attn_prefill_f32(_p(qkv), qkv.stride(0), _p(out), out.stride(0), _p(kcache), _p(vcache), _p(page_table), page_table.stride(0),
+                                         _p(seq_slot), _p(tile_seq), _p(tile_tok0), _p(tile_ntok), _p(tile_pos0), n_tiles, nh, nkv, hd,
+                                         ctypes.c_float(scale), _stream()))
+
+
 TC_PREFILL_TILE = 128  # new tokens per tile of the tcgen05 prefill kernel (AT_ROWS in attention_tc.cu)
 
 

@@ -43,6 +43,7 @@ class Attention(Part):
         self.w_qkv = self.w_o = None
         self._mma = None  # whether the mma.sync prefill kernel takes this head size (asked once a device is there)
         self._tc = None   # whether the tcgen05 prefill kernel does
+        self._f32 = None  # whether the float32 models' tensor-core prefill kernel does
 
     def sizes(self):
         out = {"heads": self.nh, "kv_heads": self.nkv, "head_dim": self.hd, **self.positions.sizes()}
@@ -92,7 +93,7 @@ class Attention(Part):
         sizes = ()
         if self._tc_prefill():
             sizes += (ops.TC_PREFILL_TILE,)
-        return sizes + ((ops.MMA_PREFILL_TILE,) if self._mma_prefill() else (self.tile_tokens,))
+        return sizes + ((ops.MMA_PREFILL_TILE,) if self._mma_prefill() else (ops.F32_PREFILL_TILE,) if self._f32_prefill() else (self.tile_tokens,))
 
     def _mma_prefill(self):
         if self._mma is None:   # (the tensor-core kernels have no lower key bound: a windowed mixer stays on the CUDA cores)
@@ -103,6 +104,11 @@ class Attention(Part):
         if self._tc is None:
             self._tc = self.window is None and ops.attn_prefill_tc_takes(self.dtype, self.hd)
         return self._tc
+
+    def _f32_prefill(self):
+        if self._f32 is None:
+            self._f32 = self.window is None and ops.attn_prefill_f32_takes(self.dtype, self.hd)
+        return self._f32
 
     def workspace_bytes(self, n_tokens, n_seqs):
         qkv = nbytes((n_tokens, (self.nh + 2 * self.nkv) * self.hd), self.dtype)
@@ -171,6 +177,11 @@ class Attention(Part):
                 ops.attn_prefill_mma(qkv, a, cache.k, cache.v, table, ctx.seq_index, tiles.seq, tiles.tok0, tiles.ntok,
                                      tiles.pos0, tiles.count, self.nh, self.nkv, self.hd, self.scale,
                                      max_keys=max(p + n for p, n in zip(ctx.seq_first_positions, ctx.seq_lengths)))
+        elif self._f32_prefill():
+            tiles = ctx.tiles(ops.F32_PREFILL_TILE)
+            with ctx.prof("attn_prefill"):
+                ops.attn_prefill_f32(qkv, a, cache.k, cache.v, table, ctx.seq_index, tiles.seq, tiles.tok0, tiles.ntok, tiles.pos0,
+                                     tiles.count, self.nh, self.nkv, self.hd, self.scale)
         else:
             tiles = ctx.tiles(self.tile_tokens)
             with ctx.prof("attn_prefill"):

@@ -992,6 +992,42 @@ def test_attn_prefill_mma(nh, nkv, hd, groups):
         t0 += n
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(3, 1, 64), (4, 4, 32), (2, 1, 96), (6, 2, 128)])
+def test_attn_prefill_f32(nh, nkv, hd):
+    """Float32 attention on the tensor cores: whole and continued prompts, tiles' and pages' edges, scores of a good size.  Per output:
+    a score's head size / 16 + 5 cut-offs and the exponent's rounding, each 2^-23 of scores up to 16 log2(e), dominate: 2^-23 x 23 x
+    sqrt(13) = 1e-5 of a weight at most; the 2-norm over all (most scores are small) stays under a tenth, and under the CUDA cores'."""
+    o = ops()
+    assert o.attn_prefill_f32_takes(torch.float32, hd) and not o.attn_prefill_f32_takes(torch.float32, 48)
+    assert not o.attn_prefill_f32_takes(torch.bfloat16, hd)
+    seqs = [(0, 5), (0, 70), (64, 1), (100, 129), (63, 2), (0, 64), (30, 200)]  # (cached before, new tokens)
+    lengths = [a + b for a, b in seqs]
+    case = PagedCase(o, torch.float32, lengths, nkv, hd, seed=nh * 10 + hd)
+    T = sum(b for _, b in seqs)
+    qkv = rnd((T, (nh + 2 * nkv) * hd), torch.float32, 81, 3.0)
+    mk = lambda x: torch.tensor(x, dtype=torch.int32, device=dev())
+    got = {}
+    for tq in (o.F32_PREFILL_TILE, max(1, 32 // (nh // nkv))):
+        tiles, t0 = [], 0
+        for s, (p0, n) in enumerate(seqs):
+            tiles += [(s, t0 + a, min(tq, n - a), p0 + a) for a in range(0, n, tq)]
+            t0 += n
+        out = torch.full((T, nh * hd), float("nan"), device=dev())
+        args = (qkv, out, case.kcache, case.vcache, case.table, case.seq_slot, *(mk([t[i] for t in tiles]) for i in range(4)), len(tiles))
+        if tq == o.F32_PREFILL_TILE:
+            o.attn_prefill_f32(*args, nh, nkv, hd, 1.0 / math.sqrt(hd))
+        else:
+            o.attn_prefill(*args, tq, nh, nkv, hd, 1.0 / math.sqrt(hd))
+        got[tq] = out.double().cpu()
+    t0, want = 0, []
+    for s, (p0, n) in enumerate(seqs):
+        want.append(attention_rows(qkv[t0:t0 + n, :nh * hd].cpu(), case.k[s], case.v[s], p0, nh, nkv, hd))
+        t0 += n
+    want = torch.cat(want)
+    errs = [float((x.reshape(want.shape) - want).norm() / want.norm()) for x in got.values()]
+    assert errs[0] < 1e-6 and errs[0] <= errs[1], errs
+
+
 def test_attn_prefill_mma_far_key_and_diagonal():
     """Scaled queries make one early key, or the token's own key, dominate: a wrong mask or page shows."""
     o = ops()
