@@ -169,9 +169,10 @@ class StateGroup:
         if device is not None:
             self.state = torch.zeros((n_entries, n_slots) + tuple(need.shape), dtype=torch.float32, device=device)
 
-    def reset(self, slot):
+    def reset(self, slot, n=1):
+        """The states of `n` slots from `slot` on start at zero."""
         if self.state is not None:
-            self.state[:, slot].zero_()
+            self.state[:, slot:slot + n].zero_()
 
 
 class SequenceCache:
@@ -240,12 +241,24 @@ class SequenceCache:
     # ------------------------------------------------------------------ sequences
     def open(self):
         """A slot for a new sequence of length 0."""
+        return self.open_many(1)[0]
+
+    def open_many(self, n):
+        """Slots for `n` new sequences of length 0; the states of neighbouring slots are zeroed together."""
         self._quiet = None
-        slot = self.slots.take()
-        self.length[slot] = 0
-        for g in self.state_groups:
-            g.reset(slot)
-        return slot
+        slots = []
+        try:
+            for _ in range(n):
+                slots.append(self.slots.take())
+        finally:     # (also the slots that were taken before there was none left)
+            run = 0
+            for i, slot in enumerate(slots):
+                self.length[slot] = 0
+                if i + 1 == len(slots) or slots[i + 1] != slot + 1:
+                    for g in self.state_groups:
+                        g.reset(slots[run], i + 1 - run)
+                    run = i + 1
+        return slots
 
     def _held(self, slot):
         if slot not in self.slots._held:

@@ -96,6 +96,23 @@ def _i32(t, name):
     _need(t.dtype == torch.int32 and t.is_cuda and t.is_contiguous(), f"{name} must be a contiguous int32 CUDA tensor")
 
 
+def lay_out_step(host, ids, ntok, pos0, slots, want, tables, tile_sizes):
+    """A step's metadata into the int32 NumPy array `host` (its sections: `edgelm_lay_out_step` in runtime.cu); returns the sections' first
+    words and the end.  ids, ntok, pos0, slots, want: contiguous int64 NumPy arrays; tables: contiguous int32 [slots, pages] ones."""
+    address = lambda a: a.__array_interface__["data"][0]
+    n, t = len(tables), len(tile_sizes)
+    ints = lambda values: (ctypes.c_int * max(1, len(values)))(*values)
+    pointers = (ctypes.c_void_p * max(1, n))(*(address(a) for a in tables))
+    sections = 7 + n + (4 * t if len(ids) != len(ntok) else 0)
+    first = (ctypes.c_int64 * (sections + 1))()
+    rc = lib().edgelm_lay_out_step(ctypes.c_void_p(address(host)), ctypes.c_longlong(host.size), ctypes.c_void_p(address(ids)), ctypes.c_longlong(len(ids)),
+                                   ctypes.c_void_p(address(ntok)), ctypes.c_void_p(address(pos0)), ctypes.c_void_p(address(slots)), len(ntok),
+                                   ctypes.c_void_p(address(want)), len(want), n, pointers, ints([a.shape[1] for a in tables]),
+                                   ints([a.shape[0] for a in tables]), t, ints(tile_sizes), first)
+    _check(rc, launches=0)
+    return list(first)
+
+
 def embed_gather(ids, table, x, err, scale=1.0):
     """x[t, :] = table[ids[t], :] * scale as float32; ids outside the table set bit 1 of `err`."""
     _i32(ids, "ids")

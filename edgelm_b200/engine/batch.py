@@ -13,6 +13,7 @@ from dataclasses import dataclass
 import numpy as np
 import torch
 
+from ..csrc import ops
 from .profiler import NULL_PROFILER
 
 
@@ -147,7 +148,6 @@ class BatchBuffers:
         self.last_bytes = 0
         self._copied = torch.cuda.Event()
         self._decode = None   # layout of the last step if it was one token per sequence: lets the next one be patched in place
-        self._tile_cols = {}  # (tokens per sequence, first positions, tile size) -> the tiles' four columns: shapes come back
 
     def fill(self, ctx, token_ids, seq_slots, seq_ntok, seq_pos0, want_rows, cache):
         """Lay out the step and copy it; sets every tensor of `ctx` (views of the device buffer)."""
@@ -156,51 +156,19 @@ class BatchBuffers:
             raise ValueError(f"a step of {T} tokens, {B} sequences and {R} wanted rows exceeds the buffers "
                              f"({self.max_tokens}, {self.max_seqs}, {self.max_want})")
         self._copied.synchronize()  # the previous step's copy has read the staging buffer
-        h = self.host_np
-        ntok = np.asarray(seq_ntok, dtype=np.int64)
-        pos0 = np.asarray(seq_pos0, dtype=np.int64)
-        o = 0
-        views = {}
-
-        def put(name, arr, n):
-            nonlocal o
-            h[o:o + n] = arr
-            views[name] = (o, n)
-            o += n
-
-        put("token_ids", np.asarray(token_ids, dtype=np.int32), T)
-        seq_of_tok = np.repeat(np.arange(B, dtype=np.int32), ntok)
-        starts = np.concatenate([[0], np.cumsum(ntok)[:-1]])
-        put("tok_pos", (np.arange(T, dtype=np.int64) - np.repeat(starts, ntok) + np.repeat(pos0, ntok)).astype(np.int32), T)
-        put("tok_seq", seq_of_tok, T)
-        put("seq_pos", (pos0 + ntok - 1).astype(np.int32), B)
-        put("seq_tok0", np.concatenate([starts, [T]]).astype(np.int32), B + 1)
-        put("want_rows", np.asarray(want_rows, dtype=np.int32), R)
-        slots = np.asarray(seq_slots, dtype=np.int64)
-        put("seq_slots", slots.astype(np.int32), B)
-        for g in self.groups:
-            s = self.stride[g.id]
-            put(("table", g.id), g.table[slots].reshape(-1), B * s)
-        tile_counts = {}
+        column = lambda values: np.ascontiguousarray(values, dtype=np.int64)
+        ntok, pos0, slots = column(seq_ntok), column(seq_pos0), column(seq_slots)
+        first = ops.lay_out_step(self.host_np, column(token_ids), ntok, pos0, slots, column(want_rows), [g.table for g in self.groups], self.tile_sizes)
+        names = ["token_ids", "tok_pos", "tok_seq", "seq_pos", "seq_tok0", "want_rows", "seq_slots"] + [("table", g.id) for g in self.groups]
         if T != B:  # steps of one token per sequence use no tiles
-            shape = (tuple(int(v) for v in ntok), tuple(int(v) for v in pos0))
-            for ts in self.tile_sizes:
-                cols = self._tile_cols.get(shape + (ts,))
-                if cols is None:
-                    if len(self._tile_cols) >= 64:
-                        self._tile_cols.clear()
-                    cols = [np.asarray(col, dtype=np.int32) for col in make_tiles(list(shape[0]), list(shape[1]), ts)]
-                    self._tile_cols[shape + (ts,)] = cols
-                tile_counts[ts] = len(cols[0])
-                for j, col in enumerate(cols):
-                    put(("tiles", ts, j), col, len(col))
+            names += [("tiles", ts, j) for ts in self.tile_sizes for j in range(4)]
+        o = first[-1]
         self.dev[:o].copy_(self.host[:o], non_blocking=True)
         self._copied.record()
         self.last_bytes = o * 4
-
-        def view(name):
-            a, n = views[name]
-            return self.dev[a:a + n]
+        views = {name: (a, b - a) for name, a, b in zip(names, first, first[1:])}
+        parts = dict(zip(names, self.dev[:o].split([n for _, n in views.values()])))
+        view = parts.__getitem__
 
         ctx.n_tokens, ctx.n_seqs = T, B
         ctx.all_single = bool(T == B and T > 0)
@@ -209,13 +177,12 @@ class BatchBuffers:
         ctx.seq_tok0 = view("seq_tok0")
         ctx.seq_index = self.seq_index_full[:B]
         ctx._tables = {g.id: view(("table", g.id)).view(B, self.stride[g.id]) for g in self.groups}
-        ctx._tiles = {ts: Tiles(view(("tiles", ts, 0)), view(("tiles", ts, 1)), view(("tiles", ts, 2)), view(("tiles", ts, 3)), n)
-                      for ts, n in tile_counts.items()}
-        ctx._seq_ntok, ctx._seq_pos0 = [int(x) for x in ntok], [int(x) for x in pos0]
+        ctx._tiles = {ts: Tiles(*(view(("tiles", ts, j)) for j in range(4)), views[("tiles", ts, 0)][1]) for ts in self.tile_sizes} if T != B else {}
+        ctx._seq_ntok, ctx._seq_pos0 = ntok.tolist(), pos0.tolist()
         ctx.seq_slots = view("seq_slots")
         self._decode = None
         if T == B and R == B:
-            self._decode = {"slots": list(seq_slots), "pos": [int(x) for x in pos0], "views": views, "words": o,
+            self._decode = {"slots": list(seq_slots), "pos": pos0.tolist(), "views": views, "words": o,
                             "version": {g.id: g.version for g in self.groups}, "slot_index": slots}
         return ctx
 

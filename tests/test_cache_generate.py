@@ -1,6 +1,7 @@
 """Host-side bookkeeping: the cache's slots and pages, and the generation loop's decisions."""
 import random
 
+import numpy as np
 import pytest
 
 from edgelm_b200.cache import CacheError, FreeList, SequenceCache, pages_for
@@ -212,6 +213,61 @@ def test_sampling_params_and_stream():
     x = s.state
     s.sample([0.0, 1.0, 2.0])
     assert xorshift64(x) == s.state
+
+
+@pytest.mark.parametrize("ntok,pos0,tiles", [([1], [0], [64]), ([5], [0], []), ([1, 1, 1], [3, 0, 200], [64, 16]), ([64, 65, 1, 130], [0, 7, 63, 64], [16, 64, 128]),
+                                             ([2048], [100], [3])])
+def test_a_steps_layout(ntok, pos0, tiles):
+    """The native layout of a step's metadata, section by section, against its definition."""
+    from edgelm_b200.csrc import ops
+    from edgelm_b200.engine.batch import make_tiles
+    rng = np.random.default_rng(len(ntok))
+    B, T = len(ntok), sum(ntok)
+    tables = [rng.integers(0, 99, (B + 2, 7)).astype(np.int32), rng.integers(0, 99, (B + 3, 4)).astype(np.int32)]
+    slots, want, ids = rng.permutation(B + 2)[:B].astype(np.int64), np.array([T - 1, 0], dtype=np.int64), rng.integers(0, 50000, T)
+    starts = np.concatenate([[0], np.cumsum(ntok)])
+    sections = [ids, np.concatenate([np.arange(p, p + n) for n, p in zip(ntok, pos0)]), np.repeat(np.arange(B), ntok), np.add(pos0, ntok) - 1, starts, want, slots]
+    sections += [t[slots].reshape(-1) for t in tables]
+    if T != B:
+        sections += [col for size in tiles for col in make_tiles(ntok, pos0, size)]
+    words = sum(len(x) for x in sections)
+    host = np.full(words + 3, -7, dtype=np.int32)
+    column = lambda a: np.array(a, dtype=np.int64)
+    first = ops.lay_out_step(host, ids, column(ntok), column(pos0), slots, want, tables, tiles)
+    assert first[-1] == words and len(first) == len(sections) + 1
+    for a, b, x in zip(first, first[1:], sections):
+        assert host[a:b].tolist() == list(x)
+    assert (host[words:] == -7).all()
+    for args in ((host[:words - 1], ids, column(ntok), slots), (host, ids[:-1], column(ntok), slots), (host, ids, column(ntok), slots + 99)):
+        before = host.copy()
+        with pytest.raises(ops.KernelError):
+            ops.lay_out_step(args[0], args[1], args[2], column(pos0), args[3], want, tables, tiles)
+        assert (host == before).all()
+
+
+def test_token_ids_from_any_sequence():
+    from edgelm_b200.engine.engine import _as_ids
+    for n in (3, 200):
+        ids = list(range(n))
+        for tokens in (ids, tuple(ids), np.array(ids, dtype=np.int32), [np.int64(i) for i in ids], [float(i) for i in ids]):
+            got = _as_ids(tokens)
+            assert got.dtype == np.int64 and got.tolist() == ids
+        with pytest.raises(OverflowError):
+            _as_ids([2 ** 70] * n)
+        assert _as_ids([[1, 2]] * n).ndim == 2
+
+
+def test_slots_opened_together():
+    needs = [StateNeed((2,)), KVNeed(1, 16)]
+    cache = SequenceCache(needs, 4 * 64, 256, device="cpu", max_seqs=4)
+    state = cache.state_groups[0].state
+    state.fill_(1.0)
+    assert cache.open_many(2) == [0, 1] and cache.open() == 2
+    cache.close(0)
+    state.fill_(1.0)
+    with pytest.raises(CacheError):       # two are free, the third is not: the two are held (and start at zero) as one by one
+        cache.open_many(3)
+    assert state[:, [0, 3]].eq(0).all() and state[:, [1, 2]].eq(1).all() and cache.slots.held() == {0, 1, 2, 3}
 
 
 def test_decode_splits_rule():
