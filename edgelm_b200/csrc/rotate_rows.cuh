@@ -1,10 +1,13 @@
 // Prompt steps: projections of many tokens through bias, filter over time, norm and rotation into queries and cache rows, for heads of
 // whole runs of 32 dimensions.  A warp owns one unit (a query head, a key head, or as many value channels) of ROT_TOKENS consecutive
-// tokens: lane l holds the dimensions l, l + 32, ... in registers, a rotation's partner lies in the same lane or a shuffle away, the
-// filter's taps and inputs stay in registers from token to token, and the angles' sines and cosines are computed once a token and block.
+// tokens: lane l holds the run of dk / 32 dimensions from l dk / 32 on (one access of 8 or 16 bytes a token where rows are aligned to a
+// run; a rotation's partner is one shuffle away, or in the lane), the filter's taps and inputs stay in registers from token to token, and the
+// angles' sines and cosines are computed once a token and block, while the rows, the three in front and the taps are on their way.
 // (A token a block, every element computing its own angle and reading its filter's inputs anew, took 271 us for 3,900 tokens of 16 heads
-// of two maps of 64 with three taps; this 156; 2,048 tokens of 64 heads of 64 94 and 45.)  The projection is read once, queries and cache rows are written once: at 45 us
-// about 1.1 TB/s, so what takes the time is a warp's chain of eight tokens and its instructions, not memory.
+// of two maps of 64 with three taps; dimensions l, l + 32, ... a lane 171, runs 104: a norm's sum is 4 shuffles instead of 20, a
+// partner needs no selection.  2,048 tokens of 64 heads of 64: 44 and 37.)  At 1.5 to 2.3 TB/s: angles, filter and norm
+// are a fifth, a fifth and an eighth of the time (the longer case without them: 45 us, 3.5 TB/s), and 16 warps an SM what 127 registers leave room
+// for; a loop over the tokens with three rows on their way holds more warps and takes 5 to 10 % longer.
 #pragma once
 #include "common.cuh"
 
@@ -38,19 +41,77 @@ constexpr int ROT_BLOCKS = 450;
 // whether the kernel takes these sizes (dk: what a head's queries and a key row hold, all maps)
 inline bool rotate_rows_takes(int n_tokens, int H, int G, int dk, int dv, int maps, int rot, int interleaved, int taps) {
   if (dk < 1 || (long long)((n_tokens + ROT_TOKENS - 1) / ROT_TOKENS) * ((H + G + G * dv / dk + ROT_WARPS - 1) / ROT_WARPS) < ROT_BLOCKS) return false;
-  if (n_tokens <= 64 || dk % 32 || dk > 128 || maps < 1 || dk % maps || (dk / maps) % 32 || rot > 128 || (G * dv) % dk || taps > 4) return false;
-  const int half = rot / 2;
-  return rot == 0 || interleaved || half % 32 == 0 || (half < 32 && (half & (half - 1)) == 0);
+  if (n_tokens <= 64 || dk % 32 || dk > 128 || maps < 1 || dk % maps || (dk / maps) % 32 || (dk == 96 && maps > 1) || rot > 128 || (G * dv) % dk || taps > 4) return false;
+  return true;
 }
 
+// M consecutive values from or to memory, in one access where `whole` says that they lie aligned to their size (M 2 or 4)
+template <int M>
+__device__ __forceinline__ void load_run(const float* p, bool whole, float* v) {
+  if (M == 4 && whole) {
+    const float4 x = *reinterpret_cast<const float4*>(p);
+    v[0] = x.x; v[M > 1 ? 1 : 0] = x.y; v[M > 2 ? 2 : 0] = x.z; v[M > 3 ? 3 : 0] = x.w;
+  } else if (M == 2 && whole) {
+    const float2 x = *reinterpret_cast<const float2*>(p);
+    v[0] = x.x; v[M > 1 ? 1 : 0] = x.y;
+  } else {
+#pragma unroll
+    for (int m = 0; m < M; ++m) v[m] = p[m];
+  }
+}
+template <int M, typename T>
+__device__ __forceinline__ void store_run(T* p, bool whole, const float* v) {
+  if (M == 4 && whole) store_piece(p, make_float4(v[0], v[M > 1 ? 1 : 0], v[M > 2 ? 2 : 0], v[M > 3 ? 3 : 0]));
+  else if (M == 2 && whole && sizeof(T) == 4) *reinterpret_cast<float2*>(p) = make_float2(v[0], v[M > 1 ? 1 : 0]);
+  else if (M == 2 && whole) *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(v[0], v[M > 1 ? 1 : 0]);
+  else {
+#pragma unroll
+    for (int m = 0; m < M; ++m) p[m] = from_f32<T>(v[m]);
+  }
+}
+
+// Whole runs: bit 0 the projections' rows, bit 1 the queries, bit 2 the cache's rows are aligned to a run of M.
 template <typename T, typename TQ, int M>      // M = dk / 32
 __global__ void __launch_bounds__(ROT_WARPS * 32)
-rotate_rows_kernel(const RotateRows a, TQ* __restrict__ q_out, T* __restrict__ kcache, T* __restrict__ vcache) {
+rotate_rows_kernel(const RotateRows a, TQ* __restrict__ q_out, T* __restrict__ kcache, T* __restrict__ vcache, int whole) {
   pdl_launch_dependents();
   pdl_wait();
   __shared__ float2 turn[ROT_TOKENS][64];
-  __shared__ int place[ROT_TOKENS], seq[ROT_TOKENS];      // page * PAGE + row of a token (-1: none)
+  __shared__ int place[ROT_TOKENS], seq[ROT_TOKENS], first[ROT_TOKENS];      // page * PAGE + row of a token (-1: none); its sequence and that one's first row
   const int t0 = blockIdx.x * ROT_TOKENS, nt = min(ROT_TOKENS, a.n_tokens - t0), lane = threadIdx.x & 31, warp = threadIdx.x >> 5, half = a.rot >> 1;
+  constexpr int DK = 32 * M;
+  const int unit = blockIdx.y * ROT_WARPS + warp, n_units = a.H + a.G + a.G * a.dv / DK;
+  const int ch0 = unit * DK + lane * M, C = (a.H + a.G) * DK + a.G * a.dv, ds = DK / a.maps;
+  const bool value = unit >= a.H + a.G, busy = unit < n_units;
+  const float* nw = value ? nullptr : unit < a.H ? a.q_norm : a.k_norm;
+  const int j0 = lane * M % ds, lanes = 32 / a.maps;      // this lane's first dimension inside its map; lanes of a map
+  // (all that memory gives is on its way while the angles are computed: rows, the three rows in front, taps, weights)
+  float in[ROT_TOKENS][M] = {}, ib[M] = {}, past[M][3] = {}, w[M][4] = {}, nwm[M];
+  if (busy) {
+#pragma unroll
+    for (int x = 0; x < ROT_TOKENS; ++x)
+      if (x < nt) load_run<M>(a.qkv + (size_t)(t0 + x) * a.ldq + ch0, whole & 1, in[x]);
+    if (a.conv_w) {
+#pragma unroll
+      for (int j = 0; j < 3; ++j)
+        if (j >= 4 - a.taps && t0 - 3 + j >= 0) {
+          float v[M];
+          load_run<M>(a.qkv + (size_t)(t0 - 3 + j) * a.ldq + ch0, whole & 1, v);
+#pragma unroll
+          for (int m = 0; m < M; ++m) past[m][j] = v[m];
+        }
+#pragma unroll
+      for (int m = 0; m < M; ++m)              // (aligned to the end: the last tap is [3], the token before [2])
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j >= 4 - a.taps) w[m][j] = a.conv_w[(size_t)(ch0 + m) * a.taps + j - (4 - a.taps)];
+    }
+    if (a.bias)
+#pragma unroll
+      for (int m = 0; m < M; ++m) ib[m] = a.bias[ch0 + m];
+#pragma unroll
+    for (int m = 0; m < M; ++m) nwm[m] = nw ? nw[j0 + m] : 1.f;
+  }
   if (threadIdx.x < ROT_TOKENS) {
     const int t = t0 + threadIdx.x, pos = threadIdx.x < nt ? a.tok_pos[t] : -1, s = threadIdx.x < nt ? a.tok_seq[t] : 0;
     int at = -1;
@@ -63,6 +124,7 @@ rotate_rows_kernel(const RotateRows a, TQ* __restrict__ q_out, T* __restrict__ k
     }
     place[threadIdx.x] = at;
     seq[threadIdx.x] = s;
+    first[threadIdx.x] = a.conv_w && threadIdx.x < nt ? a.seq_tok0[s] : 0;
   }
   for (int i = threadIdx.x; i < nt * half; i += ROT_WARPS * 32) {
     const int x = i / half, j = i - x * half;
@@ -73,37 +135,32 @@ rotate_rows_kernel(const RotateRows a, TQ* __restrict__ q_out, T* __restrict__ k
     turn[x][j] = make_float2(cs * a.mult, sn * a.mult);
   }
   __syncthreads();
-  constexpr int DK = 32 * M;
-  const int unit = blockIdx.y * ROT_WARPS + warp, n_units = a.H + a.G + a.G * a.dv / DK;
-  if (unit >= n_units) return;
-  const bool value = unit >= a.H + a.G;
-  const int ch0 = unit * DK + lane, C = (a.H + a.G) * DK + a.G * a.dv, ds = DK / a.maps;
-  float in[ROT_TOKENS][M], ib[M];
-#pragma unroll
-  for (int m = 0; m < M; ++m) ib[m] = a.bias ? a.bias[ch0 + 32 * m] : 0.f;
+  if (!busy) return;
+  // half a rotation away: in the lane `half / M` further, or (half no whole run: M 3, or fewer than a run) a dimension of some lane's
+  const bool whole_lanes = half % M == 0, front = j0 < half;
+  const int away = front ? lane + half / M : lane - half / M;
+  const int vi = ch0 - (a.H + a.G) * DK, vg = vi / a.dv, vj = vi - vg * a.dv;      // (value channels: their head and place in it)
 #pragma unroll
   for (int x = 0; x < ROT_TOKENS; ++x)
 #pragma unroll
-    for (int m = 0; m < M; ++m) in[x][m] = (x < nt ? a.qkv[(size_t)(t0 + x) * a.ldq + ch0 + 32 * m] : 0.f) + ib[m];
+    for (int m = 0; m < M; ++m) in[x][m] += ib[m];
   if (a.conv_w) {
-    float w[M][4], past[M][3];                 // (aligned to the end: the last tap is [3], the token before [2])
 #pragma unroll
     for (int m = 0; m < M; ++m)
 #pragma unroll
-      for (int j = 0; j < 4; ++j) w[m][j] = j >= 4 - a.taps ? a.conv_w[(size_t)(ch0 + 32 * m) * a.taps + j - (4 - a.taps)] : 0.f;
+      for (int j = 0; j < 3; ++j) past[m][j] = j >= 4 - a.taps ? past[m][j] + ib[m] : 0.f;
 #pragma unroll
     for (int x = 0; x < ROT_TOKENS; ++x) {
       if (x >= nt) break;
-      const int s = seq[x], k = t0 + x - a.seq_tok0[s];
-      if (x == 0 || k == 0) {                  // the inputs before this token: rows of the step, or the sequence's tail
+      const int s = seq[x], k = t0 + x - first[x];
+      if (x == 0 ? k < 3 : k == 0) {           // the inputs before this token that are no rows of the step: the sequence's tail
         const float* tail = a.conv_state + (size_t)a.seq_slot[s] * (a.taps - 1) * C;
 #pragma unroll
         for (int j = 0; j < 3; ++j) {
           const int r = k - 3 + j, row = a.taps - 1 + r;
+          if (r < 0 && j >= 4 - a.taps)
 #pragma unroll
-          for (int m = 0; m < M; ++m)
-            past[m][j] = j < 4 - a.taps ? 0.f : r >= 0 ? a.qkv[(size_t)(t0 + x - k + r) * a.ldq + ch0 + 32 * m] + ib[m]
-                                : (row >= 0 ? tail[(size_t)row * C + ch0 + 32 * m] : 0.f);
+            for (int m = 0; m < M; ++m) past[m][j] = row >= 0 ? tail[(size_t)row * C + ch0 + m] : 0.f;
         }
       }
 #pragma unroll
@@ -118,74 +175,66 @@ rotate_rows_kernel(const RotateRows a, TQ* __restrict__ q_out, T* __restrict__ k
   }
   if (value) {
 #pragma unroll
-    for (int m = 0; m < M; ++m) {
-      const int i = ch0 + 32 * m - (a.H + a.G) * DK, g = i / a.dv, j = i - g * a.dv;
+    for (int x = 0; x < ROT_TOKENS; ++x) {
+      if (x >= nt || place[x] < 0) continue;
+      T* rows = vcache + ((size_t)(place[x] / PAGE) * a.G * PAGE + place[x] % PAGE) * a.dv;
+      if (a.dv % M == 0) {                     // a lane's run lies in one head's values
+        store_run<M>(rows + (size_t)vg * PAGE * a.dv + vj, whole & 4, in[x]);
+      } else {
 #pragma unroll
-      for (int x = 0; x < ROT_TOKENS; ++x)
-        if (x < nt && place[x] >= 0) vcache[(((size_t)(place[x] / PAGE) * a.G + g) * PAGE + place[x] % PAGE) * a.dv + j] = from_f32<T>(in[x][m]);
+        for (int m = 0; m < M; ++m) {
+          const int g = (vi + m) / a.dv;
+          rows[(size_t)g * PAGE * a.dv + vi + m - g * a.dv] = from_f32<T>(in[x][m]);
+        }
+      }
     }
     return;
   }
-  const float* nw = unit < a.H ? a.q_norm : a.k_norm;
-  float nwm[M];
-#pragma unroll
-  for (int m = 0; m < M; ++m) nwm[m] = nw ? nw[lane + 32 * m % ds] : 1.f;
 #pragma unroll
   for (int x = 0; x < ROT_TOKENS; ++x) {
-    if (x >= nt || place[x] < 0) continue;
     float v[M];
 #pragma unroll
     for (int m = 0; m < M; ++m) v[m] = in[x][m];
     if (nw) {
-      float ss[M];                             // a map's sum of squares, then its factor, at each of its runs
+      float ss = 0.f;
 #pragma unroll
-      for (int m = 0; m < M; ++m) ss[m] = v[m] * v[m];
+      for (int m = 0; m < M; ++m) ss = fmaf(v[m], v[m], ss);
 #pragma unroll
-      for (int m = 1; m < M; ++m)
-        if (32 * m % ds != 0) ss[m] += ss[m - 1];
+      for (int o = 1; o < 32; o <<= 1)
+        if (o < lanes) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+      const float inv = 1.0f / sqrtf(ss / (float)ds + a.eps);
 #pragma unroll
-      for (int m = M - 2; m >= 0; --m)
-        if (32 * (m + 1) % ds != 0) ss[m] = ss[m + 1];
-#pragma unroll
-      for (int m = 0; m < M; ++m)
-        if (32 * m % ds == 0) ss[m] = 1.0f / sqrtf(warp_sum(ss[m]) / (float)ds + a.eps);
-        else ss[m] = ss[m - 1];
-#pragma unroll
-      for (int m = 0; m < M; ++m) v[m] = v[m] * ss[m] * nwm[m];
+      for (int m = 0; m < M; ++m) v[m] = v[m] * inv * nwm[m];
     }
     if (a.rot) {
-      float out[M];
+      float other[M];
+      if (a.interleaved && M % 2 == 0) {       // the other of a neighbouring pair lies in this lane
 #pragma unroll
-      for (int m = 0; m < M; ++m) {
-        const int j = lane + 32 * m % ds;      // dimension inside its map
-        // the partner: the other of a neighbouring pair, half a rotation away in this lane, or in another
-        float other;
-        int at;
-        bool first;
-        if (a.interleaved) {
-          other = __shfl_xor_sync(0xffffffffu, v[m], 1);
-          at = j >> 1;
-          first = (j & 1) == 0;
-        } else {
-          first = j < half;
-          at = first ? j : j - half;
-          if (half >= 32) {
-            other = 0.f;
+        for (int m = 0; m < M; ++m) other[m] = v[m ^ (M > 1)];
+      } else if (!a.interleaved && whole_lanes) {
 #pragma unroll
-            for (int p = 0; p < M; ++p)
-              if (p == (first ? m + half / 32 : m - half / 32)) other = v[p];
-          } else {
-            other = __shfl_xor_sync(0xffffffffu, v[m], half);
+        for (int m = 0; m < M; ++m) other[m] = __shfl_sync(0xffffffffu, v[m], away & 31);
+      } else {
+#pragma unroll
+        for (int m = 0; m < M; ++m) {
+          const int j = j0 + m, p = a.interleaved ? j ^ 1 : j < half ? j + half : j - half, d = lane * M - j0 + p;
+          other[m] = 0.f;
+#pragma unroll
+          for (int e = 0; e < M; ++e) {
+            const float got = __shfl_sync(0xffffffffu, v[e], d / M);
+            if (d % M == e) other[m] = got;
           }
-        }
-        out[m] = v[m];
-        if (j < a.rot) {
-          const float2 tr = turn[x][at];
-          out[m] = first ? v[m] * tr.x - other * tr.y : v[m] * tr.x + other * tr.y;
         }
       }
 #pragma unroll
-      for (int m = 0; m < M; ++m) v[m] = out[m];
+      for (int m = 0; m < M; ++m) {
+        const int j = j0 + m;
+        if (j < a.rot) {
+          const bool first_of = a.interleaved ? (j & 1) == 0 : j < half;
+          const float2 tr = turn[x][a.interleaved ? j >> 1 : j < half ? j : j - half];
+          v[m] = first_of ? v[m] * tr.x - other[m] * tr.y : v[m] * tr.x + other[m] * tr.y;
+        }
+      }
     }
     if (a.unit_norm) {
       float ss = 0.f;
@@ -195,25 +244,23 @@ rotate_rows_kernel(const RotateRows a, TQ* __restrict__ q_out, T* __restrict__ k
 #pragma unroll
       for (int m = 0; m < M; ++m) v[m] *= inv;
     }
-    if (unit < a.H) {
-      TQ* dst = q_out + ((size_t)(t0 + x) * a.H + unit) * DK + lane;
-#pragma unroll
-      for (int m = 0; m < M; ++m) dst[32 * m] = from_f32<TQ>(v[m]);
-    } else {
-      T* dst = kcache + (((size_t)(place[x] / PAGE) * a.G + unit - a.H) * PAGE + place[x] % PAGE) * DK + lane;
-#pragma unroll
-      for (int m = 0; m < M; ++m) dst[32 * m] = from_f32<T>(v[m]);
-    }
+    // (rows without a place are computed like the others, so that the tokens' chains interleave, and not stored)
+    if (x >= nt || place[x] < 0) continue;
+    if (unit < a.H) store_run<M>(q_out + ((size_t)(t0 + x) * a.H + unit) * DK + lane * M, whole & 2, v);
+    else store_run<M>(kcache + (((size_t)(place[x] / PAGE) * a.G + unit - a.H) * PAGE + place[x] % PAGE) * DK + lane * M, whole & 4, v);
   }
 }
 
 template <typename T, typename TQ>
 inline void launch_rotate_rows(const RotateRows& a, int dk, TQ* q_out, T* kcache, T* vcache, cudaStream_t stream) {
   const dim3 grid((a.n_tokens + ROT_TOKENS - 1) / ROT_TOKENS, (a.H + a.G + a.G * a.dv / dk + ROT_WARPS - 1) / ROT_WARPS), block(ROT_WARPS * 32);
-  if (dk == 32) rotate_rows_kernel<T, TQ, 1><<<grid, block, 0, stream>>>(a, q_out, kcache, vcache);
-  else if (dk == 64) rotate_rows_kernel<T, TQ, 2><<<grid, block, 0, stream>>>(a, q_out, kcache, vcache);
-  else if (dk == 96) rotate_rows_kernel<T, TQ, 3><<<grid, block, 0, stream>>>(a, q_out, kcache, vcache);
-  else rotate_rows_kernel<T, TQ, 4><<<grid, block, 0, stream>>>(a, q_out, kcache, vcache);
+  const auto aligned = [&](const void* p, size_t row, size_t item) { return (uintptr_t)p % (item * (dk / 32)) == 0 && row % (dk / 32) == 0; };
+  const int whole = (aligned(a.qkv, a.ldq, 4) ? 1 : 0) | (aligned(q_out, dk, sizeof(TQ)) ? 2 : 0) |
+                    (aligned(kcache, dk, sizeof(T)) && aligned(vcache, a.dv, sizeof(T)) ? 4 : 0);
+  if (dk == 32) rotate_rows_kernel<T, TQ, 1><<<grid, block, 0, stream>>>(a, q_out, kcache, vcache, whole);
+  else if (dk == 64) rotate_rows_kernel<T, TQ, 2><<<grid, block, 0, stream>>>(a, q_out, kcache, vcache, whole);
+  else if (dk == 96) rotate_rows_kernel<T, TQ, 3><<<grid, block, 0, stream>>>(a, q_out, kcache, vcache, whole);
+  else rotate_rows_kernel<T, TQ, 4><<<grid, block, 0, stream>>>(a, q_out, kcache, vcache, whole);
 }
 
 }  // namespace edgelm

@@ -383,6 +383,15 @@ def test_rotation_and_append_of_many_tokens(H, G, dk, dv, maps, rot, inter, norm
             t0 += n
 
 
+@pytest.mark.parametrize("H,G,dk,dv,maps,rot,inter,norm,taps,bias", [
+    (120, 6, 96, 96, 1, 96, False, True, 0, False), (120, 6, 96, 96, 1, 64, True, False, 3, True), (120, 8, 128, 128, 1, 6, False, True, 0, False),
+    (124, 4, 64, 64, 1, 2, False, False, 4, False), (120, 8, 128, 64, 2, 50, True, True, 0, False), (114, 6, 32, 64, 1, 22, False, False, 0, True)])
+def test_rotation_of_many_tokens_partners_of_every_kind(H, G, dk, dv, maps, rot, inter, norm, taps, bias):
+    """A partner that is no whole run of a lane's dimensions away, in this lane, or in one that no power of two leads to."""
+    for dtype in (torch.float32, torch.bfloat16):
+        test_rotation_and_append_of_many_tokens(H, G, dk, dv, maps, rot, inter, norm, taps, bias, dtype)
+
+
 @pytest.mark.parametrize("taps", [1, 2, 3, 4])
 def test_filter_inside_rotation_reads_no_token_in_front_of_its_taps(taps):
     """Steps of more than 64 tokens: an infinity in a value channel and a NaN in a query and a key channel reach `taps` tokens each."""
