@@ -1318,12 +1318,12 @@ def rglru_scratch_floats(n_tokens, n_seqs, W):
     return 2 * ((n_tokens + RGLRU_SEG - 1) // RGLRU_SEG) * W
 
 
-def rglru_scan(gates, br, bi, u, c, y, by, state, out, seq_tok0, seq_slot, n_seqs, single, tok_seq=None, scratch=None):
+def rglru_scan(gates, br, bi, u, c, y, by, state, out, seq_tok0, seq_slot, n_seqs, single, tok_seq=None, scratch=None, composed=False):
     """S_t = a S_(t-1) + sqrt(1 - a^2) i u with a = exp(c r), r = sigmoid(gates[:, :W] + br), i = sigmoid(gates[:, W:] + bi);
     out = S_t gelu_tanh(y + by).  gates [T, 2 W], u [T, W] and y (a view of W columns) float32 rows; c, br, bi, by [W];
     state [slots, W] float32, read and moved on; `single`: every sequence of the step brings one token.  Other steps name
     every token's sequence (`tok_seq` [T] int32), bring `scratch`, float32 of `rglru_scratch_floats` elements, and leave
-    decays and inputs in `gates`."""
+    decays and inputs in `gates`; `composed`: `rglru_gates_compose` left them and the scratch already."""
     for t, n in ((gates, "gates"), (br, "br"), (bi, "bi"), (c, "c"), (by, "by"), (state, "state")):
         _f32(t, n)
     T, W = out.shape
@@ -1336,8 +1336,8 @@ def rglru_scan(gates, br, bi, u, c, y, by, state, out, seq_tok0, seq_slot, n_seq
         _need(tok_seq.numel() >= T and scratch.numel() >= rglru_scratch_floats(T, int(n_seqs), W), "rglru_scan: tok_seq and scratch sizes")
     _check(lib().edgelm_rglru_scan(_p(gates), gates.stride(0), _p(br), _p(bi), _p(u), u.stride(0), _p(c), _p(y), y.stride(0), _p(by), _p(state),
                                    _p(out), _dt(out), _p(seq_tok0), _p(seq_slot), _p(tok_seq) if not single else None,
-                                   _p(scratch) if not single else None, int(n_seqs), T, W, 1 if single else 0, _stream()),
-           launches=1 if single else 2)
+                                   _p(scratch) if not single else None, int(n_seqs), T, W, 1 if single else 0, 1 if composed else 0, _stream()),
+           launches=1 if single or composed else 2)
 
 
 def rglru_gates(u, w_ra, w_ri, gates, blocks):
@@ -1354,6 +1354,30 @@ def rglru_gates(u, w_ra, w_ri, gates, blocks):
     else:
         head_matmul(u, bw, w_ra, gates[:, :W], bw)
         head_matmul(u, bw, w_ri, gates[:, W:], bw)
+
+
+def rglru_gates_compose_takes(u, w_ra, w_ri, br, bi, c, state, gates, blocks):
+    """Whether a prompt step's gate products and the first pass of its scan run as one kernel (bfloat16 matrices, aligned rows)."""
+    if w_ra.dtype != torch.bfloat16 or u.dtype != torch.float32 or u.stride(1) != 1:
+        return False
+    return bool(lib().edgelm_rglru_gates_compose_takes(_p(u), u.stride(0), _p(w_ra), _p(w_ri), _p(br), _p(bi), _p(c), _p(state), _p(gates), gates.stride(0),
+                                                       u.shape[1], int(blocks)))
+
+
+def rglru_gates_compose(u, w_ra, w_ri, br, bi, c, state, gates, blocks, seq_tok0, seq_slot, tok_seq, scratch, n_seqs):
+    """`rglru_gates` and the first pass of a prompt step's `rglru_scan` in one: gates [T, 2 W] <- decays | inputs, `scratch` <- the segments'
+    maps; the scan goes on with `composed`."""
+    for t, n in ((gates, "gates"), (br, "br"), (bi, "bi"), (c, "c"), (state, "state"), (scratch, "scratch")):
+        _f32(t, n)
+    T, W = u.shape
+    bw = W // blocks
+    _need(W % blocks == 0 and gates.shape == (T, 2 * W) and w_ra.shape == w_ri.shape == (blocks, bw, bw) and w_ra.dtype == w_ri.dtype == torch.bfloat16 and
+          w_ra.is_contiguous() and w_ri.is_contiguous() and u.dtype == torch.float32 and u.stride(1) == 1 and state.shape[1] == W and
+          br.numel() == bi.numel() == c.numel() == W, "rglru_gates_compose: shapes")
+    _i32(seq_tok0, "seq_tok0"); _i32(seq_slot, "seq_slot"); _i32(tok_seq, "tok_seq")
+    _need(tok_seq.numel() >= T and scratch.numel() >= rglru_scratch_floats(T, int(n_seqs), W), "rglru_gates_compose: tok_seq and scratch sizes")
+    _check(lib().edgelm_rglru_gates_compose(_p(u), u.stride(0), _p(w_ra), _p(w_ri), _p(br), _p(bi), _p(c), _p(state), _p(gates), gates.stride(0), _p(scratch),
+                                            _p(seq_tok0), _p(seq_slot), _p(tok_seq), T, W, int(blocks), _stream()))
 
 
 def clamped_glu(gu, mid, limit, alpha, shift=1.0, bias=None, x=None, x_bias=None):

@@ -90,13 +90,18 @@ class RGLRU(Part):
             ops.conv_act(yx, W, self.conv_w, self.conv_b, conv.state if conv is not None else self.no_tail, u,
                          ctx.tok_seq, ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs, update_state=True, in_bias=self.b_x, act=None)
         gates = ws.alloc((T, 2 * W), f32)
+        s, state = ws.alloc((T, W), self.dtype), cache["rglru"].state
+        scratch = None if ctx.all_single else ws.alloc((ops.rglru_scratch_floats(T, ctx.n_seqs, W),), f32)
+        composed = not ctx.all_single and ops.rglru_gates_compose_takes(u, self.w_ra, self.w_ri, self.b_ra, self.b_ri, self.decay, state, gates, self.blocks)
         with ctx.prof("rglru_gates"):
-            ops.rglru_gates(u, self.w_ra, self.w_ri, gates, self.blocks)
-        s = ws.alloc((T, W), self.dtype)
+            if composed:
+                ops.rglru_gates_compose(u, self.w_ra, self.w_ri, self.b_ra, self.b_ri, self.decay, state, gates, self.blocks, ctx.seq_tok0, ctx.seq_slots,
+                                        ctx.tok_seq, scratch, ctx.n_seqs)
+            else:
+                ops.rglru_gates(u, self.w_ra, self.w_ri, gates, self.blocks)
         with ctx.prof("rglru_scan"):
-            scratch = None if ctx.all_single else ws.alloc((ops.rglru_scratch_floats(T, ctx.n_seqs, W),), f32)
-            ops.rglru_scan(gates, self.b_ra, self.b_ri, u, self.decay, yx[:, :W], self.b_y, cache["rglru"].state, s,
-                           ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs, ctx.all_single, tok_seq=ctx.tok_seq, scratch=scratch)
+            ops.rglru_scan(gates, self.b_ra, self.b_ri, u, self.decay, yx[:, :W], self.b_y, state, s,
+                           ctx.seq_tok0, ctx.seq_slots, ctx.n_seqs, ctx.all_single, tok_seq=ctx.tok_seq, scratch=scratch, composed=composed)
         with ctx.prof("rglru_out_proj"):
             linear.matmul(ctx, s, self.w_o, x, epilogue=linear.EPI_RESIDUAL if accumulate else linear.EPI_STORE,
                           residual=x if accumulate else None, prefetch=ctx.weights_after)

@@ -90,6 +90,39 @@ def test_gate_products_are_float32(W, blocks, T, w_dtype):
     assert np.abs(lossy - want[0]).max() > 1e-4 * scale      # (the check above can tell the two apart)
 
 
+@pytest.mark.parametrize("W,blocks,lengths", [(16, 2, [3, 1, 70]), (160, 1, [64, 64]), (480, 3, [1, 130, 2, 66]), (128, 2, [63, 200]), (120, 3, [65])])
+def test_gates_and_first_pass_in_one(W, blocks, lengths):
+    """The fused kernel against the two it stands for, at widths of a piece, a tile and their remainders, sequences that start inside segments.
+    Per number: 3 W / blocks / 16 cut-offs of a gate's sum (2^-23 of it) through sigmoids and an exponential of slope below 8: 8 x 2^-23 x 30
+    = 3e-5 at most for sums up to 10; a segment's map is a product of up to 64 of them below 1 and their sum."""
+    g = torch.Generator().manual_seed(W)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    T, bw = sum(lengths), W // blocks
+    u, y = rnd(T, W).to(DEV), rnd(T, W).to(DEV)
+    ra, ri = ((rnd(blocks, bw, bw) / bw ** 0.5).to(device=DEV, dtype=torch.bfloat16) for _ in range(2))
+    br, bi, by = (rnd(W).to(DEV) * 0.3 for _ in range(3))
+    c = -(torch.rand(W, generator=g) * 6 + 0.05).to(DEV)
+    tok0, tok_seq = packed(lengths)
+    slots, n = i32([3, 0, 5, 1][:len(lengths)]), len(lengths)
+    left, outs, maps, gates = rnd(6, W).to(DEV), [], [], []
+    for fused in (False, True):
+        state, ab, o = left.clone(), torch.full((T, 2 * W), float("nan"), device=DEV), torch.full((T, W), float("nan"), device=DEV)
+        scratch = torch.full((ops.rglru_scratch_floats(T, n, W),), float("nan"), device=DEV)
+        assert ops.rglru_gates_compose_takes(u, ra, ri, br, bi, c, state, ab, blocks)
+        if fused:
+            ops.rglru_gates_compose(u, ra, ri, br, bi, c, state, ab, blocks, tok0, slots, tok_seq, scratch, n)
+        else:
+            ops.rglru_gates(u, ra, ri, ab, blocks)
+        ops.rglru_scan(ab, br, bi, u, c, y, by, state, o, tok0, slots, n, False, tok_seq=tok_seq, scratch=scratch, composed=fused)
+        outs.append((o, state))
+        maps.append(scratch)
+        gates.append(ab)
+    for a, b in zip(outs[0] + (maps[0], gates[0]), outs[1] + (maps[1], gates[1])):
+        assert float((a - b).abs().max()) < 3e-5 * max(1.0, float(a.abs().max()))
+    assert not ops.rglru_gates_compose_takes(u, ra.float(), ri.float(), br, bi, c, left, gates[0], blocks)
+    assert not ops.rglru_gates_compose_takes(u[:, 1:], ra, ri, br, bi, c, left, gates[0], blocks)
+
+
 # ----------------------------------------------------------------------------- residual streams
 @pytest.mark.parametrize("h_dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("S,D,T", [(3, 64, 37), (1, 50, 5), (4, 208, 130), (8, 72, 3), (2, 1030, 9)])
