@@ -1,0 +1,433 @@
+// Attention of many new tokens over bfloat16 keys and values with float32 queries, scores and softmax weights on the fifth-generation
+// tensor cores (tcgen05): what attention_mma_split.cu computes, for steps whose sequences bring enough tokens for tiles of 128.
+//
+//   S = (q1 + q2 + q3) K^T,  O += (p1 + p2 + p3) V      the float32 operand as the sum of three bfloat16 terms, exact products, float32 sums
+//
+// grid (head or head's map, query tile); a CTA takes up to 128 consecutive tokens of one sequence for one head and walks the keys that its
+// rows see in blocks of two cache pages (or of the step's own rows).  Roles: warp 0 loads the keys by TMA, warp 1 the values, warp 2 issues
+// S (A: the queries' terms, swizzled K-major tiles written once; B: the keys as they lie), warp 3 issues O (A: the weights' terms out
+// of tensor memory; B: the values as they lie, MN-major), warps 4 to 19 are the softmax: four threads a row, half a page
+// of the block each.  They exchange a row's maximum through shared memory, so that they share one reference and one accumulator; the
+// reference moves only when the maximum has outgrown it by 2^8 (then they scale the row of O in place).  A thread's weights go back over the
+// scores that they came from: its 32 columns hold terms 1 and 2, 16 further ones the third.  Tensor memory: two such buffers of 192
+// columns and O (up to 128).
+// So S of block j + 1 is computed beside the softmax of block j, and O of block j beside the softmax of block j + 1.
+//
+// Masks, sinks, gates, kept keys and maps as in attention_mma_split.cu.  Every wait is bounded as in the matrix products.
+// mma.sync takes a scheduler 16 clocks for an m16n8k16 here, four times what tcgen05 takes for as many multiply-adds, and bounds the other kernel.
+// What bounds this one is the softmax: 2,600 clocks a block, 1,750 of them the exponentials, the splitting and the stores into tensor memory
+// (with a third of either product's MMAs it takes 3 % less, without exponentials and splitting 17 %); 3 us a tile before the first block.
+// mma.sync and here, us: 9 heads of 64 over 3, 6,000 tokens 448 and 135; chunks of 512, 333 to 1,700 tokens 39.6 and 24.8; 9 heads of
+// 96 / 64 over the step's own rows, 333 to 1,700 tokens 101 and 35.5; 16 heads of two maps of 64 over values of 128, chunks of 1,024, 1,000 and
+// 2,900 tokens 243 and 121.  Distance from float64 in the float32 output of two maps: 0.5 to 1.05 of the other's.
+// Tiles of the most keys go first over all heads (a head's tiles next to each other left the last head's longest tile to the end).
+#include <math_constants.h>
+
+#include "mma_split.cuh"
+#include "tc_common.cuh"
+
+namespace edgelm {
+
+enum : int { ST_MASK_CAUSAL = 0, ST_MASK_WINDOW = 1, ST_MASK_CHUNK = 2 };
+
+constexpr int ST_ROWS = 128, ST_SOFT_WARPS = 16, ST_THREADS = 128 + ST_SOFT_WARPS * 32;
+constexpr uint32_t ST_BUF_COLS = 192, ST_O_COL = 2 * ST_BUF_COLS;
+constexpr float ST_LAZY = 8.f;
+constexpr int ST_TILE = 128 * 128;             // bytes of 128 rows of 64 bfloat16
+
+template <int DK, int DV> struct StSizes {
+  static constexpr int KC = (DK + 63) / 64, VC = (DV + 63) / 64;      // tiles of 64 dimensions
+  static constexpr int KS = 2, VS = KC == 2 && VC == 2 ? 1 : 2;       // stages of keys and values
+  static constexpr int smem = 1024 + (3 * KC + KS * KC + VS * VC) * ST_TILE + 12 * ST_ROWS * 4 + 256;
+};
+
+__device__ __forceinline__ int st_first_key(int pos, int mask, int size) {
+  if (mask == ST_MASK_WINDOW) return max(0, pos - size + 1);
+  if (mask == ST_MASK_CHUNK) return (pos / size) * size;
+  return 0;
+}
+__device__ __forceinline__ void st_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
+__device__ __forceinline__ void st_tmem_st8(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
+               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
+               : "memory");
+}
+__device__ __forceinline__ void st_tmem_ld8(uint32_t taddr, uint32_t* r) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
+}
+// D (+)= A (tensor memory) x B (shared memory)
+__device__ __forceinline__ void st_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.b32 p, %4, 0;\n\t"
+      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
+      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
+      : "memory");
+}
+
+struct SplitTcArgs {
+  const float* q;
+  int ldq;
+  void* out;
+  int ldo;
+  const int32_t* page_table;       // null: the step's own rows
+  int table_stride, n_pages;
+  const int32_t *tile_seq, *tile_tok0, *tile_ntok, *tile_pos0;
+  int n_tiles, nh, nkv, maps;
+  float scale;
+  const float* gate;
+  int ldg, mask, mask_size;
+  const float* sink;
+  int keep, gate_ch;
+  int* err;
+};
+
+template <int DK, int DV>
+__global__ void __launch_bounds__(ST_THREADS, 1)
+attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __grid_constant__ CUtensorMap map_v, const SplitTcArgs a) {
+  using Z = StSizes<DK, DV>;
+  constexpr int KC = Z::KC, VC = Z::VC, KS = Z::KS, VS = Z::VS;
+  extern __shared__ uint8_t st_raw[];
+  uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(st_raw) + 1023) & ~(uintptr_t)1023);
+  uint8_t* q_s = smem;                             // [3 terms][KC][128 rows][128 bytes]
+  uint8_t* k_s = q_s + 3 * KC * ST_TILE;           // [KS][KC][128 keys][128 bytes]
+  uint8_t* v_s = k_s + KS * KC * ST_TILE;          // [VS][VC][128 keys][128 bytes]
+  float* row_max = reinterpret_cast<float*>(v_s + VS * VC * ST_TILE);      // [block & 1][quarter of its keys][128 rows]
+  float* row_sum = row_max + 8 * ST_ROWS;          // [quarter of the keys][128 rows]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(row_sum + 4 * ST_ROWS);
+  uint64_t *q_ready = bars, *k_full = bars + 1, *k_empty = k_full + KS, *v_full = k_empty + KS, *v_empty = v_full + VS;
+  uint64_t *s_ready = v_empty + VS, *p_ready = s_ready + 2, *o_done = p_ready + 2;
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int tile = a.n_tiles - 1 - (int)blockIdx.y, head = blockIdx.x, kvh = head / (a.nh / a.nkv * a.maps), map = head % a.maps;
+  const int seq = a.tile_seq[tile], tok0 = a.tile_tok0[tile], ntok = a.tile_ntok[tile], pos0 = a.tile_pos0[tile];
+  const int n_keys = pos0 + ntok, n_pg = (n_keys + PAGE - 1) / PAGE;
+  // the pages to visit: those of the kept keys that lie ahead of the window's first, then the window's; two a block
+  const int first_page = st_first_key(pos0, a.mask, a.mask_size) / PAGE, kept_pages = min(first_page, (a.keep + PAGE - 1) / PAGE);
+  const int n_visit = kept_pages + n_pg - first_page, n_blk = (n_visit + 1) / 2;
+  auto page_at = [&](int i) { return i < kept_pages ? i : first_page + i - kept_pages; };
+
+  if (threadIdx.x == 0) {
+    for (uint64_t* b = bars; b < o_done + 2; ++b) mbar_init(smem_u32(b), b == q_ready || (b >= p_ready && b < o_done) ? ST_SOFT_WARPS : 1);
+    *abort_flag = 0;
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  if (warp == 2) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+  const uint32_t tmem = *tmem_slot;
+  auto wait = [&](uint64_t* bar, int parity) { return __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(bar), (uint32_t)parity, abort_flag, a.err)); };
+
+  if (warp < 2) {
+    const bool keys = warp == 0;
+    const CUtensorMap* m = keys ? &map_k : &map_v;
+    const int stages = keys ? KS : VS, chunks = keys ? KC : VC, dim = keys ? DK : DV;
+    uint64_t *full = keys ? k_full : v_full, *empty = keys ? k_empty : v_empty;
+    uint8_t* dst = keys ? k_s : v_s;
+    const int32_t* pages = a.page_table ? a.page_table + (size_t)seq * a.table_stride : nullptr;
+    const bool leader = elect_one();
+    for (int j = 0; j < n_blk; ++j) {
+      const int st = j % stages;
+      if (j >= stages && !wait(&empty[st], (j / stages & 1) ^ 1)) break;
+      if (leader) {
+        const uint32_t bar = smem_u32(&full[st]);
+        mbar_expect_tx(bar, chunks * ST_TILE);
+        for (int h = 0; h < 2; ++h) {
+          const int pg = page_at(2 * j + h < n_visit ? 2 * j + h : 2 * j);      // (no second page: the first again, masked)
+          int x, y;
+          if (pages) {
+            int page = pages[pg];
+            if (page < 0 || page >= a.n_pages) {
+              atomicOr(a.err, ERR_PAGE_RANGE);
+              page = 0;
+            }
+            x = keys ? map * DK : 0;
+            y = (page * a.nkv + kvh) * PAGE;
+          } else {
+            x = (keys ? kvh * a.maps + map : kvh) * dim;
+            y = tok0 - pos0 + pg * PAGE;
+          }
+          for (int c = 0; c < chunks; ++c) tma_load_2d(smem_u32(dst + (st * chunks + c) * ST_TILE + h * (ST_TILE / 2)), m, bar, x + c * 64, y);
+        }
+      }
+      __syncwarp();
+    }
+  } else if (warp == 2) {
+    constexpr uint32_t idesc = umma_idesc(ST_ROWS, 128);
+    const bool leader = elect_one();
+    const uint64_t dq = umma_desc(smem_u32(q_s));
+    bool ok = wait(q_ready, 0);
+    for (int j = 0; j < n_blk && ok; ++j) {
+      const int b = j & 1, st = j % KS;
+      if (j >= 2) ok = wait(&o_done[b], (j >> 1) - 1 & 1);            // (the block before last has left this buffer)
+      if (ok) ok = wait(&k_full[st], j / KS & 1);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint64_t dk = umma_desc(smem_u32(k_s + st * KC * ST_TILE));
+      if (leader) {
+#pragma unroll
+        for (int t = 2; t >= 0; --t)                                  // (the small terms first)
+#pragma unroll
+          for (int s = 0; s < DK / 16; ++s)
+            umma_f16(tmem + b * ST_BUF_COLS, dq + ((t * KC + s / 4) * ST_TILE >> 4) + 2 * (s % 4), dk + (s / 4 * ST_TILE >> 4) + 2 * (s % 4), idesc, t != 2 || s != 0);
+        umma_commit(smem_u32(&s_ready[b]));
+        umma_commit(smem_u32(&k_empty[st]));
+      }
+      __syncwarp();
+    }
+  } else if (warp == 3) {
+    constexpr uint32_t idesc = umma_idesc(ST_ROWS, 64) | (1u << 16);  // B (the values) is MN-major
+    const bool leader = elect_one();
+    bool ok = true;
+    for (int j = 0; j < n_blk && ok; ++j) {
+      const int b = j & 1, st = j % VS;
+      ok = wait(&p_ready[b], j >> 1 & 1) && wait(&v_full[st], j / VS & 1);
+      if (!ok) break;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+      const uint64_t dv = umma_desc(smem_u32(v_s + st * VC * ST_TILE));
+      if (leader) {
+#pragma unroll
+        for (int c = 0; c < VC; ++c)
+#pragma unroll
+          for (int t = 2; t >= 0; --t)
+#pragma unroll
+            for (int s = 0; s < 8; ++s) {                             // 16 keys: of the threads of quarter s / 2
+              const uint32_t p = tmem + b * ST_BUF_COLS + (t == 2 ? 128 + s * 8 : s / 2 * 32 + t * 16 + s % 2 * 8);
+              st_umma_ts(tmem + ST_O_COL + c * 64, p, dv + (c * ST_TILE + s * 16 * 128 >> 4), idesc, j != 0 || t != 2 || s != 0);
+            }
+        umma_commit(smem_u32(&o_done[b]));
+        umma_commit(smem_u32(&v_empty[st]));
+      }
+      __syncwarp();
+    }
+  } else {
+    const int sw = warp - 4, part = sw >> 2, half = part >> 1, quarter = warp & 3, row = quarter * 32 + lane, tid = threadIdx.x - 128;
+    const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
+    // scores in units of log 2; the scale's sign (or a scale of 0) goes to the queries, so that the largest score has the largest weight
+    const float scale2 = a.scale == 0.f ? 1.f : fabsf(a.scale) * 1.4426950408889634f, turn = a.scale < 0.f ? -1.f : a.scale > 0.f ? 1.f : 0.f;
+    for (int i = tid; i < ST_ROWS * (DK / 4); i += ST_SOFT_WARPS * 32) {
+      const int r = i / (DK / 4), d = i % (DK / 4) * 4;
+      float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+      if (r < ntok) v = *reinterpret_cast<const float4*>(a.q + (size_t)(tok0 + r) * a.ldq + head * DK + d);
+      uint2 t[3];
+      sp_split(turn * v.x, turn * v.y, t[0].x, t[1].x, t[2].x);
+      sp_split(turn * v.z, turn * v.w, t[0].y, t[1].y, t[2].y);
+      uint8_t* dst = q_s + d / 64 * ST_TILE + r * 128 + ((d % 64 / 8 ^ (r & 7)) << 4) + d % 8 * 2;
+#pragma unroll
+      for (int k = 0; k < 3; ++k) *reinterpret_cast<uint2*>(dst + k * KC * ST_TILE) = t[k];
+    }
+    asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+    __syncwarp();
+    if (lane == 0) st_arrive(smem_u32(q_ready));
+    const int pos = row < ntok ? pos0 + row : -1, first = st_first_key(max(pos, 0), a.mask, a.mask_size);
+    const int last_first = st_first_key(n_keys - 1, a.mask, a.mask_size);      // the first key of the tile's last row
+    float m = -CUDART_INF_F, l = 0.f;             // the row's reference (in units of log 2), this thread's keys' weights
+    bool ok = true;
+    for (int j = 0; j < n_blk; ++j) {             // (also behind a wait that ran out: the row's other thread may be at the exchange)
+      const int b = j & 1;
+      const bool there = 2 * j + half < n_visit;
+      const int page0 = page_at(there ? 2 * j + half : 2 * j) * PAGE, key0 = page0 + part % 2 * 32;
+      const uint32_t s_addr = tmem + lanes + b * ST_BUF_COLS + part * 32;
+      if (ok) ok = wait(&s_ready[b], j >> 1 & 1);
+      uint32_t r[32];
+      float mx = -CUDART_INF_F;
+      if (ok) {
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        tmem_ld32(s_addr, r);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (!there || key0 + 31 > pos0 || (key0 < last_first && key0 + 32 > a.keep)) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i)
+            if (!there || key0 + i > pos || (key0 + i < first && key0 + i >= a.keep)) r[i] = __float_as_uint(-CUDART_INF_F);
+        }
+        float mx1 = -CUDART_INF_F;
+#pragma unroll
+        for (int i = 0; i < 32; i += 4) {
+          mx = fmaxf(mx, fmaxf(__uint_as_float(r[i]), __uint_as_float(r[i + 1])));
+          mx1 = fmaxf(mx1, fmaxf(__uint_as_float(r[i + 2]), __uint_as_float(r[i + 3])));
+        }
+        mx = fmaxf(mx, mx1);
+      }
+      row_max[(b * 4 + part) * ST_ROWS + row] = mx;
+      asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");      // the row's four threads (warps w, w + 4, w + 8, w + 12)
+      if (!ok) continue;
+#pragma unroll
+      for (int k = 1; k < 4; ++k) mx = fmaxf(mx, row_max[(b * 4 + (part ^ k)) * ST_ROWS + row]);
+      mx = mx == -CUDART_INF_F ? mx : mx * scale2;
+      float rescale = 1.f;
+      if (j == 0) {
+        m = mx;
+      } else if (mx > m + ST_LAZY) {
+        rescale = sp_exp2(m - mx);                 // (0 if the row has seen no key so far)
+        m = mx;
+      }
+      if (__any_sync(0xffffffffu, rescale != 1.f)) {       // (rare after the first blocks; all warps of the rows take it)
+        ok = wait(&o_done[b ^ 1], (j - 1) >> 1 & 1);
+        if (!ok) continue;
+        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+        for (int c = 0; c < DV / 4; c += 8) {
+          uint32_t o[8];
+          const uint32_t at = tmem + lanes + ST_O_COL + part * (DV / 4) + c;
+          st_tmem_ld8(at, o);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * rescale);
+          st_tmem_st8(at, o);
+        }
+        l *= rescale;
+      }
+      const float ref = m == -CUDART_INF_F ? 0.f : m;
+      float sum0 = 0.f, sum1 = 0.f;
+#pragma unroll
+      for (int c = 0; c < 2; ++c) {                // 16 keys: 8 columns of each term
+        uint32_t t[3][8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const float p0 = sp_exp2(fmaf(__uint_as_float(r[c * 16 + 2 * i]), scale2, -ref)), p1 = sp_exp2(fmaf(__uint_as_float(r[c * 16 + 2 * i + 1]), scale2, -ref));
+          sum0 += p0;
+          sum1 += p1;
+          sp_split(p0, p1, t[0][i], t[1][i], t[2][i]);
+        }
+        st_tmem_st8(s_addr + c * 8, t[0]);
+        st_tmem_st8(s_addr + 16 + c * 8, t[1]);
+        st_tmem_st8(tmem + lanes + b * ST_BUF_COLS + 128 + part * 16 + c * 8, t[2]);
+      }
+      l += sum0 + sum1;
+      if (j == n_blk - 1) {
+        // value rows behind the tile's last position (or of no page) meet weights of zero: make them zero, whatever lies there
+        const int v_from = there ? min(PAGE, n_keys - page0) : 0;
+        if (v_from < PAGE) {                       // uniform over the warp
+          ok = wait(&v_full[j % VS], j / VS & 1);
+          if (!ok) continue;
+          for (int i = (sw & 7) * 32 + lane; i < (PAGE - v_from) * 8 * VC; i += 256) {
+            const int c = i / ((PAGE - v_from) * 8), e = i % ((PAGE - v_from) * 8);
+            *reinterpret_cast<uint4*>(v_s + (j % VS * VC + c) * ST_TILE + (half * PAGE + v_from + (e >> 3)) * 128 + (e & 7) * 16) = make_uint4(0, 0, 0, 0);
+          }
+          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        }
+      }
+      asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+      asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+      __syncwarp();
+      if (lane == 0) st_arrive(smem_u32(&p_ready[b]));
+    }
+    if (ok) ok = wait(&o_done[(n_blk - 1) & 1], (n_blk - 1) >> 1 & 1);
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    row_sum[part * ST_ROWS + row] = l;
+    asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");
+    float den = (row_sum[row] + row_sum[ST_ROWS + row]) + (row_sum[2 * ST_ROWS + row] + row_sum[3 * ST_ROWS + row]), fix = 1.f;
+    if (a.sink != nullptr) {                       // one more term of the denominator
+      const float s2 = a.sink[head] * 1.4426950408889634f, nm = fmaxf(m, s2);
+      fix = exp2f(m - nm);
+      den = den * fix + exp2f(s2 - nm);
+    }
+    float inv = den > 0.f ? fix / den : 0.f;
+    if (den != den) inv = den;                     // (not a number stays one)
+    const bool mine = row < ntok;
+    const size_t tok = (size_t)(tok0 + row);
+    if (a.gate != nullptr && !a.gate_ch && mine) inv *= 1.0f / (1.0f + expf(-a.gate[tok * a.ldg + head]));
+    if (ok) {
+#pragma unroll
+      for (int c = 0; c < DV / 4; c += 8) {
+        uint32_t o[8];
+        const int d = part * (DV / 4) + c;
+        st_tmem_ld8(tmem + lanes + ST_O_COL + d, o);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        if (!mine) continue;
+        float v[8];
+#pragma unroll
+        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(o[i]) * inv;
+        if (a.gate != nullptr && a.gate_ch) {
+          const float* g = a.gate + tok * a.ldg + head * DV + d;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] *= 1.0f / (1.0f + expf(-g[i]));
+        }
+        if (a.maps > 1) {
+          float4* dst = reinterpret_cast<float4*>(static_cast<float*>(a.out) + tok * a.ldo + head * DV + d);
+          dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+          dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
+          __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.out) + tok * a.ldo + head * DV + d;
+          store_piece(dst, make_float4(v[0], v[1], v[2], v[3]));
+          store_piece(dst + 4, make_float4(v[4], v[5], v[6], v[7]));
+        }
+      }
+    }
+  }
+  asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+  __syncthreads();
+  if (warp == 2) {
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512) : "memory");
+  }
+}
+
+template <int DK, int DV>
+static int launch_split_tc(const CUtensorMap& mk, const CUtensorMap& mv, const SplitTcArgs& a, cudaStream_t stream) {
+  constexpr int smem = StSizes<DK, DV>::smem;
+  static_assert(smem <= 227 * 1024, "shared memory");
+  auto kern = attn_prefill_split_tc_kernel<DK, DV>;
+  const cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  EL_REFUSE(e == cudaSuccess, "attn_prefill_split_tc: %d bytes of shared memory refused: %s", smem, cudaGetErrorString(e));
+  kern<<<dim3(a.nh * a.maps, a.n_tiles), ST_THREADS, smem, stream>>>(mk, mv, a);
+  return 0;
+}
+
+}  // namespace edgelm
+
+using namespace edgelm;
+
+// Tokens per tile that the host must cut sequences into for this kernel.
+extern "C" int edgelm_attn_prefill_split_tc_tile_tokens() { return ST_ROWS; }
+
+// 1 if the kernel takes these key and value head sizes and maps a head, else 0.
+extern "C" int edgelm_attn_prefill_split_tc_takes(int dk, int dv, int maps) {
+  if (maps == 2) return dk == 64 && (dv == 64 || dv == 128) ? 1 : 0;
+  return maps == 1 && ((dv == 64 && (dk == 64 || dk == 96 || dk == 128)) || (dv == 128 && dk == 128)) ? 1 : 0;
+}
+
+// As `edgelm_attn_prefill_split`, over tiles of at most 128 tokens; `n_pages` of the cache, or, with `page_table` null, the step's rows of
+// `kcache` and `vcache` ([rows][kv heads][...]).  `err`: the device error word (waits that run out, pages out of range).
+extern "C" int edgelm_attn_prefill_split_tc(const float* q, int ldq, void* out, int ldo, const void* kcache, const void* vcache, int n_pages,
+                                            const int32_t* page_table, int table_stride, const int32_t* tile_seq, const int32_t* tile_tok0,
+                                            const int32_t* tile_ntok, const int32_t* tile_pos0, int n_tiles, int nh, int nkv, int dk, int dv, float scale,
+                                            int mask, int mask_size, const float* sink, const float* gate, int ldg, int keep, int gate_ch, int maps,
+                                            int* err, cudaStream_t stream) {
+  if (n_tiles == 0) return 0;
+  EL_REFUSE(nh > 0 && nkv > 0 && nh % nkv == 0, "attn_prefill_split_tc: %d query heads are not a multiple of %d key/value heads", nh, nkv);
+  EL_REFUSE(edgelm_attn_prefill_split_tc_takes(dk, dv, maps), "attn_prefill_split_tc: head sizes %d / %d with %d maps", dk, dv, maps);
+  EL_REFUSE(maps == 1 || (sink == nullptr && gate == nullptr), "attn_prefill_split_tc: two maps take no sink and no gate");
+  EL_REFUSE(ldq % 4 == 0 && ldo % 4 == 0 && (uintptr_t)q % 16 == 0 && (uintptr_t)out % 16 == 0, "attn_prefill_split_tc: rows must be 16- and 8-byte aligned");
+  EL_REFUSE((uintptr_t)kcache % 16 == 0 && (uintptr_t)vcache % 16 == 0, "attn_prefill_split_tc: keys and values must be 16-byte aligned");
+  EL_REFUSE(mask == ST_MASK_CAUSAL || ((mask == ST_MASK_WINDOW || mask == ST_MASK_CHUNK) && mask_size >= 1), "attn_prefill_split_tc: mask %d of size %d", mask, mask_size);
+  EL_REFUSE(keep >= 0 && (keep == 0 || mask == ST_MASK_WINDOW) && (gate_ch == 0 || gate_ch == dv), "attn_prefill_split_tc: %d kept keys, a gate of %d channels", keep, gate_ch);
+  EL_REFUSE(err != nullptr && n_tiles > 0 && n_tiles <= 65535 && n_pages > 0 && (long long)n_pages * nkv * PAGE < (1LL << 31), "attn_prefill_split_tc: bad grid");
+  CUtensorMap mk, mv;
+  if (page_table) {
+    if (tensor_map(kcache, n_pages * nkv * PAGE, dk * maps, dk * maps, PAGE, &mk)) return -1;
+    if (tensor_map(vcache, n_pages * nkv * PAGE, dv, dv, PAGE, &mv)) return -1;
+  } else {
+    if (tensor_map(kcache, n_pages, nkv * maps * dk, nkv * maps * dk, PAGE, &mk)) return -1;
+    if (tensor_map(vcache, n_pages, nkv * dv, nkv * dv, PAGE, &mv)) return -1;
+  }
+  const SplitTcArgs a{q, ldq, out, ldo, page_table, table_stride, n_pages, tile_seq, tile_tok0, tile_ntok, tile_pos0, n_tiles, nh, nkv, maps, scale,
+                      gate, ldg, mask, mask_size, sink, keep, gate_ch, err};
+  int rc = 0;
+  if (dk == 64 && dv == 64) rc = launch_split_tc<64, 64>(mk, mv, a, stream);
+  else if (dk == 64) rc = launch_split_tc<64, 128>(mk, mv, a, stream);
+  else if (dk == 96) rc = launch_split_tc<96, 64>(mk, mv, a, stream);
+  else if (dv == 64) rc = launch_split_tc<128, 64>(mk, mv, a, stream);
+  else rc = launch_split_tc<128, 128>(mk, mv, a, stream);
+  if (rc) return rc;
+  EL_LAUNCH_CHECK("attn_prefill_split_tc");
+  return 0;
+}

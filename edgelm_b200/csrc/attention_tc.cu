@@ -97,33 +97,6 @@ __device__ __forceinline__ float at_max3(float a, float b, float c) {
   asm("max.f32 %0, %1, %2, %3;" : "=f"(d) : "f"(a), "f"(b), "f"(c));
   return d;
 }
-// A bounded wait that lets the hardware park the warp (a time hint on try_wait) and looks at the abort flag and the
-// clock only now and then: the roles of this kernel wait often and long, and their polling would take issue slots
-// from the exponentials.
-__device__ __forceinline__ bool at_wait(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err) {
-  if (mbar_try(bar, parity)) return true;
-  const long long t0 = clock64();
-  while (true) {
-#pragma unroll 1
-    for (int i = 0; i < 8; ++i) {
-      uint32_t ok;
-      asm volatile(
-          "{\n\t.reg .pred p;\n\t"
-          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
-          "selp.u32 %0, 1, 0, p;\n\t}"
-          : "=r"(ok)
-          : "r"(bar), "r"(parity), "r"(20000u)
-          : "memory");
-      if (ok) return true;
-    }
-    if (*abort_flag) return false;
-    if (clock64() - t0 > TC_WAIT_CYCLES) {
-      *abort_flag = 1;
-      atomicOr(err, ERR_WAIT_TIMEOUT);
-      return false;
-    }
-  }
-}
 __device__ __forceinline__ uint32_t at_pack(float a, float b) {
   const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
   return *reinterpret_cast<const uint32_t*>(&v);
@@ -307,7 +280,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
           p0 = p1 = 0;
         }
         const int y0 = (p0 * nkv + kvh) * PAGE, y1 = (p1 * nkv + kvh) * PAGE;
-        if (!at_wait(smem_u32(&empty[s]), par ^ 1u, abort_flag, err)) break;
+        if (!mbar_wait_parked(smem_u32(&empty[s]), par ^ 1u, abort_flag, err)) break;
         mbar_expect_tx(smem_u32(&full[s]), AT_KV_BYTES);
         tma_load_2d(smem_u32(dst + s * AT_KV_BYTES), map, smem_u32(&full[s]), 0, y0);
         tma_load_2d(smem_u32(dst + s * AT_KV_BYTES + AT_KV_BYTES / 2), map, smem_u32(&full[s]), 0, y1);
@@ -321,11 +294,11 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     // takes them from, and an issue took some 120 clocks.)
     constexpr uint32_t idesc_qk = umma_idesc(AT_ROWS, AT_KEYS);
     const uint64_t dq = umma_desc(smem_u32(q_s));
-    bool ok = __all_sync(0xffffffffu, at_wait(smem_u32(q_full), 0, abort_flag, err));
+    bool ok = __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(q_full), 0, abort_flag, err));
     for (int j = 0; j < n_blk && ok; ++j) {
       const int g = j & 1, st = j % AT_STAGES;
-      if (j >= 2 && !(ok = __all_sync(0xffffffffu, at_wait(smem_u32(&s_free[g]), (uint32_t)((j >> 1) - 1) & 1u, abort_flag, err)))) break;
-      if (!(ok = __all_sync(0xffffffffu, at_wait(smem_u32(&k_full[st]), (uint32_t)(j / AT_STAGES) & 1u, abort_flag, err)))) break;
+      if (j >= 2 && !(ok = __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(&s_free[g]), (uint32_t)((j >> 1) - 1) & 1u, abort_flag, err)))) break;
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(&k_full[st]), (uint32_t)(j / AT_STAGES) & 1u, abort_flag, err)))) break;
       if (j == 1 && n_blk >= 4) {
         // The second group starts half a block's time behind the first.  Nothing else sets the groups' offset, and it
         // stays where it starts: in step, both groups are at their exponentials together and leave the special-function
@@ -351,8 +324,8 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     bool ok = true;
     for (int j = 0; j < n_blk && ok; ++j) {
       const int g = j & 1, u = j >> 1, st = j % AT_V_STAGES;
-      if (!(ok = __all_sync(0xffffffffu, at_wait(smem_u32(&p_ready[2 * g + (u & 1)]), (uint32_t)(u >> 1) & 1u, abort_flag, err)))) break;
-      if (!(ok = __all_sync(0xffffffffu, at_wait(smem_u32(&v_full[st]), (uint32_t)(j / AT_V_STAGES) & 1u, abort_flag, err)))) break;
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(&p_ready[2 * g + (u & 1)]), (uint32_t)(u >> 1) & 1u, abort_flag, err)))) break;
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(&v_full[st]), (uint32_t)(j / AT_V_STAGES) & 1u, abort_flag, err)))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       if (tracing && lane == 0 && u < AT_TRACE_BLOCKS) trace[(g * AT_TRACE_BLOCKS + u) * 8 + 6] = clock64();   // (the issuer's view: P and V seen,
       const uint64_t dv = umma_desc(smem_u32(v_s + st * AT_KV_BYTES));
@@ -395,7 +368,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       const int key0 = j * AT_KEYS + half * AT_HALF;
       uint8_t* p_tile = p_s + (g * AT_P_BUFS + (u % AT_P_BUFS)) * AT_P_BYTES + half * (AT_P_BYTES / 2);
       stamp(u, 0);
-      if (!(ok = __all_sync(0xffffffffu, at_wait(smem_u32(&s_ready[g]), u & 1, abort_flag, err)))) break;
+      if (!(ok = __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(&s_ready[g]), u & 1, abort_flag, err)))) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       stamp(u, 1);
       float rescale;
@@ -407,7 +380,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       // it read is free for the block after this one.  (The P V of the block before last would do for the buffer,
       // and the scaling is rare; but without this wait the two groups fall into step, are at their exponentials
       // together and leave the special-function units idle together: measured a quarter slower.)
-      if (u > 0 && !(ok = __all_sync(0xffffffffu, at_wait(smem_u32(&o_ready[2 * g + ((u - 1) & 1)]), (uint32_t)((u - 1) >> 1) & 1u, abort_flag, err)))) break;
+      if (u > 0 && !(ok = __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(&o_ready[2 * g + ((u - 1) & 1)]), (uint32_t)((u - 1) >> 1) & 1u, abort_flag, err)))) break;
       stamp(u, 3);
       if (__any_sync(0xffffffffu, rescale != 1.f)) {   // rare after the first blocks
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
@@ -426,7 +399,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
       l = fmaf(l, rescale, lsum);
       if (j == n_blk - 1 && n_keys < j * AT_KEYS + AT_KEYS) {
         // value rows past the tile's last position: every weight on them is zero; make them zero too
-        if (!(ok = __all_sync(0xffffffffu, at_wait(smem_u32(&v_full[j % AT_V_STAGES]), (uint32_t)(j / AT_V_STAGES) & 1u, abort_flag, err)))) break;
+        if (!(ok = __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(&v_full[j % AT_V_STAGES]), (uint32_t)(j / AT_V_STAGES) & 1u, abort_flag, err)))) break;
         const int first = n_keys - j * AT_KEYS;   // 1 .. 127
         for (int i = (sw & 7) * 32 + lane; i < (AT_KEYS - first) * 8; i += AT_GROUP_THREADS) {
           const int r = first + (i >> 3);
@@ -444,7 +417,7 @@ attn_prefill_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_c
     // of tensor memory, so each reads its 16 dims of the row from all four accumulators; only (m, l) go through
     // shared memory (over this group's K stage: its last Q K^T is long done).
     if (ok && u > 0)
-      ok = __all_sync(0xffffffffu, at_wait(smem_u32(&o_ready[2 * g + ((u - 1) & 1)]), (uint32_t)((u - 1) >> 1) & 1u, abort_flag, err));
+      ok = __all_sync(0xffffffffu, mbar_wait_parked(smem_u32(&o_ready[2 * g + ((u - 1) & 1)]), (uint32_t)((u - 1) >> 1) & 1u, abort_flag, err));
     asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
     const int q = g * 2 + half;
     float* hand_ml = reinterpret_cast<float*>(k_s + g * AT_KV_BYTES);   // [half][row][2]

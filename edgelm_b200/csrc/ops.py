@@ -1045,6 +1045,40 @@ def attn_prefill_split_takes(dtype, dk, dv, maps=1):
     return maps == 1 and dtype == torch.bfloat16 and dk in (32, 64, 96, 128) and dv in (32, 64, 96, 128) and dv <= dk
 
 
+SPLIT_TC_TILE = 128  # new tokens per tile of the tcgen05 form of it (ST_ROWS in attention_split_tc.cu)
+# Steps whose longest sequence brings fewer new tokens than this stay on tiles of 64 and mma.sync (us there and on tcgen05: 9 heads of 96 / 64, 192
+# tokens 10.4 and 12.0, 256 12.5 and 13.0, 400 16.8 and 14.2; 16 heads of two maps, four times 192 20.9 and 22.6, 256 31 and 25, 400 80 and 49).
+SPLIT_TC_MIN_TOKENS = 256
+
+
+def attn_prefill_split_tc_takes(dtype, dk, dv, maps=1):
+    """Whether the tcgen05 form of `attn_prefill_split` takes these sizes."""
+    return dtype == torch.bfloat16 and bool(lib().edgelm_attn_prefill_split_tc_takes(int(dk), int(dv), int(maps)))
+
+
+def attn_prefill_split_tc(q, out, kcache, vcache, page_table, tile_seq, tile_tok0, tile_ntok, tile_pos0, n_tiles, nh, nkv, dk, dv, scale, err, gate=None,
+                          mask=0, mask_size=0, sink=None, keep=0, maps=1):
+    """`attn_prefill_split` on tcgen05, over tiles of at most SPLIT_TC_TILE tokens; `err`: the device error word."""
+    _f32(q, "q")
+    T = q.shape[0]
+    _need(q.shape == (T, nh * maps * dk) and out.dtype == (torch.bfloat16 if maps == 1 else torch.float32) and out.is_contiguous() and
+          out.shape == (T, nh * maps * dv), "attn_prefill_split_tc: shapes")
+    _need(vcache is not None and kcache.dtype == torch.bfloat16 and vcache.dtype == torch.bfloat16, "attn_prefill_split_tc: bfloat16 keys with values of their own")
+    if page_table is not None:
+        _masked_cache_check(kcache, vcache, nkv, maps * dk, dv, "attn_prefill_split_tc")
+        _i32(page_table, "page_table")
+    else:
+        _need(kcache.is_contiguous() and vcache.is_contiguous() and kcache.shape == (T, nkv * maps * dk) and vcache.shape == (T, nkv * dv), "attn_prefill_split_tc: the step's own keys and values")
+    _need(sink is None or (sink.dtype == torch.float32 and sink.is_cuda and sink.is_contiguous() and sink.numel() == nh), "attn_prefill_split_tc: sink")
+    gate_ch = _gate_check(gate, T, nh, dv, "attn_prefill_split_tc")
+    for t, n in ((tile_seq, "tile_seq"), (tile_tok0, "tile_tok0"), (tile_ntok, "tile_ntok"), (tile_pos0, "tile_pos0")):
+        _i32(t, n)
+    _check(lib().edgelm_attn_prefill_split_tc(_p(q), q.stride(0), _p(out), out.stride(0), _p(kcache), _p(vcache), kcache.shape[0], _p(page_table),
+                                              page_table.stride(0) if page_table is not None else 0, _p(tile_seq), _p(tile_tok0), _p(tile_ntok), _p(tile_pos0),
+                                              int(n_tiles), nh, nkv, dk, dv, ctypes.c_float(scale), int(mask), int(mask_size or 0), _p(sink),
+                                              _p(gate), gate.stride(0) if gate is not None else 0, int(keep), gate_ch, int(maps), _p(err), _stream()))
+
+
 def attn_prefill_split(q, out, kcache, vcache, page_table, tile_seq, tile_tok0, tile_ntok, tile_pos0, n_tiles, nh, nkv, dk, dv, scale, gate=None,
                        max_keys=0, mask=0, mask_size=0, sink=None, keep=0, maps=1):
     """Attention of a prompt step over bfloat16 keys and values on the tensor cores with float32 scores and softmax weights: the

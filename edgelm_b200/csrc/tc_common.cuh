@@ -46,6 +46,32 @@ __device__ __forceinline__ bool mbar_wait(uint32_t bar, uint32_t parity, volatil
     }
   }
 }
+// A bounded wait that lets the hardware park the warp (a time hint on try_wait) and looks at the abort flag and the
+// clock only now and then: for roles that wait often and long, whose polling would take issue slots from others.
+__device__ __forceinline__ bool mbar_wait_parked(uint32_t bar, uint32_t parity, volatile int* abort_flag, int* err) {
+  if (mbar_try(bar, parity)) return true;
+  const long long t0 = clock64();
+  while (true) {
+#pragma unroll 1
+    for (int i = 0; i < 8; ++i) {
+      uint32_t ok;
+      asm volatile(
+          "{\n\t.reg .pred p;\n\t"
+          "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+          "selp.u32 %0, 1, 0, p;\n\t}"
+          : "=r"(ok)
+          : "r"(bar), "r"(parity), "r"(20000u)
+          : "memory");
+      if (ok) return true;
+    }
+    if (*abort_flag) return false;
+    if (clock64() - t0 > TC_WAIT_CYCLES) {
+      *abort_flag = 1;
+      atomicOr(err, ERR_WAIT_TIMEOUT);
+      return false;
+    }
+  }
+}
 // One lane of a converged warp (the same one every time).
 __device__ __forceinline__ bool elect_one() {
   uint32_t chosen;

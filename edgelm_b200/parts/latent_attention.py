@@ -31,7 +31,7 @@ from ..config.base import ConfigError
 from ..csrc import ops
 from . import linear
 from .base import KVNeed, Part, as_matrix, as_vector, nbytes
-from .masked_attention import MASKS, MAX_SPLITS, SHARED_KEYS_MIN_GROUP, decode_splits, kept_first, most_keys, read_mask, single_token_tiles, splits_room
+from .masked_attention import MASKS, MAX_SPLITS, SHARED_KEYS_MIN_GROUP, decode_splits, kept_first, most_keys, read_mask, single_token_tiles, split_prefill, split_prefill_tiles, splits_room
 from .registry import register_mixer
 from .rope import rotary_frequencies, rotary_magnitude
 
@@ -73,7 +73,7 @@ class LatentAttention(Part):
         return ops.attn_prefill_split_takes(self.dtype, self.dq, self.dv)
 
     def tile_sizes(self):
-        return (self.tile_tokens, ops.SPLIT_PREFILL_TILE if self._on_tensor_cores() else self.EXPANDED_TILE)
+        return (self.tile_tokens,) + (split_prefill_tiles(self.dtype, self.dq, self.dv) if self._on_tensor_cores() else (self.EXPANDED_TILE,))
 
     def sizes(self):
         return {"heads": self.nh, "head_dim": self.d, "rot_dim": self.rd, "v_head_dim": self.dv, "kv_rank": self.rank,
@@ -195,10 +195,8 @@ class LatentAttention(Part):
         a = ws.alloc((T, self.nh * self.dv), self.dtype)
         with ctx.prof("attn_latent"):
             if self._on_tensor_cores():
-                tiles = ctx.tiles(ops.SPLIT_PREFILL_TILE)
-                ops.attn_prefill_split(q, a, kx, vx, None, tiles.seq, tiles.tok0, tiles.ntok, tiles.pos0, tiles.count, self.nh, self.nh, self.dq, self.dv,
-                                       self.scale, gate=gate, max_keys=max(ctx.seq_lengths), mask=self.mask, mask_size=self.mask_size, sink=self.sink,
-                                       keep=self.keep)
+                split_prefill(ctx, q, a, kx, vx, None, self.nh, self.nh, self.dq, self.dv, self.scale, max(ctx.seq_lengths), gate=gate, mask=self.mask,
+                              mask_size=self.mask_size, sink=self.sink, keep=self.keep)
             else:
                 tiles = ctx.tiles(self.EXPANDED_TILE)
                 ops.masked_attn_tiled(q, a, kx, vx, None, tiles.seq, tiles.tok0, tiles.ntok, tiles.pos0, tiles.count, self.EXPANDED_TILE,

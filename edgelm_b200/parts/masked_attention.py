@@ -115,6 +115,21 @@ def decode_splits(ctx, n_kv_heads, group, mask, mask_size, keep=0):
     return splits
 
 
+def split_prefill_tiles(dtype, dk, dv, maps=1):
+    """Tile sizes of the prompt steps' tensor-core kernels with float32 scores and weights."""
+    return (ops.SPLIT_PREFILL_TILE,) + ((ops.SPLIT_TC_TILE,) if ops.attn_prefill_split_tc_takes(dtype, dk, dv, maps) else ())
+
+
+def split_prefill(ctx, q, out, k, v, table, nh, nkv, dk, dv, scale, max_keys, maps=1, **options):
+    """Those kernels' step: on tcgen05 where it takes the sizes and some sequence brings tokens enough for its tiles, else on mma.sync."""
+    if max(ctx.seq_lengths) >= ops.SPLIT_TC_MIN_TOKENS and ops.attn_prefill_split_tc_takes(k.dtype, dk, dv, maps):
+        t = ctx.tiles(ops.SPLIT_TC_TILE)
+        ops.attn_prefill_split_tc(q, out, k, v, table, t.seq, t.tok0, t.ntok, t.pos0, t.count, nh, nkv, dk, dv, scale, ctx.err, maps=maps, **options)
+    else:
+        t = ctx.tiles(ops.SPLIT_PREFILL_TILE)
+        ops.attn_prefill_split(q, out, k, v, table, t.seq, t.tok0, t.ntok, t.pos0, t.count, nh, nkv, dk, dv, scale, max_keys=max_keys, maps=maps, **options)
+
+
 def splits_room(n_seqs, n_heads, dv):
     """Bytes of the splits' partial results for a step of `n_seqs` single tokens (sequences x splits stays under 2 SMs' worth
     of blocks plus the sequences themselves, (token, head) pairs x their splits under BLOCKS_AN_SM SMs' worth plus the pairs; 600 and
@@ -197,7 +212,7 @@ class MaskedAttention(Part):
         return ops.masked_attn_rows_takes(self.dtype, self.dk, self.dv, self.maps)
 
     def tile_sizes(self):
-        return (self.tile_tokens, ops.SPLIT_PREFILL_TILE) if self._on_tensor_cores() else (self.tile_tokens,)
+        return (self.tile_tokens,) + (split_prefill_tiles(self.dtype, self.dk, self.dv, self.maps) if self._on_tensor_cores() else ())
 
     def sizes(self):
         out = {"heads": self.nh, "kv_heads": self.nkv, "head_dim": self.dk, "v_head_dim": self.dv, "rot_dims": self.rot,
@@ -334,10 +349,9 @@ class MaskedAttention(Part):
                                 self.mask, self.mask_size, self.sink, most_keys(self.mask, self.mask_size, self.keep), maps=self.maps, gate=gate,
                                 n_splits=splits, part=part, keep=self.keep)
             elif self._on_tensor_cores():
-                tiles = ctx.tiles(ops.SPLIT_PREFILL_TILE)
-                ops.attn_prefill_split(q, a, cache.k, cache.v, table, tiles.seq, tiles.tok0, tiles.ntok, tiles.pos0, tiles.count, self.nh, self.nkv,
-                                       self.dk, self.dv, self.scale, gate=gate, mask=self.mask, mask_size=self.mask_size, sink=self.sink, keep=self.keep, maps=self.maps,
-                                       max_keys=max(p + n for p, n in zip(ctx.seq_first_positions, ctx.seq_lengths)))
+                split_prefill(ctx, q, a, cache.k, cache.v, table, self.nh, self.nkv, self.dk, self.dv, self.scale,
+                              max(p + n for p, n in zip(ctx.seq_first_positions, ctx.seq_lengths)), maps=self.maps, gate=gate, mask=self.mask,
+                              mask_size=self.mask_size, sink=self.sink, keep=self.keep)
             else:
                 tiles = ctx.tiles(self.tile_tokens)
                 ops.masked_attn_tiled(q, a, cache.k, cache.v, table, tiles.seq, tiles.tok0, tiles.ntok, tiles.pos0, tiles.count,

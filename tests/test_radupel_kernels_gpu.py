@@ -455,6 +455,50 @@ def test_tensor_core_attention_scale_of_any_sign(scale):
     assert float((outs[0] - outs[1]).abs().max()) <= 2.0 ** -7 * float(outs[1].abs().max())
 
 
+@pytest.mark.parametrize("new,first,H,G,dk,dv,maps,mask,size,keep,sink,gate,own,scale", [
+    ([1, 128, 129], [0, 0, 0], 2, 1, 64, 64, 1, 0, 0, 0, False, 1, False, 0.125), ([127, 64, 300], [1, 63, 70], 3, 3, 64, 64, 1, 0, 0, 0, True, 0, False, 0.2),
+    ([300], [200], 2, 1, 64, 64, 1, 1, 90, 70, False, 2, False, 0.1), ([257, 70], [0, 30], 2, 2, 128, 64, 1, 1, 64, 0, True, 0, False, 0.1),
+    ([400, 65], [37, 0], 4, 2, 64, 64, 1, 2, 100, 0, True, 1, False, -0.1), ([200, 130], [0, 5], 2, 1, 128, 128, 1, 2, 128, 0, False, 2, False, 0.05),
+    ([129, 260, 1], [0, 0, 0], 3, 3, 96, 64, 1, 0, 0, 0, False, 0, True, 0.1), ([300, 64], [0, 0], 2, 2, 128, 64, 1, 1, 150, 40, False, 1, True, 0.1),
+    ([300, 90], [100, 0], 2, 1, 96, 64, 1, 0, 0, 0, False, 0, False, 0.0), ([130, 300], [0, 250], 3, 1, 64, 128, 2, 2, 256, 0, False, 0, False, 0.125),
+    ([260], [3], 2, 2, 64, 64, 2, 0, 0, 0, False, 0, False, 0.125), ([300], [0], 2, 2, 64, 128, 2, 1, 70, 0, False, 0, True, 0.125)])
+def test_tcgen05_attention_over_all_its_forms(new, first, H, G, dk, dv, maps, mask, size, keep, sink, gate, own, scale):
+    """The tcgen05 kernel against the mma.sync one, which takes every form too: tiles' and pages' edges, pages that no row sees, blocks without a
+    second page, rows behind a sequence's end that hold not-a-numbers.  Both sum the same exact products in float32, cut off differently: bfloat16
+    outputs may round to neighbours (2^-8), float32 ones (two maps) differ by cut-offs, 24 a block of 128 keys of 2^-24 each: 3e-6 for up to 550 keys."""
+    g = torch.Generator().manual_seed(sum(new) + dk)
+    rnd = lambda *s: torch.randn(*s, generator=g)
+    T, lengths = sum(new), [a + b for a, b in zip(new, first)]
+    q, sk = (rnd(T, H * maps * dk) * 2).to(DEV), rnd(H).to(DEV) if sink else None
+    gt = (rnd(T, (H if gate == 1 else H * dv) + 3)).to(DEV)[:, 3:] if gate else None
+    if own:
+        k, v, table = rnd(T, G * maps * dk).to(DEV, torch.bfloat16), rnd(T, G * dv).to(DEV, torch.bfloat16), None
+    else:
+        held = [-(-n // PAGE) for n in lengths]
+        order, at = torch.randperm(sum(held) + 2, generator=g).tolist(), 0
+        rows = [[order[sum(held[:s]) + i] if i < held[s] else -1 for i in range(max(held))] for s in range(len(new))]
+        k, v = torch.full((len(order), G, PAGE, maps * dk), float("nan")), torch.full((len(order), G, PAGE, dv), float("nan"))
+        for s, n in enumerate(lengths):
+            for i in range(held[s]):
+                m = min(PAGE, n - i * PAGE)
+                k[rows[s][i], :, :m], v[rows[s][i], :, :m] = rnd(G, m, maps * dk), rnd(G, m, dv)
+        k, v, table = k.to(DEV, torch.bfloat16), v.to(DEV, torch.bfloat16), i32(rows)
+    assert ops.attn_prefill_split_tc_takes(torch.bfloat16, dk, dv, maps) and not ops.attn_prefill_split_tc_takes(torch.float32, dk, dv, maps)
+    outs, err = [], torch.zeros(1, dtype=torch.int32, device=DEV)
+    options = dict(gate=gt, mask=mask, mask_size=size, sink=sk, keep=keep, maps=maps)
+    for tile in (ops.SPLIT_PREFILL_TILE, ops.SPLIT_TC_TILE):
+        out = torch.full((T, H * maps * dv), float("nan"), dtype=torch.bfloat16 if maps == 1 else torch.float32, device=DEV)
+        tiles = make_tiles(new, first, tile)
+        if tile == ops.SPLIT_TC_TILE:
+            ops.attn_prefill_split_tc(q, out, k, v, table, *tiles, H, G, dk, dv, scale, err, **options)
+        else:
+            ops.attn_prefill_split(q, out, k, v, table, *tiles, H, G, dk, dv, scale, max_keys=max(lengths), **options)
+        outs.append(out.float())
+    assert int(err.item()) == 0
+    off, size_of = (outs[0] - outs[1]).abs(), outs[0].abs()
+    assert bool((off <= (2.0 ** -7 * size_of + 1e-5 if maps == 1 else 3e-6 * float(size_of.max()))).all())
+
+
 # ----------------------------------------------------------------------------- the scoring router and its experts
 @pytest.mark.parametrize("E,ident,top,groups,keep,negative", [(6, 3, 3, 3, 2, False), (3, 0, 1, 1, 1, False), (5, 1, 2, 2, 1, True), (7, 2, 2, 3, 1, True),
                                                               (8, 0, 4, 4, 2, False), (2, 2, 2, 1, 1, True), (12, 4, 3, 8, 2, False), (4, 2, 3, 3, 1, True)])
