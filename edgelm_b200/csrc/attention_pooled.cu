@@ -318,6 +318,135 @@ pooled_window_attn_kernel(const T* __restrict__ q, T* __restrict__ out, const T*
   }
 }
 
+// The same for key and value heads of D dimensions alike, rows of whole 16-byte pieces: a load instruction of a warp covers 32 / LPR whole
+// rows, and a warp's 32 keys and values (fewer of rows over 128 bytes) are requested together, before the first score is known.  (In the kernel above a
+// lane reads a key by itself and the warp walks its values one after the other, a trip to memory or four keys at a time: 16 tokens of 9
+// heads, window 512: 54 us.)  A warp takes a run of the window's keys and a run of the pooled rows (float32 rows: lanes of 4 dimensions),
+// each with a maximum, a denominator and an output of its own; all are merged in order through shared memory.  Bound by four trips to
+// memory in a chain (position, page, rows, merge), which is why a block has as many warps as keep a run at 32 keys where blocks are few.
+template <typename T, int D>
+struct PwRow {
+  static constexpr int EPL = 16 / sizeof(T), LPR = D / EPL, RPI = 32 / LPR;      // elements a lane, lanes a row, rows an instruction
+  static constexpr int ITS = RPI >= 4 ? 32 / RPI : 8, KEYS = ITS * RPI;                           // instructions in flight (8 at most), their rows
+};
+__device__ __forceinline__ void pw_unpack(const uint4& u, float* v, const float*) {
+  v[0] = __uint_as_float(u.x); v[1] = __uint_as_float(u.y); v[2] = __uint_as_float(u.z); v[3] = __uint_as_float(u.w);
+}
+__device__ __forceinline__ void pw_unpack(const uint4& u, float* v, const __nv_bfloat16*) {
+  const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    v[2 * i] = __uint_as_float(w[i] << 16);
+    v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
+  }
+}
+// A run of rows [begin, end) through one query: `row_of(r)` is the row's number in `keys` and `values` (-1: none).
+template <typename T, int D, typename RowOf>
+__device__ __forceinline__ void pw_run(const T* __restrict__ keys, const T* __restrict__ values, const float* qh, int begin, int end, int lane, RowOf row_of,
+                                       float& m, float& l, float* slot) {
+  using R = PwRow<T, D>;
+  const int part = lane % R::LPR, grp = lane / R::LPR;
+  float qv[R::EPL], o[R::EPL] = {};
+#pragma unroll
+  for (int e = 0; e < R::EPL; ++e) qv[e] = qh[part * R::EPL + e];
+  for (int r0 = begin; r0 < end; r0 += R::KEYS) {
+    uint4 kv[R::ITS], vv[R::ITS];
+    bool there[R::ITS];
+#pragma unroll
+    for (int i = 0; i < R::ITS; ++i) {
+      const int r = r0 + i * R::RPI + grp, row = r < end ? row_of(r) : -1;
+      there[i] = row >= 0;
+      kv[i] = there[i] ? *reinterpret_cast<const uint4*>(keys + (size_t)row * D + part * R::EPL) : make_uint4(0, 0, 0, 0);
+      vv[i] = there[i] ? *reinterpret_cast<const uint4*>(values + (size_t)row * D + part * R::EPL) : make_uint4(0, 0, 0, 0);
+    }
+    float sc[R::ITS], m_new = m;
+#pragma unroll
+    for (int i = 0; i < R::ITS; ++i) {
+      float k[R::EPL], d = 0.f;
+      pw_unpack(kv[i], k, keys);
+#pragma unroll
+      for (int e = 0; e < R::EPL; ++e) d = fmaf(qv[e], k[e], d);
+#pragma unroll
+      for (int x = 1; x < R::LPR; x <<= 1) d += __shfl_xor_sync(0xffffffffu, d, x);
+      sc[i] = there[i] ? d : -INFINITY;
+      m_new = fmaxf(m_new, sc[i]);
+    }
+    m_new = warp_max(m_new);
+    if (m_new == -INFINITY) continue;
+    const float corr = m == -INFINITY ? 0.f : expf(m - m_new);
+    float sum = 0.f;
+#pragma unroll
+    for (int e = 0; e < R::EPL; ++e) o[e] *= corr;
+#pragma unroll
+    for (int i = 0; i < R::ITS; ++i) {
+      if (!there[i]) continue;
+      float v[R::EPL];
+      const float w = expf(sc[i] - m_new);
+      sum += w;
+      pw_unpack(vv[i], v, values);
+#pragma unroll
+      for (int e = 0; e < R::EPL; ++e) o[e] = fmaf(w, v[e], o[e]);
+    }
+    l = l * corr + sum;                        // (this lane's rows)
+    m = m_new;
+  }
+#pragma unroll
+  for (int x = R::LPR; x < 32; x <<= 1) {
+    l += __shfl_xor_sync(0xffffffffu, l, x);
+#pragma unroll
+    for (int e = 0; e < R::EPL; ++e) o[e] += __shfl_xor_sync(0xffffffffu, o[e], x);
+  }
+  if (grp == 0)
+#pragma unroll
+    for (int e = 0; e < R::EPL; ++e) slot[part * R::EPL + e] = o[e];
+}
+
+constexpr int PWR_MAX_WARPS = 16;
+template <typename T, int D>
+__global__ void __launch_bounds__(PWR_MAX_WARPS * 32)
+pooled_window_attn_rows_kernel(const T* __restrict__ q, T* __restrict__ out, const T* __restrict__ kcache, const T* __restrict__ vcache,
+                               const float* __restrict__ pk, const float* __restrict__ pv, const int32_t* __restrict__ tok_pos,
+                               const int32_t* __restrict__ tok_seq, const int32_t* __restrict__ page_table, int table_stride,
+                               int n_pages, int H, int G, float scale, int window, int P, int R) {
+  pdl_launch_dependents();
+  pdl_wait();
+  __shared__ float qh[D], wm[2 * PWR_MAX_WARPS], wl[2 * PWR_MAX_WARPS], wo[2 * PWR_MAX_WARPS][D];      // (a warp's window run, its pooled run)
+  const int t = blockIdx.x, h = blockIdx.y, lane = threadIdx.x & 31, warp = threadIdx.x >> 5, NW = blockDim.x >> 5;
+  const int pos = tok_pos[t];
+  if (pos < 0) return;
+  const int g = h / (H / G);
+  const int32_t* table = page_table + (size_t)tok_seq[t] * table_stride;
+  for (int i = threadIdx.x; i < D; i += blockDim.x) qh[i] = to_f32(q[((size_t)t * H + h) * D + i]) * scale;
+  __syncthreads();
+  const int lo = max(0, pos - window + 1), n_win = pos - lo + 1;
+  const int n_blocks = (P > 0 && pos - window >= 0) ? (pos - window + 1) / P : 0;
+  float m = -INFINITY, l = 0.f;
+  pw_run<T, D>(kcache, vcache, qh, (int)((long long)n_win * warp / NW), (int)((long long)n_win * (warp + 1) / NW), lane, [&](int r) {
+    const int p = lo + r, page = table[p / PAGE];
+    return page >= 0 && page < n_pages ? (page * G + g) * PAGE + p % PAGE : -1;
+  }, m, l, wo[2 * warp]);
+  if (lane == 0) { wm[2 * warp] = m; wl[2 * warp] = l; }
+  m = -INFINITY, l = 0.f;
+  if (n_blocks)
+    pw_run<float, D>(pk, pv, qh, n_blocks * warp / NW, n_blocks * (warp + 1) / NW, lane, [&](int e) {
+      const int end = e * P + P - 1, page = table[end / PAGE];
+      return page >= 0 && page < n_pages ? (page * G + g) * R + (e - (PAGE * (end / PAGE)) / P) : -1;
+    }, m, l, wo[2 * warp + 1]);
+  if (lane == 0) { wm[2 * warp + 1] = m; wl[2 * warp + 1] = l; }
+  __syncthreads();
+  if (threadIdx.x < D) {
+    float M = -INFINITY, L = 0.f, acc = 0.f;
+    for (int w = 0; w < 2 * NW; ++w) M = fmaxf(M, wm[w]);
+    for (int w = 0; w < 2 * NW; ++w) {
+      if (wm[w] == -INFINITY) continue;
+      const float f = expf(wm[w] - M);
+      L = fmaf(wl[w], f, L);
+      acc = fmaf(wo[w][threadIdx.x], f, acc);
+    }
+    out[((size_t)t * H + h) * D + threadIdx.x] = from_f32<T>(L > 0.f ? acc * (1.0f / L) : 0.f);
+  }
+}
+
 // ---- the attention kernel of prompt steps
 // A block = up to 32 (token, query head) rows of one key/value head and of one run of consecutive tokens (a tile of the
 // step's metadata); 64 keys with their values are staged in shared memory as float32 once for all the rows: first the
@@ -770,6 +899,23 @@ extern "C" int edgelm_pooled_window_attn(const void* q, void* out, const void* k
   const int pair_v = dv % 2 == 0 && (uintptr_t)vcache % 8 == 0;
   EL_REFUSE(P == 0 || ((uintptr_t)pk % 16 == 0 && (uintptr_t)pv % 8 == 0), "pooled_window_attn: the pooled rows are not 16-byte aligned");
   EL_REFUSE((long long)n_pages * G * (PAGE > R ? PAGE : R) < (1ll << 31), "pooled_window_attn: more cache rows than a 32-bit index counts");
+  if (dk == dv && (dk == 32 || dk == 64 || dk == 128) && vec_k && (uintptr_t)vcache % 16 == 0 && (P == 0 || (uintptr_t)pv % 16 == 0)) {
+    // warps a block: a run of 32 keys a warp where blocks are few (the chain of trips counts), fewer and longer runs where there are many
+    const long long blocks = (long long)n_tokens * H;
+    const int most = blocks >= 148 * 12 ? 4 : blocks >= 148 * 4 ? 8 : PWR_MAX_WARPS, warps = max(1, min(most, (window + 31) / 32));
+    const dim3 threads(max(warps * 32, dk));
+#define EL_PWR(TT, DD) launch_pdl(pdl_bit_for_tokens(n_tokens), pooled_window_attn_rows_kernel<TT, DD>, grid, threads, (size_t)0, stream, (const TT*)q, (TT*)out, \
+      (const TT*)kcache, (const TT*)vcache, pk, pv, tok_pos, tok_seq, page_table, table_stride, n_pages, H, G, scale, window, P, R)
+    if (dtype == DT_F32) {
+      if (dk == 32) EL_PWR(float, 32); else if (dk == 64) EL_PWR(float, 64); else EL_PWR(float, 128);
+    } else if (dtype == DT_BF16) {
+      if (dk == 32) EL_PWR(__nv_bfloat16, 32); else if (dk == 64) EL_PWR(__nv_bfloat16, 64); else EL_PWR(__nv_bfloat16, 128);
+    } else
+      EL_REFUSE(false, "pooled_window_attn: unknown dtype code %d", dtype);
+#undef EL_PWR
+    EL_LAUNCH_CHECK("pooled_window_attn");
+    return 0;
+  }
   const int dvr = dv <= 64 ? 1 : (dv <= 128 ? 2 : 4);
 #define EL_PWA(TT, DVR) launch_pdl(pdl_bit_for_tokens(n_tokens), pooled_window_attn_kernel<TT, DVR>, dim3(grid), dim3(block), (size_t)(smem), stream, (const TT*)q, (TT*)out, (const TT*)kcache, (const TT*)vcache, pk, pv, \
       tok_pos, tok_seq, page_table, table_stride, n_pages, H, G, dk, dv, scale, window, P, R, vec_k, pair_v)

@@ -398,6 +398,14 @@ def test_window_attention_with_pooled_blocks(dtype, window, pool, dk, dv, H, G):
         assert np.isfinite(ot).all() and np.abs(ot - w).max() < tol * max(1.0, np.abs(w).max())
 
 
+@pytest.mark.parametrize("window,pool,d,H,G", [(9, 4, 64, 4, 2), (70, 64, 32, 3, 3), (33, 1, 128, 2, 1), (64, 5, 64, 3, 1), (40, 7, 128, 2, 2)])
+def test_window_attention_of_whole_rows(window, pool, d, H, G):
+    """Heads that the kernel of whole rows takes: runs of keys and of pooled rows that are empty, a part of a load and several loads."""
+    for dtype in (torch.float32, torch.bfloat16):
+        test_window_attention_with_pooled_blocks(dtype, window, pool, d, d, H, G)
+
+
+
 @pytest.mark.parametrize("window,pool,d,H,G", [(100, 64, 64, 4, 2), (7, 3, 32, 3, 1), (64, 1, 96, 2, 2), (200, 5, 128, 2, 1), (50, None, 64, 2, 1)])
 def test_pooled_attention_on_the_tensor_cores(window, pool, d, H, G):
     """Prompts and pieces that go on from the cache, up to 300 pooled rows, edges of pages and tiles, unwritten rows poisoned.  The
