@@ -188,6 +188,7 @@ template <> struct KVec<__nv_bfloat16> {
 };
 
 // ------------------------------------------------------------------------- decode
+// attn_decode_kernel: every head size; the ones that attention_decode_rows.cuh and attention_decode_mma.cuh take run there.
 // One new token per sequence.  grid (sequence, kv head, split), 4 warps per block.  The pages of
 // the sequence that fall to this split are cut into tiles of `tk` keys (a tile of K and of V is
 // at most 8 KB); tiles are dealt to the block's warps.  For each tile a warp
@@ -241,6 +242,67 @@ template <> struct Pair<__nv_bfloat16> {
     *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b);
   }
 };
+
+// A block's result of up to RW heads (head0 on) from its warps' partials Wp [warp][pitch][hd + 2] (values, maximum, sum):
+// folded in the order of the warps 0..3, warp r row r; written to the output, or to the splits' scratch.
+template <typename T, int NP>
+__device__ __forceinline__ void decode_fold_warps(const float* Wp, int pitch, int rows, int hd, int seq, int head0, int nh, int split,
+                                                  int n_splits, T* __restrict__ out, int ldo, float* __restrict__ part_o,
+                                                  float* __restrict__ part_ml) {
+  const int lane = threadIdx.x & 31, r = threadIdx.x >> 5, ws = hd + 2;
+  if (r >= rows) return;
+  float M = -CUDART_INF_F;
+  for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, Wp[(w * pitch + r) * ws + hd]);
+  if (M != M) M = CUDART_NAN_F;
+  float L = 0.f, o[NP][2];
+#pragma unroll
+  for (int c = 0; c < NP; ++c) o[c][0] = o[c][1] = 0.f;
+  bool bad = false;
+  for (int w = 0; w < DEC_WARPS; ++w) bad = bad || (Wp[(w * pitch + r) * ws + hd] != Wp[(w * pitch + r) * ws + hd]);
+  if (M != -CUDART_INF_F && !bad) {
+    for (int w = 0; w < DEC_WARPS; ++w) {
+      const float* p = Wp + (w * pitch + r) * ws;
+      if (p[hd] == -CUDART_INF_F) continue;
+      const float f = expf(p[hd] - M);
+      L = fmaf(p[hd + 1], f, L);
+#pragma unroll
+      for (int c = 0; c < NP; ++c) {
+        const int d = 2 * lane + 64 * c;
+        if (d < hd) {
+          o[c][0] = fmaf(p[d], f, o[c][0]);
+          o[c][1] = fmaf(p[d + 1], f, o[c][1]);
+        }
+      }
+    }
+  }
+  if (bad) {
+    M = 0.f;
+    L = CUDART_NAN_F;
+  }
+  const int head = head0 + r;
+  if (n_splits == 1) {
+    const float inv = 1.0f / L;
+#pragma unroll
+    for (int c = 0; c < NP; ++c) {
+      const int d = 2 * lane + 64 * c;
+      if (d < hd) Pair<T>::store(out + (size_t)seq * ldo + head * hd + d, o[c][0] * inv, o[c][1] * inv);
+    }
+  } else {
+    const size_t pi = ((size_t)seq * nh + head) * n_splits + split;
+#pragma unroll
+    for (int c = 0; c < NP; ++c) {
+      const int d = 2 * lane + 64 * c;
+      if (d < hd) {
+        part_o[pi * hd + d] = o[c][0];
+        part_o[pi * hd + d + 1] = o[c][1];
+      }
+    }
+    if (lane == 0) {
+      part_ml[pi * 2] = M;
+      part_ml[pi * 2 + 1] = L;
+    }
+  }
+}
 
 // Partial results of one split: part_o [seq][head][split][hd], part_ml [seq][head][split][2].
 template <typename T, int NP>  // NP = ceil(hd / 64): pairs of value dims a lane owns
@@ -485,66 +547,13 @@ attn_decode_kernel(const T* __restrict__ q, int ldq, T* __restrict__ out, int ld
       }
     }
     __syncthreads();
-    // fold the warps in the order 0..3; warp r folds row r
-    if (warp < rows) {
-      const int r = warp;
-      float M = -CUDART_INF_F;
-      for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, Wp[(w * RW + r) * ws + hd]);
-      if (M != M) M = CUDART_NAN_F;
-      float L = 0.f, o[NP][2];
-#pragma unroll
-      for (int c = 0; c < NP; ++c) o[c][0] = o[c][1] = 0.f;
-      bool bad = false;
-      for (int w = 0; w < DEC_WARPS; ++w) bad = bad || (Wp[(w * RW + r) * ws + hd] != Wp[(w * RW + r) * ws + hd]);
-      if (M != -CUDART_INF_F && !bad) {
-        for (int w = 0; w < DEC_WARPS; ++w) {
-          const float* p = Wp + (w * RW + r) * ws;
-          if (p[hd] == -CUDART_INF_F) continue;
-          const float f = expf(p[hd] - M);
-          L = fmaf(p[hd + 1], f, L);
-#pragma unroll
-          for (int c = 0; c < NP; ++c) {
-            const int d = 2 * lane + 64 * c;
-            if (d < hd) {
-              o[c][0] = fmaf(p[d], f, o[c][0]);
-              o[c][1] = fmaf(p[d + 1], f, o[c][1]);
-            }
-          }
-        }
-      }
-      if (bad) {
-        M = 0.f;
-        L = CUDART_NAN_F;
-      }
-      const int head = kvh * g + h0 + r;
-      if (n_splits == 1) {
-        const float inv = 1.0f / L;
-#pragma unroll
-        for (int c = 0; c < NP; ++c) {
-          const int d = 2 * lane + 64 * c;
-          if (d < hd) Pair<T>::store(out + (size_t)seq * ldo + head * hd + d, o[c][0] * inv, o[c][1] * inv);
-        }
-      } else {
-        const size_t pi = ((size_t)seq * nh + head) * n_splits + split;
-#pragma unroll
-        for (int c = 0; c < NP; ++c) {
-          const int d = 2 * lane + 64 * c;
-          if (d < hd) {
-            part_o[pi * hd + d] = o[c][0];
-            part_o[pi * hd + d + 1] = o[c][1];
-          }
-        }
-        if (lane == 0) {
-          part_ml[pi * 2] = M;
-          part_ml[pi * 2 + 1] = L;
-        }
-      }
-    }
+    decode_fold_warps<T, NP>(Wp, RW, rows, hd, seq, kvh * g + h0, nh, split, n_splits, out, ldo, part_o, part_ml);
   }
 }
 
 }  // namespace edgelm
 #include "attention_decode_mma.cuh"
+#include "attention_decode_rows.cuh"
 namespace edgelm {
 
 // The fold of up to Q splits whose values a thread holds all at once (see the kernel below): `ml` are the lane's
@@ -770,7 +779,31 @@ int launch_decode(const void* q, int ldq, void* out, int ldo, const void* kc, co
       }
     }
   }
-  if (!on_mma) {
+  // Rows of 8, 16 or 32 pieces of 16 bytes: the whole-rows kernel, whatever the lengths, heads and splits (measured, us,
+  // attn_decode_kernel's shared-memory tiles | whole rows.  float32: 24 sequences of 500 keys, 15 heads on 5 of 64, 3 splits 17.4 | 9.9;
+  // 1 of 700, 16 splits 9.7 | 5.6; 64 of 1,000 58.9 | 36.8; 32 heads on 32, 64 of 1,000 197 | 165; 16 on 8 of 128, 24 of 500
+  // 64.9 | 19.2; 8 on 8 of 32, 64 of 1,000 48.5 | 31.6.  bfloat16 with a window: 15 on 5 of 64, 64 of 1,000, window 512
+  // 27.9 | 17.9; 8 on 1, 8 of 1,000, window 256 22.3 | 9.8; 16 on 8 of 128, 64 of 1,000 119 | 62).  bfloat16 without a
+  // window stays on the tensor cores: 64 sequences of 1,200 keys take 103 there and 125 here (32 on 32), 19 and 37 (15 on 5).
+  constexpr int ROW_MIN = 8 * KVec<T>::N;   // the smallest head size of the whole-rows kernel: a row of 8 lanes
+  const bool on_rows = !on_mma && !g_decode_cuda_cores && (hd == ROW_MIN || hd == 2 * ROW_MIN || (hd == 4 * ROW_MIN && hd <= 128)) &&
+                       (uintptr_t)kc % 16 == 0 && (uintptr_t)vc % 16 == 0;
+  if (on_rows) {
+    auto go = [&](auto kern) {
+      return launch_pdl(2, kern, grid, dim3(DEC_WARPS * 32), 0, stream, (const T*)q, ldq, (T*)out, ldo, (T*)const_cast<void*>(kc),
+                        (T*)const_cast<void*>(vc), page_table, table_stride, seq_slot, seq_pos, nh, nkv, scale, n_splits, part_o, part_ml,
+                        err, cos_t, sin_t, max_pos, window, meta_ready);
+    };
+    auto heads = [&](auto lanes) {
+      constexpr int L = decltype(lanes)::value;
+      const int g = nh / nkv;
+      return g == 1 ? go(attn_decode_rows_kernel<T, L, 1>) : g == 2 ? go(attn_decode_rows_kernel<T, L, 2>)
+           : g == 3 ? go(attn_decode_rows_kernel<T, L, 3>) : go(attn_decode_rows_kernel<T, L, RW>);
+    };
+    if (hd == ROW_MIN) le = heads(std::integral_constant<int, 8>{});
+    else if (hd == 2 * ROW_MIN) le = heads(std::integral_constant<int, 16>{});
+    else if constexpr (sizeof(T) == 4) le = heads(std::integral_constant<int, 32>{});
+  } else if (!on_mma) {
     const int tk = decode_tile_keys(hd, sizeof(T));
     const size_t smem = decode_head_bytes(hd) + (size_t)DEC_WARPS * 2 * tk * hd * sizeof(T);
     auto kern = attn_decode_kernel<T, NP>;

@@ -359,6 +359,47 @@ def test_attention_with_a_window(dtype, nh, nkv, hd, window):
             assert rel_err(out[s_:s_ + 1], want) < (1e-5 if dtype == torch.float32 else 1e-2), (n_splits, s_, n)
 
 
+@pytest.mark.parametrize("dtype,hd,window", [(torch.float32, 32, 0), (torch.float32, 64, 0), (torch.float32, 64, 33), (torch.float32, 128, 0),
+                                             (torch.bfloat16, 64, 70), (torch.bfloat16, 128, 15)])
+@pytest.mark.parametrize("g", [1, 2, 3, 4, 6])
+def test_attn_decode_of_whole_rows(dtype, hd, window, g):
+    """Lengths at the edges of a warp's chunk (8, 16 or 32 keys), of four warps' chunks and of a page, more splits than
+    pages, a second pass of heads (g > 4); the rows past a sequence's end hold NaN values.  The fused form's own
+    token sits at those edges too.  float32: sums of at most 200 products and weights in another order, 1e-5; bfloat16:
+    a rounded result, 1e-2."""
+    o = ops()
+    nkv, nh = 2, 2 * g
+    lengths = [1, 7, 8, 9, 15, 16, 17, 31, 32, 33, 63, 64, 65, 127, 129, 200]
+    B = len(lengths)
+    case = PagedCase(o, dtype, lengths, nkv, hd, seed=g + hd)
+    fused = PagedCase(o, dtype, lengths, nkv, hd, seed=g + hd)
+    cos_t, sin_t = (torch.from_numpy(t).to(dev()) for t in plain.rope_angles(np.arange(256), hd, 5000.0))
+    raw = rnd((B, (nh + 2 * nkv) * hd), dtype, 25)
+    seq_pos = torch.tensor([n - 1 for n in lengths], dtype=torch.int32, device=dev())
+    err = torch.zeros(1, dtype=torch.int32, device=dev())
+    qkv = raw.clone()
+    o.rope_kv_append(qkv, seq_pos, torch.arange(B, dtype=torch.int32, device=dev()), case.seq_slot, case.table, cos_t, sin_t, case.kcache,
+                     case.vcache, nh, nkv, hd, err)
+    for n_splits in (1, 2, 7):
+        outs = []
+        for entry, c, q, rope in ((o.attn_decode, case, qkv, ()), (o.attn_decode_rope, fused, raw.clone(), (cos_t, sin_t))):
+            out = torch.zeros(B, nh * hd, dtype=dtype, device=dev())
+            po = torch.full((B * nh * n_splits * hd,), float("nan"), device=dev())
+            pm = torch.full((B * nh * n_splits * 2,), float("nan"), device=dev())
+            entry(q, out, c.kcache, c.vcache, c.table, c.seq_slot, seq_pos, *rope, B, nh, nkv, hd, 1.0 / math.sqrt(hd), n_splits, po, pm,
+                  err=err, window=window)
+            outs.append(out)
+        assert int(err.item()) == 0
+        # (the two rotations may contract their products differently: a last place of a query or key)
+        assert rel_err(outs[1], outs[0]) < (1e-6 if dtype == torch.float32 else 4e-3), n_splits
+        for s_, n in enumerate(lengths):
+            page = int(case.table[int(case.seq_slot[s_]), (n - 1) // o.PAGE])
+            k, v = case.k[s_].clone(), case.v[s_].clone()
+            k[n - 1], v[n - 1] = (t[page, :, (n - 1) % o.PAGE].float().cpu() for t in (case.kcache, case.vcache))
+            want = attention_rows(qkv[s_:s_ + 1, :nh * hd].float().cpu(), k, v, n - 1, nh, nkv, hd, window)
+            assert rel_err(outs[0][s_:s_ + 1], want) < (1e-5 if dtype == torch.float32 else 1e-2), (n_splits, n)
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_a_windows_edge_stands_out(dtype):
     """One key is made to dominate every query.  Placed on the window's first key the output is its value; placed one
