@@ -226,6 +226,7 @@ pooled_window_attn_kernel(const T* __restrict__ q, T* __restrict__ out, const T*
   const int n_blocks = (P > 0 && pos - window >= 0) ? (pos - window + 1) / P : 0;
   const int blk_chunks = (n_blocks + 31) >> 5, n_chunks = blk_chunks + ((n_win + 31) >> 5);
   float m = -INFINITY, l = 0.f;
+  bool nan = false;                // some key of this warp's scored not a number
   float o[2 * DVR];                // dimensions 2 lane + 64 r and the one after it
 #pragma unroll
   for (int r = 0; r < 2 * DVR; ++r) o[r] = 0.f;
@@ -253,6 +254,7 @@ pooled_window_attn_kernel(const T* __restrict__ q, T* __restrict__ out, const T*
       }
     }
     const float m_new = fmaxf(m, warp_max(sc));
+    nan = nan || __any_sync(0xffffffffu, sc != sc);     // (a maximum drops it)
     if (m_new == -INFINITY) continue;
     const float w = sc == -INFINITY ? 0.f : expf(sc - m_new);
     const float corr = m == -INFINITY ? 0.f : expf(m - m_new);
@@ -297,7 +299,7 @@ pooled_window_attn_kernel(const T* __restrict__ q, T* __restrict__ out, const T*
     }
   }
   // merge the warps' partial results in a fixed order
-  if (lane == 0) { wm[warp] = m; wl[warp] = l; }
+  if (lane == 0) { wm[warp] = nan ? NAN : m; wl[warp] = l; }
 #pragma unroll
   for (int r = 0; r < DVR; ++r) {
     const int d = 2 * lane + 64 * r;
@@ -309,7 +311,7 @@ pooled_window_attn_kernel(const T* __restrict__ q, T* __restrict__ out, const T*
   for (int w2 = 0; w2 < NW; ++w2) M = fmaxf(M, wm[w2]);
   float L = 0.f;
   for (int w2 = 0; w2 < NW; ++w2) L += wm[w2] == -INFINITY ? 0.f : wl[w2] * expf(wm[w2] - M);
-  const float inv = L > 0.f ? 1.0f / L : 0.f;
+  const float inv = L == 0.f ? 0.f : 1.0f / L;      // (0: no key was seen; a denominator that is not a number goes on)
   for (int d = threadIdx.x; d < dv; d += blockDim.x) {
     float acc = 0.f;
     for (int w2 = 0; w2 < NW; ++w2)
@@ -340,13 +342,15 @@ __device__ __forceinline__ void pw_unpack(const uint4& u, float* v, const __nv_b
     v[2 * i + 1] = __uint_as_float(w[i] & 0xffff0000u);
   }
 }
-// A run of rows [begin, end) through one query: `row_of(r)` is the row's number in `keys` and `values` (-1: none).
+// A run of rows [begin, end) through one query: `row_of(r)` is the row's number in `keys` and `values` (-1: none).  A run with a score that
+// is not a number has such a maximum: the merge hands it on (of the scores' maximum alone it would vanish where the run has no other score).
 template <typename T, int D, typename RowOf>
 __device__ __forceinline__ void pw_run(const T* __restrict__ keys, const T* __restrict__ values, const float* qh, int begin, int end, int lane, RowOf row_of,
                                        float& m, float& l, float* slot) {
   using R = PwRow<T, D>;
   const int part = lane % R::LPR, grp = lane / R::LPR;
   float qv[R::EPL], o[R::EPL] = {};
+  bool nan = false;
 #pragma unroll
   for (int e = 0; e < R::EPL; ++e) qv[e] = qh[part * R::EPL + e];
   for (int r0 = begin; r0 < end; r0 += R::KEYS) {
@@ -369,6 +373,7 @@ __device__ __forceinline__ void pw_run(const T* __restrict__ keys, const T* __re
 #pragma unroll
       for (int x = 1; x < R::LPR; x <<= 1) d += __shfl_xor_sync(0xffffffffu, d, x);
       sc[i] = there[i] ? d : -INFINITY;
+      nan = nan || sc[i] != sc[i];
       m_new = fmaxf(m_new, sc[i]);
     }
     m_new = warp_max(m_new);
@@ -390,6 +395,7 @@ __device__ __forceinline__ void pw_run(const T* __restrict__ keys, const T* __re
     l = l * corr + sum;                        // (this lane's rows)
     m = m_new;
   }
+  if (__any_sync(0xffffffffu, nan)) m = NAN;
 #pragma unroll
   for (int x = R::LPR; x < 32; x <<= 1) {
     l += __shfl_xor_sync(0xffffffffu, l, x);
@@ -443,7 +449,7 @@ pooled_window_attn_rows_kernel(const T* __restrict__ q, T* __restrict__ out, con
       L = fmaf(wl[w], f, L);
       acc = fmaf(wo[w][threadIdx.x], f, acc);
     }
-    out[((size_t)t * H + h) * D + threadIdx.x] = from_f32<T>(L > 0.f ? acc * (1.0f / L) : 0.f);
+    out[((size_t)t * H + h) * D + threadIdx.x] = from_f32<T>(L == 0.f ? 0.f : acc * (1.0f / L));   // (0: no key was seen)
   }
 }
 

@@ -405,6 +405,51 @@ def test_window_attention_of_whole_rows(window, pool, d, H, G):
         test_window_attention_with_pooled_blocks(dtype, window, pool, d, d, H, G)
 
 
+@pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
+@pytest.mark.parametrize("window,pool,d", [(9, 4, 20), (40, 7, 96), (1, 4, 64), (40, 7, 32), (33, 1, 64), (70, 64, 128), (300, 5, 64)])
+def test_window_attention_of_single_tokens_that_see_no_number(window, pool, d, dtype):
+    """One sequence a fault: a not-a-number or an infinity in a key, a value or a pooled row that the token sees, in its query, or (the last ones) where
+    it does not see it.  What the token's heads are then is what 64 bits give (not-a-numbers at the same places, infinities with their sign),
+    also where the faulty score is the only one of a warp's run (window 1: of the whole window).  Scores stay under 30, so no weight is zero."""
+    g = np.random.default_rng(window + d)
+    PAGE, n, H, G = 64, 150, 4, 2
+    R, pages = -(-PAGE // pool), -(-n // PAGE)
+    seen_blocks = max(0, (n - window) // pool)
+    bad = [("k", n - 1, np.nan), ("k", max(0, n - window), np.nan), ("k", n - 1, np.inf), ("k", n - 1, -np.inf), ("v", n - 1, np.nan), ("v", n - 1, -np.inf),
+           ("q", 0, np.nan), ("none", 0, 0.0)]
+    if seen_blocks:
+        bad += [("pk", 0, np.nan), ("pk", seen_blocks - 1, -np.inf), ("pv", seen_blocks // 2, np.inf), ("pv", 0, np.nan), ("k", n - window - 1, np.nan)]
+    B, scale = len(bad), d ** -0.5
+    q, kc, vc = g.normal(size=(B, H, d)), np.full((B * pages, G, PAGE, d), np.nan), np.full((B * pages, G, PAGE, d), np.nan)
+    pk, pv = np.full((B * pages, G, R, d), np.nan), np.full((B * pages, G, R, d), np.nan)
+    rnd = lambda a: torch.tensor(a).to(dtype).double().numpy()
+    want = np.zeros((B, H, d))
+    for s, (what, at, value) in enumerate(bad):
+        k, v, bk, bv = (g.normal(size=(m, G, d)) for m in (n, n, n // pool, n // pool))
+        {"k": k, "v": v, "pk": bk, "pv": bv, "q": q[s][None], "none": k}[what][at, :, 3] += value
+        for i in range(n):
+            kc[s * pages + i // PAGE, :, i % PAGE], vc[s * pages + i // PAGE, :, i % PAGE] = k[i], v[i]
+        for e in range(n // pool):
+            end = (e * pool + pool - 1) // PAGE
+            pk[s * pages + end, :, e - PAGE * end // pool], pv[s * pages + end, :, e - PAGE * end // pool] = bk[e], bv[e]
+        lo = max(0, n - window)
+        keys = np.concatenate([rnd(k[lo:]), np.float32(bk[:seen_blocks]).astype(np.float64)])
+        vals = np.concatenate([rnd(v[lo:]), np.float32(bv[:seen_blocks]).astype(np.float64)])
+        for h in range(H):
+            sc = torch.tensor(keys[:, h // 2]) @ torch.tensor(rnd(q[s, h])) * scale
+            want[s, h] = (torch.softmax(sc, 0)[:, None] * torch.tensor(vals[:, h // 2])).sum(0).numpy()
+    out = torch.full((B, H * d), 7.0, dtype=dtype, device=DEV)
+    cast = lambda a: f32(a).to(dtype)
+    ops.pooled_window_attn(cast(q.reshape(B, -1)), out, cast(kc), cast(vc), f32(pk), f32(pv), i32([n - 1] * B), i32(list(range(B))),
+                           i32([[s * pages + i for i in range(pages)] for s in range(B)]), H, G, d, d, scale, window, pool)
+    got = out.float().cpu().numpy().reshape(B, H, d)
+    assert np.isnan(want[:2]).all() and np.isnan(want[6]).all() and np.isfinite(want[7]).all() and (not seen_blocks or np.isfinite(want[-1]).all())
+    for s, fault in enumerate(bad):
+        assert np.array_equal(np.isnan(got[s]), np.isnan(want[s])) and np.array_equal(np.isinf(got[s]), np.isinf(want[s])), fault
+        assert np.array_equal(got[s][np.isinf(got[s])], want[s][np.isinf(got[s])]), fault
+        there = np.isfinite(want[s])
+        assert np.abs(got[s][there] - want[s][there]).max(initial=0.0) < (2e-5 if dtype == torch.float32 else 2e-2) * 4, fault
+
 
 @pytest.mark.parametrize("window,pool,d,H,G", [(100, 64, 64, 4, 2), (7, 3, 32, 3, 1), (64, 1, 96, 2, 2), (200, 5, 128, 2, 1), (50, None, 64, 2, 1)])
 def test_pooled_attention_on_the_tensor_cores(window, pool, d, H, G):
