@@ -257,8 +257,11 @@ __device__ __forceinline__ void decode_fold_warps(const float* Wp, int pitch, in
   float L = 0.f, o[NP][2];
 #pragma unroll
   for (int c = 0; c < NP; ++c) o[c][0] = o[c][1] = 0.f;
-  bool bad = false;
-  for (int w = 0; w < DEC_WARPS; ++w) bad = bad || (Wp[(w * pitch + r) * ws + hd] != Wp[(w * pitch + r) * ws + hd]);
+  bool bad = false;      // (a warp whose scores are all not a number has no maximum, but such a sum)
+  for (int w = 0; w < DEC_WARPS; ++w) {
+    const float* p = Wp + (w * pitch + r) * ws + hd;
+    bad = bad || p[0] != p[0] || p[1] != p[1];
+  }
   if (M != -CUDART_INF_F && !bad) {
     for (int w = 0; w < DEC_WARPS; ++w) {
       const float* p = Wp + (w * pitch + r) * ws;
@@ -487,9 +490,10 @@ attn_decode_kernel(const T* __restrict__ q, int ldq, T* __restrict__ out, int ld
         if (r < rows) {
           const float a = lane < valid && key0 + lane >= first_key ? s[0][r] * scale : -CUDART_INF_F;
           const float b = lane + 32 < valid && key0 + lane + 32 >= first_key ? s[1][r] * scale : -CUDART_INF_F;
-          const float mx = fmaxf(m[r], warp_max(fmaxf(a, b)));  // finite: the tile holds a key that the token sees
-          const float corr = expf(m[r] - mx);
-          const float p0 = expf(a - mx), p1 = expf(b - mx);
+          const float mx = fmaxf(m[r], warp_max(fmaxf(a, b)));
+          const float ref = mx == -CUDART_INF_F ? 0.f : mx;     // (no score above minus infinity yet: weights of zero, not of no number)
+          const float corr = expf(m[r] - ref);
+          const float p0 = expf(a - ref), p1 = expf(b - ref);
           l[r] = l[r] * corr + warp_sum(p0 + p1);
           m[r] = mx;
           pw[r * 64 + lane] = p0;

@@ -177,9 +177,10 @@ attn_decode_rows_kernel(const T* __restrict__ q, int ldq, T* __restrict__ out, i
         float mx = a;
 #pragma unroll
         for (int mask = 16; mask >= SAME; mask /= 2) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, mask));
-        mx = fmaxf(m[r], mx);              // finite: the chunk holds a key that the token sees
-        const float corr = expf(m[r] - mx);
-        p[r] = expf(a - mx);
+        mx = fmaxf(m[r], mx);
+        const float ref = mx == -CUDART_INF_F ? 0.f : mx;     // (no score above minus infinity yet: weights of zero, not of no number)
+        const float corr = expf(m[r] - ref);
+        p[r] = expf(a - ref);
         l[r] = l[r] * corr + p[r];         // (the lane's own keys; summed over the lanes at the end)
         m[r] = mx;
 #pragma unroll

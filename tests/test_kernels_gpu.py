@@ -400,6 +400,44 @@ def test_attn_decode_of_whole_rows(dtype, hd, window, g):
             assert rel_err(outs[0][s_:s_ + 1], want) < (1e-5 if dtype == torch.float32 else 1e-2), (n_splits, n)
 
 
+@pytest.mark.parametrize("dtype,hd,window", [(torch.float32, 48, 0), (torch.float32, 32, 0), (torch.float32, 64, 33), (torch.float32, 128, 0),
+                                             (torch.bfloat16, 64, 70), (torch.bfloat16, 128, 15)])
+@pytest.mark.parametrize("n_splits", [1, 3])
+def test_attn_decode_of_keys_that_score_no_number(dtype, hd, window, n_splits):
+    """Keys and values that a token sees and that are no finite number, one kind a sequence: one key, all keys of a warp's chunk (8 to 32 keys, so 32 in a
+    row from a page's start on), the last keys only.  What comes out is what 64 bits give: not-a-numbers at the same places, infinities
+    with their sign, a score of minus infinity a weight of zero.  Scores stay under 40 in float32, so no weight underflows."""
+    o = ops()
+    nkv, nh = 2, 4
+    nan, inf = float("nan"), float("inf")
+    kinds = [("k", 130, 131, nan), ("k", 128, 160, nan), ("k", 128, 160, -inf), ("k", 140, 141, inf), ("k", 165, 170, -inf), ("k", 169, 170, nan),
+             ("v", 150, 151, nan), ("v", 165, 166, -inf), ("k", 0, 0, 0.0)]
+    lengths = [170] * len(kinds)
+    case = PagedCase(o, dtype, lengths, nkv, hd, seed=hd)
+    B = len(kinds)
+    for s_, (what, a, b, value) in enumerate(kinds):
+        for j in range(a, b):
+            page = int(case.table[int(case.seq_slot[s_]), j // o.PAGE])
+            (case.kcache if what == "k" else case.vcache)[page, :, j % o.PAGE, 5] = value
+            (case.k if what == "k" else case.v)[s_][j, :, 5] = value
+    qkv = rnd((B, (nh + 2 * nkv) * hd), dtype, 31)
+    qkv[:, 5:nh * hd:hd] = qkv[:, 5:nh * hd:hd].abs() + 0.1      # (an infinite key dimension scores the same way for every head)
+    out = torch.zeros(B, nh * hd, dtype=dtype, device=dev())
+    part_o = torch.full((B * nh * n_splits * hd,), float("nan"), device=dev())
+    part_ml = torch.full((B * nh * n_splits * 2,), float("nan"), device=dev())
+    seq_pos = torch.tensor([n - 1 for n in lengths], dtype=torch.int32, device=dev())
+    o.attn_decode(qkv, out, case.kcache, case.vcache, case.table, case.seq_slot, seq_pos, B, nh, nkv, hd, 1.0 / math.sqrt(hd), n_splits, part_o,
+                  part_ml, window=window)
+    for s_, kind in enumerate(kinds):
+        want = attention_rows(qkv[s_:s_ + 1, :nh * hd].float().cpu(), case.k[s_], case.v[s_], lengths[s_] - 1, nh, nkv, hd, window)
+        got = out[s_:s_ + 1].double().cpu()
+        assert torch.equal(got.isnan(), want.isnan()), kind
+        finite = want.isfinite()
+        assert torch.equal(got[~finite & ~want.isnan()], want[~finite & ~want.isnan()]), kind
+        if finite.any():
+            assert rel_err(got[finite], want[finite]) < (1e-5 if dtype == torch.float32 else 1e-2), kind
+
+
 @pytest.mark.parametrize("dtype", DTYPES)
 def test_a_windows_edge_stands_out(dtype):
     """One key is made to dominate every query.  Placed on the window's first key the output is its value; placed one
