@@ -336,31 +336,36 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     const size_t tok = (size_t)(tok0 + row);
     if (a.gate != nullptr && !a.gate_ch && mine) inv *= 1.0f / (1.0f + expf(-a.gate[tok * a.ldg + head]));
     if (ok) {
+      // (tcgen05.ld wants the whole warp: all columns first, then the rows that there are)
+      __syncwarp();
+      uint32_t o[DV / 4];
 #pragma unroll
-      for (int c = 0; c < DV / 4; c += 8) {
-        uint32_t o[8];
-        const int d = part * (DV / 4) + c;
-        st_tmem_ld8(tmem + lanes + ST_O_COL + d, o);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (!mine) continue;
-        float v[8];
+      for (int c = 0; c < DV / 4; c += 8) st_tmem_ld8(tmem + lanes + ST_O_COL + part * (DV / 4) + c, o + c);
+      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+      if (mine) {
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(o[i]) * inv;
-        if (a.gate != nullptr && a.gate_ch) {
-          const float* g = a.gate + tok * a.ldg + head * DV + d;
+        for (int c = 0; c < DV / 4; c += 8) {
+          const int d = part * (DV / 4) + c;
+          float v[8];
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] *= 1.0f / (1.0f + expf(-g[i]));
-        }
-        if (a.maps > 1) {
-          float4* dst = reinterpret_cast<float4*>(static_cast<float*>(a.out) + tok * a.ldo + head * DV + d);
-          dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-          dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-        } else {
-          __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.out) + tok * a.ldo + head * DV + d;
-          store_piece(dst, make_float4(v[0], v[1], v[2], v[3]));
-          store_piece(dst + 4, make_float4(v[4], v[5], v[6], v[7]));
+          for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(o[c + i]) * inv;
+          if (a.gate != nullptr && a.gate_ch) {
+            const float* g = a.gate + tok * a.ldg + head * DV + d;
+#pragma unroll
+            for (int i = 0; i < 8; ++i) v[i] *= 1.0f / (1.0f + expf(-g[i]));
+          }
+          if (a.maps > 1) {
+            float4* dst = reinterpret_cast<float4*>(static_cast<float*>(a.out) + tok * a.ldo + head * DV + d);
+            dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+            dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+          } else {
+            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.out) + tok * a.ldo + head * DV + d;
+            store_piece(dst, make_float4(v[0], v[1], v[2], v[3]));
+            store_piece(dst + 4, make_float4(v[4], v[5], v[6], v[7]));
+          }
         }
       }
+      __syncwarp();
     }
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
