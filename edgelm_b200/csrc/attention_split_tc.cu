@@ -13,7 +13,8 @@
 // columns and O (up to 128).
 // So S of block j + 1 is computed beside the softmax of block j, and O of block j beside the softmax of block j + 1.
 //
-// Masks, sinks, gates, kept keys and maps as in attention_mma_split.cu.  Every wait is bounded as in the matrix products.
+// Masks, sinks, gates, kept keys and maps as in attention_mma_split.cu.  Every wait is bounded; where one runs out the block reports it, writes
+// not-a-numbers and waits for its own copies and MMAs before it gives its memory back.
 // mma.sync takes a scheduler 16 clocks for an m16n8k16 here, four times what tcgen05 takes for as many multiply-adds, and bounds the other kernel.
 // What bounds this one is the softmax: 2,600 clocks a block, 1,750 of them the exponentials, the splitting and the stores into tensor memory
 // (with a third of either product's MMAs it takes 3 % less, without exponentials and splitting 17 %); 3 us a tile before the first block.
@@ -67,6 +68,12 @@ __device__ __forceinline__ void st_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uin
       : "memory");
 }
 
+// A block's last wait for what it has in flight, bounded and without a report (the wait that ran out before has made one)
+__device__ __forceinline__ void st_drain(uint32_t bar, uint32_t parity) {
+  const long long t0 = clock64();
+  while (!mbar_try(bar, parity) && clock64() - t0 < TC_WAIT_CYCLES) {}
+}
+
 struct SplitTcArgs {
   const float* q;
   int ldq;
@@ -99,7 +106,8 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
   uint64_t* bars = reinterpret_cast<uint64_t*>(row_sum + 4 * ST_ROWS);
   uint64_t *q_ready = bars, *k_full = bars + 1, *k_empty = k_full + KS, *v_full = k_empty + KS, *v_empty = v_full + VS;
   uint64_t *s_ready = v_empty + VS, *p_ready = s_ready + 2, *o_done = p_ready + 2;
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_done + 2);
+  uint64_t* all_done = o_done + 2;                 // both issuers' MMAs
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(all_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -113,6 +121,7 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
 
   if (threadIdx.x == 0) {
     for (uint64_t* b = bars; b < o_done + 2; ++b) mbar_init(smem_u32(b), b == q_ready || (b >= p_ready && b < o_done) ? ST_SOFT_WARPS : 1);
+    mbar_init(smem_u32(all_done), 2);
     *abort_flag = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
@@ -134,9 +143,11 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     uint8_t* dst = keys ? k_s : v_s;
     const int32_t* pages = a.page_table ? a.page_table + (size_t)seq * a.table_stride : nullptr;
     const bool leader = elect_one();
+    int issued = 0;
     for (int j = 0; j < n_blk; ++j) {
       const int st = j % stages;
       if (j >= stages && !wait(&empty[st], (j / stages & 1) ^ 1)) break;
+      issued = j + 1;
       if (leader) {
         const uint32_t bar = smem_u32(&full[st]);
         mbar_expect_tx(bar, chunks * ST_TILE);
@@ -160,6 +171,8 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
       }
       __syncwarp();
     }
+    // (also where a wait ran out: no copy may be on its way when the block's memory is given back)
+    for (int i = max(0, issued - stages); i < issued; ++i) st_drain(smem_u32(&full[i % stages]), i / stages & 1);
   } else if (warp == 2) {
     constexpr uint32_t idesc = umma_idesc(ST_ROWS, 128);
     const bool leader = elect_one();
@@ -183,6 +196,9 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
       }
       __syncwarp();
     }
+    if (leader) umma_commit(smem_u32(all_done));
+    __syncwarp();
+    st_drain(smem_u32(all_done), 0);
   } else if (warp == 3) {
     constexpr uint32_t idesc = umma_idesc(ST_ROWS, 64) | (1u << 16);  // B (the values) is MN-major
     const bool leader = elect_one();
@@ -208,6 +224,9 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
       }
       __syncwarp();
     }
+    if (leader) umma_commit(smem_u32(all_done));
+    __syncwarp();
+    st_drain(smem_u32(all_done), 0);
   } else {
     const int sw = warp - 4, part = sw >> 2, half = part >> 1, quarter = warp & 3, row = quarter * 32 + lane, tid = threadIdx.x - 128;
     const uint32_t lanes = (uint32_t)(quarter * 32) << 16;
@@ -335,38 +354,41 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     const bool mine = row < ntok;
     const size_t tok = (size_t)(tok0 + row);
     if (a.gate != nullptr && !a.gate_ch && mine) inv *= 1.0f / (1.0f + expf(-a.gate[tok * a.ldg + head]));
+    // (tcgen05.ld wants the whole warp: all columns first, then the rows that there are)
+    __syncwarp();
+    uint32_t o[DV / 4];
     if (ok) {
-      // (tcgen05.ld wants the whole warp: all columns first, then the rows that there are)
-      __syncwarp();
-      uint32_t o[DV / 4];
 #pragma unroll
       for (int c = 0; c < DV / 4; c += 8) st_tmem_ld8(tmem + lanes + ST_O_COL + part * (DV / 4) + c, o + c);
       asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-      if (mine) {
+    } else {                                       // a wait that ran out: nothing that could pass for a result
 #pragma unroll
-        for (int c = 0; c < DV / 4; c += 8) {
-          const int d = part * (DV / 4) + c;
-          float v[8];
+      for (int i = 0; i < DV / 4; ++i) o[i] = 0x7fc00000u;
+    }
+    if (mine) {
 #pragma unroll
-          for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(o[c + i]) * inv;
-          if (a.gate != nullptr && a.gate_ch) {
-            const float* g = a.gate + tok * a.ldg + head * DV + d;
+      for (int c = 0; c < DV / 4; c += 8) {
+        const int d = part * (DV / 4) + c;
+        float v[8];
 #pragma unroll
-            for (int i = 0; i < 8; ++i) v[i] *= 1.0f / (1.0f + expf(-g[i]));
-          }
-          if (a.maps > 1) {
-            float4* dst = reinterpret_cast<float4*>(static_cast<float*>(a.out) + tok * a.ldo + head * DV + d);
-            dst[0] = make_float4(v[0], v[1], v[2], v[3]);
-            dst[1] = make_float4(v[4], v[5], v[6], v[7]);
-          } else {
-            __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.out) + tok * a.ldo + head * DV + d;
-            store_piece(dst, make_float4(v[0], v[1], v[2], v[3]));
-            store_piece(dst + 4, make_float4(v[4], v[5], v[6], v[7]));
-          }
+        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(o[c + i]) * inv;
+        if (a.gate != nullptr && a.gate_ch) {
+          const float* g = a.gate + tok * a.ldg + head * DV + d;
+#pragma unroll
+          for (int i = 0; i < 8; ++i) v[i] *= 1.0f / (1.0f + expf(-g[i]));
+        }
+        if (a.maps > 1) {
+          float4* dst = reinterpret_cast<float4*>(static_cast<float*>(a.out) + tok * a.ldo + head * DV + d);
+          dst[0] = make_float4(v[0], v[1], v[2], v[3]);
+          dst[1] = make_float4(v[4], v[5], v[6], v[7]);
+        } else {
+          __nv_bfloat16* dst = static_cast<__nv_bfloat16*>(a.out) + tok * a.ldo + head * DV + d;
+          store_piece(dst, make_float4(v[0], v[1], v[2], v[3]));
+          store_piece(dst + 4, make_float4(v[4], v[5], v[6], v[7]));
         }
       }
-      __syncwarp();
     }
+    __syncwarp();
   }
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
