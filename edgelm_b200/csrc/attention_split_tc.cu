@@ -7,20 +7,25 @@
 // rows see in blocks of two cache pages (or of the step's own rows).  Roles: warp 0 loads the keys by TMA, warp 1 the values, warp 2 issues
 // S (A: the queries' terms, swizzled K-major tiles written once; B: the keys as they lie), warp 3 issues O (A: the weights' terms out
 // of tensor memory; B: the values as they lie, MN-major), warps 4 to 19 are the softmax: four threads a row, half a page
-// of the block each.  They exchange a row's maximum through shared memory, so that they share one reference and one accumulator; the
-// reference moves only when the maximum has outgrown it by 2^8 (then they scale the row of O in place).  A thread's weights go back over the
-// scores that they came from: its 32 columns hold terms 1 and 2, 16 further ones the third.  Tensor memory: two such buffers of 192
-// columns and O (up to 128).
+// of the block each.  They exchange a row's maximum through shared memory, so that they share one reference; it moves only when the
+// maximum has outgrown it by 2^8.  A thread's weights go back over the scores that they came from: its 32 columns hold terms 1 and 2,
+// 16 further ones the third.  Tensor memory: two such buffers of 192 columns and O: 128 columns, or twice 64.
 // So S of block j + 1 is computed beside the softmax of block j, and O of block j beside the softmax of block j + 1.
+//
+// The tensor cores cut a sum off below its last place at every MMA, and with one accumulator over all keys these add up: O's runs are two
+// blocks long, and the softmax threads add a run to the row's output in registers, rounded to nearest (a quarter of the dimensions each; where
+// the reference moves they scale that, and a run that has begun in place).  Heads of 64 value dimensions have two accumulators, so that a run
+// waits a block long before it is added.  Distance from float64 in the float32 output of two maps of 64 over 128, of 256, 700, 2,000 and 5,000
+// tokens (2-norm; scores of standard deviation 1): 2.3e-7, 3.4e-7, 4.1e-7, 4.6e-7; one run over all keys 2.3e-7, 6.6e-7, 1.9e-6, 4.2e-6 and
+// 1 to 7 % less time; mma.sync 4.1e-7, 4.8e-7, 1.0e-6, 2.2e-6.
 //
 // Masks, sinks, gates, kept keys and maps as in attention_mma_split.cu.  Every wait is bounded; where one runs out the block reports it, writes
 // not-a-numbers and waits for its own copies and MMAs before it gives its memory back.
 // mma.sync takes a scheduler 16 clocks for an m16n8k16 here, four times what tcgen05 takes for as many multiply-adds, and bounds the other kernel.
 // What bounds this one is the softmax: 2,600 clocks a block, 1,750 of them the exponentials, the splitting and the stores into tensor memory
 // (with a third of either product's MMAs it takes 3 % less, without exponentials and splitting 17 %); 3 us a tile before the first block.
-// mma.sync and here, us: 9 heads of 64 over 3, 6,000 tokens 448 and 135; chunks of 512, 333 to 1,700 tokens 39.6 and 24.8; 9 heads of
-// 96 / 64 over the step's own rows, 333 to 1,700 tokens 101 and 35.5; 16 heads of two maps of 64 over values of 128, chunks of 1,024, 1,000 and
-// 2,900 tokens 243 and 121.  Distance from float64 in the float32 output of two maps: 0.5 to 1.05 of the other's.
+// mma.sync and here, us: 9 heads of 64 over 3, 1,000, 2,000 and 4,000 tokens 26 and 21, 78 and 34, 225 and 67; 512 behind 4,000 103 and 65; 16
+// heads of two maps of 64 over values of 128, chunks of 1,024, 1,000 and 4,000 tokens 88 and 33, 248 and 131; 32 heads of 128, 2,000 tokens 373 and 111.
 // Tiles of the most keys go first over all heads (a head's tiles next to each other left the last head's longest tile to the end).
 #include <math_constants.h>
 
@@ -47,11 +52,12 @@ __device__ __forceinline__ int st_first_key(int pos, int mask, int size) {
   if (mask == ST_MASK_CHUNK) return (pos / size) * size;
   return 0;
 }
+// O of the run (of two blocks) that block j belongs to: with room for two, the runs take turns
+template <int DV> __device__ __forceinline__ uint32_t st_run_col(int j) { return ST_O_COL + (DV == 64 ? (j >> 1 & 1) * 64 : 0); }
+__device__ __forceinline__ uint32_t st_low_bits(int n) { return n >= 32 ? ~0u : ~(~0u << max(n, 0)); }
 __device__ __forceinline__ void st_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
-__device__ __forceinline__ void st_tmem_st8(uint32_t taddr, const uint32_t* r) {
-  asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]),
-               "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7])
-               : "memory");
+__device__ __forceinline__ void st_tmem_st4(uint32_t taddr, const uint32_t* r) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
 __device__ __forceinline__ void st_tmem_ld8(uint32_t taddr, uint32_t* r) {
   asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
@@ -217,7 +223,7 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
 #pragma unroll
             for (int s = 0; s < 8; ++s) {                             // 16 keys: of the threads of quarter s / 2
               const uint32_t p = tmem + b * ST_BUF_COLS + (t == 2 ? 128 + s * 8 : s / 2 * 32 + t * 16 + s % 2 * 8);
-              st_umma_ts(tmem + ST_O_COL + c * 64, p, dv + (c * ST_TILE + s * 16 * 128 >> 4), idesc, j != 0 || t != 2 || s != 0);
+              st_umma_ts(tmem + st_run_col<DV>(j) + c * 64, p, dv + (c * ST_TILE + s * 16 * 128 >> 4), idesc, j & 1 || t != 2 || s != 0);
             }
         umma_commit(smem_u32(&o_done[b]));
         umma_commit(smem_u32(&v_empty[st]));
@@ -249,7 +255,22 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     const int pos = row < ntok ? pos0 + row : -1, first = st_first_key(max(pos, 0), a.mask, a.mask_size);
     const int last_first = st_first_key(n_keys - 1, a.mask, a.mask_size);      // the first key of the tile's last row
     float m = -CUDART_INF_F, l = 0.f;             // the row's reference (in units of log 2), this thread's keys' weights
-    bool ok = true;
+    float acc[DV / 4] = {};                       // the row's output, this thread's dimensions
+    auto gather = [&](int j) {                    // += the run that the MMAs of block j ended in tensor memory
+      if (!wait(&o_done[j & 1], j >> 1 & 1)) return false;
+      asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+      for (int c = 0; c < DV / 4; c += 16) {
+        uint32_t o[16];
+        st_tmem_ld8(tmem + lanes + st_run_col<DV>(j) + part * (DV / 4) + c, o);
+        st_tmem_ld8(tmem + lanes + st_run_col<DV>(j) + part * (DV / 4) + c + 8, o + 8);
+        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+        for (int i = 0; i < 16; ++i) acc[c + i] += __uint_as_float(o[i]);
+      }
+      return true;
+    };
+    bool ok = true, waiting = false;              // (a run is whole and not in `acc` yet)
     for (int j = 0; j < n_blk; ++j) {             // (also behind a wait that ran out: the row's other thread may be at the exchange)
       const int b = j & 1;
       const bool there = 2 * j + half < n_visit;
@@ -263,9 +284,11 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
         tmem_ld32(s_addr, r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
         if (!there || key0 + 31 > pos0 || (key0 < last_first && key0 + 32 > a.keep)) {
+          // (a bit a key: five instructions a score, with its place compared to each bound, made a masked block twice as long)
+          const uint32_t seen = (there ? st_low_bits(pos - key0 + 1) : 0u) & (~st_low_bits(first - key0) | st_low_bits(a.keep - key0));
 #pragma unroll
           for (int i = 0; i < 32; ++i)
-            if (!there || key0 + i > pos || (key0 + i < first && key0 + i >= a.keep)) r[i] = __float_as_uint(-CUDART_INF_F);
+            if (!(seen >> i & 1)) r[i] = __float_as_uint(-CUDART_INF_F);
         }
         float mx1 = -CUDART_INF_F;
 #pragma unroll
@@ -287,38 +310,48 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
       } else if (mx > m + ST_LAZY) {
         rescale = sp_exp2(m - mx);                 // (0 if the row has seen no key so far)
         m = mx;
-      }
-      if (__any_sync(0xffffffffu, rescale != 1.f)) {       // (rare after the first blocks; all warps of the rows take it)
-        ok = wait(&o_done[b ^ 1], (j - 1) >> 1 & 1);
-        if (!ok) continue;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
-#pragma unroll
-        for (int c = 0; c < DV / 4; c += 8) {
-          uint32_t o[8];
-          const uint32_t at = tmem + lanes + ST_O_COL + part * (DV / 4) + c;
-          st_tmem_ld8(at, o);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * rescale);
-          st_tmem_st8(at, o);
-        }
         l *= rescale;
+      }
+      if (j > 0 && !(j & 1)) waiting = true;       // the run before this block's is whole, or soon
+      if (__any_sync(0xffffffffu, rescale != 1.f)) {       // (rare after the first blocks; all warps of the rows take it)
+        if (waiting) ok = gather(j - 1 - (j & 1));
+        waiting = false;
+        if (ok && (j & 1)) {                       // the run's first block is in tensor memory
+          ok = wait(&o_done[0], j >> 1 & 1);
+          if (ok) {
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+#pragma unroll
+            for (int c = 0; c < DV / 4; c += 8) {
+              uint32_t o[8];
+              const uint32_t at = tmem + lanes + st_run_col<DV>(j) + part * (DV / 4) + c;
+              st_tmem_ld8(at, o);
+              asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+              for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * rescale);
+              st_tmem_st4(at, o);
+              st_tmem_st4(at + 4, o + 4);
+            }
+          }
+        }
+        if (!ok) continue;
+#pragma unroll
+        for (int i = 0; i < DV / 4; ++i) acc[i] *= rescale;
       }
       const float ref = m == -CUDART_INF_F ? 0.f : m;
       float sum0 = 0.f, sum1 = 0.f;
 #pragma unroll
-      for (int c = 0; c < 2; ++c) {                // 16 keys: 8 columns of each term
-        uint32_t t[3][8];
+      for (int c = 0; c < 4; ++c) {                // 8 keys: 4 columns of each term
+        uint32_t t[3][4];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          const float p0 = sp_exp2(fmaf(__uint_as_float(r[c * 16 + 2 * i]), scale2, -ref)), p1 = sp_exp2(fmaf(__uint_as_float(r[c * 16 + 2 * i + 1]), scale2, -ref));
+        for (int i = 0; i < 4; ++i) {
+          const float p0 = sp_exp2(fmaf(__uint_as_float(r[c * 8 + 2 * i]), scale2, -ref)), p1 = sp_exp2(fmaf(__uint_as_float(r[c * 8 + 2 * i + 1]), scale2, -ref));
           sum0 += p0;
           sum1 += p1;
           sp_split(p0, p1, t[0][i], t[1][i], t[2][i]);
         }
-        st_tmem_st8(s_addr + c * 8, t[0]);
-        st_tmem_st8(s_addr + 16 + c * 8, t[1]);
-        st_tmem_st8(tmem + lanes + b * ST_BUF_COLS + 128 + part * 16 + c * 8, t[2]);
+        st_tmem_st4(s_addr + c * 4, t[0]);
+        st_tmem_st4(s_addr + 16 + c * 4, t[1]);
+        st_tmem_st4(tmem + lanes + b * ST_BUF_COLS + 128 + part * 16 + c * 4, t[2]);
       }
       l += sum0 + sum1;
       if (j == n_blk - 1) {
@@ -334,13 +367,18 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
           asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         }
       }
+      if (waiting && (DV != 64 || (j & 1))) {      // before the next block's MMAs may take its columns
+        waiting = false;
+        ok = gather(j - 1 - (j & 1));
+        if (!ok) continue;
+      }
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
       if (lane == 0) st_arrive(smem_u32(&p_ready[b]));
     }
-    if (ok) ok = wait(&o_done[(n_blk - 1) & 1], (n_blk - 1) >> 1 & 1);
-    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (ok && waiting) ok = gather(n_blk - 2);     // (the last block has a run of its own)
+    if (ok) ok = gather(n_blk - 1);
     row_sum[part * ST_ROWS + row] = l;
     asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");
     float den = (row_sum[row] + row_sum[ST_ROWS + row]) + (row_sum[2 * ST_ROWS + row] + row_sum[3 * ST_ROWS + row]), fix = 1.f;
@@ -354,24 +392,14 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     const bool mine = row < ntok;
     const size_t tok = (size_t)(tok0 + row);
     if (a.gate != nullptr && !a.gate_ch && mine) inv *= 1.0f / (1.0f + expf(-a.gate[tok * a.ldg + head]));
-    // (tcgen05.ld wants the whole warp: all columns first, then the rows that there are)
-    __syncwarp();
-    uint32_t o[DV / 4];
-    if (ok) {
-#pragma unroll
-      for (int c = 0; c < DV / 4; c += 8) st_tmem_ld8(tmem + lanes + ST_O_COL + part * (DV / 4) + c, o + c);
-      asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-    } else {                                       // a wait that ran out: nothing that could pass for a result
-#pragma unroll
-      for (int i = 0; i < DV / 4; ++i) o[i] = 0x7fc00000u;
-    }
+    if (!ok) inv = __uint_as_float(0x7fc00000u);   // a wait that ran out: nothing that could pass for a result
     if (mine) {
 #pragma unroll
       for (int c = 0; c < DV / 4; c += 8) {
         const int d = part * (DV / 4) + c;
         float v[8];
 #pragma unroll
-        for (int i = 0; i < 8; ++i) v[i] = __uint_as_float(o[c + i]) * inv;
+        for (int i = 0; i < 8; ++i) v[i] = acc[c + i] * inv;
         if (a.gate != nullptr && a.gate_ch) {
           const float* g = a.gate + tok * a.ldg + head * DV + d;
 #pragma unroll

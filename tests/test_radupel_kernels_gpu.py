@@ -4,6 +4,8 @@ heads with a sigmoid gate; two norms of the same rows in one pass (with rows add
 biases; softmax attention with a gate per head, for prompt steps and steps of one token, reading queries, keys and values
 out of rows that hold more; the scoring router with corrections, groups and negative scores; identity experts, the shared
 expert and the clamped experts through the grouping, the products and the weighted sum."""
+import math
+
 import numpy as np
 import pytest
 import torch
@@ -497,6 +499,43 @@ def test_tcgen05_attention_over_all_its_forms(new, first, H, G, dk, dv, maps, ma
     assert int(err.item()) == 0
     off, size_of = (outs[0] - outs[1]).abs(), outs[0].abs()
     assert bool((off <= (2.0 ** -7 * size_of + 1e-5 if maps == 1 else 3e-6 * float(size_of.max()))).all())
+
+
+@pytest.mark.parametrize("dk,dv,maps", [(64, 128, 2), (64, 64, 2), (64, 64, 1), (128, 128, 1), (96, 64, 1)])
+@pytest.mark.parametrize("growth", [0.0, 10.0, -10.0])
+def test_tcgen05_attention_over_many_blocks(dk, dv, maps, growth):
+    """1,300 keys, eleven blocks of 128: the scores' maximum stays, grows by 2^10 a block (the reference moves at every block, so that runs of O that are
+    whole, begun and not begun are scaled) or falls.  Against 64 bits: float32 outputs (two maps) are no further off than the mma.sync kernel's where
+    the maximum stays (one accumulator over all keys was, 1.5 times at 1,300 keys); growing scores carry their own rounding, 2^-24 of up to 110 in units of
+    log 2, three roundings, into weights: 110 x 2^-24 x 3 x ln 2 = 1.4e-5.  bfloat16 outputs: 2^-8."""
+    g = torch.Generator().manual_seed(dk + dv)
+    H, G, n, scale = 2, 1, 1300, 0.125
+    q, k, v = (torch.randn(n, m, d, generator=g) for m, d in ((H * maps, dk), (G * maps, dk), (G, dv)))
+    q[..., 0] = 8.0
+    k[..., 0] = (torch.arange(n) // 128 * growth / 1.4427 / (8.0 * scale))[:, None]
+    v = v + 1.0
+    k, v = k.to(torch.bfloat16), v.to(torch.bfloat16)
+    kv = PagedKV([n], G, maps * dk, dv, torch.bfloat16, seed=3)
+    kv.put(0, k.reshape(n, G, -1).float().numpy(), v.float().numpy())
+    seen = torch.ones(n, n, dtype=torch.bool, device=DEV).tril()
+    want = torch.cat([torch.softmax((q[:, h].to(DEV).double() @ k[:, h % maps].to(DEV).double().T * scale).masked_fill(~seen, -math.inf), 1) @ v[:, 0].to(DEV).double()
+                      for h in range(H * maps)], 1)
+    off, err = [], torch.zeros(1, dtype=torch.int32, device=DEV)
+    for tile in (ops.SPLIT_PREFILL_TILE, ops.SPLIT_TC_TILE):
+        out = torch.full((n, H * maps * dv), float("nan"), dtype=torch.bfloat16 if maps == 1 else torch.float32, device=DEV)
+        args = (q.reshape(n, -1).to(DEV).contiguous(), out, kv.k, kv.v, i32(kv.table), *make_tiles([n], [0], tile), H, G, dk, dv, scale)
+        if tile == ops.SPLIT_TC_TILE:
+            ops.attn_prefill_split_tc(*args, err, maps=maps)
+        else:
+            ops.attn_prefill_split(*args, max_keys=n, maps=maps)
+        off.append(float((out.double() - want).norm() / want.norm()))
+    assert int(err.item()) == 0
+    if maps == 1:
+        assert off[1] < 2.0 ** -8
+    elif growth:
+        assert off[1] < 1.4e-5
+    else:
+        assert off[1] <= off[0], off
 
 
 # ----------------------------------------------------------------------------- the scoring router and its experts
