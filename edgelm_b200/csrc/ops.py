@@ -1046,14 +1046,23 @@ def attn_prefill_split_takes(dtype, dk, dv, maps=1):
 
 
 SPLIT_TC_TILE = 128  # new tokens per tile of the tcgen05 form of it (ST_ROWS in attention_split_tc.cu)
-# Steps whose longest sequence brings fewer new tokens than this stay on tiles of 64 and mma.sync (us there and on tcgen05: 9 heads of 96 / 64, 192
-# tokens 10.4 and 12.0, 256 12.5 and 13.0, 400 16.8 and 14.2; 16 heads of two maps, four times 192 20.9 and 22.6, 256 31 and 25, 400 80 and 49).
+# Steps whose longest sequence brings fewer new tokens than this stay on tiles of 64 and mma.sync, and so do those in which it sees fewer than SPLIT_TC_MIN_KEYS
+# keys and the tiles of 128 give fewer than SPLIT_TC_MIN_BLOCKS blocks.  us there and on tcgen05: 9 heads of 64 over 3, 192 tokens 8.3 and 10.8, 256 10.3
+# and 12.2, 300 11.8 and 12.0, 256 behind 1,000 32 and 25; 9 heads of 96 / 64, 192 10.1 and 11.8, 256 12.5 and 12.8, 300 14.3 and 12.7; 16 heads of two maps,
+# 192 10.4 and 11.8, 256 12.9 and 12.8, four times 256 31 and 24.5; 32 heads of 64 over 8, 256 10.3 and 10.6, four times 256 23.5 and 19.9.
 SPLIT_TC_MIN_TOKENS = 256
+SPLIT_TC_MIN_KEYS, SPLIT_TC_MIN_BLOCKS = 300, 128
 
 
 def attn_prefill_split_tc_takes(dtype, dk, dv, maps=1):
     """Whether the tcgen05 form of `attn_prefill_split` takes these sizes."""
     return dtype == torch.bfloat16 and bool(lib().edgelm_attn_prefill_split_tc_takes(int(dk), int(dv), int(maps)))
+
+
+def attn_prefill_split_tc_pays(most_tokens, most_keys, tiles, heads):
+    """Whether a step goes to the tcgen05 form: its longest run of new tokens, the most keys a sequence has, its tiles of SPLIT_TC_TILE tokens, heads (each
+    map one)."""
+    return most_tokens >= SPLIT_TC_MIN_TOKENS and (most_keys >= SPLIT_TC_MIN_KEYS or tiles * heads >= SPLIT_TC_MIN_BLOCKS)
 
 
 def attn_prefill_split_tc(q, out, kcache, vcache, page_table, tile_seq, tile_tok0, tile_ntok, tile_pos0, n_tiles, nh, nkv, dk, dv, scale, err, gate=None,

@@ -121,8 +121,8 @@ def split_prefill_tiles(dtype, dk, dv, maps=1):
 
 
 def split_prefill(ctx, q, out, k, v, table, nh, nkv, dk, dv, scale, max_keys, maps=1, **options):
-    """Those kernels' step: on tcgen05 where it takes the sizes and some sequence brings tokens enough for its tiles, else on mma.sync."""
-    if max(ctx.seq_lengths) >= ops.SPLIT_TC_MIN_TOKENS and ops.attn_prefill_split_tc_takes(k.dtype, dk, dv, maps):
+    """Those kernels' step: on tcgen05 where it takes the sizes and is the faster one, else on mma.sync."""
+    if ops.attn_prefill_split_tc_takes(k.dtype, dk, dv, maps) and ops.attn_prefill_split_tc_pays(max(ctx.seq_lengths), max_keys, ctx.tiles(ops.SPLIT_TC_TILE).count, nh * maps):
         t = ctx.tiles(ops.SPLIT_TC_TILE)
         ops.attn_prefill_split_tc(q, out, k, v, table, t.seq, t.tok0, t.ntok, t.pos0, t.count, nh, nkv, dk, dv, scale, ctx.err, maps=maps, **options)
     else:

@@ -245,6 +245,14 @@ def test_a_steps_layout(ntok, pos0, tiles):
         assert (host == before).all()
 
 
+@pytest.mark.parametrize("most,keys,tiles,heads,tcgen05", [(255, 9000, 400, 64, False), (256, 256, 2, 9, False), (256, 299, 14, 9, False), (256, 300, 2, 9, True),
+                                                           (256, 256, 8, 16, True), (256, 256, 15, 9, True), (2000, 2000, 16, 1, True)])
+def test_which_split_attention_a_step_takes(most, keys, tiles, heads, tcgen05):
+    """Too few tokens; few keys in few blocks (the tcgen05 kernel starts later, 10.3 against 12.2 us at 256 tokens of 9 heads); many keys or many blocks."""
+    from edgelm_b200.csrc import ops
+    assert ops.attn_prefill_split_tc_pays(most, keys, tiles, heads) is tcgen05
+
+
 def test_token_ids_from_any_sequence():
     from edgelm_b200.engine.engine import _as_ids
     for n in (3, 200):
