@@ -19,13 +19,17 @@
 // tokens (2-norm; scores of standard deviation 1): 2.3e-7, 3.4e-7, 4.1e-7, 4.6e-7; one run over all keys 2.3e-7, 6.6e-7, 1.9e-6, 4.2e-6 and
 // 1 to 7 % less time; mma.sync 4.1e-7, 4.8e-7, 1.0e-6, 2.2e-6.
 //
+// A value that is no finite number makes that dimension of the rows that see it none, a key their whole output; rows that do not see it are as they were
+// without it: in blocks that some row sees in part such values are taken out ahead of the MMAs by the loaders and given to their rows at the end
+// (blocks that every row sees whole need none of it; windows and chunks of 1,024, two maps of 64 over 128, 256 tokens: 27.8 -> 30.8 us, else 1 to 3 %).
+//
 // Masks, sinks, gates, kept keys and maps as in attention_mma_split.cu.  Every wait is bounded; where one runs out the block reports it, writes
 // not-a-numbers and waits for its own copies and MMAs before it gives its memory back.
 // mma.sync takes a scheduler 16 clocks for an m16n8k16 here, four times what tcgen05 takes for as many multiply-adds, and bounds the other kernel.
 // What bounds this one is the softmax: 2,600 clocks a block, 1,750 of them the exponentials, the splitting and the stores into tensor memory
 // (with a third of either product's MMAs it takes 3 % less, without exponentials and splitting 17 %); 3 us a tile before the first block.
-// mma.sync and here, us: 9 heads of 64 over 3, 1,000, 2,000 and 4,000 tokens 26 and 21, 78 and 34, 225 and 67; 512 behind 4,000 103 and 65; 16
-// heads of two maps of 64 over values of 128, chunks of 1,024, 1,000 and 4,000 tokens 88 and 33, 248 and 131; 32 heads of 128, 2,000 tokens 373 and 111.
+// mma.sync and here, us: 9 heads of 64 over 3, 1,000 and 2,000 tokens 26 and 21, 78 and 34; 512 behind 4,000 103 and 66; 16
+// heads of two maps of 64 over values of 128, chunks of 1,024, 1,000 and 2,000 tokens 88 and 34, 158 and 64; 32 heads of 128, 2,000 tokens 373 and 115.
 // Tiles of the most keys go first over all heads (a head's tiles next to each other left the last head's longest tile to the end).
 #include <math_constants.h>
 
@@ -44,6 +48,7 @@ constexpr int ST_TILE = 128 * 128;             // bytes of 128 rows of 64 bfloat
 template <int DK, int DV> struct StSizes {
   static constexpr int KC = (DK + 63) / 64, VC = (DV + 63) / 64;      // tiles of 64 dimensions
   static constexpr int KS = 2, VS = KC == 2 && VC == 2 ? 1 : 2;       // stages of keys and values
+  static constexpr int CLEANERS = VS;             // warps that clean the values
   static constexpr int smem = 1024 + (3 * KC + KS * KC + VS * VC) * ST_TILE + 12 * ST_ROWS * 4 + 256;
 };
 
@@ -54,6 +59,14 @@ __device__ __forceinline__ int st_first_key(int pos, int mask, int size) {
 }
 // O of the run (of two blocks) that block j belongs to: with room for two, the runs take turns
 template <int DV> __device__ __forceinline__ uint32_t st_run_col(int j) { return ST_O_COL + (DV == 64 ? (j >> 1 & 1) * 64 : 0); }
+// Two bfloat16 numbers: bits 15 and 31 where they are infinite or not a number; a mask of those that are numbers; these alone
+__device__ __forceinline__ uint32_t st_no_number(uint32_t w) { return ((w & 0x7f807f80u) + 0x00800080u) & 0x80008000u; }
+__device__ __forceinline__ uint32_t st_numbers_mask(uint32_t w) { return ~((st_no_number(w) >> 15) * 0xffffu); }
+__device__ __forceinline__ uint32_t st_numbers(uint32_t w) { return w & st_numbers_mask(w); }
+__device__ __forceinline__ void st_add_nothing(const uint4& v, uint32_t& sum) {
+  asm("{\n\tfma.rn.bf16x2 %0, %1, %5, %0;\n\tfma.rn.bf16x2 %0, %2, %5, %0;\n\tfma.rn.bf16x2 %0, %3, %5, %0;\n\tfma.rn.bf16x2 %0, %4, %5, %0;\n\t}"
+      : "+r"(sum) : "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(0u));
+}
 __device__ __forceinline__ uint32_t st_low_bits(int n) { return n >= 32 ? ~0u : ~(~0u << max(n, 0)); }
 __device__ __forceinline__ void st_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void st_tmem_st4(uint32_t taddr, const uint32_t* r) {
@@ -82,6 +95,7 @@ __device__ __forceinline__ void st_drain(uint32_t bar, uint32_t parity) {
 
 struct SplitTcArgs {
   const float* q;
+  const __nv_bfloat16* values;
   int ldq;
   void* out;
   int ldo;
@@ -111,10 +125,11 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
   float* row_sum = row_max + 8 * ST_ROWS;          // [quarter of the keys][128 rows]
   uint64_t* bars = reinterpret_cast<uint64_t*>(row_sum + 4 * ST_ROWS);
   uint64_t *q_ready = bars, *k_full = bars + 1, *k_empty = k_full + KS, *v_full = k_empty + KS, *v_empty = v_full + VS;
-  uint64_t *s_ready = v_empty + VS, *p_ready = s_ready + 2, *o_done = p_ready + 2;
+  uint64_t *v_clean = v_empty + VS, *s_ready = v_clean + VS, *p_ready = s_ready + 2, *o_done = p_ready + 2;
   uint64_t* all_done = o_done + 2;                 // both issuers' MMAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(all_done + 1);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
+  volatile int* taken_out = abort_flag + 1;        // some value that is no number was
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int tile = a.n_tiles - 1 - (int)blockIdx.y, head = blockIdx.x, kvh = head / (a.nh / a.nkv * a.maps), map = head % a.maps;
@@ -124,11 +139,17 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
   const int first_page = st_first_key(pos0, a.mask, a.mask_size) / PAGE, kept_pages = min(first_page, (a.keep + PAGE - 1) / PAGE);
   const int n_visit = kept_pages + n_pg - first_page, n_blk = (n_visit + 1) / 2;
   auto page_at = [&](int i) { return i < kept_pages ? i : first_page + i - kept_pages; };
+  const int last_first = st_first_key(n_keys - 1, a.mask, a.mask_size);      // the first key of the tile's last row
+  auto hidden = [&](int key0, int n) { return key0 + n - 1 > pos0 || (key0 < last_first && key0 + n > a.keep); };      // from some row: some of n keys
+  auto some_hidden = [&](int j) {                  // some key of block j from some row (or it has no second page)
+    return 2 * j + 1 >= n_visit || hidden(page_at(2 * j) * PAGE, PAGE) || hidden(page_at(2 * j + 1) * PAGE, PAGE);
+  };
 
   if (threadIdx.x == 0) {
-    for (uint64_t* b = bars; b < o_done + 2; ++b) mbar_init(smem_u32(b), b == q_ready || (b >= p_ready && b < o_done) ? ST_SOFT_WARPS : 1);
+    for (uint64_t* b = bars; b < o_done + 2; ++b)
+      mbar_init(smem_u32(b), b == q_ready || (b >= p_ready && b < o_done) ? ST_SOFT_WARPS : b >= v_clean && b < s_ready ? Z::CLEANERS : 1);
     mbar_init(smem_u32(all_done), 2);
-    *abort_flag = 0;
+    *abort_flag = *taken_out = 0;
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
   }
   if (warp == 2) {
@@ -149,6 +170,52 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     uint8_t* dst = keys ? k_s : v_s;
     const int32_t* pages = a.page_table ? a.page_table + (size_t)seq * a.table_stride : nullptr;
     const bool leader = elect_one();
+    // Values that some row of the tile must not see meet weights of zero: where there are such, rows behind the tile's last position (or of no page) become
+    // zero, whatever lies there, and so do values that are no finite number (0 x inf would be none); the rows that see such a value get it at the end.
+    // (both loaders, half of the rows each, with the next block's copies on their way; with one stage of values their loader alone)
+    constexpr int CLEANERS = Z::CLEANERS, PIECES = 32 / CLEANERS;
+    auto clean = [&](int j) {
+      const int st = j % VS;
+      if (!wait(&v_full[st], j / VS & 1)) return false;
+      if (some_hidden(j)) {
+        uint4* mine = reinterpret_cast<uint4*>(v_s + st * VC * ST_TILE) + (CLEANERS > 1 ? warp * PIECES : 0) * 32 + lane;      // four rows a warp and load
+        const int row0 = (CLEANERS > 1 ? warp * PIECES : 0) * 4 + (lane >> 3);
+        const int from0 = min(PAGE, n_keys - page_at(2 * j) * PAGE), from1 = 2 * j + 1 < n_visit ? min(PAGE, n_keys - page_at(2 * j + 1) * PAGE) : 0;
+        bool written = false;
+        if (from0 < PAGE || from1 < PAGE) {
+          for (int x = 0; x < PIECES; ++x) {
+            const int r = row0 + x * 4;
+            if ((r & (PAGE - 1)) < (r < PAGE ? from0 : from1)) continue;
+#pragma unroll
+            for (int c = 0; c < VC; ++c) mine[c * (ST_TILE / 16) + x * 32] = make_uint4(0, 0, 0, 0);
+            written = true;
+          }
+        }
+        uint32_t sum = 0;                          // (0 x a value that is no number is none, and stays)
+#pragma unroll 1
+        for (int x = 0; x < PIECES * VC; x += 8) {
+          uint4 v[8];
+#pragma unroll
+          for (int y = 0; y < 8; ++y) v[y] = mine[x / PIECES * (ST_TILE / 16) + (x % PIECES + y) * 32];
+#pragma unroll
+          for (int y = 0; y < 8; ++y) st_add_nothing(v[y], sum);
+        }
+        if (st_no_number(sum)) {
+          for (int x = 0; x < PIECES * VC; ++x) {
+            uint4* at = mine + x / PIECES * (ST_TILE / 16) + x % PIECES * 32;
+            const uint4 v = *at;
+            if ((st_no_number(v.x) | st_no_number(v.y) | st_no_number(v.z) | st_no_number(v.w)) == 0) continue;
+            *at = make_uint4(st_numbers(v.x), st_numbers(v.y), st_numbers(v.z), st_numbers(v.w));
+            written = true;
+            *taken_out = 1;
+          }
+        }
+        if (written) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+      }
+      __syncwarp();
+      if (lane == 0) st_arrive(smem_u32(&v_clean[st]));
+      return true;
+    };
     int issued = 0;
     for (int j = 0; j < n_blk; ++j) {
       const int st = j % stages;
@@ -176,7 +243,9 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
         }
       }
       __syncwarp();
+      if ((!keys || CLEANERS > 1) && j >= VS - 1 && !clean(j - (VS - 1))) break;
     }
+    if (VS > 1 && issued == n_blk) clean(n_blk - 1);
     // (also where a wait ran out: no copy may be on its way when the block's memory is given back)
     for (int i = max(0, issued - stages); i < issued; ++i) st_drain(smem_u32(&full[i % stages]), i / stages & 1);
   } else if (warp == 2) {
@@ -211,7 +280,7 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     bool ok = true;
     for (int j = 0; j < n_blk && ok; ++j) {
       const int b = j & 1, st = j % VS;
-      ok = wait(&p_ready[b], j >> 1 & 1) && wait(&v_full[st], j / VS & 1);
+      ok = wait(&p_ready[b], j >> 1 & 1) && wait(&v_clean[st], j / VS & 1);
       if (!ok) break;
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       const uint64_t dv = umma_desc(smem_u32(v_s + st * VC * ST_TILE));
@@ -253,7 +322,6 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     __syncwarp();
     if (lane == 0) st_arrive(smem_u32(q_ready));
     const int pos = row < ntok ? pos0 + row : -1, first = st_first_key(max(pos, 0), a.mask, a.mask_size);
-    const int last_first = st_first_key(n_keys - 1, a.mask, a.mask_size);      // the first key of the tile's last row
     float m = -CUDART_INF_F, l = 0.f;             // the row's reference (in units of log 2), this thread's keys' weights
     float acc[DV / 4] = {};                       // the row's output, this thread's dimensions
     auto gather = [&](int j) {                    // += the run that the MMAs of block j ended in tensor memory
@@ -283,7 +351,7 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
         asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
         tmem_ld32(s_addr, r);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (!there || key0 + 31 > pos0 || (key0 < last_first && key0 + 32 > a.keep)) {
+        if (!there || hidden(key0, 32)) {
           // (a bit a key: five instructions a score, with its place compared to each bound, made a masked block twice as long)
           const uint32_t seen = (there ? st_low_bits(pos - key0 + 1) : 0u) & (~st_low_bits(first - key0) | st_low_bits(a.keep - key0));
 #pragma unroll
@@ -354,19 +422,6 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
         st_tmem_st4(tmem + lanes + b * ST_BUF_COLS + 128 + part * 16 + c * 4, t[2]);
       }
       l += sum0 + sum1;
-      if (j == n_blk - 1) {
-        // value rows behind the tile's last position (or of no page) meet weights of zero: make them zero, whatever lies there
-        const int v_from = there ? min(PAGE, n_keys - page0) : 0;
-        if (v_from < PAGE) {                       // uniform over the warp
-          ok = wait(&v_full[j % VS], j / VS & 1);
-          if (!ok) continue;
-          for (int i = (sw & 7) * 32 + lane; i < (PAGE - v_from) * 8 * VC; i += 256) {
-            const int c = i / ((PAGE - v_from) * 8), e = i % ((PAGE - v_from) * 8);
-            *reinterpret_cast<uint4*>(v_s + (j % VS * VC + c) * ST_TILE + (half * PAGE + v_from + (e >> 3)) * 128 + (e & 7) * 16) = make_uint4(0, 0, 0, 0);
-          }
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-        }
-      }
       if (waiting && (DV != 64 || (j & 1))) {      // before the next block's MMAs may take its columns
         waiting = false;
         ok = gather(j - 1 - (j & 1));
@@ -379,6 +434,29 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     }
     if (ok && waiting) ok = gather(n_blk - 2);     // (the last block has a run of its own)
     if (ok) ok = gather(n_blk - 1);
+    if (ok && *taken_out && row < ntok) {         // (rare: values that were taken out above, to the rows that see them)
+      for (int i = 0; i < n_visit; ++i) {
+        if (!some_hidden(i / 2)) continue;
+        const int pg = page_at(i), page = a.page_table ? a.page_table[(size_t)seq * a.table_stride + pg] : 0;
+        const __nv_bfloat16* values = a.page_table ? a.values + ((size_t)(page < 0 || page >= a.n_pages ? 0 : page) * a.nkv + kvh) * PAGE * DV
+                                                   : a.values + ((size_t)(tok0 - pos0 + pg * PAGE) * a.nkv + kvh) * DV;
+        const size_t pitch = a.page_table ? DV : (size_t)a.nkv * DV;
+#pragma unroll 1
+        for (int k = 0; k < PAGE; ++k) {
+          const int key = pg * PAGE + k;
+          if (key > pos || (key < first && key >= a.keep)) continue;
+          const uint2* at = reinterpret_cast<const uint2*>(values + k * pitch + part * (DV / 4));
+#pragma unroll
+          for (int c = 0; c < DV / 16; ++c) {
+            const uint2 v = at[c];
+            if ((st_no_number(v.x) | st_no_number(v.y)) == 0) continue;
+            const uint32_t w[2] = {v.x & ~st_numbers_mask(v.x), v.y & ~st_numbers_mask(v.y)};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) acc[c * 4 + e] += __uint_as_float(e & 1 ? w[e / 2] & 0xffff0000u : w[e / 2] << 16);
+          }
+        }
+      }
+    }
     row_sum[part * ST_ROWS + row] = l;
     asm volatile("bar.sync %0, 128;" ::"r"(quarter + 1) : "memory");
     float den = (row_sum[row] + row_sum[ST_ROWS + row]) + (row_sum[2 * ST_ROWS + row] + row_sum[3 * ST_ROWS + row]), fix = 1.f;
@@ -474,7 +552,7 @@ extern "C" int edgelm_attn_prefill_split_tc(const float* q, int ldq, void* out, 
     if (tensor_map(kcache, n_pages, nkv * maps * dk, nkv * maps * dk, PAGE, &mk)) return -1;
     if (tensor_map(vcache, n_pages, nkv * dv, nkv * dv, PAGE, &mv)) return -1;
   }
-  const SplitTcArgs a{q, ldq, out, ldo, page_table, table_stride, n_pages, tile_seq, tile_tok0, tile_ntok, tile_pos0, n_tiles, nh, nkv, maps, scale,
+  const SplitTcArgs a{q, (const __nv_bfloat16*)vcache, ldq, out, ldo, page_table, table_stride, n_pages, tile_seq, tile_tok0, tile_ntok, tile_pos0, n_tiles, nh, nkv, maps, scale,
                       gate, ldg, mask, mask_size, sink, keep, gate_ch, err};
   int rc = 0;
   if (dk == 64 && dv == 64) rc = launch_split_tc<64, 64>(mk, mv, a, stream);

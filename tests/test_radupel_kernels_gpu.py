@@ -538,6 +538,46 @@ def test_tcgen05_attention_over_many_blocks(dk, dv, maps, growth):
         assert off[1] <= off[0], off
 
 
+@pytest.mark.parametrize("first,H,G,dk,dv,maps,mask,size,keep,own", [
+    (0, 2, 1, 64, 64, 1, 0, 0, 0, False), (200, 2, 1, 64, 64, 1, 1, 90, 70, False), (130, 2, 2, 128, 64, 1, 1, 200, 0, False), (60, 2, 1, 128, 128, 1, 2, 128, 0, False),
+    (0, 3, 3, 96, 64, 1, 0, 0, 0, True), (0, 2, 2, 64, 128, 2, 2, 100, 0, False), (37, 2, 1, 64, 64, 2, 0, 0, 0, False)])
+def test_tcgen05_attention_of_values_that_are_no_number(first, H, G, dk, dv, maps, mask, size, keep, own):
+    """Infinities and not-a-numbers in values and keys, at both sides of pages' and tiles' edges: the rows that see one, and no others, have an output that is no
+    finite number, in the dimensions where the value has one; all other outputs are those of 64 bits (bfloat16 2^-7 of their size, float32 3e-6)."""
+    g = torch.Generator().manual_seed(dk + first)
+    new, scale = 300, 0.125
+    n, P = first + new, -(-(first + new) // PAGE)
+    q = torch.randn(new, H * maps, dk, generator=g).to(DEV)
+    k, v = (torch.randn(n, m, d, generator=g).to(DEV, torch.bfloat16) for m, d in ((G * maps, dk), (G, dv)))
+    for i, at in enumerate((first + 5, first + 63, first + 64, first + 127, first + 128, first + 200, n - 1, max(0, first - 3))):
+        v[at, :, 3 * i + 1] = (math.inf, -math.inf, math.nan)[i % 3]
+    k[first + 250, :, 7] = math.nan
+    if own:
+        kc, vc, table = k.reshape(n, -1), v.reshape(n, -1), None
+    else:
+        kc, vc = torch.full((P, G, PAGE, maps * dk), math.nan, device=DEV, dtype=torch.bfloat16), torch.full((P, G, PAGE, dv), math.nan, device=DEV, dtype=torch.bfloat16)
+        for i in range(P):
+            m = min(PAGE, n - i * PAGE)
+            kc[i, :, :m], vc[i, :, :m] = k[i * PAGE:i * PAGE + m].view(m, G, -1).transpose(0, 1), v[i * PAGE:i * PAGE + m].transpose(0, 1)
+        table = i32([list(range(P))])
+    out, err = torch.full((new, H * maps * dv), 7.0, dtype=torch.bfloat16 if maps == 1 else torch.float32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+    ops.attn_prefill_split_tc(q.reshape(new, -1), out, kc, vc, table, *make_tiles([new], [first], ops.SPLIT_TC_TILE), H, G, dk, dv, scale, err, mask=mask, mask_size=size, keep=keep, maps=maps)
+    pos, key = torch.arange(first, n, device=DEV)[:, None], torch.arange(n, device=DEV)[None]
+    low = pos - size + 1 if mask == 1 else pos // size * size if mask == 2 else 0 * pos
+    seen = (key <= pos) & ((key >= low) | (key < keep))
+    got = out.double().view(new, H * maps, dv)
+    for h in range(H * maps):
+        kv = h // (H // G * maps)
+        kh, vh = k[:, kv * maps + h % maps].double(), v[:, kv].double()
+        weights = torch.softmax((q[:, h].double() @ kh.T * scale).masked_fill(~seen, -math.inf), 1)
+        want = weights @ vh.nan_to_num(0.0, 0.0, 0.0)
+        lost = weights.isnan().any(1)[:, None] | (seen.double() @ (~vh.isfinite()).double() > 0)
+        assert torch.equal(~got[:, h].isfinite(), lost), h
+        off = (got[:, h] - want).abs()[~lost]
+        assert bool((off <= (2.0 ** -7 * want.abs()[~lost] + 1e-5 if maps == 1 else 3e-6 * float(want[~lost].abs().max()))).all()), h
+    assert int(err.item()) == 0
+
+
 # ----------------------------------------------------------------------------- the scoring router and its experts
 @pytest.mark.parametrize("E,ident,top,groups,keep,negative", [(6, 3, 3, 3, 2, False), (3, 0, 1, 1, 1, False), (5, 1, 2, 2, 1, True), (7, 2, 2, 3, 1, True),
                                                               (8, 0, 4, 4, 2, False), (2, 2, 2, 1, 1, True), (12, 4, 3, 8, 2, False), (4, 2, 3, 3, 1, True)])
