@@ -13,7 +13,8 @@
 // chain of pages (two warps a scheduler, 384 MMAs and 800 other instructions a page each).  On the CUDA cores and here, 9 heads of 64 over
 // 3, us: prompts of 61, 381 and 701 tokens 125 and 40.6; one of 1,500 344 and 100; 8 heads of 128, 333 and 200 tokens 98 and 57; one of 17
 // 15 and 15.  Distance from float64 (2-norm) 1.5e-7 against 3.6e-7 at 1,500 keys, 8.7e-8 against 1.3e-7 at 17.
-// A key or value that is no finite number makes the rows that see it not a number.
+// A key or value that is no finite number, or rounds to none in bfloat16, shows in its last term; a tile that met one is computed again in plain
+// multiply-adds, so that it reaches the rows that see it as it does on the CUDA cores, and no others (looking takes 0 to 2 % of the time).
 #include <math_constants.h>
 
 #include "mma_split.cuh"
@@ -29,6 +30,40 @@ __device__ __forceinline__ void af_cross(float* c, const uint32_t (*a)[4], const
   constexpr int TA[5] = {2, 0, 1, 1, 0}, TB[5] = {0, 2, 1, 0, 1};
 #pragma unroll
   for (int p = 0; p < 5; ++p) sp_mma(c, a[TA[p]][0], a[TA[p]][1], a[TA[p]][2], a[TA[p]][3], b[TB[p]][0], b[TB[p]][1]);
+}
+
+// A tile whose keys or values hold a number without bfloat16 terms, in plain multiply-adds: a warp a row, a lane a key, then hd / 32 dimensions.
+__device__ __noinline__ void af_plain_tile(const float* q, int ldq, float* out, int ldo, const float* kcache, const float* vcache, const int32_t* pages, int tok0,
+                                           int ntok, int pos0, int nkv, int kvh, int head, int hd, float scale) {
+  const int lane = threadIdx.x & 31;
+  for (int r = threadIdx.x >> 5; r < ntok; r += blockDim.x >> 5) {
+    const float* qr = q + (size_t)(tok0 + r) * ldq + head * hd;
+    const int limit = pos0 + r;
+    float m = -CUDART_INF_F, l = 0.f, o[4] = {};
+    for (int key0 = 0; key0 <= limit; key0 += 32) {
+      const int page = pages[key0 / PAGE], n = min(32, limit + 1 - key0);
+      const size_t at = (((size_t)max(page, 0) * nkv + kvh) * PAGE + key0 % PAGE) * hd;
+      float s = 0.f;
+      if (lane < n && page >= 0)
+        for (int d = 0; d < hd; ++d) s = fmaf(qr[d], kcache[at + lane * hd + d], s);
+      s = lane < n ? s * scale : -CUDART_INF_F;
+      const float mx = fmaxf(m, warp_max(s)), ref = mx == -CUDART_INF_F ? 0.f : mx, corr = expf(m - ref), p = expf(s - ref);
+      l = l * corr + p;
+      m = mx;
+#pragma unroll
+      for (int c = 0; c < 4; ++c) o[c] *= corr;
+      for (int i = 0; i < n; ++i) {
+        const float w = __shfl_sync(0xffffffffu, p, i);
+#pragma unroll
+        for (int c = 0; c < 4; ++c)
+          if (32 * c < hd) o[c] = fmaf(w, page >= 0 ? vcache[at + i * hd + 32 * c + lane] : 0.f, o[c]);
+      }
+    }
+    l = warp_sum(l);
+#pragma unroll
+    for (int c = 0; c < 4; ++c)
+      if (32 * c < hd) out[(size_t)(tok0 + r) * ldo + head * hd + 32 * c + lane] = o[c] / l;
+  }
 }
 
 template <int HDT, int NG>
@@ -87,6 +122,7 @@ attn_prefill_f32_kernel(const float* __restrict__ q, int ldq, float* __restrict_
   for (int i = 0; i < HD / 8; ++i) o[i][0] = o[i][1] = o[i][2] = o[i][3] = 0.f;
   float mA = -CUDART_INF_F, mB = -CUDART_INF_F, lA = 0.f, lB = 0.f;     // (maxima of the scores as they come; sums of this lane's keys)
 
+  uint32_t nothing = 0;      // the sum of 0 x the last terms: not a number from the first key or value on whose first term is none
   if (group < n_pages) load_page(group);
   for (int pg = group; pg < n_pages; pg += NG) {
     asm volatile("cp.async.wait_group 0;" ::: "memory");
@@ -101,6 +137,7 @@ attn_prefill_f32_kernel(const float* __restrict__ q, int ldq, float* __restrict_
       *reinterpret_cast<uint2*>(dst) = t1;
       *reinterpret_cast<uint2*>(dst + PLANE) = t2;
       *reinterpret_cast<uint2*>(dst + 2 * PLANE) = t3;
+      asm("{\n\tfma.rn.bf16x2 %0, %1, %3, %0;\n\tfma.rn.bf16x2 %0, %2, %3, %0;\n\t}" : "+r"(nothing) : "r"(t3.x), "r"(t3.y), "r"(0u));
     }
     group_sync();
     if (pg + NG < n_pages) load_page(pg + NG);
@@ -194,12 +231,15 @@ attn_prefill_f32_kernel(const float* __restrict__ q, int ldq, float* __restrict_
       }
     }
   }
+  if (__syncthreads_or((nothing & 0x7fffu) > 0x7f80u || (nothing & 0x7fff0000u) > 0x7f800000u)) {
+    af_plain_tile(q, ldq, out, ldo, kcache, vcache, pages, tok0, ntok, pos0, nkv, kvh, head, HD, scale);
+    return;
+  }
   lA += __shfl_xor_sync(0xffffffffu, lA, 1);
   lA += __shfl_xor_sync(0xffffffffu, lA, 2);
   lB += __shfl_xor_sync(0xffffffffu, lB, 1);
   lB += __shfl_xor_sync(0xffffffffu, lB, 2);
   if (NG > 1) {
-    __syncthreads();
     constexpr int MP = HD + 2;
     float* mg = reinterpret_cast<float*>(af_raw);      // [NG - 1][64 rows][HD + 2]: groups 1 ..'s output, maximum, sum
     if (group > 0) {

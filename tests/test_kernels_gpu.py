@@ -1107,6 +1107,45 @@ def test_attn_prefill_f32(nh, nkv, hd):
     assert errs[0] < 1e-6 and errs[0] <= errs[1], errs
 
 
+@pytest.mark.parametrize("nh,nkv,hd", [(3, 1, 64), (2, 2, 32), (2, 1, 96), (4, 2, 128)])
+@pytest.mark.parametrize("first", [0, 75])
+def test_attn_prefill_f32_of_numbers_that_bfloat16_has_not(nh, nkv, hd, first):
+    """Infinities, not-a-numbers and numbers that bfloat16 rounds to infinity in keys and values, at the edges of pages and of warps' rows: every output
+    is what 64 bits give, not-a-numbers and infinities at the same places, and rows in front of such a key or value have nothing of it.  The bound is
+    that of test_attn_prefill_f32: 1e-5 of the largest value."""
+    o = ops()
+    nan, inf, new = float("nan"), float("inf"), 200
+    n = first + new
+    case = PagedCase(o, torch.float32, [n], nkv, hd, seed=hd + first)
+    bad = [("v", first + 5, 1, inf), ("v", first + 64, 2, nan), ("v", first + 79, 3, -inf), ("v", n - 1, 4, inf), ("v", max(0, first - 3), 5, 3.395e38), ("k", first + 150, 6, -inf),
+           ("k", first + 170, 7, nan), ("k", first + 120, 8, -inf), ("v", first + 130, 9, 3.4e38)]
+    for what, at, d, value in bad:
+        page = int(case.table[int(case.seq_slot[0]), at // o.PAGE])
+        (case.kcache if what == "k" else case.vcache)[page, :, at % o.PAGE, d] = value
+        (case.k if what == "k" else case.v)[0][at, :, d] = value
+    qkv = rnd((new, (nh + 2 * nkv) * hd), torch.float32, 83)
+    q = qkv[:, :nh * hd].view(new, nh, hd)
+    q[:, :, 6] = q[:, :, 6].abs() + 0.1            # (that key scores minus infinity: a weight of zero; the other takes either sign)
+    rows = [(0, a, min(64, new - a), first + a) for a in range(0, new, 64)]
+    out = torch.full((new, nh * hd), 7.0, device=dev())
+    o.attn_prefill_f32(qkv, out, case.kcache, case.vcache, case.table, case.seq_slot, *(torch.tensor([r[i] for r in rows], dtype=torch.int32, device=dev()) for i in range(4)),
+                       len(rows), nh, nkv, hd, 1.0 / math.sqrt(hd))
+    seen = torch.arange(n)[None] <= torch.arange(first, n)[:, None]
+    for h in range(nh):
+        kh, vh = case.k[0][:, h // (nh // nkv)].double(), case.v[0][:, h // (nh // nkv)].double()
+        weights = torch.softmax((q[:, h].double().cpu() @ kh.T / math.sqrt(hd)).masked_fill(~seen, -inf), 1)
+        want = weights @ torch.where(vh.abs() < 1e30, vh, 0.0)
+        for what, at, d, value in bad:
+            if what == "v":
+                want[:, d] += torch.where(seen[:, at], weights[:, at] * value, 0.0)
+        got = out[:, h * hd:(h + 1) * hd].double().cpu()
+        assert torch.equal(got.isnan(), want.isnan()) and torch.equal(got.isinf(), want.isinf()) and torch.equal(got[want.isinf()], want[want.isinf()]), h
+        small = want.isfinite() & (want.abs() < 1e30)
+        assert float((got - want)[small].abs().max()) < 1e-5 * float(want[small].abs().max())
+        large = want.isfinite() & ~small
+        assert bool(((got - want)[large].abs() < 1e-5 * want[large].abs()).all())
+
+
 def test_attn_prefill_mma_far_key_and_diagonal():
     """Scaled queries make one early key, or the token's own key, dominate: a wrong mask or page shows."""
     o = ops()
