@@ -167,6 +167,11 @@ def test_gemm_split_values_that_bfloat16_has_not():
     a[7, 11] = 3.4e38
     a[8] *= 1e-34
     w[9] *= 1e-30
+    a[10] *= 1e-37                             # (terms too small for bfloat16 beside large weights: sums of 1e-25 and more)
+    a[11] *= 3e-36
+    w[20] *= 1e13
+    w[21] *= 5e10
+    a[12, 3], w[22], w[23] = 3.4e38, 0.0, 0.0  # (a number that rounds to infinity beside weights of zero: a zero)
     got, want = torch.empty(M, N, device=dev()), torch.empty(M, N, device=dev())
     o.gemm_split(a, w, got)
     o.gemm_simt(a, w, want, force_kernel=2)
