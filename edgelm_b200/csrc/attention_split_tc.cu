@@ -68,25 +68,9 @@ __device__ __forceinline__ void st_add_nothing(const uint4& v, uint32_t& sum) {
       : "+r"(sum) : "r"(v.x), "r"(v.y), "r"(v.z), "r"(v.w), "r"(0u));
 }
 __device__ __forceinline__ uint32_t st_low_bits(int n) { return n >= 32 ? ~0u : ~(~0u << max(n, 0)); }
-__device__ __forceinline__ void st_arrive(uint32_t bar) { asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(bar) : "memory"); }
 __device__ __forceinline__ void st_tmem_st4(uint32_t taddr, const uint32_t* r) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x4.b32 [%0], {%1, %2, %3, %4};" ::"r"(taddr), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]) : "memory");
 }
-__device__ __forceinline__ void st_tmem_ld8(uint32_t taddr, uint32_t* r) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
-}
-// D (+)= A (tensor memory) x B (shared memory)
-__device__ __forceinline__ void st_umma_ts(uint32_t tmem_d, uint32_t tmem_a, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile(
-      "{\n\t.reg .pred p;\n\t"
-      "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::f16 [%0], [%1], %2, %3, p;\n\t}"
-      ::"r"(tmem_d), "r"(tmem_a), "l"(bdesc), "r"(idesc), "r"(accumulate)
-      : "memory");
-}
-
 // A block's last wait for what it has in flight, bounded and without a report (the wait that ran out before has made one)
 __device__ __forceinline__ void st_drain(uint32_t bar, uint32_t parity) {
   const long long t0 = clock64();
@@ -213,7 +197,7 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
         if (written) asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
       }
       __syncwarp();
-      if (lane == 0) st_arrive(smem_u32(&v_clean[st]));
+      if (lane == 0) mbar_arrive(smem_u32(&v_clean[st]));
       return true;
     };
     int issued = 0;
@@ -292,7 +276,7 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
 #pragma unroll
             for (int s = 0; s < 8; ++s) {                             // 16 keys: of the threads of quarter s / 2
               const uint32_t p = tmem + b * ST_BUF_COLS + (t == 2 ? 128 + s * 8 : s / 2 * 32 + t * 16 + s % 2 * 8);
-              st_umma_ts(tmem + st_run_col<DV>(j) + c * 64, p, dv + (c * ST_TILE + s * 16 * 128 >> 4), idesc, j & 1 || t != 2 || s != 0);
+              umma_f16_ts(tmem + st_run_col<DV>(j) + c * 64, p, (uint32_t)dv + (c * ST_TILE + s * 16 * 128 >> 4), (uint32_t)(dv >> 32), idesc, j & 1 || t != 2 || s != 0);
             }
         umma_commit(smem_u32(&o_done[b]));
         umma_commit(smem_u32(&v_empty[st]));
@@ -320,7 +304,7 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
     }
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
     __syncwarp();
-    if (lane == 0) st_arrive(smem_u32(q_ready));
+    if (lane == 0) mbar_arrive(smem_u32(q_ready));
     const int pos = row < ntok ? pos0 + row : -1, first = st_first_key(max(pos, 0), a.mask, a.mask_size);
     float m = -CUDART_INF_F, l = 0.f;             // the row's reference (in units of log 2), this thread's keys' weights
     float acc[DV / 4] = {};                       // the row's output, this thread's dimensions
@@ -330,8 +314,8 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
 #pragma unroll
       for (int c = 0; c < DV / 4; c += 16) {
         uint32_t o[16];
-        st_tmem_ld8(tmem + lanes + st_run_col<DV>(j) + part * (DV / 4) + c, o);
-        st_tmem_ld8(tmem + lanes + st_run_col<DV>(j) + part * (DV / 4) + c + 8, o + 8);
+        tmem_ld8(tmem + lanes + st_run_col<DV>(j) + part * (DV / 4) + c, o);
+        tmem_ld8(tmem + lanes + st_run_col<DV>(j) + part * (DV / 4) + c + 8, o + 8);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
         for (int i = 0; i < 16; ++i) acc[c + i] += __uint_as_float(o[i]);
@@ -392,7 +376,7 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
             for (int c = 0; c < DV / 4; c += 8) {
               uint32_t o[8];
               const uint32_t at = tmem + lanes + st_run_col<DV>(j) + part * (DV / 4) + c;
-              st_tmem_ld8(at, o);
+              tmem_ld8(at, o);
               asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
 #pragma unroll
               for (int i = 0; i < 8; ++i) o[i] = __float_as_uint(__uint_as_float(o[i]) * rescale);
@@ -430,7 +414,7 @@ attn_prefill_split_tc_kernel(const __grid_constant__ CUtensorMap map_k, const __
       asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
       asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
       __syncwarp();
-      if (lane == 0) st_arrive(smem_u32(&p_ready[b]));
+      if (lane == 0) mbar_arrive(smem_u32(&p_ready[b]));
     }
     if (ok && waiting) ok = gather(n_blk - 2);     // (the last block has a run of its own)
     if (ok) ok = gather(n_blk - 1);

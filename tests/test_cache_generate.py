@@ -245,6 +245,13 @@ def test_a_steps_layout(ntok, pos0, tiles):
         assert (host == before).all()
 
 
+def test_tile_sizes_are_the_kernels():
+    from edgelm_b200.csrc import ops
+    lib = ops.lib()
+    assert (lib.edgelm_attn_prefill_mma_tile_tokens(), lib.edgelm_attn_prefill_f32_tile_tokens(), lib.edgelm_attn_prefill_split_tile_tokens(),
+            lib.edgelm_attn_prefill_split_tc_tile_tokens()) == (ops.MMA_PREFILL_TILE, ops.F32_PREFILL_TILE, ops.SPLIT_PREFILL_TILE, ops.SPLIT_TC_TILE)
+
+
 @pytest.mark.parametrize("most,keys,tiles,heads,tcgen05", [(255, 9000, 400, 64, False), (256, 256, 2, 9, False), (256, 299, 14, 9, False), (256, 300, 2, 9, True),
                                                            (256, 256, 8, 16, True), (256, 256, 15, 9, True), (2000, 2000, 16, 1, True)])
 def test_which_split_attention_a_step_takes(most, keys, tiles, heads, tcgen05):
