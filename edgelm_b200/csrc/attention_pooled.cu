@@ -441,14 +441,21 @@ pooled_window_attn_rows_kernel(const T* __restrict__ q, T* __restrict__ out, con
   if (lane == 0) { wm[2 * warp + 1] = m; wl[2 * warp + 1] = l; }
   __syncthreads();
   if (threadIdx.x < D) {
-    float M = -INFINITY, L = 0.f, acc = 0.f;
+    // (four sums side by side: one of up to 32 runs after the other rounds more often than the runs themselves)
+    float M = -INFINITY, Ls[4] = {}, accs[4] = {};
     for (int w = 0; w < 2 * NW; ++w) M = fmaxf(M, wm[w]);
-    for (int w = 0; w < 2 * NW; ++w) {
-      if (wm[w] == -INFINITY) continue;
-      const float f = expf(wm[w] - M);
-      L = fmaf(wl[w], f, L);
-      acc = fmaf(wo[w][threadIdx.x], f, acc);
+#pragma unroll 2
+    for (int w0 = 0; w0 < 2 * NW; w0 += 4) {
+#pragma unroll
+      for (int x = 0; x < 4; ++x) {
+        const int w = min(w0 + x, 2 * NW - 1);
+        const bool on = w0 + x < 2 * NW && wm[w] != -INFINITY;
+        const float f = expf(wm[w] - M), l = fmaf(wl[w], f, Ls[x]), o = fmaf(wo[w][threadIdx.x], f, accs[x]);
+        Ls[x] = on ? l : Ls[x];
+        accs[x] = on ? o : accs[x];
+      }
     }
+    const float L = (Ls[0] + Ls[1]) + (Ls[2] + Ls[3]), acc = (accs[0] + accs[1]) + (accs[2] + accs[3]);
     out[((size_t)t * H + h) * D + threadIdx.x] = from_f32<T>(L == 0.f ? 0.f : acc * (1.0f / L));   // (0: no key was seen)
   }
 }
