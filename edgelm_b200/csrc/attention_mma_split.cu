@@ -26,6 +26,8 @@
 // 1,024, prompts of 1,000 and 2,900 tokens: 1,614 us on the CUDA cores, 248 us here.  One sequence of 6,000 tokens, 9 heads of 64:
 // 577 -> 448 us with one conversion a pair of terms, the scale folded into the exponent's multiply-add, a row's sum added over its lanes at
 // the end and the tiles of many keys first.
+// A value that is no finite number reaches rows that do not see it as a weight of zero times it: those of the same 16 rows of a warp where some row
+// sees a key of its page (up to 63 tokens in front of it, and rows past a window).  The tcgen05 form keeps it from them.
 #include <math_constants.h>
 
 #include "mma_split.cuh"

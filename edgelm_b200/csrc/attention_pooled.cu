@@ -197,8 +197,9 @@ __device__ __forceinline__ float2 load_pair(const __nv_bfloat16* p, bool pair) {
 constexpr int PW_MAX_WARPS = 8;
 
 // Dynamic shared memory: the query (dk floats, 16-byte aligned), then per warp its maximum, its denominator and dv values.
-// (Eight lanes sharing a key, so that a load instruction of the warp covers four whole rows, was built and measured: 5.2 ms
-// against 3.8 ms for 2,048 tokens of 32 heads with a window of 1,024: the extra shuffles cost more than the loads save.)
+// This one takes key and value heads of any sizes; those of 32, 64 or 128 dimensions alike go to the kernel of whole rows below, where a load
+// instruction of a warp covers whole rows.  (For 2,048 tokens at once, 32 heads, window 1,024, that costs more in shuffles than it saves in loads, 5.2
+// ms against 3.8; single tokens wait for memory, and prompt steps have kernels of their own.)
 // DVR: how many pairs of value dimensions a lane holds (value heads of up to 64 DVR dimensions).
 template <typename T, int DVR>
 __global__ void __launch_bounds__(PW_MAX_WARPS * 32)

@@ -26,8 +26,9 @@
 // Masks, sinks, gates, kept keys and maps as in attention_mma_split.cu.  Every wait is bounded; where one runs out the block reports it, writes
 // not-a-numbers and waits for its own copies and MMAs before it gives its memory back.
 // mma.sync takes a scheduler 16 clocks for an m16n8k16 here, four times what tcgen05 takes for as many multiply-adds, and bounds the other kernel.
-// What bounds this one is the softmax: 2,600 clocks a block, 1,750 of them the exponentials, the splitting and the stores into tensor memory
-// (with a third of either product's MMAs it takes 3 % less, without exponentials and splitting 17 %); 3 us a tile before the first block.
+// What bounds this one is the softmax: about 3,200 clocks a block, most of them the exponentials, the splitting and the stores into tensor memory (ncu,
+// 4,000 tokens, 9 heads of 64: issue slots 57 % busy, tensor pipe active 36 %; in the form with one run, with a third of either product's MMAs it
+// took 3 % less, without exponentials and splitting 17 %); 3 us a tile before the first block.
 // mma.sync and here, us: 9 heads of 64 over 3, 1,000 and 2,000 tokens 26 and 21, 78 and 34; 512 behind 4,000 103 and 66; 16
 // heads of two maps of 64 over values of 128, chunks of 1,024, 1,000 and 2,000 tokens 88 and 34, 158 and 64; 32 heads of 128, 2,000 tokens 373 and 115.
 // Tiles of the most keys go first over all heads (a head's tiles next to each other left the last head's longest tile to the end).
@@ -506,7 +507,9 @@ using namespace edgelm;
 // Tokens per tile that the host must cut sequences into for this kernel.
 extern "C" int edgelm_attn_prefill_split_tc_tile_tokens() { return ST_ROWS; }
 
-// 1 if the kernel takes these key and value head sizes and maps a head, else 0.
+// 1 if the kernel takes these key and value head sizes and maps a head, else 0: value sizes of whole tiles of 64 dimensions, whose columns of tensor
+// memory the softmax threads share out in pieces of 16, over key sizes from 64 on.  Value sizes of 32 and 96, and key sizes of 32, stay on mma.sync:
+// they would need other pieces, and no form of them has been built or measured.
 extern "C" int edgelm_attn_prefill_split_tc_takes(int dk, int dv, int maps) {
   if (maps == 2) return dk == 64 && (dv == 64 || dv == 128) ? 1 : 0;
   return maps == 1 && ((dv == 64 && (dk == 64 || dk == 96 || dk == 128)) || (dv == 128 && dk == 128)) ? 1 : 0;

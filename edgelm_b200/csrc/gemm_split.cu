@@ -10,7 +10,8 @@
 // accumulator of their own, and these runs are added in registers, rounded to nearest, eight of them before they join the sum; the five
 // cross products are 2^-8 of them and share an accumulator over all of K.  Distance from float64 (2-norm over the result's, normal
 // operands) beside register tiles of float32 multiply-adds summed in runs of 32: K 16 3.6e-8 and 5.7e-8, K 576 7.7e-8 and 9.9e-8,
-// K 2560 1.02e-7 and 1.12e-7 (one block a tile; less where blocks share K).
+// K 2560 1.02e-7 and 1.12e-7 (one block a tile; less where blocks share K).  Cut-offs of one sign do not cancel: where all products are positive,
+// sums are 3.8e-8 short on average at any K from 32 on, 5.6e-8 to 7.0e-8 off in all where the register tiles were 4.0e-8 to 5.3e-8.
 //
 // One CTA computes a tile of 128 rows of W (the lanes of tensor memory; for SwiGLU 64 gate rows and the 64 up rows of the same outputs)
 // by BN rows of `a`.  A unit of work is 32 k's of the tile.  Warps:
@@ -22,8 +23,9 @@
 // Then all of them do the epilogue out of shared memory, a warp's lanes at neighbouring outputs of one row of `out`.
 // Where the tiles leave SMs idle, K is shared by the blocks of a cluster, whose sums are folded out of shared memory.
 //
-// Bound by shared memory's bandwidth: 64 k's of a tile of BN 64 are 48 KB written by TMA, 48 read, 24 written as terms and 48 read by the MMAs,
-// 1,340 clocks of the 2,000 they take (the tensor cores' pipe is busy 36 % of them).  Both operands of the MMAs in shared memory would be
+// No unit is full (1,143 rows, SwiGLU N 1536, ncu: tensor pipe active 20 % of the time, issue slots half busy, shared memory's load/store path 34 %); the
+// nearest by count is shared memory, to which TMA and the MMAs come as well: 64 k's of a tile of BN 64 are 48 KB written by TMA, 48 read, 24 written as terms and 48 read
+// by the MMAs, 1,340 clocks of the 2,000 they take.  Both operands of the MMAs in shared memory would be
 // 96 KB more; 128 rows of `a` a tile take 2,200 clocks, but half as many tiles fill fewer SMs (1,143 rows, N 576 to 1536: no gain), and
 // twice the splitting threads 5 % longer at BN 64 (20 % shorter at BN 32).  Measured beside the register tiles that
 // were here (a graph of launches over different weights): 1,143 rows, K 576, N 960 43.6 -> 17.8 us, SwiGLU N 1536 130 -> 50; K 1536, N 576

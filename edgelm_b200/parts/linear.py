@@ -31,7 +31,8 @@ def _few_rows_f32(rows, w, w2, fused_norm):
     """Whether a float32 product of up to 16 rows stays on the few-rows kernel, whose time grows with the rows; the tensor-core
     product's does not, but it starts later and wants a fused norm computed ahead (2 us).  Measured, few rows | tensor cores, us: N 576, K 576 at 8
     and 16 rows 5.6 | 6.3, 6.7 | 6.3; N 576, K 1536 at 4 and 8 7.4 | 6.8, 10.9 | 6.7; N 2560 SwiGLU, K 960 with the norm at 4, 8 and 16
-    11.4, 16.1, 23.4 | 10.5; N 49152, K 576 at 2, 4, 8, 16 34.7, 42.4, 59, 110 | 35."""
+    11.4, 16.1, 23.4 | 10.5; N 49152, K 576 at 2, 4, 8, 16 34.7, 42.4, 59, 110 | 35.  (One line by rows x weights: of these sizes it leaves N 576, K 1536 at 4
+    rows 0.6 us slower than it could be, and N 576, K 576 at 16 rows where it is the faster.)"""
     return rows < 4 or rows * w.numel() * (2 if w2 is not None else 1) < (24_000_000 if fused_norm else 5_000_000)
 
 
